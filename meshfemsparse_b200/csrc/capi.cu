@@ -320,13 +320,13 @@ std::shared_ptr<DevSym> upload_symbolic(mfs_handle *h, std::shared_ptr<Symbolic>
             const idx s = S.level_list[k];
             const idx nsb = (S.w[s] + SBk - 1) / SBk;
             sb_flag[s] = nsbflags;
-            nsbflags += 2 * int(nsb);
+            nsbflags += 2 * int(nsb) + 1;
             sb_inv[s] = inv_end;
             sb_first[s] = int32_t(isb.size());
             ds->sb_fronts.push_back(int32_t(s));
             for (idx K = 0; K < nsb; ++K) {
                 const idx nr = std::min(SBk, S.w[s] - K * SBk), nrp = (nr + 63) & ~idx(63);
-                isb.push_back({int32_t(s), int32_t(K), sb_flag[s], 0, inv_end, -1, -1});
+                isb.push_back({int32_t(s), int32_t(K), sb_flag[s], 0, inv_end, -1, -1, 0, 0, 0, 0, 0, 0, 0});
                 inv_end += nrp * nrp;
             }
         }
@@ -334,12 +334,53 @@ std::shared_ptr<DevSym> upload_symbolic(mfs_handle *h, std::shared_ptr<Symbolic>
     const int32_t nsbm = int32_t(isb.size());
     std::vector<int32_t> sb_fidx(nsn, -1);
     for (size_t i = 0; i < ds->sb_fronts.size(); ++i) sb_fidx[ds->sb_fronts[i]] = int32_t(i);
+    auto sb_parts = [&](idx s, idx K) { return (std::min(SBk, S.w[s] - K * SBk) + 63) / 64; };
+    // inverse row maps of the children in their parents' fronts, and the children of each
+    // front above the cut
+    std::vector<int32_t> par(nsn);
+    std::vector<int64_t> cmap_off(nsn + 1, 0);
+    for (idx s = 0; s < nsn; ++s) {
+        par[s] = int32_t(S.sn_parent[s]);
+        cmap_off[s + 1] = cmap_off[s] + (par[s] < 0 ? 0 : S.f[par[s]] / S.vb);
+    }
+    std::vector<SbChild> kids;
+    std::vector<int32_t> sb_child0(nsn, 0), sb_nchild(nsn, 0);
+    for (int32_t s : ds->sb_fronts) {
+        sb_child0[s] = int32_t(kids.size());
+        for (idx k = S.child_ptr[s]; k < S.child_ptr[s + 1]; ++k) {
+            const idx c = S.child_list[k];
+            if (S.d[c] == 0) continue;
+            const bool above = sb_flag[c] >= 0;
+            const int32_t done = above ? sb_flag[c] + 2 * int32_t((S.w[c] + SBk - 1) / SBk) : -1;
+            kids.push_back({done, int32_t((S.f[c] - (S.w[c] & ~idx(3)) + 63) / 64), cmap_off[c], S.sol_off[c],
+                            int32_t(S.d[c]), 0});
+        }
+        sb_nchild[s] = int32_t(kids.size()) - sb_child0[s];
+    }
+    // per analysis row of these fronts: where its superblock counts (by its first scalar)
+    std::vector<int32_t> rowcnt(std::max<idx>(S.nv, 1), 0);
+    for (int32_t s : ds->sb_fronts)
+        for (idx k = 0; k < S.w[s] / S.vb; ++k) {
+            const idx K = k * S.vb / SBk;
+            rowcnt[S.sn_start[s] + k] = int32_t(4 * (sb_flag[s] + 2 * K) + sb_parts(s, K) - 1);
+        }
     // every superblock before a front's last is full (SB x SB)
     auto sb_task = [&](idx s, idx K, idx part) {
-        return SbTask{int32_t(s),         int32_t(K), sb_flag[s], int32_t(part), sb_inv[s] + K * SBk * SBk,
-                      2 * (nsbm + sb_fidx[s]), 2 * (sb_first[s] + int32_t(K))};
+        return SbTask{int32_t(s),
+                      int32_t(K),
+                      sb_flag[s],
+                      int32_t(part),
+                      K < 0 ? -1 : sb_inv[s] + K * SBk * SBk,
+                      2 * (nsbm + sb_fidx[s]),
+                      K < 0 ? -1 : 2 * (sb_first[s] + int32_t(K)),
+                      sb_child0[s],
+                      sb_nchild[s],
+                      int32_t(S.w[s]),
+                      int32_t(S.f[s]),
+                      col0[s],
+                      0,
+                      S.sol_off[s]};
     };
-    auto sb_parts = [&](idx s, idx K) { return (std::min(SBk, S.w[s] - K * SBk) + 63) / 64; };
     std::vector<SolveAsmTask> sasm;
     std::vector<SolveTask> ftri, btri;
     std::vector<StrTask> fstr, bstr;
@@ -406,33 +447,45 @@ std::shared_ptr<DevSym> upload_symbolic(mfs_handle *h, std::shared_ptr<Symbolic>
             }
         L.ftri_n = int(ftri.size()) - L.ftri_off;
         L.btri_n = int(btri.size()) - L.btri_off;
-        // superblock tasks, one per 64-row part: ascending superblock index across the
-        // level's fronts (forward), descending (backward); every dependency precedes
-        // its task and the parts of a superblock are adjacent
-        L.fsb_off = int(fsb.size());
-        L.bsb_off = int(bsb.size());
-        if (l > S.solve_cut) {
-            idx maxnsb = 0;
-            for (idx k = S.level_ptr[l]; k < S.level_ptr[l + 1]; ++k)
-                maxnsb = std::max<idx>(maxnsb, (S.w[S.level_list[k]] + SBk - 1) / SBk);
-            for (idx K = 0; K < maxnsb; ++K)
-                for (idx k = S.level_ptr[l]; k < S.level_ptr[l + 1]; ++k) {
-                    const idx s = S.level_list[k];
-                    if (K < (S.w[s] + SBk - 1) / SBk)
-                        for (idx part = 0; part < sb_parts(s, K); ++part) fsb.push_back(sb_task(s, K, part));
-                }
-            for (idx p = 0; p < maxnsb; ++p)
-                for (idx k = S.level_ptr[l]; k < S.level_ptr[l + 1]; ++k) {
-                    const idx s = S.level_list[k];
-                    const idx nsb = (S.w[s] + SBk - 1) / SBk;
-                    if (p < nsb)
-                        for (idx part = 0; part < sb_parts(s, nsb - 1 - p); ++part)
-                            bsb.push_back(sb_task(s, nsb - 1 - p, part));
-                }
-        }
-        L.fsb_n = int(fsb.size()) - L.fsb_off;
-        L.bsb_n = int(bsb.size()) - L.bsb_off;
     }
+    // Tasks of the solves above the cut, in an order in which every dependency precedes
+    // its task and the parts of a superblock are adjacent. Forward: levels ascending;
+    // inside a level the superblocks in ascending order across the fronts, each front's
+    // structure tasks right after its last superblock. Backward: levels and superblocks
+    // descending.
+    for (idx l = S.solve_cut + 1; l < S.nlevels; ++l) {
+        idx maxnsb = 0;
+        for (idx k = S.level_ptr[l]; k < S.level_ptr[l + 1]; ++k)
+            maxnsb = std::max<idx>(maxnsb, (S.w[S.level_list[k]] + SBk - 1) / SBk);
+        for (idx K = 0; K < maxnsb; ++K) {
+            for (idx k = S.level_ptr[l]; k < S.level_ptr[l + 1]; ++k) {
+                const idx s = S.level_list[k];
+                if (K < (S.w[s] + SBk - 1) / SBk)
+                    for (idx part = 0; part < sb_parts(s, K); ++part) fsb.push_back(sb_task(s, K, part));
+            }
+            for (idx k = S.level_ptr[l]; k < S.level_ptr[l + 1]; ++k) {
+                const idx s = S.level_list[k];
+                if (S.d[s] == 0 || K + 1 != (S.w[s] + SBk - 1) / SBk) continue;
+                const idx span = S.f[s] - (S.w[s] & ~idx(3));
+                for (idx b = 0; b < (span + 63) / 64; ++b) fsb.push_back(sb_task(s, -1, b));
+            }
+        }
+    }
+    for (idx l = S.nlevels - 1; l > S.solve_cut; --l) {
+        idx maxnsb = 0;
+        for (idx k = S.level_ptr[l]; k < S.level_ptr[l + 1]; ++k)
+            maxnsb = std::max<idx>(maxnsb, (S.w[S.level_list[k]] + SBk - 1) / SBk);
+        for (idx p = 0; p < maxnsb; ++p)
+            for (idx k = S.level_ptr[l]; k < S.level_ptr[l + 1]; ++k) {
+                const idx s = S.level_list[k];
+                const idx nsb = (S.w[s] + SBk - 1) / SBk;
+                if (p < nsb)
+                    for (idx part = 0; part < sb_parts(s, nsb - 1 - p); ++part)
+                        bsb.push_back(sb_task(s, nsb - 1 - p, part));
+            }
+    }
+    ds->nfsb = int(fsb.size());
+    ds->nbsb = int(bsb.size());
     ds->small_list.upload(small_list, st);
     ds->large_dev.upload(ds->large_fronts, st);
     ds->all_list.upload(all_list, st);
@@ -498,6 +551,16 @@ std::shared_ptr<DevSym> upload_symbolic(mfs_handle *h, std::shared_ptr<Symbolic>
     sd.struct_rows = ds->struct_rows.p;
     sd.rel = ds->rel.p;
     sd.vb = S.vb;
+    {
+        ds->parent.upload(par, st);
+        ds->cmap_off.upload(cmap_off, st);
+        up(ds->sb_children, kids);
+        up(ds->rowcnt, rowcnt);
+        ds->cmap.ensure(size_t(std::max<int64_t>(cmap_off[nsn], 1)));
+        launch_child_maps(ds->parent.p, ds->cmap_off.p, int(nsn), sd, ds->cmap.p, st);
+        MFS_LAUNCHED();
+        MFS_CUDA(cudaStreamSynchronize(st));
+    }
     return ds;
 }
 
@@ -568,7 +631,7 @@ void ensure_panel_maps(mfs_handle *h, DevSym &ds, const void *base, bool half, c
 }
 
 // Tensor maps of the superblock solves for the factor array `base` (elements of es
-// bytes): per superblock inverse (nrp x nrp) and per front's L11 (w x w, leading
+// bytes): per superblock inverse (nrp x nrp) and per front's panel (f x w, leading
 // dimension ld), a forward box (64 rows x FC columns) and a backward box (FC rows x
 // 64 columns), FC = 32 KB / (64 es).
 void ensure_solve_maps(mfs_handle *h, DevSym &ds, const void *base, int es) {
@@ -591,9 +654,9 @@ void ensure_solve_maps(mfs_handle *h, DevSym &ds, const void *base, int es) {
     for (size_t i = 0; i < nf && ok; ++i) {
         const int32_t s = ds.sb_fronts[i];
         const void *p = b + size_t(ds.dpan[s]) * es;
-        const uint64_t w = uint64_t(S.w[s]), ld = uint64_t(ds.dld[s]);
-        ok = encode_plain_map(&maps[2 * (nb + i)], p, es, w, w, ld, 64, FC) &&
-             encode_plain_map(&maps[2 * (nb + i) + 1], p, es, w, w, ld, FC, 64);
+        const uint64_t f = uint64_t(S.f[s]), w = uint64_t(S.w[s]), ld = uint64_t(ds.dld[s]);
+        ok = encode_plain_map(&maps[2 * (nb + i)], p, es, f, w, ld, 64, FC) &&
+             encode_plain_map(&maps[2 * (nb + i) + 1], p, es, f, w, ld, FC, 64);
     }
     if (!ok) throw StatusError(MFS_INTERNAL, "cuTensorMapEncodeTiled refused a solve tensor map");
     h->smaps.ensure(maps.size());
@@ -815,10 +878,11 @@ void run_solve(mfs_handle *h, DevSym &ds, const T *factor, double *X, int nrhs) 
     const int pass = sb ? kSbMaxRhs : kMaxSolveRhs;
     const int chunk = std::min(nrhs, pass);
     h->sol.ensure(size_t(std::max<idx>(S.sol_size, 1)) * chunk);
-    h->str_partials.ensure(size_t(std::max<int64_t>(ds.max_str_entries, 1)) * chunk);
     if (sb) {
         h->sb_scratch.ensure(size_t(std::max<idx>(S.n, 1)) * chunk);
         ensure_solve_maps(h, ds, factor, int(sizeof(T)));
+    } else {
+        h->str_partials.ensure(size_t(std::max<int64_t>(ds.max_str_entries, 1)) * chunk);
     }
     for (int r0 = 0; r0 < nrhs; r0 += pass) {
         const int nr = std::min(pass, nrhs - r0);
@@ -827,31 +891,33 @@ void run_solve(mfs_handle *h, DevSym &ds, const T *factor, double *X, int nrhs) 
         // levels <= solve_cut: whole subtrees, one per CTA
         launch_subtree_solve<T>(true, ds.subs.p, ds.nsub, ds.sub_fmax, ds.sd, factor, Xc, S.n, nr, h->sol.p, st);
         MFS_LAUNCHED();
-        for (size_t l = size_t(ds.solve_cut + 1); l < ds.levels.size(); ++l) {
-            const LevelPlan &L = ds.levels[l];
-            launch_fwd_asm(ds.sasm_tasks.p + L.sasm_off, L.sasm_n, L.sasm_tiles, ds.sd, Xc, S.n, nr, h->sol.p, st);
-            MFS_LAUNCHED();
-            if (!sb)
+        if (sb) {
+            auto above = [&](bool forward, const SbTask *tasks, int n) {
+                MFS_CUDA(launch_sb_solve<T>(forward, tasks, n, ds.sd, h->smaps.p, ds.sb_children.p, ds.cmap.p,
+                                            ds.rowcnt.p, Xc, S.n, nr, h->sol.p, h->sb_scratch.p, ds.flags.p,
+                                            h->solve_err.p, st));
+            };
+            above(true, ds.fsb_tasks.p, ds.nfsb);
+            above(false, ds.bsb_tasks.p, ds.nbsb);
+        } else {
+            for (size_t l = size_t(ds.solve_cut + 1); l < ds.levels.size(); ++l) {
+                const LevelPlan &L = ds.levels[l];
+                launch_fwd_asm(ds.sasm_tasks.p + L.sasm_off, L.sasm_n, L.sasm_tiles, ds.sd, Xc, S.n, nr, h->sol.p, st);
+                MFS_LAUNCHED();
                 MFS_CUDA(launch_diag<T>(true, ds.ftri_tasks.p + L.ftri_off, L.ftri_n, ds.sd, factor, Xc, S.n, nr,
                                         ds.flags.p, h->solve_err.p, st));
-            else
-                MFS_CUDA(launch_sb_solve<T>(true, ds.fsb_tasks.p + L.fsb_off, L.fsb_n, ds.sd, factor, h->smaps.p, Xc, S.n, nr,
-                                            h->sb_scratch.p, ds.flags.p, h->solve_err.p, st));
-            launch_str<T>(true, ds.fstr_tasks.p + L.fstr_off, L.fstr_n, ds.fred.p + L.fred_off, L.fred_n, ds.sd,
-                          factor, Xc, S.n, nr, h->sol.p, h->str_partials.p, st);
-            MFS_LAUNCHED();
-        }
-        for (size_t l = ds.levels.size(); l-- > size_t(ds.solve_cut + 1);) {
-            const LevelPlan &L = ds.levels[l];
-            launch_str<T>(false, ds.bstr_tasks.p + L.bstr_off, L.bstr_n, ds.bred.p + L.bred_off, L.bred_n, ds.sd,
-                          factor, Xc, S.n, nr, h->sol.p, h->str_partials.p, st);
-            MFS_LAUNCHED();
-            if (!sb)
+                launch_str<T>(true, ds.fstr_tasks.p + L.fstr_off, L.fstr_n, ds.fred.p + L.fred_off, L.fred_n, ds.sd,
+                              factor, Xc, S.n, nr, h->sol.p, h->str_partials.p, st);
+                MFS_LAUNCHED();
+            }
+            for (size_t l = ds.levels.size(); l-- > size_t(ds.solve_cut + 1);) {
+                const LevelPlan &L = ds.levels[l];
+                launch_str<T>(false, ds.bstr_tasks.p + L.bstr_off, L.bstr_n, ds.bred.p + L.bred_off, L.bred_n, ds.sd,
+                              factor, Xc, S.n, nr, h->sol.p, h->str_partials.p, st);
+                MFS_LAUNCHED();
                 MFS_CUDA(launch_diag<T>(false, ds.btri_tasks.p + L.btri_off, L.btri_n, ds.sd, factor, Xc, S.n, nr,
                                         ds.flags.p, h->solve_err.p, st));
-            else
-                MFS_CUDA(launch_sb_solve<T>(false, ds.bsb_tasks.p + L.bsb_off, L.bsb_n, ds.sd, factor, h->smaps.p, Xc, S.n, nr,
-                                            h->sb_scratch.p, ds.flags.p, h->solve_err.p, st));
+            }
         }
         launch_subtree_solve<T>(false, ds.subs.p, ds.nsub, ds.sub_fmax, ds.sd, factor, Xc, S.n, nr, h->sol.p, st);
         MFS_LAUNCHED();

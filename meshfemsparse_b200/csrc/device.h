@@ -150,17 +150,30 @@ struct StrTask {
 struct StrReduce {
     int32_t sn, idx, first, nchunks;
 };
-// One superblock K of a front's L11 in the diagonal-block solves: a CTA task of the
-// inverse kernel (part 0), or of the forward / backward chains for its 64-row part
-// `pad`. inv: factor-array offset of inv(L_KK) (nrp x nrp column-major, nrp = 64 *
-// ceil(rows / 64)); flag0: the front's first count (two per superblock: parts
-// solved, parts whose accumulated right-hand side is in the scratch vector);
-// pmap / imap: the first of the two tensor maps (forward box, backward box) of the
-// front's L11 / of inv(L_KK) in the solve's map array.
+// One superblock K of a front's L11 in the solves above the cut: a CTA task of the
+// inverse kernel (part 0), or of the forward / backward kernels for its 64-row part
+// `pad`; K = -1: rows [64 pad, 64 pad + 64) of the front's structure part (from w rounded
+// down to a multiple of 4; forward only). inv: factor-array offset of inv(L_KK) (nrp x
+// nrp column-major, nrp = 64 * ceil(rows / 64)); flag0: the front's first count (two
+// per superblock: parts solved, parts whose accumulated right-hand side is in the
+// scratch vector; then one: structure tasks done); pmap / imap: the first of the two
+// tensor maps (forward box, backward box) of the front's panel / of inv(L_KK) in the
+// solve's map array; child0 / nchild: the front's children with an update vector (SbChild).
 struct SbTask {
     int32_t sn, K, flag0, pad;
     int64_t inv;
     int32_t pmap, imap;
+    int32_t child0, nchild;
+    int32_t w, f, c0, pad2;             // the front's width, rows and first column
+    int64_t sol;                        // its place in the solve arena
+};
+// One child of a front above the cut: the count that says its update vector is whole, and
+// its value then (flag -1: below the cut, whole before the launch); its row map's first
+// entry, its place in the solve arena and its row count.
+struct SbChild {
+    int32_t flag, need;
+    int64_t map, sol;
+    int32_t d, pad;
 };
 constexpr int kSuperBlock = 256;        // rows per superblock
 // structure part of the solves: forward tasks are kStrRows rows x kStrCols columns
@@ -243,11 +256,17 @@ cudaError_t launch_diag(bool forward, const SolveTask *tasks, int ntasks, SnDev 
 template <typename T>
 void launch_str(bool forward, const StrTask *tasks, int ntasks, const StrReduce *red, int nred, SnDev sd,
                 const T *factor, double *X, int64_t ldx, int nrhs, double *sol, double *P, cudaStream_t st);
-// Superblock diagonal solves (cooperative launch) and the superblock inverses they apply.
+// Solves of the levels above the cut (one cooperative launch per direction and pass of
+// at most kSbMaxRhs right-hand sides) and the superblock inverses they apply. cmap: the
+// children's inverse row maps (launch_child_maps); rowcnt: per analysis row of a front
+// above the cut, 4 x its superblock's first count + its parts - 1.
 template <typename T>
-cudaError_t launch_sb_solve(bool forward, const SbTask *tasks, int ntasks, SnDev sd, const T *factor,
-                            const void *maps, double *X, int64_t ldx, int nrhs, double *scratch, int *flags, int *err,
-                            cudaStream_t st);
+cudaError_t launch_sb_solve(bool forward, const SbTask *tasks, int ntasks, SnDev sd, const void *maps,
+                            const SbChild *children, const int32_t *cmap, const int32_t *rowcnt, double *X, int64_t ldx,
+                            int nrhs, double *sol, double *scratch, int *flags, int *err, cudaStream_t st);
+// Per child c of the assembly forest, the map from its parent's front (block rows) to its
+// own structure (block index, -1: not in it), at map + off[c].
+void launch_child_maps(const int32_t *parent, const int64_t *off, int nsn, SnDev sd, int32_t *map, cudaStream_t st);
 template <typename T>
 void launch_sb_inverse(const SbTask *tasks, int ntasks, SnDev sd, T *factor, cudaStream_t st);
 int solve_rows_per_task();

@@ -88,7 +88,6 @@ struct LevelPlan {
     int sasm_off = 0, sasm_n = 0, sasm_tiles = 0;
     int ftri_off = 0, ftri_n = 0;
     int btri_off = 0, btri_n = 0;
-    int fsb_off = 0, fsb_n = 0, bsb_off = 0, bsb_n = 0;   // superblock diagonal solves (above the cut)
     int fstr_off = 0, fstr_n = 0, fred_off = 0, fred_n = 0;
     int bstr_off = 0, bstr_n = 0, bred_off = 0, bred_n = 0;
 };
@@ -115,8 +114,12 @@ struct DevSym {
     DBuf<SolveTask> ftri_tasks, btri_tasks;
     DBuf<StrTask> fstr_tasks, bstr_tasks;
     DBuf<StrReduce> fred, bred;
-    DBuf<SbTask> fsb_tasks, bsb_tasks, isb_tasks;   // superblock solves (forward, backward) and inverses
-    int nsb_inv = 0;
+    DBuf<SbTask> fsb_tasks, bsb_tasks, isb_tasks;   // solves above the cut (forward, backward) and inverses
+    int nfsb = 0, nbsb = 0, nsb_inv = 0;
+    DBuf<SbChild> sb_children;                      // the children of the fronts above the cut
+    DBuf<int32_t> parent, cmap;                     // assembly parents; children's inverse row maps
+    DBuf<int64_t> cmap_off;
+    DBuf<int32_t> rowcnt;                           // per analysis row above the cut: its superblock's count and parts
     std::vector<SbTask> isb_host;                   // the superblocks (their inverses' offsets)
     std::vector<int32_t> sb_fronts;                 // fronts with superblock solves
     int64_t max_str_entries = 0;       // structure partial sums of one level, per right-hand side

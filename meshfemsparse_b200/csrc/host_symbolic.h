@@ -183,10 +183,9 @@ struct Symbolic {
     std::vector<idx> upd_off;
     idx upd_size = 0;
     // Forward-solve update vectors u_s (d x nrhs), unit size d: offsets here are
-    // scaled by nrhs at solve time. Supernodes at levels <= solve_cut are solved
-    // by whole subtrees (contiguous postorder ranges [sub_lo, sub_hi], largest
-    // work first, fronts of at most sub_fmax rows), so their u_s live from the
-    // start of the solve until their parent's level.
+    // scaled by nrhs at solve time, one place per supernode. Supernodes at levels
+    // <= solve_cut are solved by whole subtrees (contiguous postorder ranges [sub_lo,
+    // sub_hi], largest work first, fronts of at most sub_fmax rows).
     std::vector<idx> sol_off;
     idx sol_size = 0;
     idx solve_cut = -1;

@@ -1,43 +1,67 @@
-// Diagonal-block solves of the level-scheduled triangular solves (K6) through
-// explicit inverses of 256-row superblocks of L11.
+// Triangular solves of the levels above the solve cut (K6): one persistent
+// dataflow kernel per direction.
 //
 // Reference: SparseLDL::Solve (forward L y = b, backward L^T x = y; called at
 // Solvers/CatamariFactorizer.cc:54,70) and its per-supernode kernels
-// (trs_kernels::SolveLowerTri, tests/test_catamari_solve_kernels.cc). The
-// dependency chain of a front's L11 solve is what bounds the solve: a block of y
-// cannot start before every earlier block is known. Here the chain runs over
-// superblocks of SB = 256 rows: after the numeric factorization,
-// sb_inverse_kernel writes inv(L_KK) of every superblock K of every front above
-// the solve cut (dense, column-major, nrp x nrp with nrp = 64 * ceil(rows / 64),
-// zeros above the diagonal), built from the 64 x 64 diagonal inverses by block
-// forward substitution.
+// (trs_kernels::SolveLowerTri / MultiplyLowerBlock, solve_kernels::fused_forward /
+// fused_backward, tests/test_catamari_solve_kernels.cc). The dependency chain of a
+// front's L11 solve bounds the solve: a block of y cannot start before every
+// earlier block is known. Here the chain runs over superblocks of SB = 256 rows:
+// after the numeric factorization, sb_inverse_kernel writes inv(L_KK) of every
+// superblock K of every front above the solve cut (dense, column-major, nrp x nrp
+// with nrp = 64 * ceil(rows / 64), zeros above the diagonal), built from the
+// 64 x 64 diagonal inverses by block forward substitution.
 //
-// A solve task is one 64-row part h of superblock K of one front, run by one CTA;
-// the (up to) four parts of a superblock run side by side:
-//   forward   a_h = b_h - sum_{J < K} L(rows h, superblock J) y_J (J ascending, as
-//             J's count reaches its part count), a_h to a scratch vector, count;
-//             once every part of K has counted, y_h = inv(L_KK)(rows h, :) a_K, count;
-//   backward  a_h = y_h - sum_{J > K} L(superblock J, columns h)^T x_J (J
+// Tasks (one CTA each; SbTask), v = right-hand side of the front's rows with the
+// children's update vectors added in child order (pulled through the children's
+// inverse row maps once their structure tasks have counted):
+//   forward, diagonal   64-row part h of superblock K: a_h = v_h - sum_{J < K}
+//             L(rows h, superblock J) y_J (J ascending, as J's count reaches its part
+//             count), a_h to a scratch vector, count; once every part of K has
+//             counted, y_h = inv(L_KK)(rows h, :) a_K, count;
+//   forward, structure  64 rows of L21: u = v - sum_J L21(rows, superblock J) y_J, to
+//             the solve arena, count (the parent waits for the front's total);
+//   backward            64 columns h of superblock K: a_h = y_h - L21^T x_struct (as the
+//             ancestors' superblocks are done) - sum_{J > K} L(superblock J, columns h)^T x_J (J
 //             descending), then x_h = inv(L_KK)(:, columns h)^T a_K the same way.
-// A superblock thus costs two hops between CTAs and two 64 x 256 products on the
-// chain, and what a task reads after its last dependency arrives (64 x 256 of L
-// and at most 64 x 256 of the inverse) is already on chip: L and the inverse
-// stream through shared memory in 32 KB chunks (64 rows x 128 FP32 / 64 FP64
-// columns forward, 128 / 64 rows x 64 columns backward), one 2D TMA box per chunk
-// issued by one thread through per-front / per-inverse tensor maps, completing on
-// the ring slot's mbarrier, up to six chunks in flight. A box reaching past the
-// front's L11 or past the inverse reads zeros there.
+// What bounds it: the chain of the large fronts (two hops between CTAs and two
+// 64 x 256 products a superblock) and, between the levels, the pass from a front's last
+// structure task to its parent's first part. One launch for all levels and both kinds
+// of task instead of one to four launches a level: the next level's fronts start as
+// soon as their own children are done, the structure products stream L21 while the
+// chain runs, and no partial sums go through memory. One pass over the factor in FP64
+// with one right-hand side (k = 40, 201,720 variables, 19 levels above the cut):
+// 5.56 ms before (133 launches), 1.56 ms now; FP32 with 32 of them, refined in 4 iterations
+// (k = 48, 345,744 variables): 146 ms before, 71 ms now.
+//
+// A CTA is 8 product warps and 8 warps that run ahead of them through the CTA's tasks, so
+// that a small task costs its products and not its chain of dependent loads (a structure
+// task of 64 rows x 33 columns took 4.1 us with the loads in line, 1.5 us this way):
+//   copy warp     its lane 0 streams L and the inverses through shared memory in 32 KB
+//                 chunks (64 rows x 128 FP32 / 64 FP64 columns forward, 128 / 64 rows x
+//                 64 columns backward), one 2D TMA box per chunk through per-front /
+//                 per-inverse tensor maps, across the borders of tasks: what a task reads
+//                 after its last dependency arrives is already on chip;
+//   vector warps  wait for the counts and bring y_J / x_J / x_struct, 256 rows at a time,
+//                 into VS buffers;
+//   gather warps  v of every task's own rows (forward: the children's counts, their row
+//                 maps, their u) and its sizes;
+//   count warp    publishes a structure task's results once all product warps have handed
+//                 them over.
+// Structure rows start at w rounded down to a multiple of 4 (TMA boxes start 16-byte
+// aligned); the rows before w, and what a box holds past the front, meet zeros or are not
+// stored.
 //
 // Launches are cooperative (all CTAs co-resident); every CTA walks its tasks in
 // ascending order and a task waits only on lower-numbered tasks and on the other
 // parts of its own superblock (adjacent task numbers, so on other CTAs), hence
 // the lowest unfinished task can always proceed. Counts are zeroed before each
-// solve: forward targets are the superblock's part count, backward ones twice
-// that. Waits are bounded in time: on expiry the kernel records an error and
+// solve: forward targets are eight (warps) times the superblock's part count, backward
+// ones twice that. Waits are bounded in time: on expiry the kernel records an error and
 // stops waiting; the host reports MFS_TIMEOUT. Sums run in a fixed order, so
 // results are run-to-run identical. With an FP32 factor (the preconditioner of
-// FP64 refinement) the products with off-diagonal superblocks are FP32
-// (accumulated per thread over the task, combined in FP64) and the inverse of the
+// FP64 refinement) the products are FP32, summed in FP32 over at most 256 columns
+// (forward) / 1024 rows (backward) and beyond that in FP64, and the inverse of the
 // diagonal superblock is applied in FP64; an FP64 factor keeps FP64 throughout.
 #include "device.h"
 
@@ -49,9 +73,17 @@ namespace mfs {
 namespace {
 
 constexpr int SB = kSuperBlock;
-constexpr int kSbThreads = 256;
+constexpr int kSbProducts = 256;                         // product threads (8 warps)
+constexpr int kVecWarps = 4, kGatherWarps = 2;
+constexpr int kSbThreads = kSbProducts + 32 * (2 + kVecWarps + kGatherWarps);
+constexpr int kPubSlots = 4;                             // counts under way
+constexpr int own_slots(int nr) { return nr > 4 ? 4 : 8; }   // tasks whose own rows are gathered ahead
+// A gather warp's task `it` waits for the slot's task it - slots by the parity of its
+// phase, which only tells that phase from the one before it; the warp's own last wait
+// (for task it - warps - slots) covers the earlier ones as long as warps <= slots.
+static_assert(kGatherWarps <= own_slots(8), "gather warps");
 constexpr unsigned long long kWaitNs = 2000000000ull;    // 2 s per wait at most
-static_assert(SB == kSbThreads, "one thread per superblock row");
+static_assert(SB == kSbProducts, "one product thread per superblock row");
 
 __device__ __forceinline__ int ld_acquire(const int *p) {
     int v;
@@ -66,22 +98,6 @@ __device__ __forceinline__ unsigned long long gtimer() {
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
 }
-// thread 0 waits for flag == epoch (bounded), then the whole block proceeds
-__device__ __forceinline__ void wait_flag(const int *flag, int epoch, int *err) {
-    if (threadIdx.x == 0) {
-        if (ld_acquire(flag) != epoch) {
-            const unsigned long long t0 = gtimer();
-            while (ld_acquire(flag) != epoch) {
-                if (*(volatile int *)err) break;
-                if (gtimer() - t0 > kWaitNs) {
-                    atomicExch(err, 1);
-                    break;
-                }
-            }
-        }
-    }
-    __syncthreads();
-}
 // Product type of the off-diagonal chunk sums: FP32 for an FP32 factor, FP64 otherwise.
 template <typename T>
 using PT = std::conditional_t<sizeof(T) == 4, float, double>;
@@ -94,15 +110,15 @@ struct SpChunk {
     static constexpr int ELEMS = 64 * FC;
     static constexpr int BYTES = ELEMS * int(sizeof(T));
 };
-// Shared memory: ring [NST][32 KB] | vec [NR][SB] doubles | vp [NR][SB] products' type
-// | red [4][NR][64] doubles | own [NR][64] doubles.
-template <typename T, int NST, int NR>
+// Shared memory: ring [NST][32 KB] | vp [VS][SB * NR] products' type (the vector warps'
+// buffers) | red [8][NR][64] doubles (per-warp partial sums; its start also holds the
+// exchanged a_K, [SB * NR] doubles) | own [own_slots][NR][64] doubles.
+template <typename T, int NST, int NR, int VS>
 struct SpLayout {
-    static constexpr size_t vec_off = size_t(NST) * SpChunk<T>::BYTES;
-    static constexpr size_t vp_off = vec_off + size_t(NR) * SB * sizeof(double);
-    static constexpr size_t red_off = vp_off + size_t(NR) * SB * sizeof(PT<T>);
-    static constexpr size_t own_off = red_off + size_t(4) * NR * 64 * sizeof(double);
-    static constexpr size_t bytes = own_off + size_t(NR) * 64 * sizeof(double);
+    static constexpr size_t vp_off = size_t(NST) * SpChunk<T>::BYTES;
+    static constexpr size_t red_off = vp_off + size_t(VS) * NR * SB * sizeof(PT<T>);
+    static constexpr size_t own_off = red_off + size_t(8) * NR * 64 * sizeof(double);
+    static constexpr size_t bytes = own_off + size_t(own_slots(NR)) * NR * 64 * sizeof(double);
 };
 
 // Rows of superblock K of a front with w columns, and its 64-rounded extent.
@@ -129,22 +145,27 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
-// Every thread waits for the chunk's copies (bounded; on expiry the error is
-// recorded and the chunk's contents are not trusted).
-__device__ __forceinline__ void mbar_wait_all(uint32_t bar, uint32_t parity, int *err) {
-    if (mbar_try(bar, parity)) return;
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// Bounded wait for the phase with the given parity; false on expiry (the error is
+// recorded) or once another wait has expired: what follows is not trusted then.
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int *err) {
+    if (mbar_try(bar, parity)) return true;
     const unsigned long long t0 = gtimer();
-    for (int it = 1;; ++it) {
-        if (mbar_try(bar, parity)) return;
-        if ((it & 63) == 0) {
-            if (*(volatile int *)err) return;
+    for (int it = 0;; ++it) {
+        if (mbar_try(bar, parity)) return true;
+        if ((it & 15) == 0) {                            // (at once: after an expiry every wait ends quickly)
+            if (*(volatile int *)err) return false;
             if (gtimer() - t0 > kWaitNs) {
                 atomicExch(err, 1);
-                return;
+                return false;
             }
         }
     }
 }
+// The product warps' barrier.
+__device__ __forceinline__ void psync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 // 2D tiled TMA load of one box of the tensor map at `map` (device memory written
 // before the launch), box origin (x = row, y = column), completing on `bar`.
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const char *map, int x, int y, uint32_t bar) {
@@ -155,376 +176,817 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const char *map, int x
         : "memory");
 }
 
-// After an error (a wait that gave up), the copies a CTA issued may still be in
-// flight: thread 0 waits, again bounded, for the last use of every ring slot, so
-// no copy lands in shared memory after the CTA has exited.
-template <int NST>
-__device__ __forceinline__ void ring_drain(uint64_t *bars, long long issued, const int *err) {
-    if (threadIdx.x != 0 || !*(volatile const int *)err) return;
-    for (int b = 0; b < NST; ++b) {
-        if (issued <= b) continue;
-        const long long last = b + ((issued - 1 - b) / NST) * NST;
-        const uint32_t bar = smem_u32(&bars[b]), par = uint32_t((last / NST) & 1);
+// The calling lanes wait until the count at p reaches target (bounded).
+__device__ __forceinline__ void spin_count(const int *p, int target, int *err) {
+    if (ld_acquire(p) >= target) return;
+    const unsigned long long t0 = gtimer();
+    for (int it = 1; ld_acquire(p) < target; ++it) {
+        if (it & 31) continue;                           // (each look costs a round trip to L2)
+        if (*(volatile int *)err) return;
+        if (gtimer() - t0 > kWaitNs) {
+            atomicExch(err, 1);
+            return;
+        }
+    }
+}
+// N consecutive values from shared memory with 16-byte loads (N * sizeof(V) a multiple
+// of 16, 16-byte aligned).
+template <int N>
+__device__ __forceinline__ void lds_vec(float (&x)[N], const float *p) {
+#pragma unroll
+    for (int k = 0; k < N / 4; ++k) {
+        const float4 v = reinterpret_cast<const float4 *>(p)[k];
+        x[4 * k] = v.x;
+        x[4 * k + 1] = v.y;
+        x[4 * k + 2] = v.z;
+        x[4 * k + 3] = v.w;
+    }
+}
+template <int N>
+__device__ __forceinline__ void lds_vec(double (&x)[N], const double *p) {
+#pragma unroll
+    for (int k = 0; k < N / 2; ++k) {
+        const double2 v = reinterpret_cast<const double2 *>(p)[k];
+        x[2 * k] = v.x;
+        x[2 * k + 1] = v.y;
+    }
+}
+
+// Forward product of one chunk (64 rows x FC columns, column-major): the warp's FC / 8
+// columns, two rows (2 lane, 2 lane + 1) per lane; v holds the vectors [r][SB].
+template <typename T, typename V, int NR>
+__device__ __forceinline__ void fwd_chunk(const T *ck, const V *v, V (&acc)[2][NR], int wp, int lane) {
+    constexpr int QW = SpChunk<T>::FC / 8;
+    using T2 = std::conditional_t<sizeof(T) == 4, float2, double2>;
+    const T *a = ck + wp * QW * 64 + 2 * lane;
+    const V *x = v + wp * QW;
+#pragma unroll
+    for (int j = 0; j < QW; j += 4) {
+        T2 l[4];
+        V xv[NR][4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) l[u] = *reinterpret_cast<const T2 *>(a + (j + u) * 64);
+#pragma unroll
+        for (int r = 0; r < NR; ++r) lds_vec(xv[r], x + r * SB + j);
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int r = 0; r < NR; ++r) {
+                acc[0][r] += V(l[u].x) * xv[r][u];
+                acc[1][r] += V(l[u].y) * xv[r][u];
+            }
+    }
+}
+
+// Backward products: how a warp's lanes share a chunk's rows and the right-hand sides.
+// With 8 right-hand sides the half-warps take 4 each (64 accumulators a lane otherwise).
+template <typename T, int NR>
+struct BwdLanes {
+    static constexpr int RH = NR > 4 ? 2 : 1, NL = NR / RH;          // groups of lanes, right-hand sides each
+    static constexpr int LN = 32 / RH, RV = SpChunk<T>::FC / LN;     // lanes of a group, rows per lane
+    static constexpr int N = 8 * NL;                                 // a lane's accumulators (8 columns)
+    static constexpr int NV = N > LN ? N / LN : 1;                   // sums a lane ends with
+    static constexpr int VW = 16 / int(sizeof(T));                   // rows per 16-byte load
+    // first of the chunk rows of vector load k of a lane (loads of a group are contiguous)
+    static __device__ __forceinline__ int row(int lane, int k) { return (k * LN + (lane & (LN - 1))) * VW; }
+};
+// One chunk (FC rows x 64 columns, column-major) times v ([r][SB]): the warp's 8 columns
+// from col0 on, rows below nrows.
+template <typename T, typename V, int NR>
+__device__ __forceinline__ void bwd_chunk(const T *ck, const V *v, V (&acc)[BwdLanes<T, NR>::N], int col0, int lane,
+                                          int nrows) {
+    using B = BwdLanes<T, NR>;
+    constexpr int FC = SpChunk<T>::FC, VW = B::VW;
+    const V *vr = v + (lane / B::LN) * B::NL * SB;
+#pragma unroll
+    for (int k = 0; k < B::RV / VW; ++k) {
+        const int row = B::row(lane, k);
+        if (row >= nrows) break;
+        V xv[B::NL][VW];
+#pragma unroll
+        for (int r = 0; r < B::NL; ++r) lds_vec(xv[r], vr + r * SB + row);
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            T l[VW];
+            lds_vec(l, ck + (col0 + u) * FC + row);
+#pragma unroll
+            for (int e = 0; e < VW; ++e)
+#pragma unroll
+                for (int r = 0; r < B::NL; ++r) acc[u * B::NL + r] += V(l[e]) * xv[r][e];
+        }
+    }
+}
+
+// Sum N values (a power of two) over groups of LN lanes, spreading the sums: at each step
+// a lane keeps one half of its values and hands the other to its partner. Lane `lane`
+// ends with the sums spread_index, spread_index + 1, .. (N / LN of them; one, held by
+// LN / N lanes, when N < LN).
+template <int N, int LN, typename V>
+__device__ __forceinline__ void spread_sum(V (&v)[N], int lane) {
+    int n = N;
+#pragma unroll
+    for (int o = LN / 2; o > 0; o >>= 1) {
+        if (n > 1) {
+            n >>= 1;
+            const bool up = lane & o;
+#pragma unroll
+            for (int k = 0; k < N / 2; ++k)
+                if (k < n) {
+                    const V give = up ? v[k] : v[k + n], keep = up ? v[k + n] : v[k];
+                    v[k] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+                }
+        } else {
+            v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+        }
+    }
+}
+template <int N, int LN>
+__device__ __forceinline__ int spread_index(int lane) {
+    int idx = 0, n = N;
+#pragma unroll
+    for (int o = LN / 2; o > 0; o >>= 1)
+        if (n > 1) {
+            n >>= 1;
+            if (lane & o) idx += n;
+        }
+    return idx;
+}
+// Whether this lane is the one that stores its value (N < LN: the first of its holders).
+template <int N, int LN>
+__device__ __forceinline__ bool spread_first(int lane) {
+    return N >= LN || (lane & (LN / N - 1)) == 0;
+}
+
+// Barriers of a CTA: chunk ring, vector buffers, gathered own rows (full / empty each).
+template <int NST, int VS, int OS>
+struct SpBars {
+    uint64_t full[NST], empty[NST], vfull[VS], vempty[VS], ofull[OS], oempty[OS], pfull[kPubSlots], pempty[kPubSlots];
+};
+struct SpRing {
+    uint32_t full, empty, vfull, vempty, ofull, oempty, pfull, pempty;
+};
+template <int NST, int VS, int OS>
+__device__ __forceinline__ SpRing init_bars(SpBars<NST, VS, OS> &b) {
+    const SpRing rg{smem_u32(b.full),   smem_u32(b.empty), smem_u32(b.vfull),
+                    smem_u32(b.vempty), smem_u32(b.ofull), smem_u32(b.oempty), smem_u32(b.pfull), smem_u32(b.pempty)};
+    if (threadIdx.x == 0) {
+        for (int k = 0; k < NST; ++k) {
+            mbar_init(rg.full + 8 * k, 1);
+            mbar_init(rg.empty + 8 * k, 8);
+        }
+        for (int k = 0; k < VS; ++k) {
+            mbar_init(rg.vfull + 8 * k, 64);
+            mbar_init(rg.vempty + 8 * k, 8);
+        }
+        for (int k = 0; k < OS; ++k) {
+            mbar_init(rg.ofull + 8 * k, 32);
+            mbar_init(rg.oempty + 8 * k, 8);
+        }
+        for (int k = 0; k < kPubSlots; ++k) {
+            mbar_init(rg.pfull + 8 * k, 8);
+            mbar_init(rg.pempty + 8 * k, 1);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    return rg;
+}
+
+// What a task streams. Forward: ndep chunks of earlier superblocks (diagonal tasks) or
+// of the whole width (structure tasks, K < 0), then ninv chunks of the inverse.
+template <typename T>
+struct FwdShape {
+    int w, f, R0, ndep, ninv, ngroups;
+    __device__ __forceinline__ explicit FwdShape(const SbTask &tk) : w(tk.w), f(tk.f) {
+        constexpr int FC = SpChunk<T>::FC;
+        if (tk.K < 0) {
+            R0 = (w & ~3) + tk.pad * 64;
+            ndep = (w + FC - 1) / FC;
+            ninv = 0;
+            ngroups = (w + SB - 1) / SB;
+        } else {
+            R0 = tk.K * SB + tk.pad * 64;
+            ndep = tk.K * (SB / FC);
+            ninv = ((tk.pad + 1) * 64 + FC - 1) / FC;    // up to the rows' last nonzero column
+            ngroups = tk.K;
+        }
+    }
+};
+// Backward: nstr chunks of L21 (groups of 256 rows from the last up), nql of the last superblock, then the others down to K + 1,
+// then ninv of the inverse (from row 64 h on).
+template <typename T>
+struct BwdShape {
+    static constexpr int FC = SpChunk<T>::FC, per = SB / FC;
+    int w, f, nsb, C0, nstr, nsg, nql, ndep, ninv, irows;
+    __device__ __forceinline__ explicit BwdShape(const SbTask &tk) : w(tk.w), f(tk.f) {
+        nsb = (w + SB - 1) / SB;
+        C0 = tk.K * SB + tk.pad * 64;
+        nstr = f > w ? (f - (w & ~3) + FC - 1) / FC : 0;
+        nsg = (nstr + per - 1) / per;
+        nql = tk.K < nsb - 1 ? (sb_pad(sb_rows(w, nsb - 1)) + FC - 1) / FC : 0;
+        ndep = nql > 0 ? nql + (nsb - 2 - tk.K) * per : 0;
+        irows = sb_pad(sb_rows(w, tk.K)) - tk.pad * 64;
+        ninv = (irows + FC - 1) / FC;
+    }
+    // chunk q of the superblock part: superblock J, chunk c of it
+    __device__ __forceinline__ void dep(int q, int &J, int &c) const {
+        if (q < nql) {
+            J = nsb - 1;
+            c = q;
+        } else {
+            J = nsb - 2 - (q - nql) / per;
+            c = (q - nql) % per;
+        }
+    }
+};
+
+// Copy warp, lane 0: every chunk of the CTA's tasks in order into the ring.
+template <typename T, int NST, bool FWD>
+__device__ __forceinline__ void copy_chunks(const SbTask *tasks, int ntasks, const char *maps, T *ring,
+                                            const SpRing &rg, int *err) {
+    constexpr int FC = SpChunk<T>::FC, CE = SpChunk<T>::ELEMS;
+    long long gq = 0;
+    bool ok = true;
+    auto load = [&](const char *map, int x, int y) {
+        const int slot = int(gq % NST);
+        if (gq >= NST && !mbar_wait(rg.empty + 8 * slot, uint32_t((gq / NST) - 1) & 1u, err)) ok = false;
+        if (!ok) return;
+        mbar_expect_tx(rg.full + 8 * slot, SpChunk<T>::BYTES);
+        tma_load_2d(smem_u32(ring + slot * CE), map, x, y, rg.full + 8 * slot);
+        ++gq;
+    };
+    for (int t = blockIdx.x; t < ntasks && ok; t += gridDim.x) {
+        const SbTask tk = tasks[t];
+        const char *pm = maps + size_t(tk.pmap + (FWD ? 0 : 1)) * kTensorMapBytes;
+        const char *im = maps + size_t(tk.imap + (FWD ? 0 : 1)) * kTensorMapBytes;
+        if constexpr (FWD) {
+            const FwdShape<T> sh(tk);
+            for (int q = 0; q < sh.ndep && ok; ++q) load(pm, sh.R0, q * FC);
+            for (int c = 0; c < sh.ninv && ok; ++c) load(im, tk.pad * 64, c * FC);
+        } else {
+            const BwdShape<T> sh(tk);
+            for (int g = sh.nsg - 1; g >= 0; --g)
+                for (int c = g * (SB / FC); c < min(sh.nstr, (g + 1) * (SB / FC)) && ok; ++c)
+                    load(pm, (sh.w & ~3) + c * FC, sh.C0);
+            for (int q = 0; q < sh.ndep && ok; ++q) {
+                int J, c;
+                sh.dep(q, J, c);
+                load(pm, J * SB + c * FC, sh.C0);
+            }
+            for (int c = 0; c < sh.ninv && ok; ++c) load(im, tk.pad * 64 + c * FC, tk.pad * 64);
+        }
+    }
+    // whatever happened, the copies issued land before the CTA's shared memory goes away
+    for (long long q = gq > NST ? gq - NST : 0; q < gq; ++q) {
+        const uint32_t bar = rg.full + 8 * uint32_t(q % NST), par = uint32_t(q / NST) & 1u;
         const unsigned long long t0 = gtimer();
         while (!mbar_try(bar, par) && gtimer() - t0 < kWaitNs) {
         }
     }
 }
 
-// Thread 0 waits until the count at p reaches target (bounded), then the block proceeds.
-__device__ __forceinline__ void wait_count(const int *p, int target, int *err) {
-    if (threadIdx.x == 0) {
-        if (ld_acquire(p) < target) {
-            const unsigned long long t0 = gtimer();
-            while (ld_acquire(p) < target) {
-                if (*(volatile int *)err) break;
-                if (gtimer() - t0 > kWaitNs) {
-                    atomicExch(err, 1);
-                    break;
-                }
-            }
-        }
-    }
-    __syncthreads();
+// The warp's stores so far are published and counted (diagonal tasks: the chain waits, and
+// eight warps releasing their own stores side by side are sooner done than one for all).
+__device__ __forceinline__ void warp_count(int *p, int lane) {
+    __syncwarp();
+    if (lane == 0) asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(p) : "memory");
 }
-// After a __syncthreads that follows this block's writes: publish them and count.
-__device__ __forceinline__ void count_up(int *p) {
-    if (threadIdx.x == 0) {
-        __threadfence();
-        atomicAdd(p, 1);
+// Count warp, lane 0: once all product warps have handed over a structure task's stores,
+// publish them to the GPU and count (a release waits for the stores to arrive, 0.8 us that
+// the product warps would each spend otherwise: 1.5 instead of 2.15 us for a task of 64
+// rows x 33 columns in FP64).
+__device__ __forceinline__ void publish(const SbTask *tasks, int ntasks, const SpRing &rg, int *flags, int *err) {
+    int e = 0;
+    for (int t = blockIdx.x; t < ntasks; t += gridDim.x) {
+        const SbTask tk = tasks[t];
+        if (tk.K >= 0) continue;
+        const int slot = e % kPubSlots;
+        if (!mbar_wait(rg.pfull + 8 * slot, uint32_t(e / kPubSlots) & 1u, err)) return;
+        asm volatile("fence.acq_rel.gpu;" ::: "memory");
+        asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(flags + tk.flag0 + 2 * ((tk.w + SB - 1) / SB))
+                     : "memory");
+        mbar_arrive(rg.pempty + 8 * slot);
+        ++e;
+    }
+}
+// A product warp's side: its stores so far belong to the CTA's next count.
+struct Handover {
+    const SpRing &rg;
+    int *err;
+    int e = 0;
+    __device__ __forceinline__ void operator()(int lane) {
+        const int slot = e % kPubSlots;
+        if (e >= kPubSlots) mbar_wait(rg.pempty + 8 * slot, uint32_t(e / kPubSlots - 1) & 1u, err);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(rg.pfull + 8 * slot);
+        ++e;
+    }
+};
+
+// Vector warps: the vectors of every group of 256 rows, [r][256]. Two pairs take the groups
+// in turn (a group costs a count's and a vector's round trip to L2, and small tasks have
+// one each); a warp of a pair brings 128 rows. (A pair passes every second group, so its
+// waits by parity are unambiguous with two buffers or more.)
+constexpr int VR = SB / 2 / 32;                          // rows per lane
+
+// Forward: y_J.
+template <typename T, int NR, int VS>
+__device__ __forceinline__ void fwd_vectors(const SbTask *tasks, int ntasks, const double *X,
+                                            int64_t ldx, int nrhs, PT<T> *vp, const SpRing &rg, const int *flags,
+                                            int *err, int me) {
+    using P = PT<T>;
+    const int pair = me >> 1, i0 = (me & 1) * (SB / 2) + (threadIdx.x & 31);
+    long long gv = 0;
+    for (int t = blockIdx.x; t < ntasks; t += gridDim.x) {
+        const SbTask tk = tasks[t];
+        const FwdShape<T> sh(tk);
+        const int c0 = tk.c0;
+        for (int J = 0; J < sh.ngroups; ++J, ++gv) {
+            if (int(gv & 1) != pair) continue;
+            const int slot = int(gv % VS);
+            if (gv >= VS && !mbar_wait(rg.vempty + 8 * slot, uint32_t(gv / VS - 1) & 1u, err)) return;
+            const int nrJ = sb_rows(sh.w, J);
+            spin_count(flags + tk.flag0 + 2 * J, 8 * (sb_pad(nrJ) / 64), err);
+            const double *xj = X + c0 + J * SB;
+            P *dst = vp + slot * (NR * SB);
+            double v[NR][VR];                      // (written by other CTAs: through L2)
+#pragma unroll
+            for (int r = 0; r < NR; ++r)
+#pragma unroll
+                for (int k = 0; k < VR; ++k) {
+                    const int row = i0 + 32 * k;
+                    v[r][k] = (row < nrJ && r < nrhs) ? __ldcg(xj + row + r * ldx) : 0.0;
+                }
+#pragma unroll
+            for (int r = 0; r < NR; ++r)
+#pragma unroll
+                for (int k = 0; k < VR; ++k) dst[r * SB + i0 + 32 * k] = P(v[r][k]);
+            mbar_arrive(rg.vfull + 8 * slot);
+        }
     }
 }
 
-// Forward task (s, K, h = tk.pad): rows R0 = K SB + 64 h, nrh of them. Chunks: for
-// J < K, L(rows R0.., columns J SB + c FC ..) (c < SB / FC), then the inverse's
-// rows 64 h.. of columns [c FC, c FC + FC) up to column 64 h + 63 (the rest of
-// the row is zero). Thread (i = tid % 64, part = tid / 64) sums columns
-// [part FC / 4, (part + 1) FC / 4) of every chunk for row i.
-template <typename T, int NST, int NR>
-__global__ void __launch_bounds__(kSbThreads, 1) sp_fwd_kernel(const SbTask *__restrict__ tasks, int ntasks,
-                                                               SnDev sd, const T *__restrict__ factor,
-                                                               const char *__restrict__ maps, double *__restrict__ X, int64_t ldx, int nrhs,
-                                                               double *__restrict__ scratch, int *__restrict__ flags,
-                                                               int *__restrict__ err) {
-    using Lay = SpLayout<T, NST, NR>;
+// Backward: x_struct from the last rows up (the ancestors are done from the root down, and
+// each from its last superblock on, so that most of L21 is read while the parent's chain
+// still runs), then x_J (J descending). A group's lowest row is the last to become final:
+// rowcnt gives its superblock's count and parts.
+template <typename T, int NR, int VS>
+__device__ __forceinline__ void bwd_vectors(const SbTask *tasks, int ntasks, const SnDev &sd, const int32_t *rowcnt,
+                                            const double *X, int64_t ldx, int nrhs, PT<T> *vp, const SpRing &rg,
+                                            const int *flags, int *err, int me) {
     using P = PT<T>;
-    constexpr int FC = SpChunk<T>::FC, CE = SpChunk<T>::ELEMS;
-    constexpr int per = SB / FC;                         // chunks per earlier superblock
-    constexpr int QC = FC / 4;
+    const int pair = me >> 1, i0 = (me & 1) * (SB / 2) + (threadIdx.x & 31);
+    const int vb = sd.vb;
+    long long gv = 0;
+    for (int t = blockIdx.x; t < ntasks; t += gridDim.x) {
+        const SbTask tk = tasks[t];
+        const BwdShape<T> sh(tk);
+        const int c0 = tk.c0;
+        const int32_t *rows = sd.struct_rows + sd.struct_ptr[tk.sn];
+        const int nv = sh.nsg + (sh.nsb - 1 - tk.K);
+        // the rows' places in X (-1: none) and the count to wait for, a group ahead of their use
+        int64_t next[VR];
+        int nflag = 0, nneed = 0;
+        auto places = [&](int g) {
+            if (g >= nv) return;
+            if (g < sh.nsg) {
+                const int base = (sh.w & ~3) + (sh.nsg - 1 - g) * SB;
+                const int rc = rowcnt[rows[(max(base, sh.w) - sh.w) / vb]];
+                nflag = rc >> 2;
+                nneed = 16 * ((rc & 3) + 1);
+#pragma unroll
+                for (int k = 0; k < VR; ++k) {
+                    const int row = base + i0 + 32 * k, li = row - sh.w;
+                    next[k] = row >= sh.w && row < sh.f ? int64_t(rows[li / vb]) * vb + li % vb : -1;
+                }
+            } else {
+                const int J = sh.nsb - 1 - (g - sh.nsg), nrJ = sb_rows(sh.w, J);
+                nflag = tk.flag0 + 2 * J;
+                nneed = 16 * (sb_pad(nrJ) / 64);
+#pragma unroll
+                for (int k = 0; k < VR; ++k) {
+                    const int i = i0 + 32 * k;
+                    next[k] = i < nrJ ? c0 + J * SB + i : -1;
+                }
+            }
+        };
+        places(int(gv & 1) == pair ? 0 : 1);
+        for (int g = 0; g < nv; ++g, ++gv) {
+            if (int(gv & 1) != pair) continue;
+            const int slot = int(gv % VS);
+            int64_t at[VR];
+#pragma unroll
+            for (int k = 0; k < VR; ++k) at[k] = next[k];
+            const int flag = nflag, need = nneed;
+            places(g + 2);
+            if (gv >= VS && !mbar_wait(rg.vempty + 8 * slot, uint32_t(gv / VS - 1) & 1u, err)) return;
+            spin_count(flags + flag, need, err);
+            P *dst = vp + slot * (NR * SB);
+            double v[NR][VR];
+#pragma unroll
+            for (int r = 0; r < NR; ++r)
+#pragma unroll
+                for (int k = 0; k < VR; ++k)
+                    v[r][k] = (at[k] >= 0 && r < nrhs) ? __ldcg(X + at[k] + r * ldx) : 0.0;
+#pragma unroll
+            for (int r = 0; r < NR; ++r)
+#pragma unroll
+                for (int k = 0; k < VR; ++k) dst[r * SB + i0 + 32 * k] = P(v[r][k]);
+            mbar_arrive(rg.vfull + 8 * slot);
+        }
+    }
+}
+
+// Gather warp `me`: every kGatherWarps-th task with its own rows, [r][64]. Forward: the
+// right-hand side of a diagonal task's rows plus the children's update vectors, in child
+// order; backward: y. What does not depend on a count (the task, its children, their row
+// maps) is loaded a task ahead.
+template <int NR, bool FWD>
+__device__ __forceinline__ void gather_own(const SbTask *tasks, int ntasks, int vb, const SbChild *children,
+                                           const int32_t *cmap, const double *X, int64_t ldx, int nrhs,
+                                           const double *sol, SbTask *meta, double *own, const SpRing &rg,
+                                           const int *flags, int *err, int me) {
+    constexpr int OS = own_slots(NR);
+    const int lane = threadIdx.x & 31;
+    struct Ahead {
+        SbTask tk;
+        SbChild ch[2];                                   // the first two children
+        int m[2][2];                                     // [row][child]: block of the child's structure, or -1
+    } nx;
+    auto rows = [&](const SbTask &tk, int e, int &brow, int &off) {
+        const int row = (tk.K < 0 ? (tk.w & ~3) : tk.K * SB) + tk.pad * 64 + lane + 32 * e;
+        brow = row / vb;
+        off = row - brow * vb;
+        return tk.K < 0 ? (row >= tk.w && row < tk.f) : row < tk.w;
+    };
+    auto maps = [&](const SbTask &tk, int ci, SbChild (&ch)[2], int (&m)[2][2]) {
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+            if (ci + k < tk.nchild) ch[k] = children[tk.child0 + ci + k];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            int brow, off;
+            const bool live = rows(tk, e, brow, off);
+#pragma unroll
+            for (int k = 0; k < 2; ++k) m[e][k] = (ci + k < tk.nchild && live) ? cmap[ch[k].map + brow] : -1;
+        }
+    };
+    auto ahead = [&](int t) {
+        if (t >= ntasks) return;
+        nx.tk = tasks[t];
+        if constexpr (FWD) maps(nx.tk, 0, nx.ch, nx.m);
+    };
+    const int stride = gridDim.x * kGatherWarps;
+    int it = me;
+    ahead(blockIdx.x + me * int(gridDim.x));
+    for (int t = blockIdx.x + me * gridDim.x; t < ntasks; t += stride, it += kGatherWarps) {
+        const int slot = it % OS;
+        const SbTask tk = nx.tk;
+        double v[2][NR];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            int brow, off;
+            const bool live = rows(tk, e, brow, off) && tk.K >= 0;
+            const double *x = X + tk.c0 + brow * vb + off;
+#pragma unroll
+            for (int r = 0; r < NR; ++r) v[e][r] = (live && r < nrhs) ? x[r * ldx] : 0.0;
+        }
+        if constexpr (FWD) {
+            SbChild ch[2] = {nx.ch[0], nx.ch[1]};
+            int m[2][2] = {{nx.m[0][0], nx.m[0][1]}, {nx.m[1][0], nx.m[1][1]}};
+            ahead(t + stride);
+            for (int ci = 0; ci < tk.nchild; ci += 2) {
+                if (ci) maps(tk, ci, ch, m);
+#pragma unroll
+                for (int k = 0; k < 2; ++k)
+                    if (ci + k < tk.nchild && ch[k].flag >= 0) spin_count(flags + ch[k].flag, ch[k].need, err);
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    double u[2][NR];
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        int brow, off;
+                        rows(tk, e, brow, off);
+                        const double *uc = sol + ch[k].sol * nrhs + m[e][k] * vb + off;
+#pragma unroll
+                        for (int r = 0; r < NR; ++r)
+                            u[e][r] = (m[e][k] >= 0 && r < nrhs) ? __ldcg(uc + int64_t(r) * ch[k].d) : 0.0;
+                    }
+#pragma unroll
+                    for (int e = 0; e < 2; ++e)
+#pragma unroll
+                        for (int r = 0; r < NR; ++r) v[e][r] += u[e][r];
+                }
+            }
+        } else {
+            ahead(t + stride);
+        }
+        if (it >= OS && !mbar_wait(rg.oempty + 8 * slot, uint32_t(it / OS - 1) & 1u, err)) return;
+        double *o = own + slot * (NR * 64);
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+#pragma unroll
+            for (int r = 0; r < NR; ++r) o[r * 64 + lane + 32 * e] = v[e][r];
+        if (lane == 0) meta[slot] = tk;
+        mbar_arrive(rg.ofull + 8 * slot);
+    }
+}
+
+template <typename T, int NST, int NR, int VS>
+__global__ void __launch_bounds__(kSbThreads, 1)
+    sp_fwd_kernel(const SbTask *__restrict__ tasks, int ntasks, SnDev sd, const char *__restrict__ maps,
+                  const SbChild *__restrict__ children, const int32_t *__restrict__ cmap, double *X, int64_t ldx,
+                  int nrhs, double *sol, double *scratch, int *flags, int *err) {
+    using Lay = SpLayout<T, NST, NR, VS>;
+    using P = PT<T>;
+    constexpr int FC = SpChunk<T>::FC, CE = SpChunk<T>::ELEMS, per = SB / FC;
+    constexpr int NO = (NR + 3) / 4;
     extern __shared__ __align__(128) unsigned char sp_dyn[];
-    __shared__ __align__(8) uint64_t bars[NST];
+    constexpr int OS = own_slots(NR);
+    __shared__ __align__(8) SpBars<NST, VS, OS> bars;
+    __shared__ SbTask meta[OS];
     // TMA destinations: 128-byte aligned (the launch adds 128 bytes for this)
     unsigned char *sp_raw = sp_dyn + ((128u - (smem_u32(sp_dyn) & 127u)) & 127u);
     T *ring = reinterpret_cast<T *>(sp_raw);
-    double *vec = reinterpret_cast<double *>(sp_raw + Lay::vec_off);
     P *vp = reinterpret_cast<P *>(sp_raw + Lay::vp_off);
     double *red = reinterpret_cast<double *>(sp_raw + Lay::red_off);
-    double *own = reinterpret_cast<double *>(sp_raw + Lay::own_off);
-    const int tid = threadIdx.x, i = tid & 63, part = tid >> 6;
-    if (tid == 0) {
-        for (int b = 0; b < NST; ++b) mbar_init(smem_u32(&bars[b]), 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    double *vec = red;
+    double *owns = reinterpret_cast<double *>(sp_raw + Lay::own_off);
+    const SpRing rg = init_bars(bars);
+    const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
+    if (wp == 8) {
+        if (lane == 0) copy_chunks<T, NST, true>(tasks, ntasks, maps, ring, rg, err);
+        return;
     }
-    __syncthreads();
-    long long gq = 0;                                    // chunks this CTA has consumed (ring phase)
-    for (int t = blockIdx.x; t < ntasks; t += gridDim.x) {
-        const SbTask tk = tasks[t];
-        const int s = tk.sn, K = tk.K, h = tk.pad;
-        const int w = sd.w[s], c0 = sd.col0[s];
-        const int nrK = sb_rows(w, K), nrpK = sb_pad(nrK), nhK = nrpK / 64;
-        const int R0 = K * SB + h * 64, nrh = min(64, w - R0);
-        const int icols = (h + 1) * 64;                  // nonzero columns of the inverse's rows
-        const int ndep = K * per;
-        const int nq = ndep + (icols + FC - 1) / FC;
-        int *ycnt = flags + tk.flag0;                    // [2 J]: parts of J done, [2 J + 1]: a_J parts
-        auto stage = [&](int q) {
-            const int slot = int((gq + q) % NST);
-            T *dst = ring + slot * CE;
-            const uint32_t bar = smem_u32(&bars[slot]);
-            mbar_expect_tx(bar, SpChunk<T>::BYTES);
-            if (q < ndep) {
-                const int J = q / per, c = q - J * per;
-                tma_load_2d(smem_u32(dst), maps + size_t(tk.pmap) * kTensorMapBytes, R0, J * SB + c * FC, bar);
-            } else {
-                const int c = q - ndep;
-                tma_load_2d(smem_u32(dst), maps + size_t(tk.imap) * kTensorMapBytes, h * 64, c * FC, bar);
-            }
-        };
-        __syncthreads();                                 // the previous task is done with shared memory
-        if (tid == 0)
-            for (int q = 0; q < NST - 1 && q < nq; ++q) stage(q);
-        if (tid < 64)
-            for (int r = 0; r < NR; ++r) own[r * 64 + i] = (r < nrhs && i < nrh) ? X[c0 + R0 + i + r * ldx] : 0.0;
-        P pacc[NR];
-        double dacc[NR];
-#pragma unroll
-        for (int r = 0; r < NR; ++r) {
-            pacc[r] = P(0);
-            dacc[r] = 0.0;
-        }
-        auto chunk = [&](int q) -> const T * {
-            const int slot = int((gq + q) % NST);
-            mbar_wait_all(smem_u32(&bars[slot]), uint32_t(((gq + q) / NST) & 1), err);
-            __syncthreads();                             // (also: vectors are complete)
-            return ring + slot * CE;
-        };
-        for (int q = 0; q < ndep; ++q) {
-            if (tid == 0 && q + NST - 1 < nq) stage(q + NST - 1);
-            const int J = q / per, c = q - J * per;
-            if (c == 0) {
-                // y_J: wait for its parts, then load it (written by other CTAs: through L2)
-                wait_count(ycnt + 2 * J, SB / 64, err);
-#pragma unroll
-                for (int r = 0; r < NR; ++r) {
-                    const double v = r < nrhs ? __ldcg(&X[c0 + J * SB + tid + r * ldx]) : 0.0;
-                    vec[r * SB + tid] = v;
-                    vp[r * SB + tid] = P(v);
-                }
-            }
-            const T *a = chunk(q) + part * QC * 64 + i;
-            const P *v = vp + c * FC + part * QC;
-#pragma unroll 8
-            for (int j = 0; j < QC; ++j) {
-                const P l = P(a[j * 64]);
-#pragma unroll
-                for (int r = 0; r < NR; ++r) pacc[r] += l * v[r * SB + j];
-            }
-            __syncthreads();                             // the ring slot is refilled NST - 1 chunks later
-        }
-        // every dependency is in: a_h = own - sums, to the scratch vector; count, wait
-        // for the other parts of K, load a_K
-#pragma unroll
-        for (int r = 0; r < NR; ++r) red[(part * NR + r) * 64 + i] = double(pacc[r]);
-        __syncthreads();
-        if (tid < 64)
-#pragma unroll
-            for (int r = 0; r < NR; ++r) {
-                const int e = r * 64 + i;
-                const double a = own[e] - (((red[e] + red[NR * 64 + e]) + red[2 * NR * 64 + e]) + red[3 * NR * 64 + e]);
-                if (r < nrhs && i < nrh) scratch[c0 + R0 + i + r * ldx] = a;
-            }
-        __syncthreads();
-        count_up(ycnt + 2 * K + 1);
-        wait_count(ycnt + 2 * K + 1, nhK, err);
+    if (wp > 8 && wp <= 8 + kVecWarps) {
+        fwd_vectors<T, NR, VS>(tasks, ntasks, X, ldx, nrhs, vp, rg, flags, err, wp - 9);
+        return;
+    }
+    if (wp == 9 + kVecWarps + kGatherWarps) {
+        if (lane == 0) publish(tasks, ntasks, rg, flags, err);
+        return;
+    }
+    if (wp > 8) {
+        gather_own<NR, true>(tasks, ntasks, sd.vb, children, cmap, X, ldx, nrhs, sol, meta, owns, rg, flags, err,
+                                wp - 9 - kVecWarps);
+        return;
+    }
+    const int i = tid & 63, part = tid >> 6;             // combining thread: row i, right-hand sides part + 4 o
+    long long gq = 0, gv = 0;
+    Handover handover{rg, err};
+    auto chunk = [&]() -> const T * {
+        const int slot = int(gq % NST);
+        mbar_wait(rg.full + 8 * slot, uint32_t(gq / NST) & 1u, err);
+        return ring + slot * CE;
+    };
+    auto release = [&]() {
+        __syncwarp();
+        if (lane == 0) mbar_arrive(rg.empty + 8 * uint32_t(gq % NST));
+        ++gq;
+    };
+    // per-warp partial sums to shared memory, then the sum over warps of this thread's entries
+    auto combine = [&](const double (&d)[2][NR], double (&out)[NO]) {
+        psync();                                         // red / vec of before is read
 #pragma unroll
         for (int r = 0; r < NR; ++r)
-            vec[r * SB + tid] = (r < nrhs && tid < nrK) ? __ldcg(&scratch[c0 + K * SB + tid + r * ldx]) : 0.0;
-        for (int q = ndep; q < nq; ++q) {
-            if (tid == 0 && q + NST - 1 < nq) stage(q + NST - 1);
-            const int c = q - ndep;
-            const int j0 = part * QC, j1 = min(QC, min(FC, icols - c * FC) - j0);
-            const T *a = chunk(q) + j0 * 64 + i;
-            const double *v = vec + c * FC + j0;
-            for (int j = 0; j < j1; ++j) {
-                const double l = double(a[j * 64]);
+            *reinterpret_cast<double2 *>(red + (wp * NR + r) * 64 + 2 * lane) = make_double2(d[0][r], d[1][r]);
+        psync();
 #pragma unroll
-                for (int r = 0; r < NR; ++r) dacc[r] += l * v[r * SB + j];
-            }
-            __syncthreads();
+        for (int o = 0; o < NO; ++o) {
+            const int r = part + 4 * o;
+            double s = 0.0;
+            if (r < NR)
+#pragma unroll
+                for (int k = 0; k < 8; ++k) s += red[(k * NR + r) * 64 + i];
+            out[o] = s;
         }
-        gq += nq;
+    };
+    int it = 0;
+    for (int t = blockIdx.x; t < ntasks; t += gridDim.x, ++it) {
+        const int os = it % OS;
+        mbar_wait(rg.ofull + 8 * os, uint32_t(it / OS) & 1u, err);
+        const SbTask tk = meta[os];
+        const int c0 = tk.c0;
+        const FwdShape<T> sh(tk);
+        const int w = sh.w, K = tk.K;
+        const int row = sh.R0 + i;                       // front row of this thread's entries
+        const bool live = K < 0 ? (row >= w && row < sh.f) : row < w;
+        int *cnt = flags + tk.flag0;
+        double own[NO];
 #pragma unroll
-        for (int r = 0; r < NR; ++r) red[(part * NR + r) * 64 + i] = dacc[r];
-        __syncthreads();
-        if (tid < 64)
+        for (int o = 0; o < NO; ++o) own[o] = part + 4 * o < NR ? owns[(os * NR + part + 4 * o) * 64 + i] : 0.0;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(rg.oempty + 8 * os);
+        double dacc[2][NR];
+#pragma unroll
+        for (int r = 0; r < NR; ++r) dacc[0][r] = dacc[1][r] = 0.0;
+        for (int J = 0, q = 0; J < sh.ngroups; ++J, ++gv) {
+            const int slot = int(gv % VS), qe = min(sh.ndep, q + per);
+            mbar_wait(rg.vfull + 8 * slot, uint32_t(gv / VS) & 1u, err);
+            P pacc[2][NR];
+#pragma unroll
+            for (int r = 0; r < NR; ++r) pacc[0][r] = pacc[1][r] = P(0);
+            for (int c = 0; q < qe; ++q, ++c) {
+                const T *ck = chunk();
+                if (J * SB + c * FC + wp * (FC / 8) < w)
+                    fwd_chunk<T, P, NR>(ck, vp + slot * (NR * SB) + c * FC, pacc, wp, lane);
+                release();
+            }
+            if (lane == 0) mbar_arrive(rg.vempty + 8 * slot);   // (after release's __syncwarp)
 #pragma unroll
             for (int r = 0; r < NR; ++r) {
-                const int e = r * 64 + i;
-                const double y = ((red[e] + red[NR * 64 + e]) + red[2 * NR * 64 + e]) + red[3 * NR * 64 + e];
-                if (r < nrhs && i < nrh) X[c0 + R0 + i + r * ldx] = y;
+                dacc[0][r] += double(pacc[0][r]);
+                dacc[1][r] += double(pacc[1][r]);
             }
-        __syncthreads();
-        count_up(ycnt + 2 * K);
+        }
+        double sum[NO];
+        combine(dacc, sum);
+        if (K < 0) {
+#pragma unroll
+            for (int o = 0; o < NO; ++o) {
+                const int r = part + 4 * o;
+                if (live && r < nrhs) sol[tk.sol * nrhs + (row - w) + int64_t(r) * (sh.f - w)] = own[o] - sum[o];
+            }
+            handover(lane);
+            continue;
+        }
+        // a_h; exchanged with the other parts of K through the scratch vector
+        const int nrK = sb_rows(w, K), nhK = sb_pad(nrK) / 64;
+        if (nhK > 1) {
+#pragma unroll
+            for (int o = 0; o < NO; ++o) {
+                const int r = part + 4 * o;
+                if (live && r < nrhs) scratch[c0 + row + r * ldx] = own[o] - sum[o];
+            }
+            // (this CTA's eight warps are among the counted: all have read red then)
+            warp_count(cnt + 2 * K + 1, lane);
+            spin_count(cnt + 2 * K + 1, 8 * nhK, err);
+#pragma unroll
+            for (int r = 0; r < NR; ++r)
+                vec[r * SB + tid] = (r < nrhs && tid < nrK) ? __ldcg(&scratch[c0 + K * SB + tid + r * ldx]) : 0.0;
+        } else {
+            psync();                                     // red is read, vec may be written
+#pragma unroll
+            for (int o = 0; o < NO; ++o) {
+                const int r = part + 4 * o;
+                if (r < NR) vec[r * SB + i] = (live && r < nrhs) ? own[o] - sum[o] : 0.0;
+            }
+        }
+        psync();
+#pragma unroll
+        for (int r = 0; r < NR; ++r) dacc[0][r] = dacc[1][r] = 0.0;
+        for (int c = 0; c < sh.ninv; ++c) {
+            const T *ck = chunk();
+            if (c * FC + wp * (FC / 8) < (tk.pad + 1) * 64)
+                fwd_chunk<T, double, NR>(ck, vec + c * FC, dacc, wp, lane);
+            release();
+        }
+        combine(dacc, sum);
+#pragma unroll
+        for (int o = 0; o < NO; ++o) {
+            const int r = part + 4 * o;
+            if (live && r < nrhs) X[c0 + row + r * ldx] = sum[o];
+        }
+        warp_count(cnt + 2 * K, lane);
     }
-    ring_drain<NST>(bars, gq, err);
 }
 
-// Backward task (s, K, h = tk.pad): columns C0 = K SB + 64 h, nch of them. Chunks:
-// for J = nsb - 1 down to K + 1, L(rows J SB + c FC .., columns C0..) (the last
-// superblock's rows rounded up to 64), then the inverse's columns 64 h.. from row
-// 64 h + c FC on. Warp wp sums columns 8 wp .. 8 wp + 7 of every chunk, its lanes
-// over the chunk's rows.
-template <typename T, int NST, int NR>
-__global__ void __launch_bounds__(kSbThreads, 1) sp_bwd_kernel(const SbTask *__restrict__ tasks, int ntasks,
-                                                               SnDev sd, const T *__restrict__ factor,
-                                                               const char *__restrict__ maps, double *__restrict__ X, int64_t ldx, int nrhs,
-                                                               double *__restrict__ scratch, int *__restrict__ flags,
-                                                               int *__restrict__ err) {
-    using Lay = SpLayout<T, NST, NR>;
+template <typename T, int NST, int NR, int VS>
+__global__ void __launch_bounds__(kSbThreads, 1)
+    sp_bwd_kernel(const SbTask *__restrict__ tasks, int ntasks, SnDev sd, const char *__restrict__ maps,
+                  const SbChild *__restrict__ children, const int32_t *__restrict__ rowcnt, double *X, int64_t ldx,
+                  int nrhs, double *sol, double *scratch, int *flags, int *err) {
+    using Lay = SpLayout<T, NST, NR, VS>;
     using P = PT<T>;
-    constexpr int FC = SpChunk<T>::FC, CE = SpChunk<T>::ELEMS;
-    constexpr int per = SB / FC;                         // chunks per full later superblock
-    constexpr int RL = FC / 32;                          // chunk rows per lane
+    using B = BwdLanes<T, NR>;
+    constexpr int FC = SpChunk<T>::FC, CE = SpChunk<T>::ELEMS, per = SB / FC;
+    constexpr int N = B::N, NV = B::NV;
+    constexpr int kFlush = sizeof(T) == 4 ? 1024 / FC : 1 << 30;   // chunks between FP64 sums
     extern __shared__ __align__(128) unsigned char sp_dyn[];
-    __shared__ __align__(8) uint64_t bars[NST];
-    // TMA destinations: 128-byte aligned (the launch adds 128 bytes for this)
+    constexpr int OS = own_slots(NR);
+    __shared__ __align__(8) SpBars<NST, VS, OS> bars;
+    __shared__ SbTask meta[OS];
     unsigned char *sp_raw = sp_dyn + ((128u - (smem_u32(sp_dyn) & 127u)) & 127u);
     T *ring = reinterpret_cast<T *>(sp_raw);
-    double *vec = reinterpret_cast<double *>(sp_raw + Lay::vec_off);
     P *vp = reinterpret_cast<P *>(sp_raw + Lay::vp_off);
-    double *own = reinterpret_cast<double *>(sp_raw + Lay::own_off);
+    double *vec = reinterpret_cast<double *>(sp_raw + Lay::red_off);   // a_K, [r][SB]
+    double *owns = reinterpret_cast<double *>(sp_raw + Lay::own_off);
+    const SpRing rg = init_bars(bars);
     const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
-    if (tid == 0) {
-        for (int b = 0; b < NST; ++b) mbar_init(smem_u32(&bars[b]), 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    if (wp == 8) {
+        if (lane == 0) copy_chunks<T, NST, false>(tasks, ntasks, maps, ring, rg, err);
+        return;
     }
-    __syncthreads();
-    long long gq = 0;
-    for (int t = blockIdx.x; t < ntasks; t += gridDim.x) {
-        const SbTask tk = tasks[t];
-        const int s = tk.sn, K = tk.K, h = tk.pad;
-        const int w = sd.w[s], c0 = sd.col0[s];
-        const int nsb = (w + SB - 1) / SB;
-        const int nrK = sb_rows(w, K), nrpK = sb_pad(nrK), nhK = nrpK / 64;
-        const int C0 = K * SB + h * 64, nch = min(64, w - C0);
-        const int nrl = sb_rows(w, nsb - 1), nql = (sb_pad(nrl) + FC - 1) / FC;   // last superblock
-        const int ndep = K < nsb - 1 ? nql + (nsb - 2 - K) * per : 0;
-        const int irows = nrpK - h * 64;                 // the inverse's rows from 64 h
-        const int nq = ndep + (irows + FC - 1) / FC;
-        int *ycnt = flags + tk.flag0;
-        // dependency chunk q: superblock J, chunk c
-        auto dep = [&](int q, int &J, int &c) {
-            if (q < nql) {
-                J = nsb - 1;
-                c = q;
-            } else {
-                const int m = q - nql;
-                J = nsb - 2 - m / per;
-                c = m % per;
-            }
-        };
-        auto stage = [&](int q) {
-            const int slot = int((gq + q) % NST);
-            T *dst = ring + slot * CE;
-            const uint32_t bar = smem_u32(&bars[slot]);
-            mbar_expect_tx(bar, SpChunk<T>::BYTES);
-            if (q < ndep) {
-                int J, c;
-                dep(q, J, c);
-                tma_load_2d(smem_u32(dst), maps + size_t(tk.pmap + 1) * kTensorMapBytes, J * SB + c * FC, C0, bar);
-            } else {
-                const int c = q - ndep;
-                tma_load_2d(smem_u32(dst), maps + size_t(tk.imap + 1) * kTensorMapBytes, h * 64 + c * FC, h * 64,
-                            bar);
-            }
-        };
-        __syncthreads();
-        if (tid == 0)
-            for (int q = 0; q < NST - 1 && q < nq; ++q) stage(q);
-        if (tid < 64)
-            for (int r = 0; r < NR; ++r)
-                own[r * 64 + tid] = (r < nrhs && tid < nch) ? X[c0 + C0 + tid + r * ldx] : 0.0;
-        auto chunk = [&](int q) -> const T * {
-            const int slot = int((gq + q) % NST);
-            mbar_wait_all(smem_u32(&bars[slot]), uint32_t(((gq + q) / NST) & 1), err);
-            __syncthreads();
-            return ring + slot * CE;
-        };
-        {
-            P pacc[8][NR];
+    if (wp > 8 && wp <= 8 + kVecWarps) {
+        bwd_vectors<T, NR, VS>(tasks, ntasks, sd, rowcnt, X, ldx, nrhs, vp, rg, flags, err, wp - 9);
+        return;
+    }
+    if (wp == 9 + kVecWarps + kGatherWarps) return;      // (forward only)
+    if (wp > 8) {
+        gather_own<NR, false>(tasks, ntasks, sd.vb, children, nullptr, X, ldx, nrhs, sol, meta, owns, rg, flags, err,
+                                 wp - 9 - kVecWarps);
+        return;
+    }
+    long long gq = 0, gv = 0;
+    auto chunk = [&]() -> const T * {
+        const int slot = int(gq % NST);
+        mbar_wait(rg.full + 8 * slot, uint32_t(gq / NST) & 1u, err);
+        return ring + slot * CE;
+    };
+    auto release = [&]() {
+        __syncwarp();
+        if (lane == 0) mbar_arrive(rg.empty + 8 * uint32_t(gq % NST));
+        ++gq;
+    };
+    // the sums this lane ends with: columns and right-hand sides
+    int scol[NV], srhs[NV];
+    const bool first = spread_first<N, B::LN>(lane);
 #pragma unroll
-            for (int u = 0; u < 8; ++u)
+    for (int k = 0; k < NV; ++k) {
+        const int e = spread_index<N, B::LN>(lane) + k;
+        scol[k] = wp * 8 + e / B::NL;
+        srhs[k] = (lane / B::LN) * B::NL + e % B::NL;
+    }
+    int it = 0;
+    for (int t = blockIdx.x; t < ntasks; t += gridDim.x, ++it) {
+        const int os = it % OS;
+        mbar_wait(rg.ofull + 8 * os, uint32_t(it / OS) & 1u, err);
+        const SbTask tk = meta[os];
+        const int c0 = tk.c0, K = tk.K;
+        const BwdShape<T> sh(tk);
+        const int w = sh.w;
+        const int nch = min(64, w - sh.C0), nrK = sb_rows(w, K), nhK = sb_pad(nrK) / 64;
+        int *cnt = flags + tk.flag0;
+        double *xs = X + c0 + sh.C0;
+        double own[NV], sum[NV];
 #pragma unroll
-                for (int r = 0; r < NR; ++r) pacc[u][r] = P(0);
-            for (int q = 0; q < ndep; ++q) {
-                if (tid == 0 && q + NST - 1 < nq) stage(q + NST - 1);
-                int J, c;
-                dep(q, J, c);
-                const int nrJ = sb_rows(w, J);
-                if (c == 0) {
-                    wait_count(ycnt + 2 * J, 2 * (sb_pad(nrJ) / 64), err);
-#pragma unroll
-                    for (int r = 0; r < NR; ++r) {
-                        const double v = (r < nrhs && tid < nrJ) ? __ldcg(&X[c0 + J * SB + tid + r * ldx]) : 0.0;
-                        vec[r * SB + tid] = v;
-                        vp[r * SB + tid] = P(v);
-                    }
-                }
-                const T *tl = chunk(q);
-                // rows of the chunk at or past the superblock's end are masked out
-                const int nv = nrJ - c * FC;
-                const P *v = vp + c * FC;
-#pragma unroll
-                for (int k = 0; k < RL; ++k) {
-                    const int row = lane + 32 * k;
-                    const bool ok = row < nv;
-                    P x[NR];
-#pragma unroll
-                    for (int r = 0; r < NR; ++r) x[r] = ok ? v[r * SB + row] : P(0);
-#pragma unroll
-                    for (int u = 0; u < 8; ++u) {
-                        const P l = ok ? P(tl[(wp * 8 + u) * FC + row]) : P(0);
-#pragma unroll
-                        for (int r = 0; r < NR; ++r) pacc[u][r] += l * x[r];
-                    }
-                }
-                __syncthreads();
-            }
-            __syncthreads();                             // own is complete
-#pragma unroll
-            for (int u = 0; u < 8; ++u)
-#pragma unroll
-                for (int r = 0; r < NR; ++r) {
-                    P g = pacc[u][r];
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) g += __shfl_down_sync(0xffffffffu, g, o);
-                    if (lane == 0) own[r * 64 + wp * 8 + u] -= double(g);
-                }
+        for (int k = 0; k < NV; ++k) {
+            own[k] = owns[(os * NR + srhs[k]) * 64 + scol[k]];
+            sum[k] = 0.0;
         }
-        __syncthreads();
-        if (tid < 64)
+        __syncwarp();
+        if (lane == 0) mbar_arrive(rg.oempty + 8 * os);
+        P pacc[N];
+#pragma unroll
+        for (int k = 0; k < N; ++k) pacc[k] = P(0);
+        int held = 0;
+        auto flush = [&]() {
+            spread_sum<N, B::LN>(pacc, lane);
+#pragma unroll
+            for (int k = 0; k < NV; ++k) sum[k] += double(pacc[k]);
+#pragma unroll
+            for (int k = 0; k < N; ++k) pacc[k] = P(0);
+            held = 0;
+        };
+        // one vector buffer at a time: its chunks
+        const int ngroups = sh.nsg + (sh.nsb - 1 - K);
+        for (int g = 0; g < ngroups; ++g, ++gv) {
+            const int slot = int(gv % VS);
+            const int nc = g < sh.nsg ? min(per, sh.nstr - (sh.nsg - 1 - g) * per) : g == sh.nsg ? sh.nql : per;
+            mbar_wait(rg.vfull + 8 * slot, uint32_t(gv / VS) & 1u, err);
+            for (int c = 0; c < nc; ++c) {
+                const T *ck = chunk();
+                bwd_chunk<T, P, NR>(ck, vp + slot * (NR * SB) + c * FC, pacc, wp * 8, lane, FC);
+                release();
+                if (++held == kFlush) flush();
+            }
+            if (lane == 0) mbar_arrive(rg.vempty + 8 * slot);   // (after release's __syncwarp)
+        }
+        if (held > 0) flush();
+        // a_h; exchanged with the other parts of K through the scratch vector
+        if (nhK > 1) {
+#pragma unroll
+            for (int k = 0; k < NV; ++k)
+                if (first && srhs[k] < nrhs && scol[k] < nch)
+                    scratch[c0 + sh.C0 + scol[k] + srhs[k] * ldx] = own[k] - sum[k];
+            // (this CTA's eight warps are among the counted: all are done with the vec of before)
+            warp_count(cnt + 2 * K + 1, lane);
+            spin_count(cnt + 2 * K + 1, 16 * nhK, err);
 #pragma unroll
             for (int r = 0; r < NR; ++r)
-                if (r < nrhs && tid < nch) scratch[c0 + C0 + tid + r * ldx] = own[r * 64 + tid];
-        __syncthreads();
-        count_up(ycnt + 2 * K + 1);
-        wait_count(ycnt + 2 * K + 1, 2 * nhK, err);
+                vec[r * SB + tid] = (r < nrhs && tid < nrK) ? __ldcg(&scratch[c0 + K * SB + tid + r * ldx]) : 0.0;
+        } else {
+            psync();                                     // vec of before is read
 #pragma unroll
-        for (int r = 0; r < NR; ++r)
-            vec[r * SB + tid] = (r < nrhs && tid < nrK) ? __ldcg(&scratch[c0 + K * SB + tid + r * ldx]) : 0.0;
-        double dacc[8][NR];
-#pragma unroll
-        for (int u = 0; u < 8; ++u)
-#pragma unroll
-            for (int r = 0; r < NR; ++r) dacc[u][r] = 0.0;
-        for (int q = ndep; q < nq; ++q) {
-            if (tid == 0 && q + NST - 1 < nq) stage(q + NST - 1);
-            const int c = q - ndep;
-            const T *tl = chunk(q);
-            const int nv = min(FC, irows - c * FC);
-            const double *v = vec + h * 64 + c * FC;
-#pragma unroll
-            for (int k = 0; k < RL; ++k) {
-                const int row = lane + 32 * k;
-                if (row < nv) {
-                    double x[NR];
-#pragma unroll
-                    for (int r = 0; r < NR; ++r) x[r] = v[r * SB + row];
-#pragma unroll
-                    for (int u = 0; u < 8; ++u) {
-                        const double l = double(tl[(wp * 8 + u) * FC + row]);
-#pragma unroll
-                        for (int r = 0; r < NR; ++r) dacc[u][r] += l * x[r];
-                    }
-                }
-            }
-            __syncthreads();
+            for (int k = 0; k < NV; ++k)
+                if (first)
+                    vec[srhs[k] * SB + scol[k]] = (srhs[k] < nrhs && scol[k] < nch) ? own[k] - sum[k] : 0.0;
         }
-        gq += nq;
+        psync();
+        double dacc[N];
 #pragma unroll
-        for (int u = 0; u < 8; ++u)
+        for (int k = 0; k < N; ++k) dacc[k] = 0.0;
+        for (int c = 0; c < sh.ninv; ++c) {
+            const T *ck = chunk();
+            bwd_chunk<T, double, NR>(ck, vec + tk.pad * 64 + c * FC, dacc, wp * 8, lane, sh.irows - c * FC);
+            release();
+        }
+        spread_sum<N, B::LN>(dacc, lane);
 #pragma unroll
-            for (int r = 0; r < NR; ++r) {
-                double g = dacc[u][r];
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) g += __shfl_down_sync(0xffffffffu, g, o);
-                const int col = wp * 8 + u;
-                if (lane == 0 && r < nrhs && col < nch) X[c0 + C0 + col + r * ldx] = g;
-            }
-        __syncthreads();
-        count_up(ycnt + 2 * K);
+        for (int k = 0; k < NV; ++k)
+            if (first && srhs[k] < nrhs && scol[k] < nch) xs[scol[k] + srhs[k] * ldx] = dacc[k];
+        warp_count(cnt + 2 * K, lane);
     }
-    ring_drain<NST>(bars, gq, err);
 }
 
 // inv(L_KK) of superblock K of front s (nr rows), nrp x nrp column-major at
@@ -639,50 +1101,66 @@ __global__ void __launch_bounds__(256) sb_inverse_kernel(const SbTask *__restric
     }
 }
 
-template <typename K>
-int coop_grid(K kernel, size_t smem, int ntasks) {
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kSbThreads, smem);
-    const int g = std::max(1, per_sm) * device_sm_count();
-    return std::min(g, std::max(1, ntasks));
-}
-
 // NR: the right-hand sides the vectors hold (nrhs <= NR)
-template <typename T, int NST, int NR>
-cudaError_t launch_sp_impl(bool forward, const SbTask *tasks, int ntasks, SnDev sd, const T *factor, const char *maps,
-                           double *X, int64_t ldx, int nrhs, double *scratch, int *flags, int *err, cudaStream_t st) {
-    using L = SpLayout<T, NST, NR>;
+template <typename T, int NST, int NR, int VS>
+cudaError_t launch_sp_impl(bool forward, const SbTask *tasks, int ntasks, SnDev sd, const char *maps,
+                           const SbChild *children, const int32_t *rowmap, double *X, int64_t ldx, int nrhs, double *sol, double *scratch, int *flags, int *err,
+                           cudaStream_t st) {
+    using L = SpLayout<T, NST, NR, VS>;
     constexpr size_t smem = L::bytes + 128;
-    static_assert(smem + 256 <= size_t(kMaxSmemOptin), "superblock solve shared memory");
-    void *kern = forward ? (void *)sp_fwd_kernel<T, NST, NR> : (void *)sp_bwd_kernel<T, NST, NR>;
+    static_assert(smem + 1024 <= size_t(kMaxSmemOptin), "superblock solve shared memory");
+    void *kern = forward ? (void *)sp_fwd_kernel<T, NST, NR, VS> : (void *)sp_bwd_kernel<T, NST, NR, VS>;
     static PerDeviceOnce once;
     once([] {
-        cudaFuncSetAttribute(sp_fwd_kernel<T, NST, NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-        cudaFuncSetAttribute(sp_bwd_kernel<T, NST, NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+        cudaFuncSetAttribute(sp_fwd_kernel<T, NST, NR, VS>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+        cudaFuncSetAttribute(sp_bwd_kernel<T, NST, NR, VS>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     });
-    const int grid = forward ? coop_grid(sp_fwd_kernel<T, NST, NR>, smem, ntasks)
-                             : coop_grid(sp_bwd_kernel<T, NST, NR>, smem, ntasks);
-    void *args[] = {(void *)&tasks, (void *)&ntasks, (void *)&sd,      (void *)&factor, (void *)&maps, (void *)&X,
-                    (void *)&ldx,   (void *)&nrhs,   (void *)&scratch, (void *)&flags,  (void *)&err};
+    // one CTA per SM (its shared memory); the parts of a superblock (at most four) must be
+    // on different CTAs, which a grid of min(SMs, tasks) gives
+    const int grid = std::min(device_sm_count(), ntasks);
+    void *args[] = {(void *)&tasks, (void *)&ntasks, (void *)&sd,   (void *)&maps, (void *)&children,
+                    (void *)&rowmap, (void *)&X,     (void *)&ldx,  (void *)&nrhs, (void *)&sol,
+                    (void *)&scratch, (void *)&flags, (void *)&err};
     ++g_kernel_launches;
     return cudaLaunchCooperativeKernel(kern, dim3(grid), dim3(kSbThreads), args, smem, st);
 }
 
+// Inverse row map of one child (blockIdx.x) of the assembly forest in its parent's front.
+__global__ void child_map_kernel(const int32_t *__restrict__ parent, const int64_t *__restrict__ off, SnDev sd,
+                                 int32_t *__restrict__ map) {
+    const int c = blockIdx.x, p = parent[c];
+    if (p < 0) return;
+    const int vb = sd.vb, nf = sd.f[p] / vb, nc = sd.d[c] / vb;
+    int32_t *m = map + off[c];
+    const int32_t *rel = sd.rel + sd.struct_ptr[c];
+    for (int k = threadIdx.x; k < nf; k += blockDim.x) m[k] = -1;
+    __syncthreads();
+    for (int k = threadIdx.x; k < nc; k += blockDim.x) m[rel[k] / vb] = k;
+}
+
 }  // namespace
 
+void launch_child_maps(const int32_t *parent, const int64_t *off, int nsn, SnDev sd, int32_t *map, cudaStream_t st) {
+    if (nsn <= 0) return;
+    ++g_kernel_launches;
+    child_map_kernel<<<nsn, 128, 0, st>>>(parent, off, sd, map);
+}
+
 template <typename T>
-cudaError_t launch_sb_solve(bool forward, const SbTask *tasks, int ntasks, SnDev sd, const T *factor,
-                            const void *maps, double *X, int64_t ldx, int nrhs, double *scratch, int *flags, int *err,
-                            cudaStream_t st) {
+cudaError_t launch_sb_solve(bool forward, const SbTask *tasks, int ntasks, SnDev sd, const void *maps,
+                            const SbChild *children, const int32_t *cmap, const int32_t *rowcnt, double *X, int64_t ldx,
+                            int nrhs, double *sol, double *scratch, int *flags, int *err, cudaStream_t st) {
     const char *mp = static_cast<const char *>(maps);
     if (ntasks <= 0) return cudaSuccess;
     if (nrhs > kSbMaxRhs) return cudaErrorInvalidValue;
-    // ring depth: the deepest that fits beside the vectors of nrhs right-hand sides
-    constexpr int D4 = sizeof(T) == 4 ? 6 : 5, D8 = sizeof(T) == 4 ? 5 : 4;
-    if (nrhs <= 4)
-        return launch_sp_impl<T, D4, 4>(forward, tasks, ntasks, sd, factor, mp, X, ldx, nrhs, scratch, flags, err, st);
-    return launch_sp_impl<T, D8, kSbMaxRhs>(forward, tasks, ntasks, sd, factor, mp, X, ldx, nrhs, scratch, flags, err,
-                                            st);
+    auto go = [&](auto impl) {
+        return impl(forward, tasks, ntasks, sd, mp, children, forward ? cmap : rowcnt, X, ldx, nrhs, sol, scratch, flags, err, st);
+    };
+    // ring depth and vector buffers: the most that fit beside the sums of nrhs right-hand sides
+    if (nrhs == 1) return go(launch_sp_impl<T, 6, 1, 4>);
+    if (nrhs == 2) return go(launch_sp_impl<T, 6, 2, 4>);
+    if (nrhs <= 4) return go(launch_sp_impl<T, 5, 4, 4>);
+    return go(launch_sp_impl<T, sizeof(T) == 4 ? 5 : 4, kSbMaxRhs, 2>);
 }
 
 template <typename T>
@@ -695,10 +1173,12 @@ void launch_sb_inverse(const SbTask *tasks, int ntasks, SnDev sd, T *factor, cud
     sb_inverse_kernel<T><<<dim3(ntasks, SB / 64), 256, smem, st>>>(tasks, sd, factor);
 }
 
-template cudaError_t launch_sb_solve<float>(bool, const SbTask *, int, SnDev, const float *, const void *, double *,
-                                            int64_t, int, double *, int *, int *, cudaStream_t);
-template cudaError_t launch_sb_solve<double>(bool, const SbTask *, int, SnDev, const double *, const void *, double *,
-                                             int64_t, int, double *, int *, int *, cudaStream_t);
+#define MFS_SB_INSTANTIATE(T)                                                                                      \
+    template cudaError_t launch_sb_solve<T>(bool, const SbTask *, int, SnDev, const void *, const SbChild *,       \
+                                            const int32_t *, const int32_t *, double *, int64_t, int, double *,    \
+                                            double *, int *, int *, cudaStream_t);
+MFS_SB_INSTANTIATE(float)
+MFS_SB_INSTANTIATE(double)
 template void launch_sb_inverse<float>(const SbTask *, int, SnDev, float *, cudaStream_t);
 template void launch_sb_inverse<double>(const SbTask *, int, SnDev, double *, cudaStream_t);
 

@@ -607,22 +607,16 @@ std::string analyze(idx nblocks, const idx *Ap, const idx *Ai, int bs, const idx
             }
         }
     }
-    // ---- solve arena: as the update arena, except that subtree supernodes are
-    // allocated up front and kept at least until the levels above the cut
+    // ---- solve arena: one place per supernode (the solves run the levels into one
+    // another, so no place is free before the forward pass has ended)
     {
         S.sol_off.assign(nsn, -1);
-        Arena arena;
-        std::vector<std::vector<idx>> release_at(S.nlevels + 2);
-        auto alloc_level = [&](idx s) { return S.level[s] <= S.solve_cut ? 0 : idx(S.level[s]); };
-        for (idx l = 0; l < S.nlevels; ++l) {
-            for (idx s : release_at[l]) arena.release(S.sol_off[s], S.d[s]);
-            for (idx s = 0; s < nsn; ++s) {
-                if (alloc_level(s) != l || S.d[s] == 0 || S.sn_parent[s] < 0) continue;
-                S.sol_off[s] = arena.alloc(S.d[s]);
-                release_at[std::max<idx>(S.level[S.sn_parent[s]] + 1, S.solve_cut + 1)].push_back(s);
-            }
+        S.sol_size = 0;
+        for (idx s = 0; s < nsn; ++s) {
+            if (S.d[s] == 0 || S.sn_parent[s] < 0) continue;
+            S.sol_off[s] = S.sol_size;
+            S.sol_size += S.d[s];
         }
-        S.sol_size = arena.top;
     }
 
     // ---- conversion plan
