@@ -10,21 +10,23 @@
 // the O(m nb^2) part of the TRSM runs at GEMM speed.
 //
 // The block (padded to a multiple of 32 with an identity tail) is processed in
-// 32 x 32 tiles I = 0 .. nblk-1, right-looking, two barriers per tile column:
-//   phase A  one warp per tile: the tiles below, L_RI = A_RI inv(L_II)^T, and the
-//            inverse tiles inv(L)_IJ = -inv(L_II) sum_K P_IJK (J < I).
-//   phase B  warp 0 updates tile (I+1, I+1) and at once factors it left-looking
-//            (lane = row, reciprocal square root per pivot) and inverts it
-//            (lane = column); warps 1-7 meanwhile run the other trailing updates
-//            A_RC -= L_RI L_CI^T (R >= C > I) and the products
+// 32 x 32 tiles I = 0 .. nblk-1, right-looking, three barriers per tile column:
+//   phase A  the tiles below, L_RI = A_RI inv(L_II)^T, and the inverse tiles
+//            inv(L)_IJ = -inv(L_II) sum_K P_IJK (J < I), in halves of 16 columns, one
+//            warp each;
+//   phase B  tile (I+1, I+1) -= L_{I+1,I} L_{I+1,I}^T, four columns a warp;
+//   phase C  warp 0 factors tile (I+1, I+1) (lane = row) and warp 1 inverts it (lane =
+//            column) four pivots behind; warps 2-7 meanwhile run the other trailing
+//            updates A_RC -= L_RI L_CI^T (R >= C > I) and the products
 //            P_{I+1,J,K} = L_{I+1,K} inv(L)_KJ (J <= K <= I) that the next
 //            off-diagonal inverse tiles need (they only read final tiles).
-// Every tile product runs as a warp-level register-tiled 32 x 32 x 32 GEMM
-// (each lane owns a 4 x 8 patch), so the chain of dependent work per tile is
-// the 32 pivots of its diagonal factorization and three 32-deep products.
-// The code is kept compact (rolled loops, one product routine): the work per
-// CTA is small, and fully unrolled variants spent most of their time refetching
-// instructions.
+// What bounds it is the chain of pivots of one warp: everything else is split over the
+// warps so that it does not lengthen the chain. Clocks at 128 columns in FP32: 84,800
+// with whole-tile products on the chain, the inverse in the factoring warp and
+// four-way bank conflicts in the load; 64,900 now (47 -> 34 us a launch). At 64 columns
+// in FP64: 47,300 and 35,500 (32 -> 19 us).
+// The code is kept compact (rolled loops): the work per CTA is small, and fully unrolled
+// variants spent most of their time refetching instructions.
 #include "device.h"
 
 #include <type_traits>
@@ -34,7 +36,6 @@ namespace mfs {
 namespace {
 
 constexpr int kPanelThreads = 256;
-constexpr int kPanelLoadVecs = 16;                 // 16-byte loads per thread and batch
 
 template <typename T>
 struct Vec16;
@@ -50,7 +51,7 @@ struct Vec16<double> {
 template <typename T>
 __device__ __forceinline__ T recip_sqrt(T x);
 template <>
-__device__ __forceinline__ double recip_sqrt<double>(double x) { return 1.0 / sqrt(x); }
+__device__ __forceinline__ double recip_sqrt<double>(double x) { return rsqrt(x); }
 template <>
 __device__ __forceinline__ float recip_sqrt<float>(float x) { return rsqrtf(x); }
 
@@ -65,148 +66,210 @@ __device__ __forceinline__ float round_operand<float>(float x) {
     return __uint_as_float(r);
 }
 
-// Same rule as the small-front kernel: report (plain) or perturb (refined FP32).
-// Kept out of line: it is rare, and inlined into the unrolled pivot loop it
-// stops that loop from being unrolled.
-// With an FP64 re-factor pending (sflag), a bad pivot only marks the block: the
-// FP32 pass still finishes on a floor value and the block is factored again in FP64.
+// Largest value of type T at or below x (x >= 0): p > x in FP64 exactly when p > down(x).
 template <typename T>
-__device__ __noinline__ T panel_bad_pivot(T a, int col, PivotCtl pv, int *sflag) {
-    if (col < 0) return T(1);
-    if (sflag) {
-        *sflag = 1;
-        const T floor_v = T(1e-3 * fabs(pv.dorig[col]));
-        const T m = fabs(a);
-        return (m > floor_v) ? m : (floor_v > T(0) ? floor_v : T(1));
-    }
-    if (pv.dorig) {
-        const T floor_v = T(1e-3 * fabs(pv.dorig[col]));
-        const T m = fabs(a);
-        atomicAdd(pv.perturbed, 1);
-        return (m > floor_v) ? m : (floor_v > T(0) ? floor_v : T(1));
-    }
-    atomicMin(pv.fail_col, col);
-    return T(1);
-}
+__device__ __forceinline__ T round_down(double x);
+template <>
+__device__ __forceinline__ double round_down<double>(double x) { return x; }
+template <>
+__device__ __forceinline__ float round_down<float>(double x) { return __double2float_rd(x); }
 
-// Warp-level tile product: c[r][q] += sum_{k < 32} A(4 rq + r, k) * B(8 cq + q, k)
-// with rq = lane % 8, cq = lane / 8; A(i, k) = A0[k * lda + i], B(j, k) = B0[j * sj + k * sk].
-template <typename T>
-__device__ __forceinline__ void tile_mma(T (&c)[4][8], const T *A0, int lda, const T *B0, int sj, int sk,
-                                         int lane) {
+// Warp-level tile product: c[r][q] += sum_{k < 32} A(4 rq + r, k) * B(NC cq + q, k) with
+// rq = lane % 8, cq = lane / 8: 32 rows, 4 NC columns; A(i, k) = A0[k * lda + i],
+// B(j, k) = B0[j * sj + k * sk].
+template <typename T, int NC>
+__device__ __forceinline__ void tile_mma(T (&c)[4][NC], const T *A0, int lda, const T *B0, int sj, int sk, int lane) {
     const int rq = lane & 7, cq = lane >> 3;
     const T *a = A0 + 4 * rq;
-    const T *b = B0 + 8 * cq * sj;
-#pragma unroll 2
-    for (int k = 0; k < 32; ++k) {
-        T av[4], bv[8];
-#pragma unroll
-        for (int r = 0; r < 4; ++r) av[r] = a[k * lda + r];
-#pragma unroll
-        for (int q = 0; q < 8; ++q) bv[q] = b[q * sj + k * sk];
-#pragma unroll
-        for (int r = 0; r < 4; ++r)
-#pragma unroll
-            for (int q = 0; q < 8; ++q) c[r][q] += av[r] * bv[q];
-    }
-}
-
-template <typename T>
-__device__ __forceinline__ void tile_zero(T (&c)[4][8]) {
+    const T *b = B0 + NC * cq * sj;
 #pragma unroll
     for (int r = 0; r < 4; ++r)
 #pragma unroll
-        for (int q = 0; q < 8; ++q) c[r][q] = T(0);
+        for (int q = 0; q < NC; ++q) c[r][q] = T(0);
+#pragma unroll 4
+    for (int k = 0; k < 32; ++k) {
+        T av[4], bv[NC];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) av[r] = a[k * lda + r];
+#pragma unroll
+        for (int q = 0; q < NC; ++q) bv[q] = b[q * sj + k * sk];
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+#pragma unroll
+            for (int q = 0; q < NC; ++q) c[r][q] += av[r] * bv[q];
+    }
 }
 
-// Store a lane's 4 x 8 patch into a column-major tile (element (i, j) at M[j * ldm + i]),
+// Store a lane's 4 x NC patch into a column-major tile (element (i, j) at M[j * ldm + i]),
 // scaled by s (and added to the old value when add is set).
-template <typename T>
-__device__ __forceinline__ void tile_store(T *M, int ldm, const T (&c)[4][8], T s, bool add, int lane) {
+template <typename T, int NC>
+__device__ __forceinline__ void tile_store(T *M, int ldm, const T (&c)[4][NC], T s, bool add, int lane) {
     const int rq = lane & 7, cq = lane >> 3;
 #pragma unroll
-    for (int q = 0; q < 8; ++q)
+    for (int q = 0; q < NC; ++q)
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
-            T *p = M + (8 * cq + q) * ldm + 4 * rq + r;
+            T *p = M + (NC * cq + q) * ldm + 4 * rq + r;
             *p = add ? *p + s * c[r][q] : s * c[r][q];
         }
 }
 
-// Cholesky of the 32 x 32 tile at (c0, c0) of D by one warp, then its inverse.
-// Both keep a 32-entry vector per lane in registers, processed four steps at a
-// time and then shifted by four, so the current column (row) of step k0 + t is
-// entry t: the outer step loop stays rolled (compact code) while every register
-// index is static.
-//   factor : lane = row i, r[j] = A(i, k0 + j); pivot from lane k by shuffle,
-//            reciprocal square root; column k of L goes to Lrot[k][.] rotated by k
-//            (Lrot[k][j] = L(k + j, k), zero past the tile) and comes back to every
-//            lane as 16-byte broadcast loads for the rank-1 update;
-//   inverse: lane = column c, y[i] = Y(k0 + i, c); y_k = y[t] / L(k, k), then
-//            y[t + i] -= Lrot[k][i] y_k.
+// Pivot rule of a diagonal tile, one lane per column: a bad pivot (at or below `tiny`, or
+// NaN) is replaced (by 1, or under refinement by the larger of its magnitude and `floor`)
+// and remembered by the lane; what it means is settled after the tile.
 template <typename T>
-__device__ __noinline__ void warp_diag_tile(T *D, T *Iv, T *rdiag, T *Lrot, int LDD, int c0, int nb, int lane,
-                                            int col_base, int *fail_col, int *perturbed, const double *dorig,
-                                            int *sflag) {
+struct PivotRule {
+    T tiny, floor;
+    bool perturb, bad;
+    __device__ __forceinline__ T operator()(T p, bool mine) {
+        const bool b = !(p > tiny);
+        const T m = fabs(p);
+        const T sub = !perturb ? T(1) : m > floor ? m : floor > T(0) ? floor : T(1);
+        bad |= b & mine;
+        return b ? sub : p;
+    }
+};
+
+// The four columns under way go from the factoring to the inverting warp (and back to its
+// own lanes) through two buffers of Lq: [32 rows][4] of L, then the four reciprocal pivots.
+constexpr int kLq = 32 * 4 + 4;
+__device__ __forceinline__ void pair_sync() { asm volatile("bar.sync 2, 64;" ::: "memory"); }
+
+template <typename T>
+__device__ __forceinline__ void load4(T (&c)[4], const T *p) {
     using V = typename Vec16<T>::type;
-    constexpr int E = 16 / int(sizeof(T)), NV = 32 / E;
-    const PivotCtl pv{fail_col, perturbed, dorig, nullptr};
-    T *Dt = D + c0 * LDD + c0;                       // tile element (i, j) at Dt[j * LDD + i]
-    T r[32];
+    constexpr int E = 16 / int(sizeof(T));
 #pragma unroll
-    for (int j = 0; j < 32; ++j) r[j] = (j <= lane) ? Dt[j * LDD + lane] : T(0);
-    // the re-factor test's threshold of this lane's column, loaded once (a global load
-    // per pivot would sit on the pivot chain)
-    const double tiny_lane = (sflag && c0 + lane < nb) ? kRefactorTiny * fabs(dorig[col_base + c0 + lane]) : 0.0;
-#pragma unroll 1
-    for (int k0 = 0; k0 < 32; k0 += 4) {
+    for (int v = 0; v < 4 / E; ++v) *reinterpret_cast<V *>(&c[v * E]) = reinterpret_cast<const V *>(p)[v];
+}
+template <typename T>
+__device__ __forceinline__ void store4(T *p, const T (&c)[4]) {
+    using V = typename Vec16<T>::type;
+    constexpr int E = 16 / int(sizeof(T));
 #pragma unroll
-        for (int t = 0; t < 4; ++t) {
-            const int k = k0 + t;
-            T piv = __shfl_sync(0xffffffffu, r[t], k);
-            const double tiny = __shfl_sync(0xffffffffu, tiny_lane, k);
-            const int gcol = c0 + k < nb ? col_base + c0 + k : -1;
-            const bool bad = sflag ? (gcol >= 0 && !(double(piv) > tiny)) : !(piv > T(0));
-            if (bad) piv = panel_bad_pivot(piv, gcol, pv, sflag);
-            const T rs = recip_sqrt(piv);
-            const T lik = (lane == k) ? piv * rs : r[t] * rs;
-            if (lane >= k) Dt[k * LDD + lane] = lik;
-            if (lane == k) rdiag[c0 + k] = rs;
-            T *lr = Lrot + k * 32;
-            lr[(lane - k) & 31] = lane >= k ? lik : T(0);
-            __syncwarp();
-            T c[32];
+    for (int v = 0; v < 4 / E; ++v) reinterpret_cast<V *>(p)[v] = *reinterpret_cast<const V *>(&c[v * E]);
+}
+
+// Pivots k0 .. k0 + 3 of a diagonal tile, with LEN columns left. r[j] = A(lane, k0 + j). The
+// four columns are updated among themselves through shuffles; the rank-4 update that the
+// four before left pending on r[4 ..] (l4, Lq buffer `old`) fills the chain's latency; what
+// the next four need of these is done at the end.
+template <typename T, int LEN>
+__device__ __forceinline__ void factor_steps(T (&r)[32], T (&l4)[4], T &piv, PivotRule<T> &rule, int k0, T *Dt, T *Lq,
+                                             int LDD, int lane) {
+    constexpr int P = (LEN - 4) / 4;                 // pending columns per pivot
+    const T *old = Lq + (((k0 >> 2) & 1) ^ 1) * kLq;
+    T *cur = Lq + ((k0 >> 2) & 1) * kLq;
+    T l[4], rs[4];
 #pragma unroll
-            for (int v = 0; v < NV; ++v) *reinterpret_cast<V *>(&c[v * E]) = reinterpret_cast<const V *>(lr)[v];
-#pragma unroll
-            for (int j = 1; j + t < 32; ++j) r[t + j] -= lik * c[j];
+    for (int t = 0; t < 4; ++t) {
+        const int k = k0 + t;
+        rs[t] = recip_sqrt(piv);
+        l[t] = (lane == k) ? piv * rs[t] : r[t] * rs[t];
+        if (t < 3) {
+            // the next pivot, on its own lane: nothing else of this step is on the chain
+            piv = __shfl_sync(0xffffffffu, rule(r[t + 1] - l[t] * l[t], lane == k + 1), k + 1);
         }
 #pragma unroll
-        for (int j = 0; j < 28; ++j) r[j] = r[j + 4];
+        for (int u = t + 1; u < 4; ++u) r[u] -= l[t] * __shfl_sync(0xffffffffu, l[t], k0 + u);
+        if (lane >= k) Dt[k * LDD + lane] = l[t];
+#pragma unroll
+        for (int j = 4 + t * P; j < 4 + (t + 1) * P; ++j) {
+            T c[4];                                  // (rows past the tile: not used later)
+            load4(c, old + ((k0 + j) & 31) * 4);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) r[j] -= l4[e] * c[e];
+        }
     }
+    store4(cur + lane * 4, l);
+    if (lane == 0) store4(cur + 128, rs);
+    pair_sync();
+    // the next four columns, and their first pivot
+#pragma unroll
+    for (int j = 4; j < 8; ++j) {
+        T c[4];
+        load4(c, cur + ((k0 + j) & 31) * 4);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) r[j] -= l[e] * c[e];
+    }
+    piv = __shfl_sync(0xffffffffu, rule(r[4], lane == k0 + 4), (k0 + 4) & 31);
+#pragma unroll
+    for (int j = 0; j < LEN - 4; ++j) r[j] = r[j + 4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) l4[e] = l[e];
+}
+
+// The inverting warp's part of the same pivots: lane = column, y[j] = Y(k0 + j, lane);
+// Y_k = y[t] / L(k, k), then y[j] -= L(k0 + j, k) Y_k.
+template <typename T, int LEN>
+__device__ __forceinline__ void invert_steps(T (&y)[32], int k0, T *It, const T *Lq, int LDD, int lane) {
+    const T *cur = Lq + ((k0 >> 2) & 1) * kLq;
+    pair_sync();
+    T rs[4], yk[4];
+    load4(rs, cur + 128);
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+        T c[4];
+        load4(c, cur + (k0 + t) * 4);
+#pragma unroll
+        for (int e = 0; e < t; ++e) y[t] -= c[e] * yk[e];
+        yk[t] = y[t] * rs[t];
+        if (k0 + t >= lane) It[lane * LDD + k0 + t] = yk[t];
+    }
+#pragma unroll
+    for (int j = 4; j < LEN; ++j) {
+        T c[4];
+        load4(c, cur + ((k0 + j) & 31) * 4);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) y[j] -= c[e] * yk[e];
+    }
+#pragma unroll
+    for (int j = 0; j < LEN - 4; ++j) y[j] = y[j + 4];
+}
+
+// Cholesky of the 32 x 32 tile at (c0, c0) of D by warp 0 and its inverse by warp 1. The
+// 32-entry register vectors are taken four entries at a time and then shifted by four, so
+// that every register index is static in a rolled loop; the second half holds 16. Clocks of
+// a tile: FP32 7,300, FP64 10,500 (9,829 and 12,214 with both in one warp and a
+// shared-memory round trip a pivot).
+template <typename T>
+__device__ __noinline__ void factor_tile(T *D, T *Lq, int LDD, int c0, int nb, int lane, int col_base, int *fail_col,
+                                         int *perturbed, const double *dorig, int *sflag) {
+    T *Dt = D + c0 * LDD + c0;                       // tile element (i, j) at Dt[j * LDD + i]
+    T r[32], l4[4] = {T(0), T(0), T(0), T(0)};
+#pragma unroll
+    for (int j = 0; j < 32; ++j) r[j] = (j <= lane) ? Dt[j * LDD + lane] : T(0);
+    store4(Lq + kLq + lane * 4, l4);                 // (nothing is pending at first)
     __syncwarp();
+    const bool in = c0 + lane < nb;                  // (columns past nb are the identity's)
+    const int col = col_base + c0 + lane;
+    const double d = (dorig && in) ? fabs(dorig[col]) : 0.0;
+    // with an FP64 re-factor pending (sflag) a tiny pivot is bad too; the identity's are not
+    const T tiny = !in ? T(-1) : sflag ? round_down<T>(kRefactorTiny * d) : T(0);
+    PivotRule<T> rule{tiny, T(1e-3 * d), dorig != nullptr, false};
+    T piv = __shfl_sync(0xffffffffu, rule(r[0], lane == 0), 0);
+#pragma unroll 1
+    for (int k0 = 0; k0 < 16; k0 += 4) factor_steps<T, 32>(r, l4, piv, rule, k0, Dt, Lq, LDD, lane);
+#pragma unroll 1
+    for (int k0 = 16; k0 < 32; k0 += 4) factor_steps<T, 16>(r, l4, piv, rule, k0, Dt, Lq, LDD, lane);
+    if (rule.bad) {
+        // the same rule as the small-front kernel: report (plain) or perturb (refined FP32);
+        // a block to be factored again in FP64 is only marked
+        if (sflag) *sflag = 1;
+        else if (dorig) atomicAdd(perturbed, 1);
+        else atomicMin(fail_col, col);
+    }
+}
+template <typename T>
+__device__ __noinline__ void invert_tile(T *Iv, const T *Lq, int LDD, int c0, int lane) {
     T *It = Iv + c0 * LDD + c0;
     T y[32];
 #pragma unroll
-    for (int i = 0; i < 32; ++i) y[i] = (i == lane) ? T(1) : T(0);
+    for (int j = 0; j < 32; ++j) y[j] = (j == lane) ? T(1) : T(0);
 #pragma unroll 1
-    for (int k0 = 0; k0 < 32; k0 += 4) {
-#pragma unroll
-        for (int t = 0; t < 4; ++t) {
-            const int k = k0 + t;
-            const T yk = y[t] * rdiag[c0 + k];
-            if (k >= lane) It[lane * LDD + k] = yk;
-            const T *lr = Lrot + k * 32;
-            T c[32];
-#pragma unroll
-            for (int v = 0; v < NV; ++v) *reinterpret_cast<V *>(&c[v * E]) = reinterpret_cast<const V *>(lr)[v];
-#pragma unroll
-            for (int i = 1; i + t < 32; ++i) y[t + i] -= c[i] * yk;
-        }
-#pragma unroll
-        for (int i = 0; i < 28; ++i) y[i] = y[i + 4];
-    }
-    __syncwarp();
+    for (int k0 = 0; k0 < 16; k0 += 4) invert_steps<T, 32>(y, k0, It, Lq, LDD, lane);
+#pragma unroll 1
+    for (int k0 = 16; k0 < 32; k0 += 4) invert_steps<T, 16>(y, k0, It, Lq, LDD, lane);
 }
 
 // FP64 re-factor of one FP32 diagonal block whose FP32 factorization met a
@@ -298,120 +361,126 @@ __global__ void __launch_bounds__(kPanelThreads, 1) panel_kernel(const PanelTask
     const int nb = tk.nb, ld = tk.ld;
     const int nblk = (nb + 31) / 32, NBP = nblk * 32;
     const int LDD = NBP + 1;
-    T *D = reinterpret_cast<T *>(smem_raw);          // L, column-major, ld LDD (identity-padded)
+    T *Lq = reinterpret_cast<T *>(smem_raw);         // 2 x kLq: columns of a diagonal tile in work (16-byte aligned)
+    T *D = Lq + 2 * kLq;                             // L, column-major, ld LDD (identity-padded)
     T *Iv = D + NBP * LDD;                           // inv(L), column-major, ld LDD
     T *P = Iv + NBP * LDD;                           // 6 x [32][33] partial products
-    T *rdiag = P + 6 * 32 * 33;                      // reciprocal diagonal of L
-    T *Lrot = rdiag + NBP;                           // [32][32] rotated columns of a diagonal tile (16-byte aligned)
     const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5;
     T *blk = factor + tk.off;
     __shared__ int refactor_flag;
     int *sflag = (std::is_same<T, float>::value && pv.refactored && pv.dorig) ? &refactor_flag : nullptr;
     if (tid == 0) refactor_flag = 0;
-    // Load with 16-byte vectors (panel columns, the block's first row and ld are 16-byte
-    // aligned), every load of a batch issued before the first shared-memory store.
-    {
-        using V = typename Vec16<T>::type;
-        constexpr int E = 16 / int(sizeof(T));
-        const int nvec = NBP / E, tot = NBP * nvec;
-        for (int base = 0; base < tot; base += kPanelLoadVecs * nt) {
-            V buf[kPanelLoadVecs];
+    // Load: a warp takes every eighth column, lane = row, the rows' four segments of 32; eight
+    // columns' loads are issued before the first shared-memory store (neither the loads nor
+    // the stores collide). Nothing above the diagonal is read.
+    for (int jb = warp; jb < NBP; jb += 64) {
+        T v[8][4];
 #pragma unroll
-            for (int u = 0; u < kPanelLoadVecs; ++u) {
-                const int q = base + tid + u * nt;
-                const int j = q / nvec, i0 = (q - j * nvec) * E;
-                if (q < tot && j < nb && i0 + E <= nb)
-                    buf[u] = *reinterpret_cast<const V *>(blk + int64_t(j) * ld + i0);
+        for (int u = 0; u < 8; ++u)
+#pragma unroll
+            for (int g = 0; g < 4; ++g) {
+                const int j = jb + 8 * u, i = 32 * g + lane;
+                v[u][g] = (i == j) ? T(1) : T(0);
+                if (i >= j && i < nb && j < nb) v[u][g] = blk[int64_t(j) * ld + i];
             }
 #pragma unroll
-            for (int u = 0; u < kPanelLoadVecs; ++u) {
-                const int q = base + tid + u * nt;
-                if (q >= tot) continue;
-                const int j = q / nvec, i0 = (q - j * nvec) * E;
-                const T *bv = reinterpret_cast<const T *>(&buf[u]);
-                const bool full = j < nb && i0 + E <= nb;
+        for (int u = 0; u < 8; ++u)
 #pragma unroll
-                for (int e = 0; e < E; ++e) {
-                    const int i = i0 + e;
-                    T v;
-                    if (i < nb && j < nb) v = i >= j ? (full ? bv[e] : blk[int64_t(j) * ld + i]) : T(0);
-                    else v = (i == j) ? T(1) : T(0);
-                    D[j * LDD + i] = v;
+            for (int g = 0; g < 4; ++g) {
+                const int j = jb + 8 * u, i = 32 * g + lane;
+                if (j < NBP && i < NBP) {
+                    D[j * LDD + i] = v[u][g];
                     Iv[j * LDD + i] = T(0);
                 }
             }
-        }
     }
     __syncthreads();
-    if (warp == 0)
-        warp_diag_tile(D, Iv, rdiag, Lrot, LDD, 0, nb, lane, tk.col, pv.fail_col, pv.perturbed, pv.dorig, sflag);
+    auto diag = [&](int I) {
+        if (warp == 0)
+            factor_tile(D, Lq, LDD, 32 * I, nb, lane, tk.col, pv.fail_col, pv.perturbed, pv.dorig, sflag);
+        else if (warp == 1)
+            invert_tile(Iv, Lq, LDD, 32 * I, lane);
+    };
+    diag(0);
     __syncthreads();
     for (int I = 0; I < nblk; ++I) {
         const int c0 = 32 * I;
-        // ---- phase A: tiles below (L_RI) and off-diagonal inverse tiles (inv(L)_IJ)
+        // ---- phase A: tiles below (L_RI) and off-diagonal inverse tiles (inv(L)_IJ), in
+        //      halves of 16 columns; a tile below is replaced, so its halves wait for each other
         {
-            const int nbelow = nblk - 1 - I;
-            for (int u = warp; u < nbelow + I; u += 8) {
-                T c[4][8];
-                tile_zero(c);
-                if (u < nbelow) {
-                    const int R = I + 1 + u;
-                    // B(j, k) = inv(L_II)(j, k)
-                    tile_mma(c, D + c0 * LDD + 32 * R, LDD, Iv + c0 * LDD + c0, 1, LDD, lane);
-                    __syncwarp();
-                    tile_store(D + c0 * LDD + 32 * R, LDD, c, T(1), false, lane);
-                } else {
-                    const int J = u - nbelow;
-                    // T_IJ = sum_{K=J}^{I-1} P_IJK, gathered into the K = J slot; B(j, t) = T_IJ(t, j)
+            const int nbelow = nblk - 1 - I, nhalf = 2 * (nbelow + I);
+            // T_IJ = sum_{K=J}^{I-1} P_IJK, gathered into the K = J slot
+            if (I > 1) {
+                for (int J = 0; J + 1 < I; ++J) {
                     T *Pj = P + (J * (J + 1) / 2 + J) * 32 * 33;
-                    for (int K = J + 1; K < I; ++K) {
-                        const T *Pk = P + (K * (K + 1) / 2 + J) * 32 * 33;
-                        for (int e = lane; e < 32 * 33; e += 32) Pj[e] += Pk[e];
+                    for (int e = tid; e < 32 * 33; e += nt) {
+                        T sum = Pj[e];
+                        for (int K = J + 1; K < I; ++K) sum += P[(K * (K + 1) / 2 + J) * 32 * 33 + e];
+                        Pj[e] = sum;
                     }
-                    __syncwarp();
-                    tile_mma(c, Iv + c0 * LDD + c0, LDD, Pj, 33, 1, lane);
-                    tile_store(Iv + (32 * J) * LDD + c0, LDD, c, T(-1), false, lane);
                 }
+                __syncthreads();
+            }
+            T c[4][4];
+            const int u = warp >> 1, h = 16 * (warp & 1);
+            if (warp < nhalf) {
+                if (u < nbelow) {
+                    // B(j, k) = inv(L_II)(j, k)
+                    tile_mma(c, D + c0 * LDD + 32 * (I + 1 + u), LDD, Iv + c0 * LDD + c0 + h, 1, LDD, lane);
+                } else {
+                    // B(j, t) = T_IJ(t, j)
+                    const int J = u - nbelow;
+                    tile_mma(c, Iv + c0 * LDD + c0, LDD, P + (J * (J + 1) / 2 + J) * 32 * 33 + h * 33, 33, 1, lane);
+                }
+            }
+            __syncthreads();
+            if (warp < nhalf) {
+                if (u < nbelow) tile_store(D + (c0 + h) * LDD + 32 * (I + 1 + u), LDD, c, T(1), false, lane);
+                else tile_store(Iv + (32 * (u - nbelow) + h) * LDD + c0, LDD, c, T(-1), false, lane);
             }
         }
         __syncthreads();
         if (I + 1 == nblk) break;
-        // ---- phase B: trailing updates of tile column I; tile I+1 factored and inverted
-        //      as soon as its update is in; products for the next inverse tiles
+        // ---- phase B: the next diagonal tile's update, lane = row, four columns a warp
         {
+            const T *Lr = D + c0 * LDD + c0 + 32;
+            T sum[4] = {T(0), T(0), T(0), T(0)};
+#pragma unroll 8
+            for (int k = 0; k < 32; ++k) {
+                const T a = Lr[k * LDD + lane];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) sum[q] += a * Lr[k * LDD + 4 * warp + q];
+            }
+            T *Dn = D + (c0 + 32 + 4 * warp) * LDD + c0 + 32 + lane;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) Dn[q * LDD] -= sum[q];
+        }
+        __syncthreads();
+        // ---- phase C: that tile factored and inverted; the other trailing updates of tile
+        //      column I; products for the next inverse tiles
+        if (warp < 2) {
+            diag(I + 1);
+        } else {
             const int m = nblk - 1 - I;                          // trailing tile rows / columns
             const int ntrail = m * (m + 1) / 2;                  // u = 0 is tile (I+1, I+1)
             const int nterm = (I + 1) * (I + 2) / 2;             // P_{I+1,J,K}, J <= K <= I
-            if (warp == 0) {
+            for (int u = warp - 1; u < ntrail + nterm; u += 6) {
                 T c[4][8];
-                tile_zero(c);
-                const int R = I + 1;
-                tile_mma(c, D + c0 * LDD + 32 * R, LDD, D + c0 * LDD + 32 * R, 1, LDD, lane);
-                tile_store(D + (32 * R) * LDD + 32 * R, LDD, c, T(-1), true, lane);
-                __syncwarp();
-                warp_diag_tile(D, Iv, rdiag, Lrot, LDD, 32 * R, nb, lane, tk.col, pv.fail_col, pv.perturbed,
-                               pv.dorig, sflag);
-            } else {
-                for (int u = warp; u < ntrail + nterm; u += 7) {
-                    T c[4][8];
-                    tile_zero(c);
-                    if (u < ntrail) {
-                        int a = 0;
-                        while ((a + 1) * (a + 2) / 2 <= u) ++a;
-                        const int R = I + 1 + a, C = I + 1 + (u - a * (a + 1) / 2);   // R >= C
-                        // B(j, k) = L_CI(j, k)
-                        tile_mma(c, D + c0 * LDD + 32 * R, LDD, D + c0 * LDD + 32 * C, 1, LDD, lane);
-                        tile_store(D + (32 * C) * LDD + 32 * R, LDD, c, T(-1), true, lane);
-                    } else {
-                        const int t = u - ntrail;                 // t = K (K + 1) / 2 + J
-                        int K = 0;
-                        while ((K + 1) * (K + 2) / 2 <= t) ++K;
-                        const int J = t - K * (K + 1) / 2;
-                        // B(j, k) = inv(L)_KJ(k, j)
-                        tile_mma(c, D + (32 * K) * LDD + 32 * (I + 1), LDD, Iv + (32 * J) * LDD + 32 * K, LDD, 1,
-                                 lane);
-                        tile_store(P + t * 32 * 33, 33, c, T(1), false, lane);
-                    }
+                if (u < ntrail) {
+                    int a = 0;
+                    while ((a + 1) * (a + 2) / 2 <= u) ++a;
+                    const int R = I + 1 + a, C = I + 1 + (u - a * (a + 1) / 2);   // R >= C
+                    // B(j, k) = L_CI(j, k)
+                    tile_mma(c, D + c0 * LDD + 32 * R, LDD, D + c0 * LDD + 32 * C, 1, LDD, lane);
+                    tile_store(D + (32 * C) * LDD + 32 * R, LDD, c, T(-1), true, lane);
+                } else {
+                    const int t = u - ntrail;                     // t = K (K + 1) / 2 + J
+                    int K = 0;
+                    while ((K + 1) * (K + 2) / 2 <= t) ++K;
+                    const int J = t - K * (K + 1) / 2;
+                    // B(j, k) = inv(L)_KJ(k, j)
+                    tile_mma(c, D + (32 * K) * LDD + 32 * (I + 1), LDD, Iv + (32 * J) * LDD + 32 * K, LDD, 1, lane);
+                    tile_store(P + t * 32 * 33, 33, c, T(1), false, lane);
                 }
             }
         }
@@ -425,47 +494,26 @@ __global__ void __launch_bounds__(kPanelThreads, 1) panel_kernel(const PanelTask
             return;
         }
     }
-    // L (lower triangle only: the strict upper part keeps its stored values) and inv(L)
-    // (zeros above the diagonal) with 16-byte vector stores where a vector is whole
-    {
-        using V = typename Vec16<T>::type;
-        constexpr int E = 16 / int(sizeof(T));
-        const int nvec = (nb + E - 1) / E, tot = nb * nvec;
-        for (int q = tid; q < tot; q += nt) {
-            const int j = q / nvec, i0 = (q - j * nvec) * E;
-            V lv, iv;
-            T *l = reinterpret_cast<T *>(&lv), *ivp = reinterpret_cast<T *>(&iv);
+    // L (lower triangle only: the strict upper part keeps its stored values), inv(L) (zeros
+    // above the diagonal) and the 64 x 64 diagonal blocks of inv(L) (the inverses of L's
+    // 64 x 64 diagonal blocks, zero past nb), a column a warp, lane = row
+    T *inv = tk.inv_out >= 0 ? factor + tk.inv_out : nullptr;
+    const int nb64 = (nb + 63) & ~63;
+    for (int j = warp; j < nb64; j += 8) {
+        T *dl = blk + int64_t(j) * ld;
+        T *di = inv_scratch + tk.inv_full + int64_t(j) * tk.ldi;
+        T *d64 = inv ? inv + (j >> 6) * 4096 + (j & 63) * 64 - (j & ~63) : nullptr;
 #pragma unroll
-            for (int e = 0; e < E; ++e) {
-                const int i = i0 + e;
-                l[e] = D[j * LDD + i];
-                const T v = i >= j ? Iv[j * LDD + i] : T(0);
-                ivp[e] = round_inv ? round_operand(v) : v;
+        for (int g = 0; g < 4; ++g) {
+            const int i = 32 * g + lane;
+            if (i >= nb64) continue;
+            const bool live = i < nb && j < nb;
+            const T y = live && i >= j ? Iv[j * LDD + i] : T(0);
+            if (live) {
+                di[i] = round_inv ? round_operand(y) : y;
+                if (i >= j) dl[i] = D[j * LDD + i];
             }
-            T *dl = blk + int64_t(j) * ld + i0;
-            T *di = inv_scratch + tk.inv_full + int64_t(j) * tk.ldi + i0;
-            if (i0 + E <= nb) {
-                *reinterpret_cast<V *>(di) = iv;
-                if (i0 >= j) {
-                    *reinterpret_cast<V *>(dl) = lv;
-                    continue;
-                }
-            } else {
-                for (int e = 0; e < E && i0 + e < nb; ++e) di[e] = ivp[e];
-            }
-            for (int e = 0; e < E && i0 + e < nb; ++e)
-                if (i0 + e >= j) dl[e] = l[e];
-        }
-    }
-    if (tk.inv_out >= 0) {
-        // 64 x 64 diagonal blocks of inv(L) (the inverses of L's 64 x 64 diagonal blocks)
-        const int nb64 = (nb + 63) / 64;
-        T *inv = factor + tk.inv_out;
-        for (int q = tid; q < nb64 * 4096; q += nt) {
-            const int b = q >> 12, e = q & 4095;
-            const int j = e >> 6, i = e & 63;
-            const int gi = b * 64 + i, gj = b * 64 + j;
-            inv[q] = (gi < nb && gj < nb && gi >= gj) ? Iv[gj * LDD + gi] : T(0);
+            if (d64 && (i >> 6) == (j >> 6)) d64[i] = y;
         }
     }
 }
@@ -475,7 +523,7 @@ __global__ void __launch_bounds__(kPanelThreads, 1) panel_kernel(const PanelTask
 size_t panel_smem_bytes(int nb, bool fp64) {
     const size_t el = fp64 ? 8 : 4;
     const size_t nbp = size_t((nb + 31) / 32) * 32;
-    return (2 * nbp * (nbp + 1) + 6 * 32 * 33 + nbp + 32 * 32) * el;
+    return (2 * kLq + 2 * nbp * (nbp + 1) + 6 * 32 * 33) * el;
 }
 
 template <typename T>
