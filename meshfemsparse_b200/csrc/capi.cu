@@ -175,12 +175,11 @@ std::shared_ptr<DevSym> upload_symbolic(mfs_handle *h, std::shared_ptr<Symbolic>
             // tile starts at the 8-element aligned element at or before the operand
             // (panel leading dimensions are multiples of 8, so the shift is the same
             // for every column).
-            int da = 0, db = 0;
-            if (!f64) {
-                if ((lda & 3) || (ldb & 3)) throw StatusError(MFS_INTERNAL, "unaligned GEMM operand");
-                da = int(a_off & 7);
-                db = int(b_off & 7);
-            }
+            // FP64: two elements.
+            if ((lda & 3) || (ldb & 3)) throw StatusError(MFS_INTERNAL, "unaligned GEMM operand");
+            const int align = f64 ? 1 : 7;
+            const int da = int(a_off & align), db = int(b_off & align);
+            if (mode == 1 && n + db > TN) throw StatusError(MFS_INTERNAL, "row solve wider than the GEMM tile");
             g.shift = da | (db << 8);
             g.tiles_m = int32_t((m + da + TM - 1) / TM);
             g.tiles_n = int32_t((n + db + TN - 1) / TN);

@@ -56,6 +56,8 @@ extern "C" mfs_status mfs_debug_gemm(int32_t device, int32_t precision, int32_t 
     const int TM = gemm_tile_m(f64), TN = gemm_tile_n(f64);
     std::vector<GemmTask> gt(static_cast<size_t>(ntasks));
     int base = 0;
+    // FP64 operands whose columns do not start 16-byte aligned are copied to padded arrays
+    bool copy64 = f64 && ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15));
     for (int64_t t = 0; t < ntasks; ++t) {
         const int64_t *q = tasks + t * MFS_GEMM_TASK_FIELDS;
         const int64_t a_off = q[0], b_off = q[1], c_off = q[2], lda = q[3], ldb = q[4], ldc = q[5];
@@ -74,7 +76,11 @@ extern "C" mfs_status mfs_debug_gemm(int32_t device, int32_t precision, int32_t 
             return MFS_INVALID_ARG;
         }
         int da = 0, db = 0;
-        if (!f64) {
+        if (f64) {
+            da = int(a_off & 1);
+            db = int(b_off & 1);
+            copy64 |= (lda & 1) || (ldb & 1);
+        } else {
             // 16-byte aligned columns; tiles start at the 8-element boundary at or before
             // the operand, as in the factorization
             const int64_t al = half ? 7 : 3;
@@ -91,7 +97,7 @@ extern "C" mfs_status mfs_debug_gemm(int32_t device, int32_t precision, int32_t 
         }
         // the kernels read A rows [a_off - da, a_off + m) of columns 0..k-1, B likewise,
         // and write C rows [0, m) of columns 0..n-1
-        if (a_off - da < 0 || b_off - db < 0 || c_off < 0 || a_off + (k - 1) * lda + m > a_ext ||
+        if ((!f64 && (a_off - da < 0 || b_off - db < 0)) || a_off < 0 || b_off < 0 || c_off < 0 || a_off + (k - 1) * lda + m > a_ext ||
             b_off + (k - 1) * ldb + n > b_ext || c_off + (n - 1) * ldc + m > c_len) {
             put_error(err_buf, err_len, id + "an access falls outside the arrays");
             return MFS_INVALID_ARG;
@@ -168,6 +174,7 @@ extern "C" mfs_status mfs_debug_gemm(int32_t device, int32_t precision, int32_t 
     TensorMapBlob *dmaps = nullptr;
     void *h16s = nullptr, *h16l = nullptr;
     int32_t *dsexp = nullptr;
+    double *padA = nullptr, *padB = nullptr;
     auto fail = [&](cudaError_t e) {
         put_error(err_buf, err_len, cudaGetErrorString(e));
         if (dt) cudaFree(dt);
@@ -176,10 +183,43 @@ extern "C" mfs_status mfs_debug_gemm(int32_t device, int32_t precision, int32_t 
         if (h16s) cudaFree(h16s);
         if (h16l) cudaFree(h16l);
         if (dsexp) cudaFree(dsexp);
+        if (padA) cudaFree(padA);
+        if (padB) cudaFree(padB);
         return MFS_CUDA_ERROR;
     };
     cudaError_t e = cudaSetDevice(device);
     if (e != cudaSuccess) return fail(e);
+    if (copy64) {
+        int64_t na = 0, nb = 0;
+        for (GemmTask &g : gt) {
+            const int da = g.shift & 255, db = g.shift >> 8;
+            const int64_t lda = (g.m + da + 1) & ~1, ldb = (g.n + db + 1) & ~1;
+            na += lda * g.k;
+            nb += ldb * g.k;
+        }
+        if ((e = cudaMalloc(&padA, size_t(na) * 8)) != cudaSuccess) return fail(e);
+        if ((e = cudaMalloc(&padB, size_t(nb) * 8)) != cudaSuccess) return fail(e);
+        na = nb = 0;
+        for (GemmTask &g : gt) {
+            const int da = g.shift & 255, db = g.shift >> 8;
+            const int64_t lda = (g.m + da + 1) & ~1, ldb = (g.n + db + 1) & ~1;
+            if ((e = cudaMemcpy2D(padA + na + da, size_t(lda) * 8, static_cast<const double *>(A) + g.a_off,
+                                  size_t(g.lda) * 8, size_t(g.m) * 8, size_t(g.k), cudaMemcpyDeviceToDevice)) !=
+                    cudaSuccess ||
+                (e = cudaMemcpy2D(padB + nb + db, size_t(ldb) * 8, static_cast<const double *>(B) + g.b_off,
+                                  size_t(g.ldb) * 8, size_t(g.n) * 8, size_t(g.k), cudaMemcpyDeviceToDevice)) !=
+                    cudaSuccess)
+                return fail(e);
+            g.a_off = na + da;
+            g.b_off = nb + db;
+            g.lda = int32_t(lda);
+            g.ldb = int32_t(ldb);
+            na += lda * g.k;
+            nb += ldb * g.k;
+        }
+        A = padA;
+        B = padB;
+    }
     if ((e = cudaMalloc(&dt, gt.size() * sizeof(GemmTask))) != cudaSuccess) return fail(e);
     if ((e = cudaMalloc(&derr, sizeof(int))) != cudaSuccess) return fail(e);
     if ((e = cudaMemcpy(dt, gt.data(), gt.size() * sizeof(GemmTask), cudaMemcpyHostToDevice)) != cudaSuccess)
@@ -216,6 +256,8 @@ extern "C" mfs_status mfs_debug_gemm(int32_t device, int32_t precision, int32_t 
     if (h16s) cudaFree(h16s);
     if (h16l) cudaFree(h16l);
     if (dsexp) cudaFree(dsexp);
+    if (padA) cudaFree(padA);
+    if (padB) cudaFree(padB);
     if (herr) {
         put_error(err_buf, err_len, "a tensor-core pipeline wait timed out");
         return MFS_TIMEOUT;

@@ -11,8 +11,8 @@
 // (tcgen05, kernels_gemm_tc.cu); the split 3xTF32 form (a = a_hi + a_lo, three
 // products, FP32-level accuracy) and a legacy single-pass form run here on
 // mma.sync m16n8k8. FP64 factors run on the FP64 tensor-core path (mma.sync
-// m8n8k4 DMMA). Tiles are staged through shared memory with 4/8-byte cp.async,
-// double buffered. An FP32 task tile is 128 x 256 (the tcgen05 tile); the
+// m8n8k4 DMMA). Tiles are staged through shared memory with cp.async (FP32 4 bytes,
+// double buffered; FP64 16 bytes, four stages). An FP32 task tile is 128 x 256 (the tcgen05 tile); the
 // mma.sync kernel covers it as two 128 x 128 halves and ignores the tcgen05
 // alignment shift (its extra tiles find no rows or columns).
 #include "device.h"
@@ -32,10 +32,10 @@ __device__ __forceinline__ void cp_async4(void *dst, const void *src, bool valid
     const int sz = valid ? 4 : 0;
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(sz) : "memory");
 }
-__device__ __forceinline__ void cp_async8(void *dst, const void *src, bool valid) {
+// 16-byte copy of `bytes` (0, 8 or 16) source bytes, zero-filling the rest.
+__device__ __forceinline__ void cp_async16(void *dst, const void *src, int bytes) {
     const uint32_t d = smem_u32(dst);
-    const int sz = valid ? 8 : 0;
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(sz) : "memory");
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
@@ -202,96 +202,128 @@ __global__ void __launch_bounds__(256) gemm_tf32_kernel(const GemmTask *__restri
 }
 
 // ---------------------------------------------------------------- FP64 ----
-constexpr int DBM = 128, DBN = 64, DBK = 16, DLDA = DBM + 4, DLDB = DBN + 4;
-constexpr int kF64Smem = 2 * DBK * (DLDA + DLDB) * 8;
+// DMMA m8n8k4; a CTA tile is 128 x 64, warps 4 x 2 of 32 x 32, two CTAs per SM. What
+// bounds it: the tensor pipe for the large updates (37 TFLOP/s measured for DMMA alone),
+// latency for the column-block chain, whose launches have a few tiles and k of 64 to 192.
+// The operands come by 16-byte cp.async through a ring of DST stages of 16 k (a tile starts
+// at the 2-element aligned row at or before its operand, the extra row and column are
+// not stored), and C is loaded in two batches: written as C -= acc element by element, each
+// load waited for the store before it, most of a 25 us launch at k = 64. (Accumulators that
+// start as -C, so that its loads overlap the ring's first fill, were slower: the level SYRKs
+// at 24 instead of 26 TFLOP/s.) All GEMM launches of a factorization of the 48-sided cube:
+// 123 ms with 8-byte copies, two stages and the element-by-element epilogue, 105 ms now
+// (level SYRKs 26, the largest 30 TFLOP/s).
+constexpr int DBM = 128, DBN = 64, DBK = 16, DST = 4;
+constexpr int DLDA = DBM + 4, DLDB = DBN + 4;                 // 8 bytes x (4 k + row): conflict-free fragments
+constexpr int kF64Stage = DBK * (DLDA + DLDB);               // doubles
+constexpr int kF64Smem = DST * kF64Stage * 8;
 
-__global__ void __launch_bounds__(256) gemm_f64_kernel(const GemmTask *__restrict__ tasks, int ntasks,
-                                                       const double *Abase, const double *__restrict__ Bbase,
-                                                       double *Cbase) {
+__global__ void __launch_bounds__(256, 2) gemm_f64_kernel(const GemmTask *__restrict__ tasks, int ntasks,
+                                                          const double *Abase, const double *__restrict__ Bbase,
+                                                          double *Cbase) {
     extern __shared__ __align__(16) double smd[];
-    double *As = smd;                          // [2][DBK][DLDA]
-    double *Bs = smd + 2 * DBK * DLDA;         // [2][DBK][DLDB]
     const int t = blockIdx.x;
     const GemmTask tk = tasks[find_task(tasks, ntasks, t)];
     const int local = t - tk.tile_base;
     const int ti = local % tk.tiles_m, tj = local / tk.tiles_m;
-    const int i0 = ti * DBM, j0 = tj * DBN;
-    if (tk.lower && i0 + DBM - 1 < j0) return;
+    const int da = tk.shift & 255, db = tk.shift >> 8;       // shifted row x is operand row x - d
+    const int i0 = ti * DBM, j0 = tj * DBN;                  // tile origin in shifted coordinates
+    if (tk.lower && i0 + DBM - 1 - da < j0 - db) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int wm = warp & 3, wn = warp >> 2;        // 4 x 2 warps, warp tile 32 x 32
+    const int wm = warp & 3, wn = warp >> 2;
     const int gid = lane >> 2, tig = lane & 3;
-    const double *A = Abase + tk.a_off;
-    const double *B = Bbase + tk.b_off;
-    const int K = tk.k;
-
-    auto load = [&](int stage, int k0) {
-        double *as = As + stage * DBK * DLDA;
-        double *bs = Bs + stage * DBK * DLDB;
+    const double *A = Abase + (tk.a_off - da) + i0;
+    const double *B = Bbase + (tk.b_off - db) + j0;
+    const int am = tk.m + da - i0, bn = tk.n + db - j0;      // rows / columns left in shifted coordinates
+    const int K = tk.k, nk = (K + DBK - 1) / DBK;
+    // copies: 64 (A) / 32 (B) 16-byte chunks a k row; a thread has one chunk and every fourth
+    // (eighth) k row
+    const int ca = (tid & 63) * 2, ka = tid >> 6, cb = (tid & 31) * 2, kb0 = tid >> 5;
+    const int na = min(2, max(0, am - ca)) * 8, nb = min(2, max(0, bn - cb)) * 8;
+    auto load = [&](int kc) {
+        double *as = smd + (kc % DST) * kF64Stage;
+        double *bs = as + DBK * DLDA;
+        const int k0 = kc * DBK;
 #pragma unroll
-        for (int r = 0; r < (DBK * DBM) / 256; ++r) {
-            const int l = tid + 256 * r;
-            const int kk = l / DBM, ii = l % DBM;
-            const int gk = k0 + kk;
-            const bool va = (i0 + ii < tk.m) && gk < K;
-            cp_async8(as + kk * DLDA + ii, va ? A + int64_t(gk) * tk.lda + i0 + ii : A, va);
+        for (int r = 0; r < DBK / 4; ++r) {
+            const int k = ka + 4 * r, n = k0 + k < K ? na : 0;
+            cp_async16(as + k * DLDA + ca, n ? A + int64_t(k0 + k) * tk.lda + ca : Abase, n);
         }
 #pragma unroll
-        for (int r = 0; r < (DBK * DBN) / 256; ++r) {
-            const int l = tid + 256 * r;
-            const int kk = l / DBN, jj = l % DBN;
-            const int gk = k0 + kk;
-            const bool vb = (j0 + jj < tk.n) && gk < K;
-            cp_async8(bs + kk * DLDB + jj, vb ? B + int64_t(gk) * tk.ldb + j0 + jj : B, vb);
+        for (int r = 0; r < DBK / 8; ++r) {
+            const int k = kb0 + 8 * r, n = k0 + k < K ? nb : 0;
+            cp_async16(bs + k * DLDB + cb, n ? B + int64_t(k0 + k) * tk.ldb + cb : Bbase, n);
         }
-        cp_commit();
     };
-
+#pragma unroll
+    for (int kc = 0; kc < DST - 1; ++kc) {
+        if (kc < nk) load(kc);
+        cp_commit();
+    }
     double acc[4][4][2];
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
+    for (int mt = 0; mt < 4; ++mt)
 #pragma unroll
-        for (int b = 0; b < 4; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
-
-    const int nk = (K + DBK - 1) / DBK;
-    load(0, 0);
+        for (int nt = 0; nt < 4; ++nt) acc[mt][nt][0] = acc[mt][nt][1] = 0.0;
     for (int kc = 0; kc < nk; ++kc) {
-        if (kc + 1 < nk) {
-            load((kc + 1) & 1, (kc + 1) * DBK);
-            cp_wait<1>();
-        } else {
-            cp_wait<0>();
-        }
-        __syncthreads();
-        const double *as = As + (kc & 1) * DBK * DLDA;
-        const double *bs = Bs + (kc & 1) * DBK * DLDB;
+        cp_wait<DST - 2>();
+        __syncthreads();                                     // (also: stage kc - 1 is read)
+        if (kc + DST - 1 < nk) load(kc + DST - 1);
+        cp_commit();
+        const double *as = smd + (kc % DST) * kF64Stage + wm * 32 + gid;
+        const double *bs = smd + (kc % DST) * kF64Stage + DBK * DLDA + wn * 32 + gid;
 #pragma unroll
         for (int k4 = 0; k4 < DBK; k4 += 4) {
             double a[4], b[4];
 #pragma unroll
-            for (int mt = 0; mt < 4; ++mt) a[mt] = as[(k4 + tig) * DLDA + wm * 32 + mt * 8 + gid];
+            for (int mt = 0; mt < 4; ++mt) a[mt] = as[(k4 + tig) * DLDA + mt * 8];
 #pragma unroll
-            for (int nt = 0; nt < 4; ++nt) b[nt] = bs[(k4 + tig) * DLDB + wn * 32 + nt * 8 + gid];
+            for (int nt = 0; nt < 4; ++nt) b[nt] = bs[(k4 + tig) * DLDB + nt * 8];
 #pragma unroll
             for (int mt = 0; mt < 4; ++mt)
 #pragma unroll
                 for (int nt = 0; nt < 4; ++nt) mma_f64(acc[mt][nt], a[mt], b[nt]);
         }
-        __syncthreads();
     }
+    cp_wait<0>();
+    // an in-place row solve (C = A, the tile spans its columns) has read all of its rows
+    __syncthreads();
     double *C = Cbase + tk.c_off;
+    const int ib = i0 - da + wm * 32 + gid, jb = j0 - db + wn * 32 + tig * 2;
+    auto live = [&](int mt, int nt, int e) {
+        const int i = ib + mt * 8, j = jb + nt * 8 + e;
+        return i >= 0 && i < tk.m && j >= 0 && j < tk.n && !(tk.lower && i < j);
+    };
+    auto at = [&](int mt, int nt, int e) { return C + int64_t(jb + nt * 8 + e) * tk.ldc + ib + mt * 8; };
+    if (tk.mode == 0) {
+        // half of the tile's C at a time (registers): every load before the first store
 #pragma unroll
-    for (int mt = 0; mt < 4; ++mt)
+        for (int h = 0; h < 2; ++h) {
+            double c[2][4][2];
 #pragma unroll
-        for (int nt = 0; nt < 4; ++nt)
+            for (int m = 0; m < 2; ++m)
 #pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const int i = i0 + wm * 32 + mt * 8 + gid;
-                const int j = j0 + wn * 32 + nt * 8 + tig * 2 + e;
-                if (i >= tk.m || j >= tk.n || (tk.lower && i < j)) continue;
-                double *p = C + int64_t(j) * tk.ldc + i;
-                if (tk.mode == 0) *p -= acc[mt][nt][e];
-                else *p = acc[mt][nt][e];
-            }
+                for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e)
+                        if (live(2 * h + m, nt, e)) c[m][nt][e] = *at(2 * h + m, nt, e);
+#pragma unroll
+            for (int m = 0; m < 2; ++m)
+#pragma unroll
+                for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e)
+                        if (live(2 * h + m, nt, e)) *at(2 * h + m, nt, e) = c[m][nt][e] - acc[2 * h + m][nt][e];
+        }
+    } else {
+#pragma unroll
+        for (int mt = 0; mt < 4; ++mt)
+#pragma unroll
+            for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+                for (int e = 0; e < 2; ++e)
+                    if (live(mt, nt, e)) *at(mt, nt, e) = acc[mt][nt][e];
+    }
 }
 
 }  // namespace

@@ -23,7 +23,7 @@
 // What bounds it is the chain of pivots of one warp: everything else is split over the
 // warps so that it does not lengthen the chain. Clocks at 128 columns in FP32: 84,800
 // with whole-tile products on the chain, the inverse in the factoring warp and
-// four-way bank conflicts in the load; 64,900 now (47 -> 34 us a launch). At 64 columns
+// four-way bank conflicts in the load; 67,600 now (47 -> 35 us a launch). At 64 columns
 // in FP64: 47,300 and 35,500 (32 -> 19 us).
 // The code is kept compact (rolled loops): the work per CTA is small, and fully unrolled
 // variants spent most of their time refetching instructions.
