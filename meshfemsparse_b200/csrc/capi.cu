@@ -119,6 +119,15 @@ std::shared_ptr<DevSym> upload_symbolic(mfs_handle *h, std::shared_ptr<Symbolic>
     const int small_max = small_front_limit(h);
     std::vector<int32_t> small_list, all_list;
     std::vector<AssembleTask> asm_tasks;
+    // inverse row maps of the children in their parents' fronts
+    std::vector<int32_t> par(nsn);
+    std::vector<int64_t> cmap_off(nsn + 1, 0);
+    for (idx s = 0; s < nsn; ++s) {
+        par[s] = int32_t(S.sn_parent[s]);
+        cmap_off[s + 1] = cmap_off[s] + (par[s] < 0 ? 0 : S.f[par[s]] / S.vb);
+    }
+    std::vector<AsmChild> asm_children;
+    std::vector<AssembleTile> asm_tiles;
     std::vector<PanelTask> potrf_tasks;
     std::vector<GemmTask> gemm_tasks;
     ds->levels.resize(S.nlevels);
@@ -144,19 +153,26 @@ std::shared_ptr<DevSym> upload_symbolic(mfs_handle *h, std::shared_ptr<Symbolic>
         L.large_count = int(large.size());
         ds->num_large += L.large_count;
         if (large.empty()) continue;
-        L.asm_off = int(asm_tasks.size());
-        int base = 0;
-        idx maxw = 0;
+        L.asm_off = int(asm_tiles.size());
+        idx maxw = 0, maxf = 0;
+        for (idx s : large) maxf = std::max(maxf, S.f[s]);
+        L.asm_rows = maxf <= kAsmSmallFront ? kAsmRowsSmall : kAsmRows;
         for (idx s : large) {
             ds->large_fronts.push_back(int32_t(s));
             inv_off[s] = inv_end;
             inv_end += ((S.w[s] + 63) / 64) * 4096;
-            asm_tasks.push_back({int32_t(s), base});
-            base += int((S.f[s] + kAsmCols - 1) / kAsmCols);
+            const int32_t child0 = int32_t(asm_children.size());
+            for (idx k = S.child_ptr[s]; k < S.child_ptr[s + 1]; ++k) {
+                const idx c = S.child_list[k];
+                if (S.d[c] > 0) asm_children.push_back({cmap_off[c], S.upd_off[c], int32_t(S.d[c]), 0});
+            }
+            for (idx c0 = 0; c0 < S.f[s]; c0 += kAsmCols)
+                for (idx r0 = c0; r0 < S.f[s]; r0 += L.asm_rows)
+                    asm_tiles.push_back({int32_t(asm_tasks.size()), int32_t(c0), int32_t(r0)});
+            asm_tasks.push_back({int32_t(s), child0, int32_t(asm_children.size()) - child0});
             maxw = std::max(maxw, S.w[s]);
         }
-        L.asm_n = int(large.size());
-        L.asm_tiles = base;
+        L.asm_tiles = int(asm_tiles.size()) - L.asm_off;
         const bool f64 = h->opt.precision != MFS_PREC_FP32;
         const int NB = f64 ? 64 : 128;                  // column block of the large-front factorization
         const int TM = gemm_tile_m(f64), TN = gemm_tile_n(f64);
@@ -334,14 +350,7 @@ std::shared_ptr<DevSym> upload_symbolic(mfs_handle *h, std::shared_ptr<Symbolic>
     std::vector<int32_t> sb_fidx(nsn, -1);
     for (size_t i = 0; i < ds->sb_fronts.size(); ++i) sb_fidx[ds->sb_fronts[i]] = int32_t(i);
     auto sb_parts = [&](idx s, idx K) { return (std::min(SBk, S.w[s] - K * SBk) + 63) / 64; };
-    // inverse row maps of the children in their parents' fronts, and the children of each
-    // front above the cut
-    std::vector<int32_t> par(nsn);
-    std::vector<int64_t> cmap_off(nsn + 1, 0);
-    for (idx s = 0; s < nsn; ++s) {
-        par[s] = int32_t(S.sn_parent[s]);
-        cmap_off[s + 1] = cmap_off[s] + (par[s] < 0 ? 0 : S.f[par[s]] / S.vb);
-    }
+    // the children of each front above the cut
     std::vector<SbChild> kids;
     std::vector<int32_t> sb_child0(nsn, 0), sb_nchild(nsn, 0);
     for (int32_t s : ds->sb_fronts) {
@@ -497,6 +506,8 @@ std::shared_ptr<DevSym> upload_symbolic(mfs_handle *h, std::shared_ptr<Symbolic>
             MFS_CUDA(cudaMemcpyAsync(buf.p, vec.data(), vec.size() * sizeof(vec[0]), cudaMemcpyHostToDevice, st));
     };
     up(ds->asm_tasks, asm_tasks);
+    up(ds->asm_children, asm_children);
+    up(ds->asm_tiles, asm_tiles);
     up(ds->potrf_tasks, potrf_tasks);
     up(ds->gemm_tasks, gemm_tasks);
     // algorithmic flops per task: 2 m n k for an update (the lower triangle only for
@@ -751,7 +762,8 @@ void run_factor(mfs_handle *h, DevSym &ds, T *factor, T *upd, T *dscr, const dou
             MFS_LAUNCHED();
         }
         if (L.large_count == 0) continue;
-        launch_assemble_large<T>(ds.asm_tasks.p + L.asm_off, L.asm_n, L.asm_tiles, ds.sd, factor, upd, st);
+        launch_assemble_large<T>(ds.asm_tiles.p + L.asm_off, L.asm_tiles, L.asm_rows, ds.asm_tasks.p, ds.sd,
+                                 ds.asm_children.p, ds.cmap.p, factor, upd, st);
         MFS_LAUNCHED();
         // One-group look-ahead: the column-block chain (left-looking update, panel, row
         // solve) and the update of the next group's columns run on a high-priority

@@ -124,10 +124,21 @@ struct PanelTask {
     int32_t ldi;                        // leading dimension of inv(L) in scratch (nb rounded up to 4)
 };
 
-// Extend-add of all children of a large supernode, split by front columns.
+// Extend-add of all children of a large supernode: its tiles of kAsmCols columns from c0 on
+// and kAsmRows (kAsmRowsSmall) rows from r0 on, tiles without an element of the lower
+// triangle left out.
 struct AssembleTask {
     int32_t sn;
-    int32_t tile_base;                  // prefix over tasks of column chunks
+    int32_t child0, nchild;             // the front's children with an update matrix (AsmChild)
+};
+struct AssembleTile {
+    int32_t task, c0, r0;
+};
+// A child in the extend-add: its inverse row map's first entry, its update matrix in the
+// arena and that matrix's order.
+struct AsmChild {
+    int64_t map, upd;
+    int32_t d, pad;
 };
 
 // Solve tasks: one 64-row block of a front (blk < ceil(w/64): diagonal block,
@@ -186,7 +197,10 @@ constexpr int kSolveAsmRows = 256;      // front rows per forward extend-add CTA
 constexpr int kMaxSolveRhs = 16;        // right-hand sides per solve pass (more are chunked)
 constexpr int kSbMaxRhs = 8;            // right-hand sides per pass of the superblock solves
 
-constexpr int kAsmCols = 32;            // front columns per assemble CTA
+constexpr int kAsmCols = 32;            // front columns and rows per assemble CTA (rows from the
+constexpr int kAsmRows = 512;           // columns' diagonal on); the small form for levels whose
+constexpr int kAsmRowsSmall = 128;      // fronts have at most kAsmSmallFront rows (a front of 250
+constexpr int kAsmSmallFront = 1024;    // rows left most of a 512-row tile's threads idle)
 constexpr int kMaxSmemOptin = 232448;   // opt-in dynamic shared memory per CTA (227 KB)
 
 // ---------------------------------------------------------------- launchers
@@ -203,8 +217,8 @@ template <typename T>
 void launch_small_factor(const int32_t *list, int count, int max_front, SnDev sd, T *factor, T *upd,
                          PivotCtl pv, cudaStream_t st);
 template <typename T>
-void launch_assemble_large(const AssembleTask *tasks, int ntasks, int ntiles, SnDev sd, T *factor, T *upd,
-                           cudaStream_t st);
+void launch_assemble_large(const AssembleTile *tiles, int ntiles, int tile_rows, const AssembleTask *tasks, SnDev sd,
+                           const AsmChild *children, const int32_t *cmap, T *factor, T *upd, cudaStream_t st);
 template <typename T>
 void launch_panel(const PanelTask *tasks, int ntasks, int max_nb, T *factor, T *inv_scratch, PivotCtl pv,
                   bool round_inv, cudaStream_t st);

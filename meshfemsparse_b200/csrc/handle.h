@@ -74,7 +74,7 @@ struct LevelPlan {
     int small_off = 0, small_count = 0, small_max_front = 0;
     int all_off = 0, all_count = 0, all_max_front = 0;
     int large_count = 0;
-    int asm_off = 0, asm_n = 0, asm_tiles = 0;
+    int asm_off = 0, asm_tiles = 0, asm_rows = 0;   // extend-add: the level's tiles, rows of a tile
     struct Step {
         int left_off, left_n, left_tiles;   // the block's columns updated by the earlier blocks of its group
         int potrf_off, potrf_n, potrf_maxnb;
@@ -108,6 +108,8 @@ struct DevSym {
     DBuf<PlanEntryDev> plan_cat;         // the same plan in the catamari layout (built on the GPU)
     DBuf<int64_t> plan_ptr_dev;          // its bucket offsets
     DBuf<AssembleTask> asm_tasks;
+    DBuf<AssembleTile> asm_tiles;
+    DBuf<AsmChild> asm_children;         // the children of the large fronts
     DBuf<PanelTask> potrf_tasks;
     DBuf<GemmTask> gemm_tasks;
     DBuf<SolveAsmTask> sasm_tasks;

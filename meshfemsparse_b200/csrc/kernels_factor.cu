@@ -151,86 +151,114 @@ __global__ void __launch_bounds__(256) small_factor_kernel(const int32_t *__rest
     }
 }
 
-// Large fronts: zero U_s and extend-add every child into the columns
-// [c0, c0 + kAsmCols) of the front (panel part or U_s part).
-// child_rel with the analysis block size known at compile time (1 or 3), else vb.
-template <int VB>
-__device__ __forceinline__ int child_rel_vb(const int32_t *rel, int i, int vb) {
-    if constexpr (VB > 0) return rel[i / VB] + i % VB;
-    return rel[i / vb] + i % vb;
-}
-
-template <typename T, int VB>
-__global__ void __launch_bounds__(256) assemble_large_kernel(const AssembleTask *__restrict__ tasks, int ntasks,
-                                                             SnDev sd, T *__restrict__ factor,
-                                                             T *__restrict__ upd) {
-    const int t = blockIdx.x;
-    int lo = 0, hi = ntasks - 1;
-    while (lo < hi) {
-        int mid = (lo + hi + 1) >> 1;
-        if (tasks[mid].tile_base <= t) lo = mid; else hi = mid - 1;
-    }
-    const int s = tasks[lo].sn;
-    const int chunk = t - tasks[lo].tile_base;
-    const int w = sd.w[s], d = sd.d[s], f = w + d;
-    const int c0 = chunk * kAsmCols, c1 = min(f, c0 + kAsmCols);
+// Extend-add of a large front: every element of its lower triangle is the injected value
+// (panel columns) or zero (U_s) plus the children's update matrices, in child order, pulled
+// through the children's inverse row maps. HBM-bound for the large fronts: each child's
+// triangle is read and U_s written once (with scatters from the children U_s was zeroed
+// whole and then read and written once per child: 4 d^2 against 1.5 d^2 elements for two
+// children of the same size), latency-bound for the small ones. A thread has two rows of
+// the tile's columns, eight columns at a time: 16 independent loads per child in flight at
+// 4 (FP64 2) CTAs per SM, the row maps loaded once. (32 columns at once left one CTA per SM,
+// 50 ms; tiles of 8 columns spent their time on the maps, 23 ms; tiles found by a search
+// over the tasks and 512 rows for every front, 18.7 ms.)
+// k = 64 in FP32 (23 launches): 22.3 ms before, 16.5 ms now; k = 20 in FP64: 53 us a
+// launch before, 32 us now.
+template <typename T, int VB, int NT, int RW>
+__global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 1024 : 512) / NT)
+    assemble_large_kernel(const AssembleTile *__restrict__ tiles, const AssembleTask *__restrict__ tasks, SnDev sd,
+                          const AsmChild *__restrict__ children, const int32_t *__restrict__ cmap,
+                          T *__restrict__ factor, T *upd) {
+    const AssembleTile tile = tiles[blockIdx.x];
+    const AssembleTask tk = tasks[tile.task];
+    const int s = tk.sn;
+    const int w = sd.w[s], d = sd.d[s], f = w + d, ld = sd.ld[s];
+    const int c0 = tile.c0, r0 = tile.r0 + threadIdx.x;
+    const int vb = VB > 0 ? VB : sd.vb;
+    constexpr int G = 8;
     T *pan = factor + sd.pan_off[s];
-    const int ld = sd.ld[s];
-    T *Us = (d > 0 && sd.upd_off[s] >= 0) ? upd + sd.upd_off[s] : nullptr;
-    const int tid = threadIdx.x, nt = blockDim.x;
-    // zero the U_s columns of this chunk
-    if (Us) {
-        const int u0 = max(c0, w) - w, u1 = c1 - w;
-        for (int64_t k = int64_t(u0) * d + tid; k < int64_t(max(u1, u0)) * d; k += nt) Us[k] = T(0);
-    }
-    __syncthreads();
-    const int vb = sd.vb;
-    for (int ci = sd.child_ptr[s]; ci < sd.child_ptr[s + 1]; ++ci) {
-        const int c = sd.child_list[ci];
-        const int dc = sd.d[c];
-        const T *U = upd + sd.upd_off[c];
-        const int32_t *rel = sd.rel + sd.struct_ptr[c];
-        const int nblk = dc / vb;
-        // first block entry whose last scalar column reaches c0
-        int a = 0, b = nblk;
-        while (a < b) { int mid = (a + b) >> 1; if (rel[mid] + vb - 1 < c0) a = mid + 1; else b = mid; }
-        int e = a;
-        while (e < nblk && rel[e] < c1) ++e;
-        const int jc0 = a * vb, jc1 = e * vb;
-        const int ncols = jc1 - jc0;
-        if (ncols > 0) {
-            // One warp per child column (columns jc0 + warp, + 8, ...), lanes over the
-            // rows ic >= jc with 8 read-modify-writes in flight per lane. Targets are
-            // distinct (child_rel_indices is injective).
-            const int lane = tid & 31, warp = tid >> 5, nwarps = nt >> 5;
-            for (int jj = warp; jj < ncols; jj += nwarps) {
-                const int jc = jc0 + jj;
-                const int rj = child_rel_vb<VB>(rel, jc, vb);
-                if (rj < c0 || rj >= c1) continue;
-                const T *Ucol = U + int64_t(jc) * dc;
-                T *dcol = (rj < w) ? pan + int64_t(rj) * ld : Us + int64_t(rj - w) * d - w;
-                for (int ib = jc + lane; ib < dc; ib += 8 * 32) {
-                    T v[8], old[8];
-                    int ri[8];
+    T *Us = d > 0 && sd.upd_off[s] >= 0 ? upd + sd.upd_off[s] : nullptr;
+    // this thread's rows in a child (-1: none); kept for the first two children
+    auto row_maps = [&](const AsmChild &ch, int (&mi)[RW]) {
 #pragma unroll
-                    for (int u = 0; u < 8; ++u) {
-                        const int ic = ib + 32 * u;
-                        ri[u] = -1;
-                        if (ic < dc) {
-                            ri[u] = child_rel_vb<VB>(rel, ic, vb);
-                            v[u] = Ucol[ic];
-                        }
-                    }
-#pragma unroll
-                    for (int u = 0; u < 8; ++u)
-                        if (ri[u] >= 0) old[u] = dcol[ri[u]];
-#pragma unroll
-                    for (int u = 0; u < 8; ++u)
-                        if (ri[u] >= 0) dcol[ri[u]] = old[u] + v[u];
-                }
+        for (int q = 0; q < RW; ++q) {
+            const int i = r0 + NT * q;
+            mi[q] = -1;
+            if (i < f) {
+                const int b = i / vb, m = cmap[ch.map + b];
+                if (m >= 0) mi[q] = m * vb + i - b * vb;
             }
         }
-        __syncthreads();
+    };
+    AsmChild kept[2];
+    int kmi[2][RW];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        if (k >= tk.nchild) break;
+        kept[k] = children[tk.child0 + k];
+        row_maps(kept[k], kmi[k]);
+    }
+#pragma unroll 1
+    for (int cg = c0; cg < min(f, c0 + kAsmCols); cg += G) {
+        T acc[RW][G];
+        unsigned touched = 0;                            // columns with a child's contribution
+        // the panel's columns hold the injected values
+#pragma unroll
+        for (int q = 0; q < RW; ++q)
+#pragma unroll
+            for (int j = 0; j < G; ++j) {
+                const int i = r0 + NT * q;
+                acc[q][j] = T(0);
+                if (cg + j < w && i >= cg + j && i < f) acc[q][j] = pan[int64_t(cg + j) * ld + i];
+            }
+        auto add = [&](const AsmChild &ch, const int (&mi)[RW]) {
+            int mj[G], most = -1;                        // the columns in the child
+#pragma unroll
+            for (int j = 0; j < G; ++j) {
+                mj[j] = -1;
+                if (cg + j < f) {
+                    const int b = (cg + j) / vb, m = cmap[ch.map + b];
+                    if (m >= 0) mj[j] = m * vb + (cg + j) - b * vb;
+                }
+                most = max(most, mj[j]);
+            }
+            if (most < 0) return;                        // (the same for every thread)
+            const T *U = upd + ch.upd;
+            T v[RW][G];
+#pragma unroll
+            for (int j = 0; j < G; ++j) {
+                if (mj[j] >= 0) touched |= 1u << j;
+                const T *col = U + int64_t(mj[j]) * ch.d;
+#pragma unroll
+                for (int q = 0; q < RW; ++q) {
+                    v[q][j] = T(0);
+                    if (mj[j] >= 0 && mi[q] >= mj[j]) v[q][j] = col[mi[q]];
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < RW; ++q)
+#pragma unroll
+                for (int j = 0; j < G; ++j) acc[q][j] += v[q][j];
+        };
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+            if (k < tk.nchild) add(kept[k], kmi[k]);
+        for (int ci = 2; ci < tk.nchild; ++ci) {
+            const AsmChild ch = children[tk.child0 + ci];
+            int mi[RW];
+            row_maps(ch, mi);
+            add(ch, mi);
+        }
+#pragma unroll
+        for (int j = 0; j < G; ++j) {
+            const int col = cg + j;
+#pragma unroll
+            for (int q = 0; q < RW; ++q) {
+                const int i = r0 + NT * q;
+                if (col >= f || i < col || i >= f) continue;
+                if (col >= w) Us[int64_t(col - w) * d + (i - w)] = acc[q][j];
+                else if (touched >> j & 1) pan[int64_t(col) * ld + i] = acc[q][j];
+            }
+        }
     }
 }
 
@@ -278,13 +306,18 @@ void launch_small_factor(const int32_t *list, int count, int max_front, SnDev sd
 }
 
 template <typename T>
-void launch_assemble_large(const AssembleTask *tasks, int ntasks, int ntiles, SnDev sd, T *factor, T *upd,
-                           cudaStream_t st) {
+void launch_assemble_large(const AssembleTile *tiles, int ntiles, int tile_rows, const AssembleTask *tasks, SnDev sd,
+                           const AsmChild *children, const int32_t *cmap, T *factor, T *upd, cudaStream_t st) {
     if (ntiles <= 0) return;
     ++g_kernel_launches;
-    if (sd.vb == 3) assemble_large_kernel<T, 3><<<ntiles, 256, 0, st>>>(tasks, ntasks, sd, factor, upd);
-    else if (sd.vb == 1) assemble_large_kernel<T, 1><<<ntiles, 256, 0, st>>>(tasks, ntasks, sd, factor, upd);
-    else assemble_large_kernel<T, 0><<<ntiles, 256, 0, st>>>(tasks, ntasks, sd, factor, upd);
+    auto go = [&](auto narrow, auto wide) {
+        if (tile_rows == kAsmRowsSmall) narrow<<<ntiles, 128, 0, st>>>(tiles, tasks, sd, children, cmap, factor, upd);
+        else wide<<<ntiles, 256, 0, st>>>(tiles, tasks, sd, children, cmap, factor, upd);
+    };
+    static_assert(kAsmRowsSmall == 128 && kAsmRows == 512, "rows of a tile: threads x rows per thread");
+    if (sd.vb == 3) go(assemble_large_kernel<T, 3, 128, 1>, assemble_large_kernel<T, 3, 256, 2>);
+    else if (sd.vb == 1) go(assemble_large_kernel<T, 1, 128, 1>, assemble_large_kernel<T, 1, 256, 2>);
+    else go(assemble_large_kernel<T, 0, 128, 1>, assemble_large_kernel<T, 0, 256, 2>);
 }
 
 template <typename T>
@@ -300,7 +333,8 @@ void launch_extract_diag(const int64_t *diag_off, int64_t n, const T *factor, do
                                    T *, cudaStream_t);                                                            \
     template void launch_diag_shift<T>(const int64_t *, int64_t, double, T *, cudaStream_t);                       \
     template void launch_small_factor<T>(const int32_t *, int, int, SnDev, T *, T *, PivotCtl, cudaStream_t);      \
-    template void launch_assemble_large<T>(const AssembleTask *, int, int, SnDev, T *, T *, cudaStream_t);         \
+    template void launch_assemble_large<T>(const AssembleTile *, int, int, const AssembleTask *, SnDev,            \
+                                           const AsmChild *, const int32_t *, T *, T *, cudaStream_t);                                               \
     template void launch_extract_diag<T>(const int64_t *, int64_t, const T *, double *, cudaStream_t);
 
 MFS_INSTANTIATE(double)

@@ -562,12 +562,14 @@ std::string analyze(idx nblocks, const idx *Ap, const idx *Ai, int bs, const idx
     // largest subtree bounds the phase: aim for kManySubtrees (16 per SM of a
     // 148-SM B200, the measured optimum on the 811k-DOF cube; for a forest of many
     // independent meshes 48 per tree, measured on a batch of 256: the solve 103.5 ->
-    // 87.9 ms against 2368), else settle for kMinSubtrees (one per SM).
+    // 87.9 ms against 2368), else settle for kFewSubtrees (four per SM: a solve of the
+    // 20-sided cube 0.38 ms instead of 0.73 ms with the 148 largest), else for kMinSubtrees
+    // (one per SM).
     {
         idx nroots = 0;
         for (idx s = 0; s < nsn; ++s) nroots += S.sn_parent[s] < 0 ? 1 : 0;
         const idx kManySubtrees = opt.solve_subtrees > 0 ? opt.solve_subtrees : std::max<idx>(2368, 48 * nroots);
-        constexpr idx kMinSubtrees = 148, kSubFmax = 2048;
+        constexpr idx kFewSubtrees = 592, kMinSubtrees = 148, kSubFmax = 2048;
         S.solve_cut = -1;
         std::vector<idx> fmax_le(S.nlevels, 0);           // max front at levels <= l
         for (idx s = 0; s < nsn; ++s) fmax_le[S.level[s]] = std::max(fmax_le[S.level[s]], S.f[s]);
@@ -576,7 +578,7 @@ std::string analyze(idx nblocks, const idx *Ap, const idx *Ai, int bs, const idx
         for (idx s = 0; s < nsn; ++s)
             for (idx l = S.level[s]; l < (S.sn_parent[s] < 0 ? S.nlevels : S.level[S.sn_parent[s]]); ++l)
                 ++roots_at[l];
-        for (idx want : {kManySubtrees, kMinSubtrees}) {
+        for (idx want : {kManySubtrees, kFewSubtrees, kMinSubtrees}) {
             for (idx l = S.nlevels - 2; l >= 0; --l) {
                 if (fmax_le[l] > kSubFmax || roots_at[l] < want) continue;
                 S.solve_cut = l;
