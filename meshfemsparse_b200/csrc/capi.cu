@@ -117,7 +117,8 @@ std::shared_ptr<DevSym> upload_symbolic(mfs_handle *h, std::shared_ptr<Symbolic>
 
     // level schedule and tiled task lists
     const int small_max = small_front_limit(h);
-    std::vector<int32_t> small_list, all_list;
+    std::vector<int32_t> all_list;
+    std::vector<SmallTask> small_tasks;
     std::vector<AssembleTask> asm_tasks;
     // inverse row maps of the children in their parents' fronts
     std::vector<int32_t> par(nsn);
@@ -126,7 +127,17 @@ std::shared_ptr<DevSym> upload_symbolic(mfs_handle *h, std::shared_ptr<Symbolic>
         par[s] = int32_t(S.sn_parent[s]);
         cmap_off[s + 1] = cmap_off[s] + (par[s] < 0 ? 0 : S.f[par[s]] / S.vb);
     }
+    // ... and the children with an update matrix of every front
     std::vector<AsmChild> asm_children;
+    std::vector<int32_t> child0(nsn, 0), nchild(nsn, 0);
+    for (idx s = 0; s < nsn; ++s) {
+        child0[s] = int32_t(asm_children.size());
+        for (idx k = S.child_ptr[s]; k < S.child_ptr[s + 1]; ++k) {
+            const idx c = S.child_list[k];
+            if (S.d[c] > 0) asm_children.push_back({cmap_off[c], S.upd_off[c], int32_t(S.d[c]), 0});
+        }
+        nchild[s] = int32_t(asm_children.size()) - child0[s];
+    }
     std::vector<AssembleTile> asm_tiles;
     std::vector<PanelTask> potrf_tasks;
     std::vector<GemmTask> gemm_tasks;
@@ -137,18 +148,19 @@ std::shared_ptr<DevSym> upload_symbolic(mfs_handle *h, std::shared_ptr<Symbolic>
     for (idx l = 0; l < S.nlevels; ++l) {
         LevelPlan &L = ds->levels[l];
         std::vector<idx> large;
-        L.small_off = int(small_list.size());
+        L.small_off = int(small_tasks.size());
         L.all_off = int(all_list.size());
         for (idx k = S.level_ptr[l]; k < S.level_ptr[l + 1]; ++k) {
             idx s = S.level_list[k];
             all_list.push_back(int32_t(s));
             L.all_max_front = std::max<int>(L.all_max_front, int(S.f[s]));
             if (S.f[s] <= small_max) {
-                small_list.push_back(int32_t(s));
+                small_tasks.push_back({int32_t(S.w[s]), int32_t(S.f[s]), dld[s], col0[s], child0[s], nchild[s], dpan[s],
+                                       S.upd_off[s]});
                 L.small_max_front = std::max<int>(L.small_max_front, int(S.f[s]));
             } else large.push_back(s);
         }
-        L.small_count = int(small_list.size()) - L.small_off;
+        L.small_count = int(small_tasks.size()) - L.small_off;
         L.all_count = int(all_list.size()) - L.all_off;
         L.large_count = int(large.size());
         ds->num_large += L.large_count;
@@ -161,15 +173,10 @@ std::shared_ptr<DevSym> upload_symbolic(mfs_handle *h, std::shared_ptr<Symbolic>
             ds->large_fronts.push_back(int32_t(s));
             inv_off[s] = inv_end;
             inv_end += ((S.w[s] + 63) / 64) * 4096;
-            const int32_t child0 = int32_t(asm_children.size());
-            for (idx k = S.child_ptr[s]; k < S.child_ptr[s + 1]; ++k) {
-                const idx c = S.child_list[k];
-                if (S.d[c] > 0) asm_children.push_back({cmap_off[c], S.upd_off[c], int32_t(S.d[c]), 0});
-            }
             for (idx c0 = 0; c0 < S.f[s]; c0 += kAsmCols)
                 for (idx r0 = c0; r0 < S.f[s]; r0 += L.asm_rows)
                     asm_tiles.push_back({int32_t(asm_tasks.size()), int32_t(c0), int32_t(r0)});
-            asm_tasks.push_back({int32_t(s), child0, int32_t(asm_children.size()) - child0});
+            asm_tasks.push_back({int32_t(s), child0[s], nchild[s]});
             maxw = std::max(maxw, S.w[s]);
         }
         L.asm_tiles = int(asm_tiles.size()) - L.asm_off;
@@ -494,7 +501,6 @@ std::shared_ptr<DevSym> upload_symbolic(mfs_handle *h, std::shared_ptr<Symbolic>
     }
     ds->nfsb = int(fsb.size());
     ds->nbsb = int(bsb.size());
-    ds->small_list.upload(small_list, st);
     ds->large_dev.upload(ds->large_fronts, st);
     ds->all_list.upload(all_list, st);
     ds->inv_off.upload(inv_off, st);
@@ -505,6 +511,7 @@ std::shared_ptr<DevSym> upload_symbolic(mfs_handle *h, std::shared_ptr<Symbolic>
         if (!vec.empty())
             MFS_CUDA(cudaMemcpyAsync(buf.p, vec.data(), vec.size() * sizeof(vec[0]), cudaMemcpyHostToDevice, st));
     };
+    up(ds->small_tasks, small_tasks);
     up(ds->asm_tasks, asm_tasks);
     up(ds->asm_children, asm_children);
     up(ds->asm_tiles, asm_tiles);
@@ -757,8 +764,8 @@ void run_factor(mfs_handle *h, DevSym &ds, T *factor, T *upd, T *dscr, const dou
     }
     for (const LevelPlan &L : ds.levels) {
         if (L.small_count > 0) {
-            launch_small_factor<T>(ds.small_list.p + L.small_off, L.small_count, L.small_max_front, ds.sd, factor,
-                                   upd, pv, st);
+            launch_small_factor<T>(ds.small_tasks.p + L.small_off, L.small_count, L.small_max_front, S.vb,
+                                   ds.asm_children.p, ds.cmap.p, factor, upd, pv, st);
             MFS_LAUNCHED();
         }
         if (L.large_count == 0) continue;

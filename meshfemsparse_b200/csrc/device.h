@@ -134,6 +134,12 @@ struct AssembleTask {
 struct AssembleTile {
     int32_t task, c0, r0;
 };
+// A front factored whole by one CTA: sizes, panel leading dimension, first column, children
+// with an update matrix, panel and update-matrix offsets (-1: none).
+struct SmallTask {
+    int32_t w, f, ld, col0, child0, nchild;
+    int64_t pan, upd;
+};
 // A child in the extend-add: its inverse row map's first entry, its update matrix in the
 // arena and that matrix's order.
 struct AsmChild {
@@ -214,8 +220,8 @@ void launch_diag_shift(const int64_t *diag_off, int64_t n, double sigma, T *fact
 template <typename T>
 void launch_extract_diag(const int64_t *diag_off, int64_t n, const T *factor, double *out, cudaStream_t st);
 template <typename T>
-void launch_small_factor(const int32_t *list, int count, int max_front, SnDev sd, T *factor, T *upd,
-                         PivotCtl pv, cudaStream_t st);
+void launch_small_factor(const SmallTask *tasks, int count, int max_front, int vb, const AsmChild *children,
+                         const int32_t *cmap, T *factor, T *upd, PivotCtl pv, cudaStream_t st);
 template <typename T>
 void launch_assemble_large(const AssembleTile *tiles, int ntiles, int tile_rows, const AssembleTask *tasks, SnDev sd,
                            const AsmChild *children, const int32_t *cmap, T *factor, T *upd, cudaStream_t st);

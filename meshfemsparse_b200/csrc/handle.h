@@ -101,15 +101,16 @@ struct DevSym {
         return ++counter;
     }
     std::shared_ptr<Symbolic> S;
-    DBuf<int32_t> w, d, f, ld, col0, child_ptr, child_list, struct_rows, rel, small_list, all_list;
+    DBuf<int32_t> w, d, f, ld, col0, child_ptr, child_list, struct_rows, rel, all_list;
     DBuf<int64_t> pan_off, upd_off, sol_off, struct_ptr, diag_off;
     DBuf<int64_t> inv_off;               // 64 x 64 diagonal inverses of large fronts (-1: none)
     DBuf<PlanEntryDev> plan;
     DBuf<PlanEntryDev> plan_cat;         // the same plan in the catamari layout (built on the GPU)
     DBuf<int64_t> plan_ptr_dev;          // its bucket offsets
+    DBuf<SmallTask> small_tasks;         // fronts factored whole in shared memory, level by level
     DBuf<AssembleTask> asm_tasks;
     DBuf<AssembleTile> asm_tiles;
-    DBuf<AsmChild> asm_children;         // the children of the large fronts
+    DBuf<AsmChild> asm_children;         // the children of every front, front by front
     DBuf<PanelTask> potrf_tasks;
     DBuf<GemmTask> gemm_tasks;
     DBuf<SolveAsmTask> sasm_tasks;
@@ -148,7 +149,7 @@ struct DevSym {
     DBuf<int32_t> large_dev;                 // the same list on the device
     size_t bytes() const {
         return w.bytes() * 5 + col0.bytes() + child_ptr.bytes() + child_list.bytes() + struct_rows.bytes() +
-               rel.bytes() + small_list.bytes() + all_list.bytes() + pan_off.bytes() + upd_off.bytes() +
+               rel.bytes() + all_list.bytes() + pan_off.bytes() + upd_off.bytes() +
                sol_off.bytes() + struct_ptr.bytes() + diag_off.bytes() + inv_off.bytes() + plan.bytes() + asm_tasks.bytes() +
                potrf_tasks.bytes() + gemm_tasks.bytes() + spmv_ptr.bytes() +
                spmv_src.bytes() + spmv_col.bytes() + spmv_flag.bytes() + prrfr.bytes() + sperm.bytes();

@@ -26,11 +26,11 @@ namespace mfs {
 namespace {
 
 template <typename T>
-__device__ __forceinline__ T dev_sqrt(T x);
+__device__ __forceinline__ T dev_rsqrt(T x);
 template <>
-__device__ __forceinline__ double dev_sqrt<double>(double x) { return sqrt(x); }
+__device__ __forceinline__ double dev_rsqrt<double>(double x) { return rsqrt(x); }
 template <>
-__device__ __forceinline__ float dev_sqrt<float>(float x) { return sqrtf(x); }
+__device__ __forceinline__ float dev_rsqrt<float>(float x) { return rsqrtf(x); }
 
 template <typename T>
 __global__ void zero_kernel(T *p, int64_t n) {
@@ -65,8 +65,6 @@ __global__ void diag_shift_kernel(const int64_t *__restrict__ diag_off, int64_t 
         factor[diag_off[i]] = T(double(factor[diag_off[i]]) + sigma);
 }
 
-__device__ __forceinline__ int child_rel(const int32_t *rel, int i, int vb) { return rel[i / vb] + i % vb; }
-
 // A non-positive (or NaN) pivot. Without perturbation (plain solves, the
 // reference's semantics) the smallest failing column is recorded and 1 is used
 // so the launch completes; the host then reports the failure. With
@@ -93,61 +91,183 @@ __global__ void extract_diag_kernel(const int64_t *__restrict__ diag_off, int64_
         out[i] = double(factor[diag_off[i]]);
 }
 
-// Small fronts: the whole (w+d)^2 front lives in shared memory.
-template <typename T>
-__global__ void __launch_bounds__(256) small_factor_kernel(const int32_t *__restrict__ list, SnDev sd,
-                                                           T *__restrict__ factor, T *__restrict__ upd,
-                                                           PivotCtl pv) {
+// Small fronts: the front's lower triangle lives in shared memory, packed by columns.
+// Assembly pulls the children through their inverse row maps (a warp has four columns, a
+// lane the rows lane + 32 g); the factorization takes four columns at a time: every thread
+// factors the 4 x 4 diagonal block for itself, one thread per row solves the row against it
+// (to the factor and to Lp), then the rank-4 update of the trailing triangle, a warp per
+// column. Two barriers per four columns; bound by the chain of pivots (four reciprocal square
+// roots in a row) for narrow fronts and by the triangle's read and write in shared memory
+// for wide ones, hence rank 4 and not 1. With rank-1 steps, a division per element and three
+// barriers a column over the whole square the 20-sided cube took 587 us in FP64 (5
+// launches), 150 us now; the batch of 48 cubes in FP32 4,550 us (9 launches), 1,070 us now.
+constexpr int kSmallCols = 4;
+template <typename T, int VB, int NSEG, int MINB>
+__global__ void __launch_bounds__(256, MINB)
+    small_factor_kernel(const SmallTask *__restrict__ tasks, int vb_, int lp, const AsmChild *__restrict__ children,
+                        const int32_t *__restrict__ cmap, T *__restrict__ factor, T *upd, PivotCtl pv) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    T *F = reinterpret_cast<T *>(smem_raw);
-    const int s = list[blockIdx.x];
-    const int w = sd.w[s], d = sd.d[s], f = w + d;
-    const int tid = threadIdx.x, nt = blockDim.x;
-    T *pan = factor + sd.pan_off[s];
-    const int ld = sd.ld[s];
-    const int fw = f * w;
-    for (int k = tid; k < f * f; k += nt) F[k] = k < fw ? pan[(k / f) * ld + k % f] : T(0);
+    T *Lp = reinterpret_cast<T *>(smem_raw);             // [4][lp]: the four columns under way
+    T *F = Lp + kSmallCols * lp;
+    const SmallTask tk = tasks[blockIdx.x];
+    const int w = tk.w, f = tk.f, d = f - w, ld = tk.ld;
+    const int vb = VB > 0 ? VB : vb_;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    T *pan = factor + tk.pan;
+    // packed triangle: (i, j) at F[col(j) + i], i >= j
+    auto col = [f](int j) { return j * f - ((j * (j + 1)) >> 1); };
+    {
+        auto row_maps = [&](const AsmChild &ch, int (&mi)[NSEG]) {
+#pragma unroll
+            for (int g = 0; g < NSEG; ++g) {
+                const int i = lane + 32 * g;
+                mi[g] = -1;
+                if (i < f) {
+                    const int b = i / vb, m = cmap[ch.map + b];
+                    if (m >= 0) mi[g] = m * vb + i - b * vb;
+                }
+            }
+        };
+        AsmChild kept[2];
+        int kmi[2][NSEG];
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            if (k >= tk.nchild) break;
+            kept[k] = children[tk.child0 + k];
+            row_maps(kept[k], kmi[k]);
+        }
+        for (int j0 = 4 * warp; j0 < f; j0 += 32) {
+            T v[4][NSEG];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+#pragma unroll
+                for (int g = 0; g < NSEG; ++g) {
+                    const int j = j0 + u, i = lane + 32 * g;
+                    v[u][g] = T(0);
+                    if (j < w && i >= j && i < f) v[u][g] = pan[int64_t(j) * ld + i];
+                }
+            auto add = [&](const AsmChild &ch, const int (&mi)[NSEG]) {
+                int mj[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    mj[u] = -1;
+                    if (j0 + u < f) {
+                        const int b = (j0 + u) / vb, m = cmap[ch.map + b];
+                        if (m >= 0) mj[u] = m * vb + (j0 + u) - b * vb;
+                    }
+                }
+                const T *U = upd + ch.upd;
+                T x[4][NSEG];
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+#pragma unroll
+                    for (int g = 0; g < NSEG; ++g) {
+                        x[u][g] = T(0);
+                        if (mj[u] >= 0 && mi[g] >= mj[u]) x[u][g] = U[mj[u] * ch.d + mi[g]];
+                    }
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+#pragma unroll
+                    for (int g = 0; g < NSEG; ++g) v[u][g] += x[u][g];
+            };
+#pragma unroll
+            for (int k = 0; k < 2; ++k)
+                if (k < tk.nchild) add(kept[k], kmi[k]);
+            for (int ci = 2; ci < tk.nchild; ++ci) {
+                const AsmChild ch = children[tk.child0 + ci];
+                int mi[NSEG];
+                row_maps(ch, mi);
+                add(ch, mi);
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+#pragma unroll
+                for (int g = 0; g < NSEG; ++g) {
+                    const int j = j0 + u, i = lane + 32 * g;
+                    if (j < f && i >= j && i < f) F[col(j) + i] = v[u][g];
+                }
+        }
+    }
     __syncthreads();
-    const int vb = sd.vb;
-    for (int ci = sd.child_ptr[s]; ci < sd.child_ptr[s + 1]; ++ci) {
-        const int c = sd.child_list[ci];
-        const int dc = sd.d[c];
-        const T *U = upd + sd.upd_off[c];
-        const int32_t *rel = sd.rel + sd.struct_ptr[c];
-        for (int k = tid; k < dc * dc; k += nt) {
-            const int j = k / dc, i = k - j * dc;
-            if (i < j) continue;
-            F[child_rel(rel, j, vb) * f + child_rel(rel, i, vb)] += U[k];
+    for (int k = 0; k < w; k += kSmallCols) {
+        const int nb = min(kSmallCols, w - k);
+        T a[4][4], rs[4];                                // a: lower triangle of the block, then of its L
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int t = u; t < 4; ++t) a[t][u] = (t < nb) ? F[col(k + u) + k + t] : T(0);
+        const int i = k + tid;                           // this thread's row
+        T l[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) l[u] = (u < nb && i >= k + nb && i < f) ? F[col(k + u) + i] : T(0);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            rs[u] = T(0);
+            if (u < nb) {
+                T p = a[u][u];
+                if (!(p > T(0))) p = bad_pivot(p, tk.col0 + k + u, pv, tid == 0);
+                rs[u] = dev_rsqrt(p);
+                a[u][u] = p * rs[u];
+#pragma unroll
+                for (int t = u + 1; t < 4; ++t) {
+                    a[t][u] *= rs[u];
+#pragma unroll
+                    for (int v = u + 1; v <= t; ++v) a[t][v] -= a[t][u] * a[v][u];
+                }
+            }
+        }
+        if (i >= k + nb) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+#pragma unroll
+                for (int v = 0; v < u; ++v) l[u] -= l[v] * a[u][v];
+                l[u] *= rs[u];
+            }
+        } else {
+#pragma unroll
+            for (int t = 0; t < 4; ++t)
+#pragma unroll
+                for (int u = 0; u <= t; ++u)
+                    if (tid == t) l[u] = a[t][u];
+        }
+        if (i < f) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                Lp[u * lp + i] = l[u];
+                if (u < nb && i >= k + u) pan[int64_t(k + u) * ld + i] = l[u];
+            }
+        }
+        __syncthreads();
+        T li[4][NSEG];
+#pragma unroll
+        for (int g = 0; g < NSEG; ++g)
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int r = lane + 32 * g;
+                li[u][g] = (r >= k + nb && r < f) ? Lp[u * lp + r] : T(0);
+            }
+        for (int j = k + nb + warp; j < f; j += 8) {
+            T lj[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) lj[u] = Lp[u * lp + j];
+            T *Fj = F + col(j);
+#pragma unroll
+            for (int g = 0; g < NSEG; ++g) {
+                const int r = lane + 32 * g;
+                if (r >= j && r < f) {
+                    T x = Fj[r];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) x -= li[u][g] * lj[u];
+                    Fj[r] = x;
+                }
+            }
         }
         __syncthreads();
     }
-    for (int k = 0; k < w; ++k) {
-        T *colk = F + k * f;
-        if (tid == 0) {
-            T a = colk[k];
-            if (!(a > T(0))) a = bad_pivot(a, sd.col0[s] + k, pv, true);
-            colk[k] = dev_sqrt(a);
-        }
-        __syncthreads();
-        const T piv = colk[k];
-        for (int i = k + 1 + tid; i < f; i += nt) colk[i] = colk[i] / piv;
-        __syncthreads();
-        const int m = f - k - 1;
-        for (int t = tid; t < m * m; t += nt) {
-            const int jj = t / m, ii = t - jj * m;
-            if (ii < jj) continue;
-            const int j = k + 1 + jj, i = k + 1 + ii;
-            F[j * f + i] -= colk[i] * colk[j];
-        }
-        __syncthreads();
-    }
-    for (int k = tid; k < fw; k += nt) pan[(k / f) * ld + k % f] = F[k];
-    if (d > 0 && sd.upd_off[s] >= 0) {
-        T *U = upd + sd.upd_off[s];
-        for (int k = tid; k < d * d; k += nt) {
-            const int j = k / d, i = k - j * d;
-            U[k] = F[(w + j) * f + (w + i)];
-        }
+    if (d > 0 && tk.upd >= 0) {
+        T *U = upd + tk.upd;
+        for (int j = w + warp; j < f; j += 8)
+            for (int i = j + lane; i < f; i += 32) U[(j - w) * d + (i - w)] = F[col(j) + i];
     }
 }
 
@@ -295,14 +415,34 @@ void launch_diag_shift(const int64_t *diag_off, int64_t n, double sigma, T *fact
 }
 
 template <typename T>
-void launch_small_factor(const int32_t *list, int count, int max_front, SnDev sd, T *factor, T *upd, PivotCtl pv,
-                         cudaStream_t st) {
+void launch_small_factor(const SmallTask *tasks, int count, int max_front, int vb, const AsmChild *children,
+                         const int32_t *cmap, T *factor, T *upd, PivotCtl pv, cudaStream_t st) {
     if (count <= 0) return;
-    const size_t smem = size_t(max_front) * max_front * sizeof(T);
-    static PerDeviceOnce once;
-    once([] { cudaFuncSetAttribute(small_factor_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmemOptin); });
+    const int lp = (max_front + 3) & ~3;
+    const size_t smem = (size_t(kSmallCols) * lp + size_t(max_front) * (max_front + 1) / 2) * sizeof(T);
+    auto go = [&](auto kern, PerDeviceOnce &once) {
+        once([kern] { cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmemOptin); });
+        kern<<<count, 256, smem, st>>>(tasks, vb, lp, children, cmap, factor, upd, pv);
+    };
+    // rows per lane from the level's largest front
+    auto by_front = [&](auto k2, auto k3, auto k5, auto k8, PerDeviceOnce(&once)[4]) {
+        if (max_front <= 64) go(k2, once[0]);
+        else if (max_front <= 96) go(k3, once[1]);
+        else if (max_front <= 160) go(k5, once[2]);
+        else go(k8, once[3]);
+    };
     ++g_kernel_launches;
-    small_factor_kernel<T><<<count, 256, smem, st>>>(list, sd, factor, upd, pv);
+    static PerDeviceOnce once3[4], once1[4], once0[4];
+    constexpr int B2 = sizeof(T) == 4 ? 4 : 3, B5 = sizeof(T) == 4 ? 3 : 2;
+    if (vb == 3)
+        by_front(small_factor_kernel<T, 3, 2, B2>, small_factor_kernel<T, 3, 3, B2>, small_factor_kernel<T, 3, 5, B5>,
+                 small_factor_kernel<T, 3, 8, 1>, once3);
+    else if (vb == 1)
+        by_front(small_factor_kernel<T, 1, 2, B2>, small_factor_kernel<T, 1, 3, B2>, small_factor_kernel<T, 1, 5, B5>,
+                 small_factor_kernel<T, 1, 8, 1>, once1);
+    else
+        by_front(small_factor_kernel<T, 0, 2, B2>, small_factor_kernel<T, 0, 3, B2>, small_factor_kernel<T, 0, 5, B5>,
+                 small_factor_kernel<T, 0, 8, 1>, once0);
 }
 
 template <typename T>
@@ -332,7 +472,8 @@ void launch_extract_diag(const int64_t *diag_off, int64_t n, const T *factor, do
     template void launch_inject<T>(const PlanEntryDev *, int64_t, int, int, const double *, const double *, double, \
                                    T *, cudaStream_t);                                                            \
     template void launch_diag_shift<T>(const int64_t *, int64_t, double, T *, cudaStream_t);                       \
-    template void launch_small_factor<T>(const int32_t *, int, int, SnDev, T *, T *, PivotCtl, cudaStream_t);      \
+    template void launch_small_factor<T>(const SmallTask *, int, int, int, const AsmChild *, const int32_t *, T *, \
+                                         T *, PivotCtl, cudaStream_t);                                            \
     template void launch_assemble_large<T>(const AssembleTile *, int, int, const AssembleTask *, SnDev,            \
                                            const AsmChild *, const int32_t *, T *, T *, cudaStream_t);                                               \
     template void launch_extract_diag<T>(const int64_t *, int64_t, const T *, double *, cudaStream_t);
