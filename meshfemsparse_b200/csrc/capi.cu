@@ -959,12 +959,13 @@ void solve_current(mfs_handle *h, double *X, int nrhs) {
 }
 
 // Y = (A + sigma I | A + sigma B) X on the permuted reduced system.
+// dotp (optional): partial sums of X . Y per column.
 void apply_current(mfs_handle *h, const double *Ax, const double *Bx, double sigma, const double *X, double *Y,
-                   int nrhs) {
+                   int nrhs, double *dotp = nullptr) {
     DevSym &ds = *h->cur.sym;
     const Symbolic &S = *ds.S;
     launch_spmv(ds.spmv_ptr.p, ds.spmv_src.p, ds.spmv_col.p, ds.spmv_flag.p, S.nv, S.vb, S.src_ld, Ax, X, Y, S.n,
-                nrhs, h->stream);
+                nrhs, h->stream, sigma == 0.0 ? dotp : nullptr);
     MFS_LAUNCHED();
     if (sigma == 0.0) return;
     const int64_t cnt = int64_t(S.n) * nrhs;
@@ -976,6 +977,7 @@ void apply_current(mfs_handle *h, const double *Ax, const double *Bx, double sig
     } else {
         launch_axpy(Y, X, sigma, cnt, h->stream);
     }
+    if (dotp) launch_coldot_partial(X, Y, S.n, nrhs, dotp, h->stream);
     MFS_LAUNCHED();
 }
 
@@ -993,24 +995,29 @@ void refine_solve(mfs_handle *h, const double *B, double *X, int nrhs) {
     h->work_p.ensure(sz);
     h->work_ap.ensure(sz);
     const int np = reduce_partials_count();
-    h->partials.ensure(size_t(np) * 64);
+    h->partials.ensure(size_t(2 * np) * 64);
     h->dots.ensure(4 * 64);
     h->active.ensure(64);
-    double *bb = h->dots.p, *rz = h->dots.p + 64, *rz2 = h->dots.p + 128, *pap = h->dots.p + 192;
+    if (!h->xr_count.p) {
+        h->xr_count.ensure(1);
+        MFS_CUDA(cudaMemsetAsync(h->xr_count.p, 0, sizeof(unsigned), st));
+    }
+    double *bb = h->dots.p, *rz = h->dots.p + 64, *rz2 = h->dots.p + 128, *rr = h->dots.p + 192;
+    double *part = h->partials.p, *npart = part + size_t(np) * 64;
     if (!h->cur.ax) throw StatusError(MFS_NO_FACTOR, "matrix values of the current factor are not available");
     const double *Ax = h->cur.ax->p;
     const double *Bx = h->cur.bx ? h->cur.bx->p : nullptr;
     const double sigma = h->cur.sigma;
     std::vector<int> act(nrhs, 1);
     MFS_CUDA(cudaMemcpyAsync(h->active.p, act.data(), nrhs * sizeof(int), cudaMemcpyHostToDevice, st));
-    launch_colnorm2(B, n, nrhs, h->partials.p, bb, st);
+    launch_colnorm2(B, n, nrhs, part, bb, st);
     MFS_CUDA(cudaMemsetAsync(X, 0, sz * sizeof(double), st));
     launch_copy(h->work_r.p, B, int64_t(sz), st);
     launch_copy(h->work_z.p, B, int64_t(sz), st);
     MFS_LAUNCHED();
     solve_current(h, h->work_z.p, nrhs);
     launch_copy(h->work_p.p, h->work_z.p, int64_t(sz), st);
-    launch_coldot(h->work_r.p, h->work_z.p, n, nrhs, h->partials.p, rz, st);
+    launch_coldot(h->work_r.p, h->work_z.p, n, nrhs, part, rz, st);
     MFS_LAUNCHED();
     std::vector<double> hb(nrhs), hr(nrhs);
     MFS_CUDA(cudaMemcpyAsync(hb.data(), bb, nrhs * sizeof(double), cudaMemcpyDeviceToHost, st));
@@ -1023,12 +1030,11 @@ void refine_solve(mfs_handle *h, const double *B, double *X, int nrhs) {
     for (int r = 0; r < nrhs; ++r) if (hb[r] == 0.0) act[r] = 0;
     while (it < maxit) {
         ++it;
-        apply_current(h, Ax, Bx, sigma, h->work_p.p, h->work_ap.p, nrhs);
-        launch_coldot(h->work_p.p, h->work_ap.p, n, nrhs, h->partials.p, pap, st);
-        launch_pcg_update_x_r(X, h->work_r.p, h->work_p.p, h->work_ap.p, rz, pap, h->active.p, n, nrhs, st);
-        launch_colnorm2(h->work_r.p, n, nrhs, h->partials.p, rz2, st);
+        apply_current(h, Ax, Bx, sigma, h->work_p.p, h->work_ap.p, nrhs, part);
+        launch_pcg_update_x_r(X, h->work_r.p, h->work_p.p, h->work_ap.p, rz, part, h->active.p, n, nrhs, h->work_z.p,
+                              npart, rr, h->xr_count.p, nullptr, nullptr, st);
         MFS_LAUNCHED();
-        MFS_CUDA(cudaMemcpyAsync(hr.data(), rz2, nrhs * sizeof(double), cudaMemcpyDeviceToHost, st));
+        MFS_CUDA(cudaMemcpyAsync(hr.data(), rr, nrhs * sizeof(double), cudaMemcpyDeviceToHost, st));
         MFS_CUDA(cudaStreamSynchronize(st));
         check_solve_error(h);
         worst = 0.0;
@@ -1041,13 +1047,11 @@ void refine_solve(mfs_handle *h, const double *B, double *X, int nrhs) {
         }
         if (all_done) break;
         MFS_CUDA(cudaMemcpyAsync(h->active.p, act.data(), nrhs * sizeof(int), cudaMemcpyHostToDevice, st));
-        launch_copy(h->work_z.p, h->work_r.p, int64_t(sz), st);
-        MFS_LAUNCHED();
         solve_current(h, h->work_z.p, nrhs);
-        launch_coldot(h->work_r.p, h->work_z.p, n, nrhs, h->partials.p, rz2, st);
-        launch_pcg_update_p(h->work_p.p, h->work_z.p, rz2, rz, h->active.p, n, nrhs, st);
+        launch_coldot_partial(h->work_r.p, h->work_z.p, n, nrhs, part, st);
+        launch_pcg_update_p(h->work_p.p, h->work_z.p, part, rz, rz2, h->active.p, n, nrhs, nullptr, st);
         MFS_LAUNCHED();
-        MFS_CUDA(cudaMemcpyAsync(rz, rz2, nrhs * sizeof(double), cudaMemcpyDeviceToDevice, st));
+        std::swap(rz, rz2);
     }
     h->stats.refine_iterations = it;
     h->stats.residual = worst;

@@ -44,6 +44,8 @@ struct LWorkDev {
     DBuf<double> ax, bp, xp, bs, xs, z, y, e, t, gy, gz, r, pz, p, ap;
     DBuf<double> partials, dots;
     DBuf<int> active;
+    DBuf<PcgState> state;
+    DBuf<unsigned> count;
     LWork w{};
 };
 
@@ -115,7 +117,7 @@ LWorkDev &work_of(mfs_handle *h, const LGraphDev &gd, int nrhs) {
         for (DBuf<double> *b : {&W.bp, &W.xp, &W.bs, &W.xs, &W.z, &W.y, &W.e, &W.t, &W.gy, &W.gz, &W.r, &W.pz, &W.p,
                                 &W.ap})
             b->ensure(sz);
-        W.partials.ensure(size_t(reduce_partials_count()) * nrhs);
+        W.partials.ensure(size_t(2 * reduce_partials_count()) * nrhs);
         W.dots.ensure(size_t(4) * nrhs);
         W.active.ensure(size_t(nrhs));
         W.nrhs = nrhs;
@@ -185,11 +187,12 @@ void scatter_out(mfs_handle *h, const double *src, double *out, bool dev, int mo
         MFS_CUDA(cudaMemcpyAsync(out, h->io.p, size_t(ld) * nrhs * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
 }
 
-void spmv(mfs_handle *h, const double *Ax, const double *X, double *Y, int nrhs) {
+void spmv(mfs_handle *h, const double *Ax, const double *X, double *Y, int nrhs, double *dotp = nullptr,
+          const int *stop = nullptr) {
     DevSym &ds = *h->cur.sym;
     const Symbolic &S = *ds.S;
     launch_spmv(ds.spmv_ptr.p, ds.spmv_src.p, ds.spmv_col.p, ds.spmv_flag.p, S.nv, S.vb, S.src_ld, Ax, X, Y, S.n,
-                nrhs, h->stream);
+                nrhs, h->stream, dotp, stop);
     MFS_LAUNCHED();
 }
 
@@ -398,59 +401,61 @@ mfs_status mfs_pcg_solve(mfs_handle *h, mfs_lpc *net, const double *Ax, const do
         lpc_features(g, ax, W.w, st);
         if (net) lpc_forward(g, net->wb.p, W.w, st);
         MFS_LAUNCHED();
-        // z = M^{-1} r: D^{-1/2} G^T G D^{-1/2} r, or D^{-1} r without a network
+        const int np = reduce_partials_count();
+        double *part = W.partials.p, *npart = part + size_t(np) * nr;
+        double *bb = W.dots.p, *rz = W.dots.p + nr, *rz2 = W.dots.p + 2 * nr, *rr = W.dots.p + 3 * nr;
+        W.state.ensure(1);
+        if (!W.count.p) {
+            W.count.ensure(1);
+            MFS_CUDA(cudaMemsetAsync(W.count.p, 0, sizeof(unsigned), st));
+        }
+        PcgState state{0, 0, 0.0, tol};
+        MFS_CUDA(cudaMemcpyAsync(W.state.p, &state, sizeof(state), cudaMemcpyHostToDevice, st));
+        const int *stop = &W.state.p->stop;
+        // z = M^{-1} r: D^{-1/2} G^T G D^{-1/2} r, or D^{-1} r without a network; partial sums of r . z
         auto precond = [&](const double *r, double *z) {
             if (net) {
-                lpc_gmv(g, W.G.p, false, r, W.t.p, n, nr, W.dinv.p, nullptr, st);
-                lpc_gmv(g, W.G.p, true, W.t.p, z, n, nr, nullptr, W.dinv.p, st);
+                lpc_gmv(g, W.G.p, false, r, W.t.p, n, nr, W.dinv.p, nullptr, st, nullptr, nullptr, stop);
+                lpc_gmv(g, W.G.p, true, W.t.p, z, n, nr, nullptr, W.dinv.p, st, r, part, stop);
             } else {
-                lpc_scale_rows(r, W.dinv.p, false, W.t.p, n, nr, n, st);
-                lpc_scale_rows(W.t.p, W.dinv.p, false, z, n, nr, n, st);
+                launch_pcg_jacobi(r, W.dinv.p, z, n, nr, part, stop, st);
             }
         };
-        double *bb = W.dots.p, *rz = W.dots.p + nr, *rz2 = W.dots.p + 2 * nr, *pap = W.dots.p + 3 * nr;
         std::vector<int> act(static_cast<size_t>(nr), 1);
-        launch_colnorm2(W.bp.p, n, nr, W.partials.p, bb, st);
+        launch_colnorm2(W.bp.p, n, nr, part, bb, st);
         MFS_CUDA(cudaMemsetAsync(W.xp.p, 0, sz * sizeof(double), st));
         launch_copy(W.r.p, W.bp.p, int64_t(sz), st);
         precond(W.r.p, W.pz.p);
         launch_copy(W.p.p, W.pz.p, int64_t(sz), st);
-        launch_coldot(W.r.p, W.pz.p, n, nr, W.partials.p, rz, st);
+        launch_coldot(W.r.p, W.pz.p, n, nr, part, rz, st);
         MFS_LAUNCHED();
-        std::vector<double> hb(static_cast<size_t>(nr)), hr(static_cast<size_t>(nr));
+        std::vector<double> hb(static_cast<size_t>(nr));
         MFS_CUDA(cudaMemcpyAsync(hb.data(), bb, nr * sizeof(double), cudaMemcpyDeviceToHost, st));
         MFS_CUDA(cudaStreamSynchronize(st));
         for (int r = 0; r < nr; ++r)
             if (hb[r] == 0.0) act[r] = 0;
         MFS_CUDA(cudaMemcpyAsync(W.active.p, act.data(), nr * sizeof(int), cudaMemcpyHostToDevice, st));
-        int it = 0;
         bool done = std::none_of(act.begin(), act.end(), [](int a) { return a != 0; });
-        double worst = 0.0;
-        while (!done && it < maxit) {
-            ++it;
-            spmv(h, ax, W.p.p, W.ap.p, nr);
-            launch_coldot(W.p.p, W.ap.p, n, nr, W.partials.p, pap, st);
-            launch_pcg_update_x_r(W.xp.p, W.r.p, W.p.p, W.ap.p, rz, pap, W.active.p, n, nr, st);
-            launch_colnorm2(W.r.p, n, nr, W.partials.p, rz2, st);
-            MFS_LAUNCHED();
-            MFS_CUDA(cudaMemcpyAsync(hr.data(), rz2, nr * sizeof(double), cudaMemcpyDeviceToHost, st));
-            MFS_CUDA(cudaStreamSynchronize(st));
-            worst = 0.0;
-            done = true;
-            for (int r = 0; r < nr; ++r) {
-                const double rel = hb[r] > 0 ? std::sqrt(hr[r] / hb[r]) : 0.0;
-                if (act[r] && rel <= tol) act[r] = 0;
-                if (act[r]) done = false;
-                worst = std::max(worst, rel);
+        // Iterations are launched ahead, a few and then more at a time: convergence is settled
+        // on the device, and what was launched past it returns at once. (A look after every
+        // iteration left the GPU idle for half of it.)
+        for (int launched = 0, ahead = 4; !done && launched < maxit; ahead = std::min(2 * ahead, 32)) {
+            const int end = std::min(maxit, launched + ahead);
+            for (; launched < end; ++launched) {
+                spmv(h, ax, W.p.p, W.ap.p, nr, part, stop);
+                launch_pcg_update_x_r(W.xp.p, W.r.p, W.p.p, W.ap.p, rz, part, W.active.p, n, nr, nullptr, npart, rr,
+                                      W.count.p, bb, W.state.p, st);
+                precond(W.r.p, W.pz.p);
+                launch_pcg_update_p(W.p.p, W.pz.p, part, rz, rz2, W.active.p, n, nr, W.state.p, st);
+                std::swap(rz, rz2);
             }
-            if (done) break;
-            MFS_CUDA(cudaMemcpyAsync(W.active.p, act.data(), nr * sizeof(int), cudaMemcpyHostToDevice, st));
-            precond(W.r.p, W.pz.p);
-            launch_coldot(W.r.p, W.pz.p, n, nr, W.partials.p, rz2, st);
-            launch_pcg_update_p(W.p.p, W.pz.p, rz2, rz, W.active.p, n, nr, st);
             MFS_LAUNCHED();
-            MFS_CUDA(cudaMemcpyAsync(rz, rz2, nr * sizeof(double), cudaMemcpyDeviceToDevice, st));
+            MFS_CUDA(cudaMemcpyAsync(&state, W.state.p, sizeof(state), cudaMemcpyDeviceToHost, st));
+            MFS_CUDA(cudaStreamSynchronize(st));
+            done = state.stop != 0;
         }
+        const int it = state.it;
+        const double worst = state.worst;
         h->stats.pcg_iterations = it;
         h->stats.residual = worst;
         if (done) {

@@ -297,10 +297,11 @@ template <typename T>
 void launch_subtree_solve(bool forward, const int2 *subs, int nsub, int fmax, SnDev sd, const T *factor, double *X,
                           int64_t ldx, int nrhs, double *sol, cudaStream_t st);
 
-// Symmetric block SpMV over permuted reduced rows: Y = A X (both ld = n).
+// Symmetric block SpMV over permuted reduced rows: Y = A X (both ld = n); dotp: partial sums of
+// X . Y per column (reduce_partials_count each); stop: nothing is done once it is set.
 void launch_spmv(const int64_t *ptr, const int64_t *src, const int32_t *col, const int32_t *flag, int64_t nrows,
                  int vb, int src_ld, const double *Ax, const double *X, double *Y, int64_t ld, int nrhs,
-                 cudaStream_t st);
+                 cudaStream_t st, double *dotp = nullptr, const int *stop = nullptr);
 
 // Gather/scatter between the caller's (full or reduced) order and the permuted reduced order.
 void launch_gather_rows(const int64_t *map, int64_t n_in, const double *in, int64_t ld_in, double *out,
@@ -313,14 +314,25 @@ void launch_assemble_elements(const int64_t *slot_ptr, const int64_t *contrib, i
                               double *Ax, cudaStream_t st);
 
 // Refinement / PCG vector kernels (column-wise over nrhs columns, ld = n).
-void launch_residual(const double *B, const double *AX, double *R, int64_t n, int nrhs, cudaStream_t st);
 void launch_colnorm2(const double *X, int64_t n, int nrhs, double *partials, double *out, cudaStream_t st);
 void launch_coldot(const double *X, const double *Y, int64_t n, int nrhs, double *partials, double *out,
                    cudaStream_t st);
+void launch_coldot_partial(const double *X, const double *Y, int64_t n, int nrhs, double *partials, cudaStream_t st);
+// Convergence of a PCG whose iterations are launched ahead of the host's look at them.
+struct PcgState {
+    int stop, it;
+    double worst, tol;
+};
+// x, r and (Z, optional) a copy of r; pAp as partial sums. The squared norms of r go to hr;
+// count: a zeroed counter that returns to zero. With a state, convergence against hb (the
+// right-hand sides' squared norms) is settled on the device.
 void launch_pcg_update_x_r(double *X, double *R, const double *P, const double *AP, const double *rz,
-                           const double *pap, const int *active, int64_t n, int nrhs, cudaStream_t st);
-void launch_pcg_update_p(double *P, const double *Z, const double *rz_new, const double *rz_old, const int *active,
-                         int64_t n, int nrhs, cudaStream_t st);
+                           const double *pap_part, int *active, int64_t n, int nrhs, double *Z, double *norm_part,
+                           double *hr, unsigned *count, const double *hb, PcgState *state, cudaStream_t st);
+void launch_pcg_update_p(double *P, const double *Z, const double *rz_part, const double *rz_old, double *rz_new,
+                         const int *active, int64_t n, int nrhs, const PcgState *state, cudaStream_t st);
+void launch_pcg_jacobi(const double *R, const double *s, double *Z, int64_t n, int nrhs, double *rz_part,
+                       const int *stop, cudaStream_t st);
 void launch_copy(double *dst, const double *src, int64_t count, cudaStream_t st);
 void launch_axpy(double *y, const double *x, double alpha, int64_t count, cudaStream_t st);
 

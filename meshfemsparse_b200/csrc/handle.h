@@ -195,6 +195,7 @@ struct mfs_handle {
     std::shared_ptr<DBuf<double>> asm_spare;   // an earlier assembly buffer, reused once nothing holds it
     DBuf<double> rhs, work_r, work_z, work_p, work_ap, work_x, work_s, io;
     DBuf<double> partials, dots;
+    DBuf<unsigned> xr_count;      // zero between launches (blocks of the PCG update that are done)
     DBuf<int> active;
     DBuf<int> fail;
     DBuf<int> perturbed;          // pivots perturbed in the last numeric factorization

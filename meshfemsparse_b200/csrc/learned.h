@@ -54,9 +54,11 @@ int lpc_head_parts();
 void lpc_features(const LGraph &g, const double *Ax, LWork &w, cudaStream_t st);
 void lpc_forward(const LGraph &g, const __nv_bfloat16 *wb, LWork &w, cudaStream_t st);
 void lpc_backward(const LGraph &g, const __nv_bfloat16 *wb, LWork &w, float *grad, cudaStream_t st);
-// Y = G X or G^T X over 3 nv rows (ld, nrhs); pre scales X rows, post scales Y rows (nullable)
+// Y = G X or G^T X over 3 nv rows (ld, nrhs); pre scales X rows, post scales Y rows (nullable);
+// dotv, dotp: partial sums of dotv . Y per column; stop: nothing is done once it is set
 void lpc_gmv(const LGraph &g, const float *G, bool trans, const double *X, double *Y, int64_t ld, int nrhs,
-             const double *pre, const double *post, cudaStream_t st);
+             const double *pre, const double *post, cudaStream_t st, const double *dotv = nullptr,
+             double *dotp = nullptr, const int *stop = nullptr);
 void lpc_scale_rows(const double *in, const double *s, bool inv, double *out, int64_t n, int nrhs, int64_t ld,
                     cudaStream_t st);
 void lpc_dg(const LGraph &g, const double *Z, const double *GY, const double *GZ, const double *BS, int64_t ld,
