@@ -213,83 +213,98 @@ __global__ void __launch_bounds__(256) gemm_tf32_kernel(const GemmTask *__restri
 // at 24 instead of 26 TFLOP/s.) All GEMM launches of a factorization of the 48-sided cube:
 // 123 ms with 8-byte copies, two stages and the element-by-element epilogue, 105 ms now
 // (level SYRKs 26, the largest 30 TFLOP/s).
+// Launches of at most kF64FewTiles tiles (the column-block chain of the large fronts) split
+// every tile into four of 32 rows (all of its columns: a row solve is in place), since a
+// tile alone takes 1.1 us of its SM per 16 k: left-looking updates of the 20-sided cube
+// 19 us a launch on whole tiles, 12 us split; with more tiles than SMs the split only
+// costs reads of B.
 constexpr int DBM = 128, DBN = 64, DBK = 16, DST = 4;
-constexpr int DLDA = DBM + 4, DLDB = DBN + 4;                 // 8 bytes x (4 k + row): conflict-free fragments
-constexpr int kF64Stage = DBK * (DLDA + DLDB);               // doubles
-constexpr int kF64Smem = DST * kF64Stage * 8;
+constexpr int kF64FewTiles = 148;
+template <int BM>
+struct F64Tile {
+    static constexpr int LDA = BM + 4, LDB = DBN + 4;         // 8 bytes x (4 k + row): conflict-free fragments
+    static constexpr int STAGE = DBK * (LDA + LDB);          // doubles
+    static constexpr int SMEM = DST * STAGE * 8;
+    static constexpr int WM = BM == 128 ? 4 : 2, WN = 8 / WM; // warps along m, n
+    static constexpr int MT = BM / WM / 8, NT = DBN / WN / 8; // 8 x 8 products per warp
+};
 
+template <int BM>
 __global__ void __launch_bounds__(256, 2) gemm_f64_kernel(const GemmTask *__restrict__ tasks, int ntasks,
                                                           const double *Abase, const double *__restrict__ Bbase,
                                                           double *Cbase) {
+    using S = F64Tile<BM>;
+    constexpr int LDA = S::LDA, LDB = S::LDB, MT = S::MT, NT = S::NT, PARTS = DBM / BM;
     extern __shared__ __align__(16) double smd[];
-    const int t = blockIdx.x;
+    const int t = blockIdx.x / PARTS;
     const GemmTask tk = tasks[find_task(tasks, ntasks, t)];
     const int local = t - tk.tile_base;
     const int ti = local % tk.tiles_m, tj = local / tk.tiles_m;
     const int da = tk.shift & 255, db = tk.shift >> 8;       // shifted row x is operand row x - d
-    const int i0 = ti * DBM, j0 = tj * DBN;                  // tile origin in shifted coordinates
-    if (tk.lower && i0 + DBM - 1 - da < j0 - db) return;
+    const int i0 = ti * DBM + int(blockIdx.x % PARTS) * BM, j0 = tj * DBN;   // tile origin in shifted coordinates
+    if (i0 >= tk.m + da || (tk.lower && i0 + BM - 1 - da < j0 - db)) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int wm = warp & 3, wn = warp >> 2;
+    const int wm = warp % S::WM, wn = warp / S::WM;
     const int gid = lane >> 2, tig = lane & 3;
     const double *A = Abase + (tk.a_off - da) + i0;
     const double *B = Bbase + (tk.b_off - db) + j0;
     const int am = tk.m + da - i0, bn = tk.n + db - j0;      // rows / columns left in shifted coordinates
     const int K = tk.k, nk = (K + DBK - 1) / DBK;
-    // copies: 64 (A) / 32 (B) 16-byte chunks a k row; a thread has one chunk and every fourth
-    // (eighth) k row
-    const int ca = (tid & 63) * 2, ka = tid >> 6, cb = (tid & 31) * 2, kb0 = tid >> 5;
+    // copies: BM / 2 (A) and 32 (B) 16-byte chunks a k row; a thread has one chunk and every
+    // KA-th (eighth) k row
+    constexpr int CA = BM / 2, KA = 256 / CA;
+    const int ca = (tid % CA) * 2, ka = tid / CA, cb = (tid & 31) * 2, kb0 = tid >> 5;
     const int na = min(2, max(0, am - ca)) * 8, nb = min(2, max(0, bn - cb)) * 8;
     auto load = [&](int kc) {
-        double *as = smd + (kc % DST) * kF64Stage;
-        double *bs = as + DBK * DLDA;
+        double *as = smd + (kc % DST) * S::STAGE;
+        double *bs = as + DBK * LDA;
         const int k0 = kc * DBK;
 #pragma unroll
-        for (int r = 0; r < DBK / 4; ++r) {
-            const int k = ka + 4 * r, n = k0 + k < K ? na : 0;
-            cp_async16(as + k * DLDA + ca, n ? A + int64_t(k0 + k) * tk.lda + ca : Abase, n);
+        for (int r = 0; r < DBK / KA; ++r) {
+            const int k = ka + KA * r, n = k0 + k < K ? na : 0;
+            cp_async16(as + k * LDA + ca, n ? A + int64_t(k0 + k) * tk.lda + ca : Abase, n);
         }
 #pragma unroll
         for (int r = 0; r < DBK / 8; ++r) {
             const int k = kb0 + 8 * r, n = k0 + k < K ? nb : 0;
-            cp_async16(bs + k * DLDB + cb, n ? B + int64_t(k0 + k) * tk.ldb + cb : Bbase, n);
+            cp_async16(bs + k * LDB + cb, n ? B + int64_t(k0 + k) * tk.ldb + cb : Bbase, n);
         }
     };
+    double acc[MT][NT][2];
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) acc[mt][nt][0] = acc[mt][nt][1] = 0.0;
 #pragma unroll
     for (int kc = 0; kc < DST - 1; ++kc) {
         if (kc < nk) load(kc);
         cp_commit();
     }
-    double acc[4][4][2];
-#pragma unroll
-    for (int mt = 0; mt < 4; ++mt)
-#pragma unroll
-        for (int nt = 0; nt < 4; ++nt) acc[mt][nt][0] = acc[mt][nt][1] = 0.0;
     for (int kc = 0; kc < nk; ++kc) {
         cp_wait<DST - 2>();
         __syncthreads();                                     // (also: stage kc - 1 is read)
         if (kc + DST - 1 < nk) load(kc + DST - 1);
         cp_commit();
-        const double *as = smd + (kc % DST) * kF64Stage + wm * 32 + gid;
-        const double *bs = smd + (kc % DST) * kF64Stage + DBK * DLDA + wn * 32 + gid;
+        const double *as = smd + (kc % DST) * S::STAGE + wm * (8 * MT) + gid;
+        const double *bs = smd + (kc % DST) * S::STAGE + DBK * LDA + wn * (8 * NT) + gid;
 #pragma unroll
         for (int k4 = 0; k4 < DBK; k4 += 4) {
-            double a[4], b[4];
+            double a[MT], b[NT];
 #pragma unroll
-            for (int mt = 0; mt < 4; ++mt) a[mt] = as[(k4 + tig) * DLDA + mt * 8];
+            for (int mt = 0; mt < MT; ++mt) a[mt] = as[(k4 + tig) * LDA + mt * 8];
 #pragma unroll
-            for (int nt = 0; nt < 4; ++nt) b[nt] = bs[(k4 + tig) * DLDB + nt * 8];
+            for (int nt = 0; nt < NT; ++nt) b[nt] = bs[(k4 + tig) * LDB + nt * 8];
 #pragma unroll
-            for (int mt = 0; mt < 4; ++mt)
+            for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
-                for (int nt = 0; nt < 4; ++nt) mma_f64(acc[mt][nt], a[mt], b[nt]);
+                for (int nt = 0; nt < NT; ++nt) mma_f64(acc[mt][nt], a[mt], b[nt]);
         }
     }
     cp_wait<0>();
     // an in-place row solve (C = A, the tile spans its columns) has read all of its rows
     __syncthreads();
     double *C = Cbase + tk.c_off;
-    const int ib = i0 - da + wm * 32 + gid, jb = j0 - db + wn * 32 + tig * 2;
+    const int ib = i0 - da + wm * (8 * MT) + gid, jb = j0 - db + wn * (8 * NT) + tig * 2;
     auto live = [&](int mt, int nt, int e) {
         const int i = ib + mt * 8, j = jb + nt * 8 + e;
         return i >= 0 && i < tk.m && j >= 0 && j < tk.n && !(tk.lower && i < j);
@@ -297,29 +312,30 @@ __global__ void __launch_bounds__(256, 2) gemm_f64_kernel(const GemmTask *__rest
     auto at = [&](int mt, int nt, int e) { return C + int64_t(jb + nt * 8 + e) * tk.ldc + ib + mt * 8; };
     if (tk.mode == 0) {
         // half of the tile's C at a time (registers): every load before the first store
+        constexpr int H = MT / 2;
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            double c[2][4][2];
+            double c[H][NT][2];
 #pragma unroll
-            for (int m = 0; m < 2; ++m)
+            for (int m = 0; m < H; ++m)
 #pragma unroll
-                for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-                    for (int e = 0; e < 2; ++e)
-                        if (live(2 * h + m, nt, e)) c[m][nt][e] = *at(2 * h + m, nt, e);
-#pragma unroll
-            for (int m = 0; m < 2; ++m)
-#pragma unroll
-                for (int nt = 0; nt < 4; ++nt)
+                for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
                     for (int e = 0; e < 2; ++e)
-                        if (live(2 * h + m, nt, e)) *at(2 * h + m, nt, e) = c[m][nt][e] - acc[2 * h + m][nt][e];
+                        if (live(H * h + m, nt, e)) c[m][nt][e] = *at(H * h + m, nt, e);
+#pragma unroll
+            for (int m = 0; m < H; ++m)
+#pragma unroll
+                for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e)
+                        if (live(H * h + m, nt, e)) *at(H * h + m, nt, e) = c[m][nt][e] - acc[H * h + m][nt][e];
         }
     } else {
 #pragma unroll
-        for (int mt = 0; mt < 4; ++mt)
+        for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
-            for (int nt = 0; nt < 4; ++nt)
+            for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
                 for (int e = 0; e < 2; ++e)
                     if (live(mt, nt, e)) *at(mt, nt, e) = acc[mt][nt][e];
@@ -359,8 +375,14 @@ void launch_gemm<double>(const GemmTask *tasks, int ntasks, int ntiles, const do
     if (ntiles <= 0) return;
     ++g_kernel_launches;
     static PerDeviceOnce once;
-    once([] { cudaFuncSetAttribute(gemm_f64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kF64Smem); });
-    gemm_f64_kernel<<<ntiles, 256, kF64Smem, st>>>(tasks, ntasks, A, B, C);
+    once([] {
+        cudaFuncSetAttribute(gemm_f64_kernel<DBM>, cudaFuncAttributeMaxDynamicSharedMemorySize, F64Tile<DBM>::SMEM);
+        cudaFuncSetAttribute(gemm_f64_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, F64Tile<32>::SMEM);
+    });
+    if (ntiles <= kF64FewTiles)
+        gemm_f64_kernel<32><<<ntiles * (DBM / 32), 256, F64Tile<32>::SMEM, st>>>(tasks, ntasks, A, B, C);
+    else
+        gemm_f64_kernel<DBM><<<ntiles, 256, F64Tile<DBM>::SMEM, st>>>(tasks, ntasks, A, B, C);
 }
 
 }  // namespace mfs
