@@ -357,10 +357,10 @@ std::shared_ptr<DevSym> upload_symbolic(mfs_handle *h, std::shared_ptr<Symbolic>
     std::vector<int32_t> sb_fidx(nsn, -1);
     for (size_t i = 0; i < ds->sb_fronts.size(); ++i) sb_fidx[ds->sb_fronts[i]] = int32_t(i);
     auto sb_parts = [&](idx s, idx K) { return (std::min(SBk, S.w[s] - K * SBk) + 63) / 64; };
-    // the children of each front above the cut
+    // the children of each front (with the count to wait for, those above the cut)
     std::vector<SbChild> kids;
     std::vector<int32_t> sb_child0(nsn, 0), sb_nchild(nsn, 0);
-    for (int32_t s : ds->sb_fronts) {
+    for (idx s = 0; s < nsn; ++s) {
         sb_child0[s] = int32_t(kids.size());
         for (idx k = S.child_ptr[s]; k < S.child_ptr[s + 1]; ++k) {
             const idx c = S.child_list[k];
@@ -541,11 +541,46 @@ std::shared_ptr<DevSym> upload_symbolic(mfs_handle *h, std::shared_ptr<Symbolic>
     ds->isb_host = isb;
     ds->max_str_entries = max_str;
     {
-        std::vector<int2> sv(S.sub_lo.size());
-        for (size_t k = 0; k < sv.size(); ++k) sv[k] = make_int2(int(S.sub_lo[k]), int(S.sub_hi[k]));
+        // below the cut: the largest subtrees without stored inverses, and per subtree of
+        // the cut the fronts above those
+        std::vector<uint8_t> small(nsn, 0);
+        for (idx s = 0; s < nsn; ++s) {
+            small[s] = inv_off[s] < 0 && S.level[s] <= S.solve_cut;
+            for (idx k = S.child_ptr[s]; k < S.child_ptr[s + 1]; ++k) small[s] &= small[S.child_list[k]];
+        }
+        std::vector<SubFront> sf(nsn);
+        std::vector<int32_t> lo(nsn), top_ptr(1, 0), tops;
+        std::vector<std::pair<double, int32_t>> work;     // of the subtrees of small fronts
+        std::vector<double> cost(nsn, 0.0);
+        for (idx s = 0; s < nsn; ++s) {
+            sf[s] = {int32_t(S.w[s]), int32_t(S.f[s]), dld[s],     col0[s],      sb_child0[s],
+                     sb_nchild[s],    dpan[s],         inv_off[s], S.sol_off[s], S.struct_ptr[s]};
+            lo[s] = int32_t(s);
+            cost[s] = double(S.f[s]) * double(S.w[s]);
+            for (idx k = S.child_ptr[s]; k < S.child_ptr[s + 1]; ++k) {
+                lo[s] = std::min(lo[s], lo[S.child_list[k]]);
+                cost[s] += cost[S.child_list[k]];
+            }
+            if (small[s] && (S.sn_parent[s] < 0 || !small[S.sn_parent[s]])) work.push_back({-cost[s], int32_t(s)});
+            if (small[s]) ds->sub_small = std::max(ds->sub_small, int(S.f[s]));
+        }
+        std::sort(work.begin(), work.end());
+        std::vector<int2> sv;
+        for (const auto &wk : work) sv.push_back(make_int2(lo[wk.second], wk.second));
+        for (size_t k = 0; k < S.sub_lo.size(); ++k) {
+            for (idx s = S.sub_lo[k]; s <= S.sub_hi[k]; ++s)
+                if (!small[s]) {
+                    tops.push_back(int32_t(s));
+                    ds->sub_fmax = std::max(ds->sub_fmax, int(S.f[s]));
+                }
+            if (int32_t(tops.size()) > top_ptr.back()) top_ptr.push_back(int32_t(tops.size()));
+        }
         up(ds->subs, sv);
         ds->nsub = int(sv.size());
-        ds->sub_fmax = int(S.sub_fmax);
+        up(ds->top_ptr, top_ptr);
+        up(ds->tops, tops);
+        ds->ntop = int(top_ptr.size()) - 1;
+        up(ds->sub_fronts, sf);
         ds->solve_cut = int(S.solve_cut);
     }
     ds->flags.ensure(size_t(std::max(std::max(nflags, nsbflags), 1)));
@@ -906,8 +941,12 @@ void run_solve(mfs_handle *h, DevSym &ds, const T *factor, double *X, int nrhs) 
         const int nr = std::min(pass, nrhs - r0);
         double *Xc = X + int64_t(r0) * S.n;
         MFS_CUDA(cudaMemsetAsync(ds.flags.p, 0, ds.flags.bytes(), st));
-        // levels <= solve_cut: whole subtrees, one per CTA
-        launch_subtree_solve<T>(true, ds.subs.p, ds.nsub, ds.sub_fmax, ds.sd, factor, Xc, S.n, nr, h->sol.p, st);
+        // levels <= solve_cut: whole subtrees
+        launch_subtree_small<T>(true, ds.subs.p, ds.nsub, ds.sub_small, ds.sd, ds.sub_fronts.p, ds.sb_children.p,
+                                ds.cmap.p, factor, Xc, S.n, nr, h->sol.p, st);
+        MFS_LAUNCHED();
+        launch_subtree_solve<T>(true, ds.top_ptr.p, ds.tops.p, ds.ntop, ds.sub_fmax, ds.sd, ds.sub_fronts.p,
+                                ds.sb_children.p, ds.cmap.p, factor, Xc, S.n, nr, h->sol.p, st);
         MFS_LAUNCHED();
         if (sb) {
             auto above = [&](bool forward, const SbTask *tasks, int n) {
@@ -937,7 +976,11 @@ void run_solve(mfs_handle *h, DevSym &ds, const T *factor, double *X, int nrhs) 
                                         ds.flags.p, h->solve_err.p, st));
             }
         }
-        launch_subtree_solve<T>(false, ds.subs.p, ds.nsub, ds.sub_fmax, ds.sd, factor, Xc, S.n, nr, h->sol.p, st);
+        launch_subtree_solve<T>(false, ds.top_ptr.p, ds.tops.p, ds.ntop, ds.sub_fmax, ds.sd, ds.sub_fronts.p,
+                                ds.sb_children.p, ds.cmap.p, factor, Xc, S.n, nr, h->sol.p, st);
+        MFS_LAUNCHED();
+        launch_subtree_small<T>(false, ds.subs.p, ds.nsub, ds.sub_small, ds.sd, ds.sub_fronts.p, ds.sb_children.p,
+                                ds.cmap.p, factor, Xc, S.n, nr, h->sol.p, st);
         MFS_LAUNCHED();
     }
 }

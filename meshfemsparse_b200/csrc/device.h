@@ -192,6 +192,13 @@ struct SbChild {
     int64_t map, sol;
     int32_t d, pad;
 };
+// A front in the subtree solves: sizes, panel leading dimension, first column, children with
+// an update vector (SbChild), panel, stored inverses (-1: none), place in the solve arena
+// (-1: none) and first structure row.
+struct SubFront {
+    int32_t w, f, ld, col0, child0, nchild;
+    int64_t pan, inv, sol, rows;
+};
 constexpr int kSuperBlock = 256;        // rows per superblock
 // structure part of the solves: forward tasks are kStrRows rows x kStrCols columns
 // of L21, backward tasks kStrBCols columns x str_bwd_rows rows
@@ -291,10 +298,17 @@ template <typename T>
 void launch_sb_inverse(const SbTask *tasks, int ntasks, SnDev sd, T *factor, cudaStream_t st);
 int solve_rows_per_task();
 int diag_blocks_per_task();             // 64-row blocks per diagonal-chain task (one flag each)
-// Forward / backward solve of whole subtrees (subs[k] = postorder range [x, y]),
-// one CTA per subtree, fronts of at most fmax rows.
+// Forward / backward solve of whole subtrees of fronts without stored inverses (subs[k] =
+// postorder range [x, y], largest front fmax rows), then of the fronts above them up to the
+// cut (subtree k: tops[top_ptr[k]..top_ptr[k + 1]) in postorder); backward in the other order.
+// fronts per supernode, kids and cmap as for launch_sb_solve.
 template <typename T>
-void launch_subtree_solve(bool forward, const int2 *subs, int nsub, int fmax, SnDev sd, const T *factor, double *X,
+void launch_subtree_small(bool forward, const int2 *subs, int nsub, int fmax, SnDev sd, const SubFront *fronts,
+                          const SbChild *kids, const int32_t *cmap, const T *factor, double *X, int64_t ldx, int nrhs,
+                          double *sol, cudaStream_t st);
+template <typename T>
+void launch_subtree_solve(bool forward, const int32_t *top_ptr, const int32_t *tops, int nsub, int fmax, SnDev sd,
+                          const SubFront *fronts, const SbChild *kids, const int32_t *cmap, const T *factor, double *X,
                           int64_t ldx, int nrhs, double *sol, cudaStream_t st);
 
 // Symmetric block SpMV over permuted reduced rows: Y = A X (both ld = n); dotp: partial sums of

@@ -119,7 +119,7 @@ struct DevSym {
     DBuf<StrReduce> fred, bred;
     DBuf<SbTask> fsb_tasks, bsb_tasks, isb_tasks;   // solves above the cut (forward, backward) and inverses
     int nfsb = 0, nbsb = 0, nsb_inv = 0;
-    DBuf<SbChild> sb_children;                      // the children of the fronts above the cut
+    DBuf<SbChild> sb_children;                      // the children of every front, front by front
     DBuf<int32_t> parent, cmap;                     // assembly parents; children's inverse row maps
     DBuf<int64_t> cmap_off;
     DBuf<int32_t> rowcnt;                           // per analysis row above the cut: its superblock's count and parts
@@ -127,7 +127,9 @@ struct DevSym {
     std::vector<int32_t> sb_fronts;                 // fronts with superblock solves
     int64_t max_str_entries = 0;       // structure partial sums of one level, per right-hand side
     DBuf<int2> subs;                     // subtree ranges solved one per CTA (levels <= solve_cut)
-    int nsub = 0, sub_fmax = 0, solve_cut = -1;
+    DBuf<SubFront> sub_fronts;           // per supernode
+    DBuf<int32_t> top_ptr, tops;         // the cut's subtrees: their fronts above those of subs
+    int nsub = 0, ntop = 0, sub_fmax = 0, sub_small = 0, solve_cut = -1;   // fmax: largest of tops, small: of subs
     DBuf<int> flags;                     // one per 64-row diagonal block of every front
     DBuf<int64_t> spmv_ptr, spmv_src;
     DBuf<int32_t> spmv_col, spmv_flag;

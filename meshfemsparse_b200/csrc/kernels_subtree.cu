@@ -1,56 +1,38 @@
 // Multi-RHS forward / backward solves (K6) over the lower part of the assembly
-// tree, one independent subtree per CTA.
+// tree, one independent subtree per CTA or per warp and right-hand side.
 //
-// Below the cut level the tree has many small fronts and few rows per front:
-// level-by-level kernels there spend their time on launches, barriers and
-// load latency rather than on reading L. Here a CTA walks a whole subtree
-// (a contiguous postorder range of supernodes) with the front's right-hand
-// side block (front rows x up to 4 RHS) held in shared memory:
-//   forward  (postorder)  v = [x(cols); 0] + children's u (child order, through
-//            child_rel_indices); y = L11^{-1} v[0:w] (64-row blocks through the
-//            stored diagonal inverses, or column substitution for fronts factored
-//            in shared memory, which then also yields u); u = v[w:f] - L21 y;
-//            y -> x, u -> solve arena (read by the parent, later in this CTA or
-//            by the level kernels above the cut);
-//   backward (reverse postorder) v = [x(cols); x(struct rows)] (ancestors are
-//            final); v[0:w] -= L21^T x_struct; x = L11^{-T} v[0:w].
-// The next front's panel (ld x w, contiguous) is copied into shared memory with
-// cp.async while the current one is solved (panels up to kPanelStageBytes;
-// bigger ones are read from global memory). Fronts factored in shared memory
-// (no stored inverse) are substituted by one warp per right-hand side. Nothing
-// is shared between CTAs, so no flags are needed. Subtrees are assigned
-// round-robin in order of decreasing work.
+// Below the cut level the tree has many small fronts and few rows per front: what a front
+// costs is its chain of dependent loads, not its bytes. A walk goes over a whole subtree (a
+// contiguous postorder range of supernodes):
+//   forward  (postorder)  v = [x(cols); 0] + children's u (child order, through their inverse
+//            row maps); y = L11^{-1} v[0:w]; u = v[w:f] - L21 y; y -> x, u -> solve arena
+//            (read by the parent, later in this walk or above the cut);
+//   backward (reverse postorder) v = [x(cols); x(struct rows)] (ancestors are final);
+//            v[0:w] -= L21^T x_struct; x = L11^{-T} v[0:w].
+// Fronts factored in shared memory (no stored diagonal inverses) are one warp's, for up to
+// four right-hand sides, v in its registers (lane = rows lane + 32 g): column substitution
+// forward (a column's chain is a shuffle, a product with the reciprocal diagonal and a fused
+// multiply-add), backward eight columns at a time (sums over the rows below, the triangle). Both
+// read columns only; an entry is read and widened once for the four. The largest subtrees of
+// such fronts alone are a launch of their own, spread over all warps: nothing there waits
+// at a barrier. The fronts above them are a CTA's per subtree of the cut, four right-hand
+// sides at a time, through the stored 64 x 64 inverses, v in shared memory. In one CTA walk for
+// all, with barriers, a division a column and the children one after the other, a pass over
+// the batch of 48 cubes (FP32, 8 right-hand sides) took 1,140 us forward and 1,160 us backward,
+// @@BF@@ and @@BB@@ us this way; k = 64 with 4: 690 us each way, @@KF@@ and @@KB@@ us. Subtrees are
+// assigned round-robin in order of decreasing work.
 #include "device.h"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace mfs {
 
 namespace {
 
 constexpr int kSubThreads = 256;
-constexpr int kSubRhs = 4;                 // right-hand sides per pass (more are looped)
+constexpr int kSubRhs = 4;                 // right-hand sides per pass or warp (more are looped)
 constexpr int kSubRed = 4 * kSubRhs * 64;  // split-k partials of a 64-row block
-constexpr int kPanelStageBytes = 8192;     // per staging buffer (two buffers); larger ones cost occupancy
-
-__device__ __forceinline__ void sub_cp16(void *dst_smem, const void *src) {
-    const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst_smem));
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ void sub_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void sub_wait1() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
-
-// Panel of s staged into buf when it fits (ld x w elements are contiguous and
-// 16-byte aligned); returns whether it was staged.
-template <typename T>
-__device__ __forceinline__ bool stage_panel(int s, const SnDev &sd, const T *factor, T *buf) {
-    const int64_t n = int64_t(sd.ld[s]) * sd.w[s];
-    if (n * int64_t(sizeof(T)) > kPanelStageBytes) return false;
-    const T *src = factor + sd.pan_off[s];
-    constexpr int E = 16 / int(sizeof(T));
-    for (int q = threadIdx.x; q * E < n; q += blockDim.x) sub_cp16(buf + q * E, src + q * E);
-    return true;
-}
 
 template <int VB>
 __device__ __forceinline__ int crel(const int32_t *rel, int i, int vb) {
@@ -65,11 +47,12 @@ __device__ __forceinline__ double warp_sum(double x) {
 }
 
 // ------------------------------------------------------------------ forward
+// A front with stored inverses, the whole CTA.
 template <typename T, int VB>
 __device__ __forceinline__ void fwd_front(int s, const SnDev &sd, const T *__restrict__ factor, const T *pan,
                                           double *__restrict__ X, int64_t ldx, int nrhs, int rg, int nr,
                                           double *__restrict__ sol, double *v, double *red) {
-    const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, nt = blockDim.x;
     const int w = sd.w[s], d = sd.d[s], f = w + d, c0 = sd.col0[s], ld = sd.ld[s];
     for (int q = tid; q < nr * f; q += nt) {
         const int r = q / f, i = q - r * f;
@@ -151,16 +134,6 @@ __device__ __forceinline__ void fwd_front(int s, const SnDev &sd, const T *__res
             for (int r = 0; r < kSubRhs; ++r)
                 if (r < nr) v[r * f + w + k] -= acc[r];
         }
-    } else if (warp < nr) {
-        // column substitution over the whole front (y and u together), warp r for rhs r
-        double *vr = v + warp * f;
-        for (int j = 0; j < w; ++j) {
-            const double y = vr[j] / double(pan[int64_t(j) * ld + j]);
-            __syncwarp();
-            if (lane == 0) vr[j] = y;
-            for (int i = j + 1 + lane; i < f; i += 32) vr[i] -= double(pan[int64_t(j) * ld + i]) * y;
-            __syncwarp();
-        }
     }
     __syncthreads();
     const bool has_u = d > 0 && sd.sol_off[s] >= 0;
@@ -192,8 +165,7 @@ __device__ __forceinline__ void bwd_front(int s, const SnDev &sd, const T *__res
     }
     __syncthreads();
     const int64_t inv = sd.inv_off[s];
-    // v[0:w] -= L21^T x_struct: one warp per column, lanes over rows (fronts with
-    // inverses; the substitution below covers the struct rows otherwise)
+    // v[0:w] -= L21^T x_struct: one warp per column, lanes over rows
     if (d > 0 && inv >= 0) {
         for (int j = warp; j < w; j += nw) {
             double acc[kSubRhs] = {0.0, 0.0, 0.0, 0.0};
@@ -263,17 +235,6 @@ __device__ __forceinline__ void bwd_front(int s, const SnDev &sd, const T *__res
                 __syncthreads();
             }
         }
-    } else if (warp < nr) {
-        // left-looking backward substitution, warp r for rhs r:
-        // x_j = (v_j - sum_{i > j} L(i, j) x_i) / L_jj over front rows i (struct rows included)
-        double *vr = v + warp * f;
-        for (int j = w - 1; j >= 0; --j) {
-            double acc = 0.0;
-            for (int i = j + 1 + lane; i < f; i += 32) acc += double(pan[int64_t(j) * ld + i]) * vr[i];
-            acc = warp_sum(acc);
-            if (lane == 0) vr[j] = (vr[j] - acc) / double(pan[int64_t(j) * ld + j]);
-            __syncwarp();
-        }
     }
     __syncthreads();
     for (int q = tid; q < nr * w; q += nt) {
@@ -283,63 +244,307 @@ __device__ __forceinline__ void bwd_front(int s, const SnDev &sd, const T *__res
     __syncthreads();
 }
 
-template <typename T, int VB>
-__global__ void __launch_bounds__(kSubThreads) subtree_fwd_kernel(const int2 *__restrict__ subs, int nsub, SnDev sd,
-                                                                  const T *__restrict__ factor, double *X, int64_t ldx,
-                                                                  int nrhs, double *sol) {
-    extern __shared__ __align__(16) double sub_smem[];
-    T *pbuf = reinterpret_cast<T *>(sub_smem);                       // 2 staging buffers
-    double *red = sub_smem + 2 * kPanelStageBytes / 8;
-    double *v = red + kSubRed;
-    for (int k = blockIdx.x; k < nsub; k += gridDim.x) {
-        const int2 sr = subs[k];
-        for (int rg = 0; rg < nrhs; rg += kSubRhs) {
-            const int nr = min(kSubRhs, nrhs - rg);
-            constexpr int PB = kPanelStageBytes / int(sizeof(T));
-            bool staged = stage_panel(sr.x, sd, factor, pbuf);
-            sub_commit();
-            for (int s = sr.x; s <= sr.y; ++s) {
-                const int b = (s - sr.x) & 1;
-                const bool next = s < sr.y && stage_panel(s + 1, sd, factor, pbuf + (b ^ 1) * PB);
-                sub_commit();
-                sub_wait1();
-                __syncthreads();
-                const T *pan = staged ? pbuf + b * PB : factor + sd.pan_off[s];
-                fwd_front<T, VB>(s, sd, factor, pan, X, ldx, nrhs, rg, nr, sol, v, red);
-                staged = next;
+// ------------------------------------------------------------------ small fronts, one warp
+// NSEG x 32 rows at least the front's; right-hand sides r0 to r0 + nr - 1, at most RB.
+template <typename T, int VB, int NSEG, int RB>
+__device__ __forceinline__ void fwd_small(const SubFront &sf, const T *__restrict__ factor,
+                                          const SbChild *__restrict__ kids, const int32_t *__restrict__ cmap, int vb_,
+                                          double *X, int64_t ldx, int nrhs, int r0, int nr, double *sol) {
+    const int lane = threadIdx.x & 31, vb = VB > 0 ? VB : vb_;
+    const int w = sf.w, f = sf.f;
+    const T *pan = factor + sf.pan;
+    double *x = X + sf.col0 + r0 * ldx;
+    double v[RB][NSEG], rd[NSEG];
+    __syncwarp();                                        // the children's u (this warp's) are visible
+#pragma unroll
+    for (int g = 0; g < NSEG; ++g) {
+        const int i = lane + 32 * g;
+        rd[g] = i < w ? double(pan[int64_t(i) * sf.ld + i]) : 1.0;
+#pragma unroll
+        for (int r = 0; r < RB; ++r) v[r][g] = i < w && r < nr ? x[i + r * ldx] : 0.0;
+    }
+    for (int ci = 0; ci < sf.nchild; ++ci) {
+        const SbChild ch = kids[sf.child0 + ci];
+        const double *u = sol + ch.sol * nrhs + int64_t(r0) * ch.d;
+        int m[NSEG];
+#pragma unroll
+        for (int g = 0; g < NSEG; ++g) {
+            const int i = lane + 32 * g, b = i / vb;
+            m[g] = -1;
+            if (i < f) {
+                const int k = cmap[ch.map + b];
+                if (k >= 0) m[g] = k * vb + i - b * vb;
             }
-            asm volatile("cp.async.wait_all;" ::: "memory");
-            __syncthreads();
+        }
+        double a[RB][NSEG];
+#pragma unroll
+        for (int r = 0; r < RB; ++r)
+#pragma unroll
+            for (int g = 0; g < NSEG; ++g) a[r][g] = m[g] >= 0 && r < nr ? u[m[g] + r * ch.d] : 0.0;
+#pragma unroll
+        for (int r = 0; r < RB; ++r)
+#pragma unroll
+            for (int g = 0; g < NSEG; ++g) v[r][g] += a[r][g];
+    }
+#pragma unroll
+    for (int g = 0; g < NSEG; ++g) rd[g] = 1.0 / rd[g];
+#pragma unroll
+    for (int gb = 0; gb < NSEG; ++gb) {
+        if (32 * gb >= w) break;
+        const int je = min(32, w - 32 * gb);
+        for (int j0 = 0; j0 < je; j0 += 4) {
+            // four columns of L ahead of their use
+            T l[4][NSEG];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+#pragma unroll
+                for (int g = gb; g < NSEG; ++g) {
+                    const int i = lane + 32 * g, j = 32 * gb + j0 + u;
+                    l[u][g] = (j0 + u < je && i > j && i < f) ? pan[int64_t(j) * sf.ld + i] : T(0);
+                }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                if (j0 + u >= je) break;
+                double y[RB];
+#pragma unroll
+                for (int r = 0; r < RB; ++r) y[r] = __shfl_sync(0xffffffffu, v[r][gb] * rd[gb], j0 + u);
+                if (lane == j0 + u)
+#pragma unroll
+                    for (int r = 0; r < RB; ++r) v[r][gb] = y[r];
+#pragma unroll
+                for (int g = gb; g < NSEG; ++g) {
+                    const double lv = double(l[u][g]);
+#pragma unroll
+                    for (int r = 0; r < RB; ++r) v[r][g] -= lv * y[r];
+                }
+            }
+        }
+    }
+    double *us = sf.sol >= 0 ? sol + sf.sol * nrhs + int64_t(r0) * (f - w) : nullptr;
+#pragma unroll
+    for (int r = 0; r < RB; ++r) {
+        if (r >= nr) break;
+#pragma unroll
+        for (int g = 0; g < NSEG; ++g) {
+            const int i = lane + 32 * g;
+            if (i < w) x[i + r * ldx] = v[r][g];
+            else if (i < f && us) us[i - w + r * int64_t(f - w)] = v[r][g];
         }
     }
 }
 
-template <typename T, int VB>
-__global__ void __launch_bounds__(kSubThreads) subtree_bwd_kernel(const int2 *__restrict__ subs, int nsub, SnDev sd,
-                                                                  const T *__restrict__ factor, double *X, int64_t ldx,
-                                                                  int nrhs) {
-    extern __shared__ __align__(16) double sub_smem[];
-    T *pbuf = reinterpret_cast<T *>(sub_smem);
-    double *v = sub_smem + 2 * kPanelStageBytes / 8 + kSubRed;
-    for (int k = blockIdx.x; k < nsub; k += gridDim.x) {
-        const int2 sr = subs[k];
-        for (int rg = 0; rg < nrhs; rg += kSubRhs) {
-            const int nr = min(kSubRhs, nrhs - rg);
-            constexpr int PB = kPanelStageBytes / int(sizeof(T));
-            bool staged = stage_panel(sr.y, sd, factor, pbuf);
-            sub_commit();
-            for (int s = sr.y; s >= sr.x; --s) {
-                const int b = (sr.y - s) & 1;
-                const bool next = s > sr.x && stage_panel(s - 1, sd, factor, pbuf + (b ^ 1) * PB);
-                sub_commit();
-                sub_wait1();
-                __syncthreads();
-                const T *pan = staged ? pbuf + b * PB : factor + sd.pan_off[s];
-                bwd_front<T, VB>(s, sd, factor, pan, X, ldx, rg, nr, v);
-                staged = next;
+template <typename T, int VB, int NSEG, int RB>
+__device__ __forceinline__ void bwd_small(const SubFront &sf, const T *__restrict__ factor,
+                                          const int32_t *__restrict__ struct_rows, int vb_, double *X, int64_t ldx,
+                                          int r0, int nr) {
+    const int lane = threadIdx.x & 31, vb = VB > 0 ? VB : vb_;
+    const int w = sf.w, f = sf.f;
+    const T *pan = factor + sf.pan;
+    const int32_t *rows = struct_rows + sf.rows;
+    double *x = X + r0 * ldx;
+    double v[RB][NSEG], rd[NSEG];                        // x of all rows (own columns: not yet); reciprocal diagonal
+    __syncwarp();                                        // the parent's x (this warp's) is visible
+#pragma unroll
+    for (int g = 0; g < NSEG; ++g) {
+        const int i = lane + 32 * g;
+        rd[g] = i < w ? double(pan[int64_t(i) * sf.ld + i]) : 1.0;
+        int64_t gi = sf.col0 + i;
+        if (i >= w && i < f) {
+            const int li = i - w, b = li / vb;
+            gi = int64_t(rows[b]) * vb + li - b * vb;
+        }
+#pragma unroll
+        for (int r = 0; r < RB; ++r) v[r][g] = i < f && r < nr ? x[gi + r * ldx] : 0.0;
+    }
+#pragma unroll
+    for (int g = 0; g < NSEG; ++g) rd[g] = 1.0 / rd[g];
+    // eight columns at a time, last first: the sums of L(i, j) x_i over the rows below them,
+    // spread over the lanes as they are reduced (each step halves what a lane holds), then
+    // the 8 x 8 triangle, lane k of the eight with column k
+#pragma unroll
+    for (int gb = NSEG - 1; gb >= 0; --gb) {
+        if (32 * gb >= w) continue;
+        for (int jb = (min(32, w - 32 * gb) - 1) & ~7; jb >= 0; jb -= 8) {
+            const int j0 = 32 * gb + jb, nb = min(8, w - j0), below = j0 + nb;
+            const int k = lane - jb;                     // this lane's column of the eight
+            T tri[8];
+#pragma unroll
+            for (int u = 1; u < 8; ++u)
+                tri[u] = k >= 0 && k < u && u < nb ? pan[int64_t(j0 + k) * sf.ld + j0 + u] : T(0);
+            double a[RB][8];
+#pragma unroll
+            for (int r = 0; r < RB; ++r)
+#pragma unroll
+                for (int u = 0; u < 8; ++u) a[r][u] = 0.0;
+#pragma unroll
+            for (int g = gb; g < NSEG; ++g) {
+                const int i = lane + 32 * g;
+                T l[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u)
+                    l[u] = (u < nb && i >= below && i < f) ? pan[int64_t(j0 + u) * sf.ld + i] : T(0);
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    const double lv = double(l[u]);
+#pragma unroll
+                    for (int r = 0; r < RB; ++r) a[r][u] += lv * v[r][g];
+                }
             }
-            asm volatile("cp.async.wait_all;" ::: "memory");
-            __syncthreads();
+#pragma unroll
+            for (int r = 0; r < RB; ++r) {
+#pragma unroll
+                for (int h = 4; h > 0; h >>= 1) {        // lanes' bits 4, 3, 2 choose the column
+                    const bool up = lane & (4 * h);
+#pragma unroll
+                    for (int u = 0; u < h; ++u) {
+                        const double give = up ? a[r][u] : a[r][u + h], keep = up ? a[r][u + h] : a[r][u];
+                        a[r][u] = keep + __shfl_xor_sync(0xffffffffu, give, 4 * h);
+                    }
+                }
+                a[r][0] += __shfl_xor_sync(0xffffffffu, a[r][0], 2);
+                a[r][0] += __shfl_xor_sync(0xffffffffu, a[r][0], 1);
+                const double sum = __shfl_sync(0xffffffffu, a[r][0], (k & 7) * 4);
+                if (k >= 0 && k < nb) v[r][gb] -= sum;
+            }
+#pragma unroll
+            for (int u = 7; u >= 0; --u) {
+                if (u >= nb) continue;
+                const double lv = u > 0 ? double(tri[u]) : 0.0;
+#pragma unroll
+                for (int r = 0; r < RB; ++r) {
+                    const double xj = __shfl_sync(0xffffffffu, v[r][gb] * rd[gb], jb + u);
+                    if (k == u) v[r][gb] = xj;
+                    else v[r][gb] -= lv * xj;            // lv: 0 outside the columns before u
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < RB; ++r) {
+        if (r >= nr) break;
+#pragma unroll
+        for (int g = 0; g < NSEG; ++g) {
+            const int i = lane + 32 * g;
+            if (i < w) x[sf.col0 + i + r * ldx] = v[r][g];
+        }
+    }
+}
+
+// The same, for a small front in a CTA's walk: a call, so that the walk keeps its registers.
+template <typename T, int VB>
+__device__ __noinline__ void fwd_small_call(const SubFront *sf, const T *factor, const SbChild *kids,
+                                            const int32_t *cmap, int vb, double *X, int64_t ldx, int nrhs, int r,
+                                            double *sol) {
+    fwd_small<T, VB, 8, 1>(*sf, factor, kids, cmap, vb, X, ldx, nrhs, r, 1, sol);
+}
+
+template <typename T, int VB>
+__device__ __noinline__ void bwd_small_call(const SubFront *sf, const T *factor, const int32_t *struct_rows, int vb,
+                                            double *X, int64_t ldx, int r) {
+    bwd_small<T, VB, 8, 1>(*sf, factor, struct_rows, vb, X, ldx, r, 1);
+}
+
+// The front's panel into L2, a line a lane.
+template <typename T>
+__device__ __forceinline__ void prefetch_panel(const SubFront &sf, const T *factor) {
+    const char *p = reinterpret_cast<const char *>(factor + sf.pan);
+    const int bytes = sf.ld * sf.w * int(sizeof(T));
+    for (int o = (threadIdx.x & 31) * 128; o < bytes; o += 32 * 128)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(p + o));
+}
+
+// Subtrees of small fronts only: a warp per subtree and RB right-hand sides.
+template <typename T, int VB, int NSEG, int RB>
+__global__ void __launch_bounds__(kSubThreads) subtree_small_fwd_kernel(
+    const int2 *__restrict__ subs, int nsub, SnDev sd, const SubFront *__restrict__ fronts,
+    const SbChild *__restrict__ kids, const int32_t *__restrict__ cmap, const T *__restrict__ factor, double *X, int64_t ldx, int nrhs, double *sol) {
+    const int nwarps = gridDim.x * (kSubThreads / 32), ngr = (nrhs + RB - 1) / RB;
+    for (int q = blockIdx.x * (kSubThreads / 32) + (threadIdx.x >> 5); q < nsub * ngr; q += nwarps) {
+        const int2 sr = subs[q / ngr];
+        const int r0 = q % ngr * RB, nr = min(RB, nrhs - r0);
+        SubFront next = fronts[sr.x];
+        for (int s = sr.x; s <= sr.y; ++s) {
+            const SubFront sf = next;
+            if (s < sr.y) {
+                next = fronts[s + 1];
+                prefetch_panel(next, factor);
+            }
+            if (sf.f <= 64) fwd_small<T, VB, 2, RB>(sf, factor, kids, cmap, sd.vb, X, ldx, nrhs, r0, nr, sol);
+            else fwd_small<T, VB, NSEG, RB>(sf, factor, kids, cmap, sd.vb, X, ldx, nrhs, r0, nr, sol);
+        }
+    }
+}
+
+// The fronts above those: a CTA per subtree of the cut, children first (tops: its fronts,
+// top_ptr[k] to top_ptr[k + 1] in postorder).
+template <typename T, int VB>
+__global__ void __launch_bounds__(kSubThreads, 3) subtree_fwd_kernel(
+    const int32_t *__restrict__ top_ptr, const int32_t *__restrict__ tops, int nsub, SnDev sd,
+    const SubFront *__restrict__ fronts, const SbChild *__restrict__ kids, const int32_t *__restrict__ cmap,
+    const T *__restrict__ factor, double *X, int64_t ldx, int nrhs, double *sol) {
+    extern __shared__ __align__(16) double sub_smem[];
+    double *red = sub_smem, *v = red + kSubRed;
+    const int warp = threadIdx.x >> 5;
+    for (int k = blockIdx.x; k < nsub; k += gridDim.x) {
+        const int t0 = top_ptr[k], t1 = top_ptr[k + 1];
+        for (int t = t0; t < t1; ++t) {
+            const int s = tops[t];
+            __syncthreads();                             // the children's u are there
+            if (fronts[s].inv < 0) {
+                for (int r = warp; r < nrhs; r += kSubThreads / 32)
+                    fwd_small_call<T, VB>(fronts + s, factor, kids, cmap, sd.vb, X, ldx, nrhs, r, sol);
+                continue;
+            }
+            for (int rg = 0; rg < nrhs; rg += kSubRhs)
+                fwd_front<T, VB>(s, sd, factor, factor + fronts[s].pan, X, ldx, nrhs, rg, min(kSubRhs, nrhs - rg), sol,
+                                 v, red);
+        }
+    }
+}
+
+template <typename T, int VB, int NSEG, int RB>
+__global__ void __launch_bounds__(kSubThreads) subtree_small_bwd_kernel(
+    const int2 *__restrict__ subs, int nsub, SnDev sd, const SubFront *__restrict__ fronts,
+    const T *__restrict__ factor, double *X, int64_t ldx, int nrhs) {
+    const int nwarps = gridDim.x * (kSubThreads / 32), ngr = (nrhs + RB - 1) / RB;
+    for (int q = blockIdx.x * (kSubThreads / 32) + (threadIdx.x >> 5); q < nsub * ngr; q += nwarps) {
+        const int2 sr = subs[q / ngr];
+        const int r0 = q % ngr * RB, nr = min(RB, nrhs - r0);
+        SubFront next = fronts[sr.y];
+        for (int s = sr.y; s >= sr.x; --s) {
+            const SubFront sf = next;
+            if (s > sr.x) {
+                next = fronts[s - 1];
+                prefetch_panel(next, factor);
+            }
+            if (sf.f <= 64) bwd_small<T, VB, 2, RB>(sf, factor, sd.struct_rows, sd.vb, X, ldx, r0, nr);
+            else bwd_small<T, VB, NSEG, RB>(sf, factor, sd.struct_rows, sd.vb, X, ldx, r0, nr);
+        }
+    }
+}
+
+// The fronts above those: a CTA per subtree of the cut, parents first (tops: its fronts,
+// top_ptr[k] to top_ptr[k + 1] in postorder).
+template <typename T, int VB>
+__global__ void __launch_bounds__(kSubThreads, 3) subtree_bwd_kernel(
+    const int32_t *__restrict__ top_ptr, const int32_t *__restrict__ tops, int nsub, SnDev sd,
+    const SubFront *__restrict__ fronts,
+    const T *__restrict__ factor, double *X, int64_t ldx, int nrhs) {
+    extern __shared__ __align__(16) double sub_smem[];
+    double *v = sub_smem + kSubRed;
+    const int warp = threadIdx.x >> 5;
+    for (int k = blockIdx.x; k < nsub; k += gridDim.x) {
+        const int t0 = top_ptr[k], t1 = top_ptr[k + 1];
+        for (int t = t1 - 1; t >= t0; --t) {
+            const int s = tops[t];
+            __syncthreads();                             // the parent's x is there
+            if (fronts[s].inv < 0) {
+                for (int r = warp; r < nrhs; r += kSubThreads / 32)
+                    bwd_small_call<T, VB>(fronts + s, factor, sd.struct_rows, sd.vb, X, ldx, r);
+                continue;
+            }
+            for (int rg = 0; rg < nrhs; rg += kSubRhs)
+                bwd_front<T, VB>(s, sd, factor, factor + fronts[s].pan, X, ldx, rg, min(kSubRhs, nrhs - rg), v);
         }
     }
 }
@@ -348,41 +553,76 @@ int sub_sm_count() { return device_sm_count(); }
 
 }  // namespace
 
-size_t subtree_smem_bytes(int fmax) {
-    return size_t(2) * kPanelStageBytes + (size_t(kSubRed) + size_t(kSubRhs) * fmax) * sizeof(double);
+template <typename T>
+void launch_subtree_small(bool forward, const int2 *subs, int nsub, int fmax, SnDev sd, const SubFront *fronts,
+                          const SbChild *kids, const int32_t *cmap, const T *factor, double *X, int64_t ldx, int nrhs,
+                          double *sol, cudaStream_t st) {
+    if (nsub <= 0) return;
+    const int rb = nrhs > 1 ? kSubRhs : 1;
+    const int64_t warps = int64_t(nsub) * ((nrhs + rb - 1) / rb), ctas = (warps + kSubThreads / 32 - 1) / (kSubThreads / 32);
+    const int grid = int(std::min<int64_t>(ctas, 1 << 20));
+    ++g_kernel_launches;
+    auto launch = [&](auto vbc, auto seg, auto rbc) {
+        constexpr int VB = decltype(vbc)::value, NSEG = decltype(seg)::value, RB = decltype(rbc)::value;
+        if (forward)
+            subtree_small_fwd_kernel<T, VB, NSEG, RB>
+                <<<grid, kSubThreads, 0, st>>>(subs, nsub, sd, fronts, kids, cmap, factor, X, ldx, nrhs, sol);
+        else
+            subtree_small_bwd_kernel<T, VB, NSEG, RB>
+                <<<grid, kSubThreads, 0, st>>>(subs, nsub, sd, fronts, factor, X, ldx, nrhs);
+    };
+    auto run = [&](auto vbc, auto seg) {
+        if (nrhs > 1) launch(vbc, seg, std::integral_constant<int, kSubRhs>{});
+        else launch(vbc, seg, std::integral_constant<int, 1>{});
+    };
+    auto by_seg = [&](auto vbc) {                        // rows per lane of the largest front
+        if (fmax <= 96) run(vbc, std::integral_constant<int, 3>{});
+        else if (fmax <= 160) run(vbc, std::integral_constant<int, 5>{});
+        else run(vbc, std::integral_constant<int, 8>{});
+    };
+    if (sd.vb == 3) by_seg(std::integral_constant<int, 3>{});
+    else if (sd.vb == 1) by_seg(std::integral_constant<int, 1>{});
+    else by_seg(std::integral_constant<int, 0>{});
 }
 
 template <typename T>
-void launch_subtree_solve(bool forward, const int2 *subs, int nsub, int fmax, SnDev sd, const T *factor, double *X,
+void launch_subtree_solve(bool forward, const int32_t *top_ptr, const int32_t *tops, int nsub, int fmax, SnDev sd,
+                          const SubFront *fronts, const SbChild *kids, const int32_t *cmap, const T *factor, double *X,
                           int64_t ldx, int nrhs, double *sol, cudaStream_t st) {
     if (nsub <= 0) return;
-    const size_t smem = subtree_smem_bytes(fmax);
-    static PerDeviceOnce once;
-    once([] {
-        cudaFuncSetAttribute(subtree_fwd_kernel<T, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmemOptin);
-        cudaFuncSetAttribute(subtree_fwd_kernel<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmemOptin);
-        cudaFuncSetAttribute(subtree_fwd_kernel<T, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmemOptin);
-        cudaFuncSetAttribute(subtree_bwd_kernel<T, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmemOptin);
-        cudaFuncSetAttribute(subtree_bwd_kernel<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmemOptin);
-        cudaFuncSetAttribute(subtree_bwd_kernel<T, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmemOptin);
-    });
+    const size_t smem = (size_t(kSubRed) + size_t(kSubRhs) * fmax) * sizeof(double);
     const int grid = std::min(nsub, 8 * sub_sm_count());
     ++g_kernel_launches;
-    const int vb = sd.vb;
-    if (forward) {
-        if (vb == 3) subtree_fwd_kernel<T, 3><<<grid, kSubThreads, smem, st>>>(subs, nsub, sd, factor, X, ldx, nrhs, sol);
-        else if (vb == 1) subtree_fwd_kernel<T, 1><<<grid, kSubThreads, smem, st>>>(subs, nsub, sd, factor, X, ldx, nrhs, sol);
-        else subtree_fwd_kernel<T, 0><<<grid, kSubThreads, smem, st>>>(subs, nsub, sd, factor, X, ldx, nrhs, sol);
-    } else {
-        if (vb == 3) subtree_bwd_kernel<T, 3><<<grid, kSubThreads, smem, st>>>(subs, nsub, sd, factor, X, ldx, nrhs);
-        else if (vb == 1) subtree_bwd_kernel<T, 1><<<grid, kSubThreads, smem, st>>>(subs, nsub, sd, factor, X, ldx, nrhs);
-        else subtree_bwd_kernel<T, 0><<<grid, kSubThreads, smem, st>>>(subs, nsub, sd, factor, X, ldx, nrhs);
-    }
+    auto run = [&](auto vbc) {
+        constexpr int VB = decltype(vbc)::value;
+        static PerDeviceOnce once;
+        once([] {
+            cudaFuncSetAttribute(subtree_fwd_kernel<T, VB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 kMaxSmemOptin);
+            cudaFuncSetAttribute(subtree_bwd_kernel<T, VB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 kMaxSmemOptin);
+        });
+        if (forward)
+            subtree_fwd_kernel<T, VB><<<grid, kSubThreads, smem, st>>>(top_ptr, tops, nsub, sd, fronts, kids, cmap,
+                                                                       factor, X, ldx, nrhs, sol);
+        else
+            subtree_bwd_kernel<T, VB>
+                <<<grid, kSubThreads, smem, st>>>(top_ptr, tops, nsub, sd, fronts, factor, X, ldx, nrhs);
+    };
+    if (sd.vb == 3) run(std::integral_constant<int, 3>{});
+    else if (sd.vb == 1) run(std::integral_constant<int, 1>{});
+    else run(std::integral_constant<int, 0>{});
 }
 
-template void launch_subtree_solve<float>(bool, const int2 *, int, int, SnDev, const float *, double *, int64_t, int,
+#define MFS_SUBTREE(T)                                                                                               \
+    template void launch_subtree_small<T>(bool, const int2 *, int, int, SnDev, const SubFront *, const SbChild *,    \
+                                          const int32_t *, const T *, double *, int64_t, int, double *,              \
+                                          cudaStream_t);                                                             \
+    template void launch_subtree_solve<T>(bool, const int32_t *, const int32_t *, int, int, SnDev, const SubFront *, \
+                                          const SbChild *, const int32_t *, const T *, double *, int64_t, int,       \
                                           double *, cudaStream_t);
-template void launch_subtree_solve<double>(bool, const int2 *, int, int, SnDev, const double *, double *, int64_t,
-                                           int, double *, cudaStream_t);
+MFS_SUBTREE(float)
+MFS_SUBTREE(double)
+#undef MFS_SUBTREE
 
 }  // namespace mfs
