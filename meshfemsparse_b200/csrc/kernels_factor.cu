@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(256, MINB)
                 T p = a[u][u];
                 if (!(p > T(0))) p = bad_pivot(p, tk.col0 + k + u, pv, tid == 0);
                 rs[u] = dev_rsqrt(p);
-                a[u][u] = p * rs[u];
+                a[u][u] = rs[u] > T(0) ? p * rs[u] : p;  // (an infinite pivot: L = inf, zeros below)
 #pragma unroll
                 for (int t = u + 1; t < 4; ++t) {
                     a[t][u] *= rs[u];
