@@ -51,6 +51,14 @@ mfs_status mfs_debug_gemm(int32_t device, int32_t precision, int32_t kernel, int
  * *count receives the number of launches; at most max_launches are written. */
 mfs_status mfs_debug_gemm_launches(const mfs_handle *h, int64_t max_launches, double *out, int64_t *count);
 
+/* Adds delta to a count that the solves above the cut wait for: forward, from the
+ * children's structure rows (in every front with a child above the cut); backward, from
+ * the superblocks of the structure rows (in parts; a superblock of at most three parts
+ * is never complete then). With delta 1 a solve's wait runs into its limit (two seconds)
+ * and the solve returns MFS_TIMEOUT; delta -1 puts the counts back. Replaces no reference
+ * entry point: tests make the bounded waits of the solve kernels expire with it. */
+mfs_status mfs_debug_solve_counts(mfs_handle *h, int32_t forward, int32_t delta);
+
 /* The temporal nested-dissection reuse rule on its own (host only, no device): for a
  * previous separator forest (ncomp components, cparent postordered with -1 for roots,
  * cmember[v] the component of vertex v) and a new symmetric graph on the same n

@@ -28,7 +28,7 @@ EXPORTED = [
     "mfs_set_options", "mfs_apply_noalloc", "mfs_lpc_param_count", "mfs_lpc_create", "mfs_lpc_destroy",
     "mfs_lpc_get_weights", "mfs_lpc_set_weights", "mfs_lpc_loss_grad", "mfs_lpc_train_step", "mfs_pcg_solve",
     "mfs_debug_gemm", "mfs_build_pattern_device", "mfs_conversion_plan_device", "mfs_debug_gemm_launches",
-    "mfs_debug_dirty_subtrees", "mfs_debug_hierarchical_order",
+    "mfs_debug_dirty_subtrees", "mfs_debug_hierarchical_order", "mfs_debug_solve_counts",
 ]
 GEMM_TASK_FIELDS = 12
 
@@ -108,6 +108,7 @@ def load() -> C.CDLL:
                                   C.POINTER(C.c_int32)]
     lib.mfs_debug_gemm.argtypes = [C.c_int32, C.c_int32, C.c_int32, C.c_int64, i64p, P, C.c_int64, P, C.c_int64,
                                    P, C.c_int64, C.c_char_p, C.c_size_t]
+    lib.mfs_debug_solve_counts.argtypes = [P, C.c_int32, C.c_int32]
     lib.mfs_debug_gemm_launches.argtypes = [P, C.c_int64, C.POINTER(C.c_double), C.POINTER(C.c_int64)]
     lib.mfs_debug_hierarchical_order.argtypes = [C.c_int64, i64p, i64p, C.c_int64, i64p, i64p, C.c_int32, i64p,
                                                  i64p]

@@ -3,6 +3,7 @@
 // host before the launch.
 #include "../../include/mfs_b200_testing.h"
 #include "device.h"
+#include "handle.h"
 #include "host_symbolic.h"
 
 #include <cuda_runtime.h>
@@ -337,4 +338,21 @@ extern "C" mfs_status mfs_debug_hierarchical_order(int64_t n, const int64_t *xad
     } catch (const std::bad_alloc &) {
         return MFS_OOM;
     }
+}
+
+extern "C" mfs_status mfs_debug_solve_counts(mfs_handle *h, int32_t forward, int32_t delta) {
+    if (!h || !h->cur.sym) return MFS_INVALID_ARG;
+    DevSym &ds = *h->cur.sym;
+    if (cudaSetDevice(h->opt.device) != cudaSuccess || cudaStreamSynchronize(h->stream) != cudaSuccess)
+        return MFS_CUDA_ERROR;
+    auto change = [&](auto &buf, auto &&fn) {
+        std::vector<std::remove_reference_t<decltype(*buf.p)>> v(buf.n);
+        if (v.empty()) return true;
+        if (cudaMemcpy(v.data(), buf.p, buf.bytes(), cudaMemcpyDeviceToHost) != cudaSuccess) return false;
+        for (auto &e : v) fn(e);
+        return cudaMemcpy(buf.p, v.data(), buf.bytes(), cudaMemcpyHostToDevice) == cudaSuccess;
+    };
+    const bool ok = forward ? change(ds.sb_children, [&](SbChild &c) { c.need += delta; })
+                            : change(ds.rowcnt, [&](int32_t &c) { c += delta; });
+    return ok ? MFS_OK : MFS_CUDA_ERROR;
 }

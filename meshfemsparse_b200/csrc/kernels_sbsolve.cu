@@ -45,7 +45,7 @@
 //   vector warps  wait for the counts and bring y_J / x_J / x_struct, 256 rows at a time,
 //                 into VS buffers;
 //   gather warps  v of every task's own rows (forward: the children's counts, their row
-//                 maps, their u) and its sizes;
+//                 maps, their u);
 //   count warp    publishes a structure task's results once all product warps have handed
 //                 them over.
 // Structure rows start at w rounded down to a multiple of 4 (TMA boxes start 16-byte
@@ -58,8 +58,10 @@
 // the lowest unfinished task can always proceed. Counts are zeroed before each
 // solve: forward targets are eight (warps) times the superblock's part count, backward
 // ones twice that. Waits are bounded in time: on expiry the kernel records an error and
-// stops waiting; the host reports MFS_TIMEOUT. Sums run in a fixed order, so
-// results are run-to-run identical. With an FP32 factor (the preconditioner of
+// stops waiting; the host reports MFS_TIMEOUT. What a warp does and where it stores follows
+// from the task list alone, never from what a wait was for, so that after an expiry only
+// values are wrong; the product warps of a launch after one return at once. Sums run in a fixed
+// order, so results are run-to-run identical. With an FP32 factor (the preconditioner of
 // FP64 refinement) the products are FP32, summed in FP32 over at most 256 columns
 // (forward) / 1024 rows (backward) and beyond that in FP64, and the inverse of the
 // diagonal superblock is applied in FP64; an FP64 factor keeps FP64 throughout.
@@ -164,8 +166,20 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int *er
         }
     }
 }
-// The product warps' barrier.
+// The product warps' barrier, and one that tells all of them whether any thread says so.
 __device__ __forceinline__ void psync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+__device__ __forceinline__ bool psync_or(int pred) {
+    int any;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.s32 p, %1, 0;\n\t"
+        "bar.red.or.pred q, 1, 256, p;\n\t"
+        "selp.s32 %0, 1, 0, q;\n\t}"
+        : "=r"(any)
+        : "r"(pred)
+        : "memory");
+    return any != 0;
+}
 // 2D tiled TMA load of one box of the tensor map at `map` (device memory written
 // before the launch), box origin (x = row, y = column), completing on `bar`.
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const char *map, int x, int y, uint32_t bar) {
@@ -352,6 +366,19 @@ __device__ __forceinline__ SpRing init_bars(SpBars<NST, VS, OS> &b) {
     return rg;
 }
 
+// The product warps' tasks, by the last two bits of their number: four threads copy a task
+// two ahead of its use, and a product barrier of the task in between makes it visible.
+static_assert(sizeof(SbTask) == 64, "a task is four 16-byte copies");
+__device__ __forceinline__ void fetch_task(SbTask (&meta)[4], int it, const SbTask *tasks, int t, int ntasks, int tid) {
+    if (tid < 4 && t < ntasks)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(smem_u32(&meta[it & 3]) + 16 * tid),
+                     "l"(reinterpret_cast<const char *>(tasks + t) + 16 * tid)
+                     : "memory");
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+// (all but the newest copy have landed)
+__device__ __forceinline__ void task_landed() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
+
 // What a task streams. Forward: ndep chunks of earlier superblocks (diagonal tasks) or
 // of the whole width (structure tasks, K < 0), then ninv chunks of the inverse.
 template <typename T>
@@ -409,7 +436,11 @@ __device__ __forceinline__ void copy_chunks(const SbTask *tasks, int ntasks, con
     bool ok = true;
     auto load = [&](const char *map, int x, int y) {
         const int slot = int(gq % NST);
-        if (gq >= NST && !mbar_wait(rg.empty + 8 * slot, uint32_t((gq / NST) - 1) & 1u, err)) ok = false;
+        // its last copy has landed (warps whose waits have expired hand slots back before
+        // that, and a barrier takes one copy at a time), and it is read
+        const uint32_t before = uint32_t((gq / NST) - 1) & 1u;
+        if (gq >= NST && !(mbar_wait(rg.full + 8 * slot, before, err) && mbar_wait(rg.empty + 8 * slot, before, err)))
+            ok = false;
         if (!ok) return;
         mbar_expect_tx(rg.full + 8 * slot, SpChunk<T>::BYTES);
         tma_load_2d(smem_u32(ring + slot * CE), map, x, y, rg.full + 8 * slot);
@@ -604,7 +635,7 @@ __device__ __forceinline__ void bwd_vectors(const SbTask *tasks, int ntasks, con
 template <int NR, bool FWD>
 __device__ __forceinline__ void gather_own(const SbTask *tasks, int ntasks, int vb, const SbChild *children,
                                            const int32_t *cmap, const double *X, int64_t ldx, int nrhs,
-                                           const double *sol, SbTask *meta, double *own, const SpRing &rg,
+                                           const double *sol, double *own, const SpRing &rg,
                                            const int *flags, int *err, int me) {
     constexpr int OS = own_slots(NR);
     const int lane = threadIdx.x & 31;
@@ -687,7 +718,6 @@ __device__ __forceinline__ void gather_own(const SbTask *tasks, int ntasks, int 
         for (int e = 0; e < 2; ++e)
 #pragma unroll
             for (int r = 0; r < NR; ++r) o[r * 64 + lane + 32 * e] = v[e][r];
-        if (lane == 0) meta[slot] = tk;
         mbar_arrive(rg.ofull + 8 * slot);
     }
 }
@@ -704,7 +734,7 @@ __global__ void __launch_bounds__(kSbThreads, 1)
     extern __shared__ __align__(128) unsigned char sp_dyn[];
     constexpr int OS = own_slots(NR);
     __shared__ __align__(8) SpBars<NST, VS, OS> bars;
-    __shared__ SbTask meta[OS];
+    __shared__ __align__(16) SbTask meta[4];
     // TMA destinations: 128-byte aligned (the launch adds 128 bytes for this)
     unsigned char *sp_raw = sp_dyn + ((128u - (smem_u32(sp_dyn) & 127u)) & 127u);
     T *ring = reinterpret_cast<T *>(sp_raw);
@@ -712,8 +742,11 @@ __global__ void __launch_bounds__(kSbThreads, 1)
     double *red = reinterpret_cast<double *>(sp_raw + Lay::red_off);
     double *vec = red;
     double *owns = reinterpret_cast<double *>(sp_raw + Lay::own_off);
-    const SpRing rg = init_bars(bars);
     const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
+    const int expired = tid == 0 ? *(volatile int *)err : 0;   // a wait of an earlier launch
+    fetch_task(meta, 0, tasks, blockIdx.x, ntasks, tid);
+    fetch_task(meta, 1, tasks, blockIdx.x + gridDim.x, ntasks, tid);
+    const SpRing rg = init_bars(bars);
     if (wp == 8) {
         if (lane == 0) copy_chunks<T, NST, true>(tasks, ntasks, maps, ring, rg, err);
         return;
@@ -727,10 +760,12 @@ __global__ void __launch_bounds__(kSbThreads, 1)
         return;
     }
     if (wp > 8) {
-        gather_own<NR, true>(tasks, ntasks, sd.vb, children, cmap, X, ldx, nrhs, sol, meta, owns, rg, flags, err,
-                                wp - 9 - kVecWarps);
+        gather_own<NR, true>(tasks, ntasks, sd.vb, children, cmap, X, ldx, nrhs, sol, owns, rg, flags, err,
+                              wp - 9 - kVecWarps);
         return;
     }
+    task_landed();
+    if (psync_or(expired)) return;                       // (the other warps' waits end too)
     const int i = tid & 63, part = tid >> 6;             // combining thread: row i, right-hand sides part + 4 o
     long long gq = 0, gv = 0;
     Handover handover{rg, err};
@@ -764,8 +799,9 @@ __global__ void __launch_bounds__(kSbThreads, 1)
     int it = 0;
     for (int t = blockIdx.x; t < ntasks; t += gridDim.x, ++it) {
         const int os = it % OS;
+        fetch_task(meta, it + 2, tasks, t + 2 * gridDim.x, ntasks, tid);
+        const SbTask tk = meta[it & 3];
         mbar_wait(rg.ofull + 8 * os, uint32_t(it / OS) & 1u, err);
-        const SbTask tk = meta[os];
         const int c0 = tk.c0;
         const FwdShape<T> sh(tk);
         const int w = sh.w, K = tk.K;
@@ -799,6 +835,7 @@ __global__ void __launch_bounds__(kSbThreads, 1)
                 dacc[1][r] += double(pacc[1][r]);
             }
         }
+        task_landed();
         double sum[NO];
         combine(dacc, sum);
         if (K < 0) {
@@ -865,14 +902,17 @@ __global__ void __launch_bounds__(kSbThreads, 1)
     extern __shared__ __align__(128) unsigned char sp_dyn[];
     constexpr int OS = own_slots(NR);
     __shared__ __align__(8) SpBars<NST, VS, OS> bars;
-    __shared__ SbTask meta[OS];
+    __shared__ __align__(16) SbTask meta[4];
     unsigned char *sp_raw = sp_dyn + ((128u - (smem_u32(sp_dyn) & 127u)) & 127u);
     T *ring = reinterpret_cast<T *>(sp_raw);
     P *vp = reinterpret_cast<P *>(sp_raw + Lay::vp_off);
     double *vec = reinterpret_cast<double *>(sp_raw + Lay::red_off);   // a_K, [r][SB]
     double *owns = reinterpret_cast<double *>(sp_raw + Lay::own_off);
-    const SpRing rg = init_bars(bars);
     const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
+    const int expired = tid == 0 ? *(volatile int *)err : 0;   // a wait of an earlier launch
+    fetch_task(meta, 0, tasks, blockIdx.x, ntasks, tid);
+    fetch_task(meta, 1, tasks, blockIdx.x + gridDim.x, ntasks, tid);
+    const SpRing rg = init_bars(bars);
     if (wp == 8) {
         if (lane == 0) copy_chunks<T, NST, false>(tasks, ntasks, maps, ring, rg, err);
         return;
@@ -883,10 +923,12 @@ __global__ void __launch_bounds__(kSbThreads, 1)
     }
     if (wp == 9 + kVecWarps + kGatherWarps) return;      // (forward only)
     if (wp > 8) {
-        gather_own<NR, false>(tasks, ntasks, sd.vb, children, nullptr, X, ldx, nrhs, sol, meta, owns, rg, flags, err,
-                                 wp - 9 - kVecWarps);
+        gather_own<NR, false>(tasks, ntasks, sd.vb, children, nullptr, X, ldx, nrhs, sol, owns, rg, flags, err,
+                               wp - 9 - kVecWarps);
         return;
     }
+    task_landed();
+    if (psync_or(expired)) return;                       // (the other warps' waits end too)
     long long gq = 0, gv = 0;
     auto chunk = [&]() -> const T * {
         const int slot = int(gq % NST);
@@ -910,8 +952,9 @@ __global__ void __launch_bounds__(kSbThreads, 1)
     int it = 0;
     for (int t = blockIdx.x; t < ntasks; t += gridDim.x, ++it) {
         const int os = it % OS;
+        fetch_task(meta, it + 2, tasks, t + 2 * gridDim.x, ntasks, tid);
+        const SbTask tk = meta[it & 3];
         mbar_wait(rg.ofull + 8 * os, uint32_t(it / OS) & 1u, err);
-        const SbTask tk = meta[os];
         const int c0 = tk.c0, K = tk.K;
         const BwdShape<T> sh(tk);
         const int w = sh.w;
@@ -953,6 +996,7 @@ __global__ void __launch_bounds__(kSbThreads, 1)
             if (lane == 0) mbar_arrive(rg.vempty + 8 * slot);   // (after release's __syncwarp)
         }
         if (held > 0) flush();
+        task_landed();
         // a_h; exchanged with the other parts of K through the scratch vector
         if (nhK > 1) {
 #pragma unroll
