@@ -34,11 +34,14 @@ constexpr int kSubThreads = 256;
 constexpr int kSubRhs = 4;                 // right-hand sides per pass or warp (more are looped)
 constexpr int kSubRed = 4 * kSubRhs * 64;  // split-k partials of a 64-row block
 
-template <int VB>
-__device__ __forceinline__ int crel(const int32_t *rel, int i, int vb) {
-    if constexpr (VB > 0) return rel[i / VB] + i % VB;
-    return rel[i / vb] + i % vb;
-}
+// Division by the block size as a product: exact for rows of a front below the cut (at most
+// 2048 of them, so at most 2048 a block).
+struct BlockDiv {
+    int vb;
+    uint32_t m;                            // ceil(2^26 / vb)
+    explicit BlockDiv(int v) : vb(v), m(((1u << 26) + uint32_t(v) - 1) / uint32_t(v)) {}
+    __device__ __forceinline__ int operator()(int i) const { return int((uint64_t(uint32_t(i)) * m) >> 26); }
+};
 
 __device__ __forceinline__ double warp_sum(double x) {
 #pragma unroll
@@ -48,9 +51,9 @@ __device__ __forceinline__ double warp_sum(double x) {
 
 // ------------------------------------------------------------------ forward
 // A front with stored inverses, the whole CTA.
-template <typename T, int VB>
-__device__ __forceinline__ void fwd_front(int s, const SnDev &sd, const T *__restrict__ factor, const T *pan,
-                                          double *__restrict__ X, int64_t ldx, int nrhs, int rg, int nr,
+template <typename T>
+__device__ __forceinline__ void fwd_front(int s, const SnDev &sd, BlockDiv div, const T *__restrict__ factor,
+                                          const T *pan, double *__restrict__ X, int64_t ldx, int nrhs, int rg, int nr,
                                           double *__restrict__ sol, double *v, double *red) {
     const int tid = threadIdx.x, nt = blockDim.x;
     const int w = sd.w[s], d = sd.d[s], f = w + d, c0 = sd.col0[s], ld = sd.ld[s];
@@ -66,8 +69,8 @@ __device__ __forceinline__ void fwd_front(int s, const SnDev &sd, const T *__res
         const int32_t *rel = sd.rel + sd.struct_ptr[c];
         const double *uc = sol + sd.sol_off[c] * nrhs;
         for (int q = tid; q < nr * dc; q += nt) {
-            const int r = q / dc, i = q - r * dc;
-            v[r * f + crel<VB>(rel, i, sd.vb)] += uc[i + int64_t(rg + r) * dc];
+            const int r = q / dc, i = q - r * dc, b = div(i);
+            v[r * f + rel[b] + i - b * div.vb] += uc[i + int64_t(rg + r) * dc];
         }
         __syncthreads();
     }
@@ -146,20 +149,20 @@ __device__ __forceinline__ void fwd_front(int s, const SnDev &sd, const T *__res
 }
 
 // ------------------------------------------------------------------ backward
-template <typename T, int VB>
-__device__ __forceinline__ void bwd_front(int s, const SnDev &sd, const T *__restrict__ factor, const T *pan,
-                                          double *__restrict__ X, int64_t ldx, int rg, int nr, double *v) {
+template <typename T>
+__device__ __forceinline__ void bwd_front(int s, const SnDev &sd, BlockDiv div, const T *__restrict__ factor,
+                                          const T *pan, double *__restrict__ X, int64_t ldx, int rg, int nr,
+                                          double *v) {
     const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
     const int w = sd.w[s], d = sd.d[s], f = w + d, c0 = sd.col0[s], ld = sd.ld[s];
     const int32_t *rows = sd.struct_rows + sd.struct_ptr[s];
-    const int vb = sd.vb;
     for (int q = tid; q < nr * f; q += nt) {
         const int r = q / f, i = q - r * f;
         int64_t gi;
         if (i < w) gi = c0 + i;
         else {
-            const int li = i - w;
-            gi = int64_t(rows[li / (VB > 0 ? VB : vb)]) * (VB > 0 ? VB : vb) + li % (VB > 0 ? VB : vb);
+            const int li = i - w, b = div(li);
+            gi = int64_t(rows[b]) * div.vb + li - b * div.vb;
         }
         v[q] = X[gi + int64_t(rg + r) * ldx];
     }
@@ -245,21 +248,26 @@ __device__ __forceinline__ void bwd_front(int s, const SnDev &sd, const T *__res
 }
 
 // ------------------------------------------------------------------ small fronts, one warp
-// NSEG x 32 rows at least the front's; right-hand sides r0 to r0 + nr - 1, at most RB.
-template <typename T, int VB, int NSEG, int RB>
+// NSEG x 32 rows at least the front's; right-hand sides r0 to r0 + nr - 1, at most RB. A lane
+// holds the rows from the 32 columns under way on (v[r][g]: row jb + lane + 32 g), moved by
+// one entry from one such block of columns to the next, so that the loop over the blocks
+// is rolled: unrolled, with the block sizes 1 and 3 as template parameters, this file took
+// 674 s to compile and half of the object code was never run.
+template <typename T, int NSEG, int RB>
 __device__ __forceinline__ void fwd_small(const SubFront &sf, const T *__restrict__ factor,
-                                          const SbChild *__restrict__ kids, const int32_t *__restrict__ cmap, int vb_,
-                                          double *X, int64_t ldx, int nrhs, int r0, int nr, double *sol) {
-    const int lane = threadIdx.x & 31, vb = VB > 0 ? VB : vb_;
+                                          const SbChild *__restrict__ kids, const int32_t *__restrict__ cmap,
+                                          BlockDiv div, double *X, int64_t ldx, int nrhs, int r0, int nr, double *sol) {
+    const int lane = threadIdx.x & 31;
     const int w = sf.w, f = sf.f;
     const T *pan = factor + sf.pan;
     double *x = X + sf.col0 + r0 * ldx;
-    double v[RB][NSEG], rd[NSEG];
+    auto diagonal = [&](int i) { return i < w ? double(pan[int64_t(i) * sf.ld + i]) : 1.0; };
+    double v[RB][NSEG];
     __syncwarp();                                        // the children's u (this warp's) are visible
+    double d = diagonal(lane);
 #pragma unroll
     for (int g = 0; g < NSEG; ++g) {
         const int i = lane + 32 * g;
-        rd[g] = i < w ? double(pan[int64_t(i) * sf.ld + i]) : 1.0;
 #pragma unroll
         for (int r = 0; r < RB; ++r) v[r][g] = i < w && r < nr ? x[i + r * ldx] : 0.0;
     }
@@ -269,11 +277,11 @@ __device__ __forceinline__ void fwd_small(const SubFront &sf, const T *__restric
         int m[NSEG];
 #pragma unroll
         for (int g = 0; g < NSEG; ++g) {
-            const int i = lane + 32 * g, b = i / vb;
+            const int i = lane + 32 * g, b = div(i);
             m[g] = -1;
             if (i < f) {
                 const int k = cmap[ch.map + b];
-                if (k >= 0) m[g] = k * vb + i - b * vb;
+                if (k >= 0) m[g] = (k - b) * div.vb + i;
             }
         }
         double a[RB][NSEG];
@@ -286,20 +294,21 @@ __device__ __forceinline__ void fwd_small(const SubFront &sf, const T *__restric
 #pragma unroll
             for (int g = 0; g < NSEG; ++g) v[r][g] += a[r][g];
     }
-#pragma unroll
-    for (int g = 0; g < NSEG; ++g) rd[g] = 1.0 / rd[g];
-#pragma unroll
-    for (int gb = 0; gb < NSEG; ++gb) {
-        if (32 * gb >= w) break;
-        const int je = min(32, w - 32 * gb);
+    int jb = 0;
+#pragma unroll 1
+    for (;; jb += 32) {
+        const double rd = 1.0 / d;
+        d = diagonal(jb + 32 + lane);
+        const int je = min(32, w - jb);
+#pragma unroll 1
         for (int j0 = 0; j0 < je; j0 += 4) {
             // four columns of L ahead of their use
             T l[4][NSEG];
 #pragma unroll
             for (int u = 0; u < 4; ++u)
 #pragma unroll
-                for (int g = gb; g < NSEG; ++g) {
-                    const int i = lane + 32 * g, j = 32 * gb + j0 + u;
+                for (int g = 0; g < NSEG; ++g) {
+                    const int i = jb + lane + 32 * g, j = jb + j0 + u;
                     l[u][g] = (j0 + u < je && i > j && i < f) ? pan[int64_t(j) * sf.ld + i] : T(0);
                 }
 #pragma unroll
@@ -307,17 +316,25 @@ __device__ __forceinline__ void fwd_small(const SubFront &sf, const T *__restric
                 if (j0 + u >= je) break;
                 double y[RB];
 #pragma unroll
-                for (int r = 0; r < RB; ++r) y[r] = __shfl_sync(0xffffffffu, v[r][gb] * rd[gb], j0 + u);
+                for (int r = 0; r < RB; ++r) y[r] = __shfl_sync(0xffffffffu, v[r][0] * rd, j0 + u);
                 if (lane == j0 + u)
 #pragma unroll
-                    for (int r = 0; r < RB; ++r) v[r][gb] = y[r];
+                    for (int r = 0; r < RB; ++r) v[r][0] = y[r];
 #pragma unroll
-                for (int g = gb; g < NSEG; ++g) {
+                for (int g = 0; g < NSEG; ++g) {
                     const double lv = double(l[u][g]);
 #pragma unroll
                     for (int r = 0; r < RB; ++r) v[r][g] -= lv * y[r];
                 }
             }
+        }
+        if (jb + 32 >= w) break;
+#pragma unroll
+        for (int r = 0; r < RB; ++r) {
+            if (r < nr) x[jb + lane + r * ldx] = v[r][0];
+#pragma unroll
+            for (int g = 0; g + 1 < NSEG; ++g) v[r][g] = v[r][g + 1];
+            v[r][NSEG - 1] = 0.0;
         }
     }
     double *us = sf.sol >= 0 ? sol + sf.sol * nrhs + int64_t(r0) * (f - w) : nullptr;
@@ -326,47 +343,53 @@ __device__ __forceinline__ void fwd_small(const SubFront &sf, const T *__restric
         if (r >= nr) break;
 #pragma unroll
         for (int g = 0; g < NSEG; ++g) {
-            const int i = lane + 32 * g;
+            const int i = jb + lane + 32 * g;
             if (i < w) x[i + r * ldx] = v[r][g];
             else if (i < f && us) us[i - w + r * int64_t(f - w)] = v[r][g];
         }
     }
 }
 
-template <typename T, int VB, int NSEG, int RB>
+template <typename T, int NSEG, int RB>
 __device__ __forceinline__ void bwd_small(const SubFront &sf, const T *__restrict__ factor,
-                                          const int32_t *__restrict__ struct_rows, int vb_, double *X, int64_t ldx,
+                                          const int32_t *__restrict__ struct_rows, BlockDiv div, double *X, int64_t ldx,
                                           int r0, int nr) {
-    const int lane = threadIdx.x & 31, vb = VB > 0 ? VB : vb_;
-    const int w = sf.w, f = sf.f;
+    const int lane = threadIdx.x & 31;
+    const int w = sf.w, f = sf.f, wb = div(w);
     const T *pan = factor + sf.pan;
-    const int32_t *rows = struct_rows + sf.rows;
+    const int32_t *rows = struct_rows + sf.rows - wb;
     double *x = X + r0 * ldx;
-    double v[RB][NSEG], rd[NSEG];                        // x of all rows (own columns: not yet); reciprocal diagonal
+    auto diagonal = [&](int i) { return i < w ? double(pan[int64_t(i) * sf.ld + i]) : 1.0; };
+    double v[RB][NSEG];                                  // x of the rows (own columns: not yet)
     __syncwarp();                                        // the parent's x (this warp's) is visible
+    int jb = (w - 1) & ~31;
+    double d = diagonal(jb + lane);
 #pragma unroll
     for (int g = 0; g < NSEG; ++g) {
-        const int i = lane + 32 * g;
-        rd[g] = i < w ? double(pan[int64_t(i) * sf.ld + i]) : 1.0;
+        const int i = jb + lane + 32 * g;
         int64_t gi = sf.col0 + i;
         if (i >= w && i < f) {
-            const int li = i - w, b = li / vb;
-            gi = int64_t(rows[b]) * vb + li - b * vb;
+            const int b = div(i);
+            gi = int64_t(rows[b]) * div.vb + i - b * div.vb;
         }
 #pragma unroll
         for (int r = 0; r < RB; ++r) v[r][g] = i < f && r < nr ? x[gi + r * ldx] : 0.0;
     }
+    // the blocks of 32 columns, last first; in each, eight columns at a time, last first: the
+    // sums of L(i, j) x_i over the rows below them, spread over the lanes as they are
+    // reduced (each step halves what a lane holds), then the 8 x 8 triangle, lane k of the
+    // eight with column k
+#pragma unroll 1
+    for (;; jb -= 32) {
+        const double rd = 1.0 / d;
+        double vn[RB];                                   // the rows of the next block of columns
 #pragma unroll
-    for (int g = 0; g < NSEG; ++g) rd[g] = 1.0 / rd[g];
-    // eight columns at a time, last first: the sums of L(i, j) x_i over the rows below them,
-    // spread over the lanes as they are reduced (each step halves what a lane holds), then
-    // the 8 x 8 triangle, lane k of the eight with column k
-#pragma unroll
-    for (int gb = NSEG - 1; gb >= 0; --gb) {
-        if (32 * gb >= w) continue;
-        for (int jb = (min(32, w - 32 * gb) - 1) & ~7; jb >= 0; jb -= 8) {
-            const int j0 = 32 * gb + jb, nb = min(8, w - j0), below = j0 + nb;
-            const int k = lane - jb;                     // this lane's column of the eight
+        for (int r = 0; r < RB; ++r) vn[r] = jb > 0 && r < nr ? x[sf.col0 + jb - 32 + lane + r * ldx] : 0.0;
+        if (jb > 0) d = diagonal(jb - 32 + lane);
+#pragma unroll 1
+        for (int c0 = (min(32, w - jb) - 1) & ~7; c0 >= 0; c0 -= 8) {
+            const int j0 = jb + c0, nb = min(8, w - j0), below = j0 + nb;
+            const int k = lane - c0;                     // this lane's column of the eight
             T tri[8];
 #pragma unroll
             for (int u = 1; u < 8; ++u)
@@ -377,8 +400,8 @@ __device__ __forceinline__ void bwd_small(const SubFront &sf, const T *__restric
 #pragma unroll
                 for (int u = 0; u < 8; ++u) a[r][u] = 0.0;
 #pragma unroll
-            for (int g = gb; g < NSEG; ++g) {
-                const int i = lane + 32 * g;
+            for (int g = 0; g < NSEG; ++g) {
+                const int i = jb + lane + 32 * g;
                 T l[8];
 #pragma unroll
                 for (int u = 0; u < 8; ++u)
@@ -404,7 +427,7 @@ __device__ __forceinline__ void bwd_small(const SubFront &sf, const T *__restric
                 a[r][0] += __shfl_xor_sync(0xffffffffu, a[r][0], 2);
                 a[r][0] += __shfl_xor_sync(0xffffffffu, a[r][0], 1);
                 const double sum = __shfl_sync(0xffffffffu, a[r][0], (k & 7) * 4);
-                if (k >= 0 && k < nb) v[r][gb] -= sum;
+                if (k >= 0 && k < nb) v[r][0] -= sum;
             }
 #pragma unroll
             for (int u = 7; u >= 0; --u) {
@@ -412,36 +435,38 @@ __device__ __forceinline__ void bwd_small(const SubFront &sf, const T *__restric
                 const double lv = u > 0 ? double(tri[u]) : 0.0;
 #pragma unroll
                 for (int r = 0; r < RB; ++r) {
-                    const double xj = __shfl_sync(0xffffffffu, v[r][gb] * rd[gb], jb + u);
-                    if (k == u) v[r][gb] = xj;
-                    else v[r][gb] -= lv * xj;            // lv: 0 outside the columns before u
+                    const double xj = __shfl_sync(0xffffffffu, v[r][0] * rd, c0 + u);
+                    if (k == u) v[r][0] = xj;
+                    else v[r][0] -= lv * xj;             // lv: 0 outside the columns before u
                 }
             }
         }
-    }
+        if (jb + lane < w)
 #pragma unroll
-    for (int r = 0; r < RB; ++r) {
-        if (r >= nr) break;
+            for (int r = 0; r < RB; ++r)
+                if (r < nr) x[sf.col0 + jb + lane + r * ldx] = v[r][0];
+        if (jb == 0) break;
 #pragma unroll
-        for (int g = 0; g < NSEG; ++g) {
-            const int i = lane + 32 * g;
-            if (i < w) x[sf.col0 + i + r * ldx] = v[r][g];
+        for (int r = 0; r < RB; ++r) {
+#pragma unroll
+            for (int g = NSEG - 1; g > 0; --g) v[r][g] = v[r][g - 1];
+            v[r][0] = vn[r];
         }
     }
 }
 
 // The same, for a small front in a CTA's walk: a call, so that the walk keeps its registers.
-template <typename T, int VB>
+template <typename T>
 __device__ __noinline__ void fwd_small_call(const SubFront *sf, const T *factor, const SbChild *kids,
-                                            const int32_t *cmap, int vb, double *X, int64_t ldx, int nrhs, int r,
-                                            double *sol) {
-    fwd_small<T, VB, 8, 1>(*sf, factor, kids, cmap, vb, X, ldx, nrhs, r, 1, sol);
+                                            const int32_t *cmap, BlockDiv div, double *X, int64_t ldx, int nrhs,
+                                            int r, double *sol) {
+    fwd_small<T, 8, 1>(*sf, factor, kids, cmap, div, X, ldx, nrhs, r, 1, sol);
 }
 
-template <typename T, int VB>
-__device__ __noinline__ void bwd_small_call(const SubFront *sf, const T *factor, const int32_t *struct_rows, int vb,
-                                            double *X, int64_t ldx, int r) {
-    bwd_small<T, VB, 8, 1>(*sf, factor, struct_rows, vb, X, ldx, r, 1);
+template <typename T>
+__device__ __noinline__ void bwd_small_call(const SubFront *sf, const T *factor, const int32_t *struct_rows,
+                                            BlockDiv div, double *X, int64_t ldx, int r) {
+    bwd_small<T, 8, 1>(*sf, factor, struct_rows, div, X, ldx, r, 1);
 }
 
 // The front's panel into L2, a line a lane.
@@ -454,10 +479,11 @@ __device__ __forceinline__ void prefetch_panel(const SubFront &sf, const T *fact
 }
 
 // Subtrees of small fronts only: a warp per subtree and RB right-hand sides.
-template <typename T, int VB, int NSEG, int RB>
+template <typename T, int NSEG, int RB>
 __global__ void __launch_bounds__(kSubThreads) subtree_small_fwd_kernel(
-    const int2 *__restrict__ subs, int nsub, SnDev sd, const SubFront *__restrict__ fronts,
-    const SbChild *__restrict__ kids, const int32_t *__restrict__ cmap, const T *__restrict__ factor, double *X, int64_t ldx, int nrhs, double *sol) {
+    const int2 *__restrict__ subs, int nsub, BlockDiv div, const SubFront *__restrict__ fronts,
+    const SbChild *__restrict__ kids, const int32_t *__restrict__ cmap, const T *__restrict__ factor, double *X,
+    int64_t ldx, int nrhs, double *sol) {
     const int nwarps = gridDim.x * (kSubThreads / 32), ngr = (nrhs + RB - 1) / RB;
     for (int q = blockIdx.x * (kSubThreads / 32) + (threadIdx.x >> 5); q < nsub * ngr; q += nwarps) {
         const int2 sr = subs[q / ngr];
@@ -469,17 +495,17 @@ __global__ void __launch_bounds__(kSubThreads) subtree_small_fwd_kernel(
                 next = fronts[s + 1];
                 prefetch_panel(next, factor);
             }
-            if (sf.f <= 64) fwd_small<T, VB, 2, RB>(sf, factor, kids, cmap, sd.vb, X, ldx, nrhs, r0, nr, sol);
-            else fwd_small<T, VB, NSEG, RB>(sf, factor, kids, cmap, sd.vb, X, ldx, nrhs, r0, nr, sol);
+            if (sf.f <= 64) fwd_small<T, 2, RB>(sf, factor, kids, cmap, div, X, ldx, nrhs, r0, nr, sol);
+            else fwd_small<T, NSEG, RB>(sf, factor, kids, cmap, div, X, ldx, nrhs, r0, nr, sol);
         }
     }
 }
 
 // The fronts above those: a CTA per subtree of the cut, children first (tops: its fronts,
 // top_ptr[k] to top_ptr[k + 1] in postorder).
-template <typename T, int VB>
+template <typename T>
 __global__ void __launch_bounds__(kSubThreads, 3) subtree_fwd_kernel(
-    const int32_t *__restrict__ top_ptr, const int32_t *__restrict__ tops, int nsub, SnDev sd,
+    const int32_t *__restrict__ top_ptr, const int32_t *__restrict__ tops, int nsub, SnDev sd, BlockDiv div,
     const SubFront *__restrict__ fronts, const SbChild *__restrict__ kids, const int32_t *__restrict__ cmap,
     const T *__restrict__ factor, double *X, int64_t ldx, int nrhs, double *sol) {
     extern __shared__ __align__(16) double sub_smem[];
@@ -492,20 +518,20 @@ __global__ void __launch_bounds__(kSubThreads, 3) subtree_fwd_kernel(
             __syncthreads();                             // the children's u are there
             if (fronts[s].inv < 0) {
                 for (int r = warp; r < nrhs; r += kSubThreads / 32)
-                    fwd_small_call<T, VB>(fronts + s, factor, kids, cmap, sd.vb, X, ldx, nrhs, r, sol);
+                    fwd_small_call<T>(fronts + s, factor, kids, cmap, div, X, ldx, nrhs, r, sol);
                 continue;
             }
             for (int rg = 0; rg < nrhs; rg += kSubRhs)
-                fwd_front<T, VB>(s, sd, factor, factor + fronts[s].pan, X, ldx, nrhs, rg, min(kSubRhs, nrhs - rg), sol,
-                                 v, red);
+                fwd_front<T>(s, sd, div, factor, factor + fronts[s].pan, X, ldx, nrhs, rg, min(kSubRhs, nrhs - rg), sol,
+                             v, red);
         }
     }
 }
 
-template <typename T, int VB, int NSEG, int RB>
+template <typename T, int NSEG, int RB>
 __global__ void __launch_bounds__(kSubThreads) subtree_small_bwd_kernel(
-    const int2 *__restrict__ subs, int nsub, SnDev sd, const SubFront *__restrict__ fronts,
-    const T *__restrict__ factor, double *X, int64_t ldx, int nrhs) {
+    const int2 *__restrict__ subs, int nsub, BlockDiv div, const int32_t *__restrict__ struct_rows,
+    const SubFront *__restrict__ fronts, const T *__restrict__ factor, double *X, int64_t ldx, int nrhs) {
     const int nwarps = gridDim.x * (kSubThreads / 32), ngr = (nrhs + RB - 1) / RB;
     for (int q = blockIdx.x * (kSubThreads / 32) + (threadIdx.x >> 5); q < nsub * ngr; q += nwarps) {
         const int2 sr = subs[q / ngr];
@@ -517,19 +543,18 @@ __global__ void __launch_bounds__(kSubThreads) subtree_small_bwd_kernel(
                 next = fronts[s - 1];
                 prefetch_panel(next, factor);
             }
-            if (sf.f <= 64) bwd_small<T, VB, 2, RB>(sf, factor, sd.struct_rows, sd.vb, X, ldx, r0, nr);
-            else bwd_small<T, VB, NSEG, RB>(sf, factor, sd.struct_rows, sd.vb, X, ldx, r0, nr);
+            if (sf.f <= 64) bwd_small<T, 2, RB>(sf, factor, struct_rows, div, X, ldx, r0, nr);
+            else bwd_small<T, NSEG, RB>(sf, factor, struct_rows, div, X, ldx, r0, nr);
         }
     }
 }
 
 // The fronts above those: a CTA per subtree of the cut, parents first (tops: its fronts,
 // top_ptr[k] to top_ptr[k + 1] in postorder).
-template <typename T, int VB>
+template <typename T>
 __global__ void __launch_bounds__(kSubThreads, 3) subtree_bwd_kernel(
-    const int32_t *__restrict__ top_ptr, const int32_t *__restrict__ tops, int nsub, SnDev sd,
-    const SubFront *__restrict__ fronts,
-    const T *__restrict__ factor, double *X, int64_t ldx, int nrhs) {
+    const int32_t *__restrict__ top_ptr, const int32_t *__restrict__ tops, int nsub, SnDev sd, BlockDiv div,
+    const SubFront *__restrict__ fronts, const T *__restrict__ factor, double *X, int64_t ldx, int nrhs) {
     extern __shared__ __align__(16) double sub_smem[];
     double *v = sub_smem + kSubRed;
     const int warp = threadIdx.x >> 5;
@@ -540,16 +565,14 @@ __global__ void __launch_bounds__(kSubThreads, 3) subtree_bwd_kernel(
             __syncthreads();                             // the parent's x is there
             if (fronts[s].inv < 0) {
                 for (int r = warp; r < nrhs; r += kSubThreads / 32)
-                    bwd_small_call<T, VB>(fronts + s, factor, sd.struct_rows, sd.vb, X, ldx, r);
+                    bwd_small_call<T>(fronts + s, factor, sd.struct_rows, div, X, ldx, r);
                 continue;
             }
             for (int rg = 0; rg < nrhs; rg += kSubRhs)
-                bwd_front<T, VB>(s, sd, factor, factor + fronts[s].pan, X, ldx, rg, min(kSubRhs, nrhs - rg), v);
+                bwd_front<T>(s, sd, div, factor, factor + fronts[s].pan, X, ldx, rg, min(kSubRhs, nrhs - rg), v);
         }
     }
 }
-
-int sub_sm_count() { return device_sm_count(); }
 
 }  // namespace
 
@@ -561,28 +584,24 @@ void launch_subtree_small(bool forward, const int2 *subs, int nsub, int fmax, Sn
     const int rb = nrhs > 1 ? kSubRhs : 1;
     const int64_t warps = int64_t(nsub) * ((nrhs + rb - 1) / rb), ctas = (warps + kSubThreads / 32 - 1) / (kSubThreads / 32);
     const int grid = int(std::min<int64_t>(ctas, 1 << 20));
+    const BlockDiv div(sd.vb);
     ++g_kernel_launches;
-    auto launch = [&](auto vbc, auto seg, auto rbc) {
-        constexpr int VB = decltype(vbc)::value, NSEG = decltype(seg)::value, RB = decltype(rbc)::value;
+    auto launch = [&](auto seg, auto rbc) {
+        constexpr int NSEG = decltype(seg)::value, RB = decltype(rbc)::value;
         if (forward)
-            subtree_small_fwd_kernel<T, VB, NSEG, RB>
-                <<<grid, kSubThreads, 0, st>>>(subs, nsub, sd, fronts, kids, cmap, factor, X, ldx, nrhs, sol);
+            subtree_small_fwd_kernel<T, NSEG, RB>
+                <<<grid, kSubThreads, 0, st>>>(subs, nsub, div, fronts, kids, cmap, factor, X, ldx, nrhs, sol);
         else
-            subtree_small_bwd_kernel<T, VB, NSEG, RB>
-                <<<grid, kSubThreads, 0, st>>>(subs, nsub, sd, fronts, factor, X, ldx, nrhs);
+            subtree_small_bwd_kernel<T, NSEG, RB>
+                <<<grid, kSubThreads, 0, st>>>(subs, nsub, div, sd.struct_rows, fronts, factor, X, ldx, nrhs);
     };
-    auto run = [&](auto vbc, auto seg) {
-        if (nrhs > 1) launch(vbc, seg, std::integral_constant<int, kSubRhs>{});
-        else launch(vbc, seg, std::integral_constant<int, 1>{});
+    auto run = [&](auto seg) {                           // rows per lane of the largest front
+        if (nrhs > 1) launch(seg, std::integral_constant<int, kSubRhs>{});
+        else launch(seg, std::integral_constant<int, 1>{});
     };
-    auto by_seg = [&](auto vbc) {                        // rows per lane of the largest front
-        if (fmax <= 96) run(vbc, std::integral_constant<int, 3>{});
-        else if (fmax <= 160) run(vbc, std::integral_constant<int, 5>{});
-        else run(vbc, std::integral_constant<int, 8>{});
-    };
-    if (sd.vb == 3) by_seg(std::integral_constant<int, 3>{});
-    else if (sd.vb == 1) by_seg(std::integral_constant<int, 1>{});
-    else by_seg(std::integral_constant<int, 0>{});
+    if (fmax <= 96) run(std::integral_constant<int, 3>{});
+    else if (fmax <= 160) run(std::integral_constant<int, 5>{});
+    else run(std::integral_constant<int, 8>{});
 }
 
 template <typename T>
@@ -591,27 +610,20 @@ void launch_subtree_solve(bool forward, const int32_t *top_ptr, const int32_t *t
                           int64_t ldx, int nrhs, double *sol, cudaStream_t st) {
     if (nsub <= 0) return;
     const size_t smem = (size_t(kSubRed) + size_t(kSubRhs) * fmax) * sizeof(double);
-    const int grid = std::min(nsub, 8 * sub_sm_count());
+    const int grid = std::min(nsub, 8 * device_sm_count());
+    const BlockDiv div(sd.vb);
+    static PerDeviceOnce once;
+    once([] {
+        cudaFuncSetAttribute(subtree_fwd_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmemOptin);
+        cudaFuncSetAttribute(subtree_bwd_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmemOptin);
+    });
     ++g_kernel_launches;
-    auto run = [&](auto vbc) {
-        constexpr int VB = decltype(vbc)::value;
-        static PerDeviceOnce once;
-        once([] {
-            cudaFuncSetAttribute(subtree_fwd_kernel<T, VB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 kMaxSmemOptin);
-            cudaFuncSetAttribute(subtree_bwd_kernel<T, VB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 kMaxSmemOptin);
-        });
-        if (forward)
-            subtree_fwd_kernel<T, VB><<<grid, kSubThreads, smem, st>>>(top_ptr, tops, nsub, sd, fronts, kids, cmap,
-                                                                       factor, X, ldx, nrhs, sol);
-        else
-            subtree_bwd_kernel<T, VB>
-                <<<grid, kSubThreads, smem, st>>>(top_ptr, tops, nsub, sd, fronts, factor, X, ldx, nrhs);
-    };
-    if (sd.vb == 3) run(std::integral_constant<int, 3>{});
-    else if (sd.vb == 1) run(std::integral_constant<int, 1>{});
-    else run(std::integral_constant<int, 0>{});
+    if (forward)
+        subtree_fwd_kernel<T><<<grid, kSubThreads, smem, st>>>(top_ptr, tops, nsub, sd, div, fronts, kids, cmap, factor,
+                                                               X, ldx, nrhs, sol);
+    else
+        subtree_bwd_kernel<T><<<grid, kSubThreads, smem, st>>>(top_ptr, tops, nsub, sd, div, fronts, factor, X, ldx,
+                                                               nrhs);
 }
 
 #define MFS_SUBTREE(T)                                                                                               \
