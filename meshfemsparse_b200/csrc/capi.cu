@@ -536,9 +536,29 @@ std::shared_ptr<DevSym> upload_symbolic(mfs_handle *h, std::shared_ptr<Symbolic>
     up(ds->bred, bred);
     up(ds->fsb_tasks, fsb);
     up(ds->bsb_tasks, bsb);
-    up(ds->isb_tasks, isb);
-    ds->nsb_inv = int(isb.size());
     ds->isb_host = isb;
+    {
+        // many diagonal blocks without a stored inverse: inverted first, and a superblock of
+        // one such block is complete then
+        auto rows = [&](const SbTask &t) { return int(std::min<idx>(SBk, S.w[t.sn] - t.K * SBk)); };
+        std::vector<SbTask> diag;
+        for (const SbTask &t : isb)
+            for (int a = 0; inv_off[t.sn] < 0 && 64 * a < rows(t); ++a) {
+                diag.push_back(t);
+                diag.back().pad = a;
+                ds->sb_diag_rows = std::max(ds->sb_diag_rows, std::min(64, rows(t) - 64 * a));
+            }
+        if (diag.size() <= size_t(kSbDiagMany)) diag.clear();
+        else
+            isb.erase(std::remove_if(isb.begin(), isb.end(),
+                                     [&](const SbTask &t) { return inv_off[t.sn] < 0 && rows(t) <= 64; }),
+                      isb.end());
+        for (const SbTask &t : isb) ds->sb_rows = std::max(ds->sb_rows, rows(t));
+        ds->nsb_inv = int(isb.size());
+        ds->nsb_diag = int(diag.size());
+        isb.insert(isb.end(), diag.begin(), diag.end());
+        up(ds->isb_tasks, isb);
+    }
     ds->max_str_entries = max_str;
     {
         // below the cut: the largest subtrees without stored inverses, and per subtree of
@@ -853,7 +873,7 @@ void run_factor(mfs_handle *h, DevSym &ds, T *factor, T *upd, T *dscr, const dou
         }
     }
     // inverses of the superblocks of L11 that the diagonal solves apply
-    launch_sb_inverse<T>(ds.isb_tasks.p, ds.nsb_inv, ds.sd, factor, st);
+    launch_sb_inverse<T>(ds.isb_tasks.p, ds.nsb_inv, ds.sb_rows, ds.nsb_diag, ds.sb_diag_rows, ds.sd, factor, st);
     MFS_LAUNCHED();
 }
 

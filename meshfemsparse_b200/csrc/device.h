@@ -294,8 +294,16 @@ cudaError_t launch_sb_solve(bool forward, const SbTask *tasks, int ntasks, SnDev
 // Per child c of the assembly forest, the map from its parent's front (block rows) to its
 // own structure (block index, -1: not in it), at map + off[c].
 void launch_child_maps(const int32_t *parent, const int64_t *off, int nsn, SnDev sd, int32_t *map, cudaStream_t st);
+// The superblock inverses: ntasks superblocks of at most max_rows rows, after them in the
+// list ndiag diagonal blocks (of at most diag_rows rows) to be inverted before those.
 template <typename T>
-void launch_sb_inverse(const SbTask *tasks, int ntasks, SnDev sd, T *factor, cudaStream_t st);
+void launch_sb_inverse(const SbTask *tasks, int ntasks, int max_rows, int ndiag, int diag_rows, SnDev sd, T *factor,
+                       cudaStream_t st);
+// More diagonal blocks without stored inverses than this (one an SM) are inverted first, a
+// CTA each: whole FP64 factorizations of 300 fronts of 15 rows 62 -> 34 us, of 63 rows 241 ->
+// 103 us. Up to it the substitution inside the other kernel is one launch less: 74 fronts of
+// 15 rows 30 us instead of 34.
+constexpr int kSbDiagMany = 148;
 int solve_rows_per_task();
 int diag_blocks_per_task();             // 64-row blocks per diagonal-chain task (one flag each)
 // Forward / backward solve of whole subtrees of fronts without stored inverses (subs[k] =

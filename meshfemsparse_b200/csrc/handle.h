@@ -118,7 +118,8 @@ struct DevSym {
     DBuf<StrTask> fstr_tasks, bstr_tasks;
     DBuf<StrReduce> fred, bred;
     DBuf<SbTask> fsb_tasks, bsb_tasks, isb_tasks;   // solves above the cut (forward, backward) and inverses
-    int nfsb = 0, nbsb = 0, nsb_inv = 0;
+    int nfsb = 0, nbsb = 0;
+    int nsb_inv = 0, nsb_diag = 0, sb_rows = 0, sb_diag_rows = 0;   // inverses: superblocks, then diagonal blocks
     DBuf<SbChild> sb_children;                      // the children of every front, front by front
     DBuf<int32_t> parent, cmap;                     // assembly parents; children's inverse row maps
     DBuf<int64_t> cmap_off;

@@ -1037,7 +1037,8 @@ __global__ void __launch_bounds__(kSbThreads, 1)
 // factor + tk.inv, one CTA per 16 columns of it (blockIdx.y; columns of 64-column block b):
 //   X_bb = D_b, X_ab = -D_a sum_{c=b}^{a-1} L_ac X_cb for a > b, X_ab = 0 for a < b,
 // with D_a = inv(L_aa) the 64 x 64 diagonal inverses: the panel kernel's stored ones when
-// the front has them, else by substitution on L_aa (all threads, a barrier a row). The
+// the front has them, else (given) what sb_diagonal_kernel left in place, else by
+// substitution on L_aa (all threads, a barrier a row). The
 // columns' blocks X_cb stay in shared memory; each L_ac and D_a is loaded into registers
 // while the product before runs and staged there for its own 64 x 64 x 16 one (thread = row
 // i, 4 columns). Bound by the chain of up to nine products of a superblock where there are
@@ -1045,7 +1046,8 @@ __global__ void __launch_bounds__(kSbThreads, 1)
 // substitution, 90 us for the 7-sided cube and 120 us for the 20-sided one in FP64, 34
 // and 87 us this way.
 template <typename T>
-__global__ void __launch_bounds__(256) sb_inverse_kernel(const SbTask *__restrict__ tasks, SnDev sd, T *factor) {
+__global__ void __launch_bounds__(256) sb_inverse_kernel(const SbTask *__restrict__ tasks, SnDev sd, bool given,
+                                                         T *factor) {
     constexpr int LD = 65, NC = 16;
     extern __shared__ __align__(16) double inv_smem[];
     T *Xc = reinterpret_cast<T *>(inv_smem);              // [4][NC][LD]: X_cb, c = b .. nbk - 1
@@ -1062,17 +1064,18 @@ __global__ void __launch_bounds__(256) sb_inverse_kernel(const SbTask *__restric
     const int r0 = K * SB;
     const int tid = threadIdx.x, i = tid & 63, jg = tid >> 6;
     const int64_t dinv = sd.inv_off[s];
-    // block (a, c) of L_KK, or D_a for a == c when it is stored: a column a quarter, lane = row
+    // block (a, c) of L_KK, or D_a for a == c when it is there: a column a quarter, lane = row
     T v[16];
     auto fetch = [&](int a, int c) {
         if (a >= nbk) return;
-        const bool stored = a == c && dinv >= 0;
-        const T *src = factor + dinv + int64_t(K * (SB / 64) + a) * 4096;
+        const bool stored = a == c && (dinv >= 0 || given);
+        const T *src = dinv >= 0 ? factor + dinv + int64_t(K * (SB / 64) + a) * 4096 : out + int64_t(a * 64) * nrp + a * 64;
+        const int lds = dinv >= 0 ? 64 : nrp;
 #pragma unroll
         for (int u = 0; u < 16; ++u) {
             const int m = jg + 4 * u, gi = a * 64 + i, gj = c * 64 + m;
             v[u] = T(0);
-            if (gi < nr && gj < nr) v[u] = stored ? src[m * 64 + i] : pan[int64_t(r0 + gj) * ld + r0 + gi];
+            if (gi < nr && gj < nr) v[u] = stored ? src[m * lds + i] : pan[int64_t(r0 + gj) * ld + r0 + gi];
         }
     };
     auto stage = [&](T *dst) {
@@ -1082,7 +1085,7 @@ __global__ void __launch_bounds__(256) sb_inverse_kernel(const SbTask *__restric
     // D_a from the staged block in Ds: itself, or by substitution into Ls
     auto diagonal = [&](int a) -> const T * {
         __syncthreads();
-        if (dinv >= 0) return Ds;
+        if (dinv >= 0 || given) return Ds;
         // rows k in order: every thread has column j and every fourth row below; row k stays
         // unscaled until the end, so that a step needs one barrier
         const int nb = min(64, nr - a * 64), j = i;
@@ -1118,7 +1121,7 @@ __global__ void __launch_bounds__(256) sb_inverse_kernel(const SbTask *__restric
             const int j = jg * 4 + u;
             const T x = D[(j0 + j) * LD + i];
             Xc[j * LD + i] = x;
-            out[int64_t(b * 64 + j0 + j) * nrp + b * 64 + i] = x;
+            if (dinv >= 0 || !given) out[int64_t(b * 64 + j0 + j) * nrp + b * 64 + i] = x;
         }
     }
     for (int a = b + 1; a < nbk; ++a) {
@@ -1158,6 +1161,45 @@ __global__ void __launch_bounds__(256) sb_inverse_kernel(const SbTask *__restric
             out[int64_t(b * 64 + j0 + j) * nrp + a * 64 + i] = acc[u];
         }
     }
+}
+
+// Diagonal block `pad` of a superblock without stored 64 x 64 inverses, inverted to its place
+// in inv(L_KK): four threads a column, rows in order. For many of them (fronts factored whole
+// above the cut: forests of small systems), since the kernel above substitutes again for every
+// 16 columns. Whole factorizations of 5,000 fronts of 15 rows: 613 us in FP32 and 711 us in
+// FP64 without it (271 and 498 us with 64 columns a CTA there), 121 and 162 us with it; 3,000
+// fronts of 120 rows 4.46 and 5.52 ms (3.89 and 6.37 ms), 1.74 and 2.54 ms with it.
+template <typename T>
+__global__ void __launch_bounds__(256) sb_diagonal_kernel(const SbTask *__restrict__ tasks, SnDev sd, int LD,
+                                                          T *factor) {
+    extern __shared__ __align__(16) double inv_smem[];
+    T *Ls = reinterpret_cast<T *>(inv_smem);              // [LD][LD]: the block of L, column-major
+    T *Y = Ls + LD * LD;                                  // [LD][LD]: its inverse, row-major
+    const SbTask tk = tasks[blockIdx.x];
+    const int s = tk.sn, ld = sd.ld[s], a0 = 64 * tk.pad, r0 = tk.K * SB + a0;
+    const int rows = sb_rows(sd.w[s], tk.K), nrp = sb_pad(rows), nr = min(64, rows - a0);
+    const int tid = threadIdx.x, i = tid & 63;
+    const T *pan = factor + sd.pan_off[s] + int64_t(r0) * ld + r0;
+    T *out = factor + tk.inv + int64_t(a0) * nrp + a0;
+#pragma unroll 4
+    for (int c = tid >> 6; c < nr; c += 4)
+        if (i >= c && i < nr) Ls[c * LD + i] = pan[int64_t(c) * ld + i];
+    __syncthreads();
+    const int j = tid >> 2, part = tid & 3, j0 = j & ~7;   // a warp has eight columns
+    if (j0 < nr)
+        for (int k = j0; k < nr; ++k) {
+            T y = T(0);
+#pragma unroll 2
+            for (int m = j0 + part; m < k; m += 4)
+                if (m >= j && j < nr) y -= Ls[m * LD + k] * Y[m * LD + j];
+            y += __shfl_xor_sync(0xffffffffu, y, 1);
+            y += __shfl_xor_sync(0xffffffffu, y, 2);
+            if (k == j) y = T(1);
+            if (part == 0 && j < nr) Y[k * LD + j] = k >= j ? y / Ls[k * LD + k] : T(0);
+            __syncwarp();
+        }
+    __syncthreads();
+    for (int c = tid >> 6; c < 64; c += 4) out[int64_t(c) * nrp + i] = i >= c && i < nr ? Y[i * LD + c] : T(0);
 }
 
 // NR: the right-hand sides the vectors hold (nrhs <= NR)
@@ -1223,13 +1265,25 @@ cudaError_t launch_sb_solve(bool forward, const SbTask *tasks, int ntasks, SnDev
 }
 
 template <typename T>
-void launch_sb_inverse(const SbTask *tasks, int ntasks, SnDev sd, T *factor, cudaStream_t st) {
+void launch_sb_inverse(const SbTask *tasks, int ntasks, int max_rows, int ndiag, int diag_rows, SnDev sd, T *factor,
+                       cudaStream_t st) {
+    if (ndiag > 0) {
+        const int ld = diag_rows | 1;
+        const size_t smem = size_t(2) * ld * ld * sizeof(T);
+        static PerDeviceOnce once;
+        once([] {
+            cudaFuncSetAttribute(sb_diagonal_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 int(2 * 65 * 65 * sizeof(T)));
+        });
+        ++g_kernel_launches;
+        sb_diagonal_kernel<T><<<ndiag, 256, smem, st>>>(tasks + ntasks, sd, ld, factor);
+    }
     if (ntasks <= 0) return;
     const size_t smem = size_t(5 * 16 + 2 * 64) * 65 * sizeof(T);
     static PerDeviceOnce once;
     once([smem] { cudaFuncSetAttribute(sb_inverse_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)); });
     ++g_kernel_launches;
-    sb_inverse_kernel<T><<<dim3(ntasks, SB / 16), 256, smem, st>>>(tasks, sd, factor);
+    sb_inverse_kernel<T><<<dim3(ntasks, 4 * ((max_rows + 63) / 64)), 256, smem, st>>>(tasks, sd, ndiag > 0, factor);
 }
 
 #define MFS_SB_INSTANTIATE(T)                                                                                      \
@@ -1238,7 +1292,7 @@ void launch_sb_inverse(const SbTask *tasks, int ntasks, SnDev sd, T *factor, cud
                                             double *, int *, int *, cudaStream_t);
 MFS_SB_INSTANTIATE(float)
 MFS_SB_INSTANTIATE(double)
-template void launch_sb_inverse<float>(const SbTask *, int, SnDev, float *, cudaStream_t);
-template void launch_sb_inverse<double>(const SbTask *, int, SnDev, double *, cudaStream_t);
+template void launch_sb_inverse<float>(const SbTask *, int, int, int, int, SnDev, float *, cudaStream_t);
+template void launch_sb_inverse<double>(const SbTask *, int, int, int, int, SnDev, double *, cudaStream_t);
 
 }  // namespace mfs
