@@ -49,8 +49,8 @@
 //   count warp    publishes a structure task's results once all product warps have handed
 //                 them over.
 // Structure rows start at w rounded down to a multiple of 4 (TMA boxes start 16-byte
-// aligned); the rows before w, and what a box holds past the front, meet zeros or are not
-// stored.
+// aligned); the rows before w are not stored forward and cleared backward, and what a box
+// holds past the front is zero.
 //
 // Launches are cooperative (all CTAs co-resident); every CTA walks its tasks in
 // ascending order and a task waits only on lower-numbered tasks and on the other
@@ -989,6 +989,16 @@ __global__ void __launch_bounds__(kSbThreads, 1)
             mbar_wait(rg.vfull + 8 * slot, uint32_t(gv / VS) & 1u, err);
             for (int c = 0; c < nc; ++c) {
                 const T *ck = chunk();
+                if (g == sh.nsg - 1 && c == 0 && (w & 3)) {
+                    // L11's last rows, for the boxes' alignment: they meet zeros, but an infinite
+                    // pivot among them does not (each warp clears the columns that it reads)
+                    T *own_cols = ring + int(gq % NST) * CE + (wp * 8 + (lane & 7)) * FC;
+                    if (lane < 8)
+                        for (int e = 0; e < (w & 3); ++e) own_cols[e] = T(0);
+                    // (before the slot's next copy)
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    __syncwarp();
+                }
                 bwd_chunk<T, P, NR>(ck, vp + slot * (NR * SB) + c * FC, pacc, wp * 8, lane, FC);
                 release();
                 if (++held == kFlush) flush();
