@@ -120,23 +120,57 @@ std::shared_ptr<DevSym> upload_symbolic(mfs_handle *h, std::shared_ptr<Symbolic>
     std::vector<int32_t> all_list;
     std::vector<SmallTask> small_tasks;
     std::vector<AssembleTask> asm_tasks;
-    // inverse row maps of the children in their parents' fronts
+    // the fronts with many children have lists of them per block row ...
+    std::vector<int32_t> many(nsn, -1);
+    std::vector<ManyFront> many_fronts;
+    std::vector<ManyTask> many_tasks;
+    for (idx s = 0; s < nsn; ++s) {
+        idx n = 0;
+        for (idx k = S.child_ptr[s]; k < S.child_ptr[s + 1]; ++k) n += S.d[S.child_list[k]] > 0;
+        if (n <= kManyChildren) continue;
+        many[s] = int32_t(many_fronts.size());
+        many_fronts.push_back({});
+    }
+    // ... the children of the others inverse row maps in their parents' fronts
     std::vector<int32_t> par(nsn);
     std::vector<int64_t> cmap_off(nsn + 1, 0);
     for (idx s = 0; s < nsn; ++s) {
-        par[s] = int32_t(S.sn_parent[s]);
+        par[s] = S.sn_parent[s] < 0 || S.d[s] == 0 || many[S.sn_parent[s]] >= 0 ? -1 : int32_t(S.sn_parent[s]);
         cmap_off[s + 1] = cmap_off[s] + (par[s] < 0 ? 0 : S.f[par[s]] / S.vb);
     }
-    // ... and the children with an update matrix of every front
+    // the children with an update matrix of every front (nchild: of those with maps)
     std::vector<AsmChild> asm_children;
     std::vector<int32_t> child0(nsn, 0), nchild(nsn, 0);
+    std::vector<int64_t> many_ptr;
+    std::vector<int2> many_ent;
     for (idx s = 0; s < nsn; ++s) {
         child0[s] = int32_t(asm_children.size());
         for (idx k = S.child_ptr[s]; k < S.child_ptr[s + 1]; ++k) {
             const idx c = S.child_list[k];
-            if (S.d[c] > 0) asm_children.push_back({cmap_off[c], S.upd_off[c], int32_t(S.d[c]), 0});
+            if (S.d[c] > 0)
+                asm_children.push_back({many[s] >= 0 ? int64_t(S.struct_ptr[c]) : cmap_off[c], S.upd_off[c],
+                                        int32_t(S.d[c]), 0});
         }
-        nchild[s] = int32_t(asm_children.size()) - child0[s];
+        const int32_t n = int32_t(asm_children.size()) - child0[s];
+        if (many[s] < 0) {
+            nchild[s] = n;
+            continue;
+        }
+        const size_t rows = many_ptr.size();
+        many_fronts[many[s]] = {int64_t(rows), child0[s], n};
+        many_ptr.resize(rows + S.f[s] / S.vb + 1, 0);
+        int64_t *ptr = many_ptr.data() + rows;
+        auto each = [&](auto fn) {
+            for (int32_t k = child0[s]; k < child0[s] + n; ++k)
+                for (int32_t m = 0; m < asm_children[k].d / S.vb; ++m)
+                    fn(S.rel[asm_children[k].map + m] / S.vb, make_int2(k, m));
+        };
+        each([&](idx b, int2) { ++ptr[b + 1]; });
+        ptr[0] = int64_t(many_ent.size());
+        for (idx b = 0; b < S.f[s] / S.vb; ++b) ptr[b + 1] += ptr[b];
+        many_ent.resize(size_t(ptr[S.f[s] / S.vb]));
+        std::vector<int64_t> next(ptr, ptr + S.f[s] / S.vb);
+        each([&](idx b, int2 e) { many_ent[next[b]++] = e; });
     }
     std::vector<AssembleTile> asm_tiles;
     std::vector<PanelTask> potrf_tasks;
@@ -150,13 +184,14 @@ std::shared_ptr<DevSym> upload_symbolic(mfs_handle *h, std::shared_ptr<Symbolic>
         std::vector<idx> large;
         L.small_off = int(small_tasks.size());
         L.all_off = int(all_list.size());
+        L.many_off = int(many_tasks.size());
         for (idx k = S.level_ptr[l]; k < S.level_ptr[l + 1]; ++k) {
             idx s = S.level_list[k];
             all_list.push_back(int32_t(s));
             L.all_max_front = std::max<int>(L.all_max_front, int(S.f[s]));
             if (S.f[s] <= small_max) {
-                small_tasks.push_back({int32_t(S.w[s]), int32_t(S.f[s]), dld[s], col0[s], child0[s], nchild[s], dpan[s],
-                                       S.upd_off[s]});
+                small_tasks.push_back({int32_t(S.w[s]), int32_t(S.f[s]), dld[s], col0[s], child0[s], nchild[s],
+                                       many[s], 0, dpan[s], S.upd_off[s]});
                 L.small_max_front = std::max<int>(L.small_max_front, int(S.f[s]));
             } else large.push_back(s);
         }
@@ -177,9 +212,12 @@ std::shared_ptr<DevSym> upload_symbolic(mfs_handle *h, std::shared_ptr<Symbolic>
                 for (idx r0 = c0; r0 < S.f[s]; r0 += L.asm_rows)
                     asm_tiles.push_back({int32_t(asm_tasks.size()), int32_t(c0), int32_t(r0)});
             asm_tasks.push_back({int32_t(s), child0[s], nchild[s]});
+            for (idx b = 0; many[s] >= 0 && b < S.f[s] / S.vb; b += 8)
+                many_tasks.push_back({int32_t(s), many[s], int32_t(b), 0});
             maxw = std::max(maxw, S.w[s]);
         }
         L.asm_tiles = int(asm_tiles.size()) - L.asm_off;
+        L.many_n = int(many_tasks.size()) - L.many_off;
         const bool f64 = h->opt.precision != MFS_PREC_FP32;
         const int NB = f64 ? 64 : 128;                  // column block of the large-front factorization
         const int TM = gemm_tile_m(f64), TN = gemm_tile_n(f64);
@@ -371,6 +409,12 @@ std::shared_ptr<DevSym> upload_symbolic(mfs_handle *h, std::shared_ptr<Symbolic>
                             int32_t(S.d[c]), 0});
         }
         sb_nchild[s] = int32_t(kids.size()) - sb_child0[s];
+        if (many[s] >= 0) {
+            bool wait = false;
+            for (int32_t k = sb_child0[s]; k < sb_child0[s] + sb_nchild[s]; ++k) wait |= kids[k].flag >= 0;
+            if (!wait) many_fronts[many[s]].nwait = 0;
+            sb_nchild[s] = 0;
+        }
     }
     // per analysis row of these fronts: where its superblock counts (by its first scalar)
     std::vector<int32_t> rowcnt(std::max<idx>(S.nv, 1), 0);
@@ -393,7 +437,7 @@ std::shared_ptr<DevSym> upload_symbolic(mfs_handle *h, std::shared_ptr<Symbolic>
                       int32_t(S.w[s]),
                       int32_t(S.f[s]),
                       col0[s],
-                      0,
+                      many[s],
                       S.sol_off[s]};
     };
     std::vector<SolveAsmTask> sasm;
@@ -514,6 +558,10 @@ std::shared_ptr<DevSym> upload_symbolic(mfs_handle *h, std::shared_ptr<Symbolic>
     up(ds->small_tasks, small_tasks);
     up(ds->asm_tasks, asm_tasks);
     up(ds->asm_children, asm_children);
+    up(ds->many_tasks, many_tasks);
+    up(ds->many_fronts, many_fronts);
+    up(ds->many_ptr, many_ptr);
+    up(ds->many_ent, many_ent);
     up(ds->asm_tiles, asm_tiles);
     up(ds->potrf_tasks, potrf_tasks);
     up(ds->gemm_tasks, gemm_tasks);
@@ -561,11 +609,11 @@ std::shared_ptr<DevSym> upload_symbolic(mfs_handle *h, std::shared_ptr<Symbolic>
     }
     ds->max_str_entries = max_str;
     {
-        // below the cut: the largest subtrees without stored inverses, and per subtree of
-        // the cut the fronts above those
+        // below the cut: the largest subtrees without stored inverses or many children, and
+        // per subtree of the cut the fronts above those
         std::vector<uint8_t> small(nsn, 0);
         for (idx s = 0; s < nsn; ++s) {
-            small[s] = inv_off[s] < 0 && S.level[s] <= S.solve_cut;
+            small[s] = inv_off[s] < 0 && many[s] < 0 && S.level[s] <= S.solve_cut;
             for (idx k = S.child_ptr[s]; k < S.child_ptr[s + 1]; ++k) small[s] &= small[S.child_list[k]];
         }
         std::vector<SubFront> sf(nsn);
@@ -573,8 +621,8 @@ std::shared_ptr<DevSym> upload_symbolic(mfs_handle *h, std::shared_ptr<Symbolic>
         std::vector<std::pair<double, int32_t>> work;     // of the subtrees of small fronts
         std::vector<double> cost(nsn, 0.0);
         for (idx s = 0; s < nsn; ++s) {
-            sf[s] = {int32_t(S.w[s]), int32_t(S.f[s]), dld[s],     col0[s],      sb_child0[s],
-                     sb_nchild[s],    dpan[s],         inv_off[s], S.sol_off[s], S.struct_ptr[s]};
+            sf[s] = {int32_t(S.w[s]), int32_t(S.f[s]), dld[s],  col0[s],    sb_child0[s], sb_nchild[s],
+                     many[s],         0,               dpan[s], inv_off[s], S.sol_off[s], S.struct_ptr[s]};
             lo[s] = int32_t(s);
             cost[s] = double(S.f[s]) * double(S.w[s]);
             for (idx k = S.child_ptr[s]; k < S.child_ptr[s + 1]; ++k) {
@@ -623,6 +671,7 @@ std::shared_ptr<DevSym> upload_symbolic(mfs_handle *h, std::shared_ptr<Symbolic>
     sd.struct_rows = ds->struct_rows.p;
     sd.rel = ds->rel.p;
     sd.vb = S.vb;
+    ds->many = {ds->many_fronts.p, ds->many_ptr.p, ds->many_ent.p, ds->rel.p};
     {
         ds->parent.upload(par, st);
         ds->cmap_off.upload(cmap_off, st);
@@ -820,12 +869,15 @@ void run_factor(mfs_handle *h, DevSym &ds, T *factor, T *upd, T *dscr, const dou
     for (const LevelPlan &L : ds.levels) {
         if (L.small_count > 0) {
             launch_small_factor<T>(ds.small_tasks.p + L.small_off, L.small_count, L.small_max_front, S.vb,
-                                   ds.asm_children.p, ds.cmap.p, factor, upd, pv, st);
+                                   ds.asm_children.p, ds.cmap.p, ds.many, factor, upd, pv, st);
             MFS_LAUNCHED();
         }
         if (L.large_count == 0) continue;
         launch_assemble_large<T>(ds.asm_tiles.p + L.asm_off, L.asm_tiles, L.asm_rows, ds.asm_tasks.p, ds.sd,
                                  ds.asm_children.p, ds.cmap.p, factor, upd, st);
+        MFS_LAUNCHED();
+        launch_assemble_many<T>(ds.many_tasks.p + L.many_off, L.many_n, ds.sd, ds.many, ds.asm_children.p, factor, upd,
+                                st);
         MFS_LAUNCHED();
         // One-group look-ahead: the column-block chain (left-looking update, panel, row
         // solve) and the update of the next group's columns run on a high-priority
@@ -966,12 +1018,12 @@ void run_solve(mfs_handle *h, DevSym &ds, const T *factor, double *X, int nrhs) 
                                 ds.cmap.p, factor, Xc, S.n, nr, h->sol.p, st);
         MFS_LAUNCHED();
         launch_subtree_solve<T>(true, ds.top_ptr.p, ds.tops.p, ds.ntop, ds.sub_fmax, ds.sd, ds.sub_fronts.p,
-                                ds.sb_children.p, ds.cmap.p, factor, Xc, S.n, nr, h->sol.p, st);
+                                ds.sb_children.p, ds.cmap.p, ds.many, factor, Xc, S.n, nr, h->sol.p, st);
         MFS_LAUNCHED();
         if (sb) {
             auto above = [&](bool forward, const SbTask *tasks, int n) {
                 MFS_CUDA(launch_sb_solve<T>(forward, tasks, n, ds.sd, h->smaps.p, ds.sb_children.p, ds.cmap.p,
-                                            ds.rowcnt.p, Xc, S.n, nr, h->sol.p, h->sb_scratch.p, ds.flags.p,
+                                            ds.many, ds.rowcnt.p, Xc, S.n, nr, h->sol.p, h->sb_scratch.p, ds.flags.p,
                                             h->solve_err.p, st));
             };
             above(true, ds.fsb_tasks.p, ds.nfsb);
@@ -997,7 +1049,7 @@ void run_solve(mfs_handle *h, DevSym &ds, const T *factor, double *X, int nrhs) 
             }
         }
         launch_subtree_solve<T>(false, ds.top_ptr.p, ds.tops.p, ds.ntop, ds.sub_fmax, ds.sd, ds.sub_fronts.p,
-                                ds.sb_children.p, ds.cmap.p, factor, Xc, S.n, nr, h->sol.p, st);
+                                ds.sb_children.p, ds.cmap.p, ds.many, factor, Xc, S.n, nr, h->sol.p, st);
         MFS_LAUNCHED();
         launch_subtree_small<T>(false, ds.subs.p, ds.nsub, ds.sub_small, ds.sd, ds.sub_fronts.p, ds.sb_children.p,
                                 ds.cmap.p, factor, Xc, S.n, nr, h->sol.p, st);

@@ -135,13 +135,14 @@ struct AssembleTile {
     int32_t task, c0, r0;
 };
 // A front factored whole by one CTA: sizes, panel leading dimension, first column, children
-// with an update matrix, panel and update-matrix offsets (-1: none).
+// with an update matrix (none here for a front of ManyDev, whose place is `many`, else -1),
+// panel and update-matrix offsets (-1: none).
 struct SmallTask {
-    int32_t w, f, ld, col0, child0, nchild;
+    int32_t w, f, ld, col0, child0, nchild, many, pad;
     int64_t pan, upd;
 };
-// A child in the extend-add: its inverse row map's first entry, its update matrix in the
-// arena and that matrix's order.
+// A child in the extend-add: its inverse row map's first entry (of a front of ManyDev: its
+// first structure row), its update matrix in the arena and that matrix's order.
 struct AsmChild {
     int64_t map, upd;
     int32_t d, pad;
@@ -181,7 +182,8 @@ struct SbTask {
     int64_t inv;
     int32_t pmap, imap;
     int32_t child0, nchild;
-    int32_t w, f, c0, pad2;             // the front's width, rows and first column
+    int32_t w, f, c0, many;             // the front's width, rows and first column; place in ManyDev (-1: none;
+                                        // else nchild is 0)
     int64_t sol;                        // its place in the solve arena
 };
 // One child of a front above the cut: the count that says its update vector is whole, and
@@ -193,11 +195,36 @@ struct SbChild {
     int32_t d, pad;
 };
 // A front in the subtree solves: sizes, panel leading dimension, first column, children with
-// an update vector (SbChild), panel, stored inverses (-1: none), place in the solve arena
-// (-1: none) and first structure row.
+// an update vector (SbChild; none for a front of ManyDev, whose place is `many`, else -1),
+// panel, stored inverses (-1: none), place in the solve arena (-1: none) and first structure row.
 struct SubFront {
-    int32_t w, f, ld, col0, child0, nchild;
+    int32_t w, f, ld, col0, child0, nchild, many, pad;
     int64_t pan, inv, sol, rows;
+};
+// Fronts with more children than kManyChildren (a wide separator over many small parts). An
+// inverse map per child would be children x rows of the front: instead each block row of the
+// front has the list of the children that have it, in child order, {index in the child arrays,
+// block row of the child}: list of row b of front k at ent[ptr[fronts[k].rows + b] ..
+// ptr[fronts[k].rows + b + 1]). What a row or column costs is then what it is given, and not
+// a look at every child: 3,000 children of 18 rows under 600 rows factored in 11.0 ms with
+// maps in FP32 (3.0 ms with the scatters from one child after the other that the maps had
+// replaced), 0.68 ms with lists; 20,000 of 8 rows under 600 in 32.7 (17.5) and 0.73 ms. Up to
+// kManyChildren the maps are read without the lists' extra step: 300 fronts of 12 children
+// 82.9 us, of 30 children 118 us with maps and 111 us with lists.
+struct ManyFront {
+    int64_t rows;
+    int32_t child0, nwait;               // its children; how many of them to look at for a count to wait for
+};
+struct ManyDev {
+    const ManyFront *fronts;
+    const int64_t *ptr;
+    const int2 *ent;
+    const int32_t *rel;                  // the structure rows' places in the parent's front (scalars)
+};
+constexpr int kManyChildren = 16;
+// Column block of a large front of ManyDev in the extend-add: eight block columns from b on.
+struct ManyTask {
+    int32_t sn, many, b, pad;
 };
 constexpr int kSuperBlock = 256;        // rows per superblock
 // structure part of the solves: forward tasks are kStrRows rows x kStrCols columns
@@ -228,7 +255,11 @@ template <typename T>
 void launch_extract_diag(const int64_t *diag_off, int64_t n, const T *factor, double *out, cudaStream_t st);
 template <typename T>
 void launch_small_factor(const SmallTask *tasks, int count, int max_front, int vb, const AsmChild *children,
-                         const int32_t *cmap, T *factor, T *upd, PivotCtl pv, cudaStream_t st);
+                         const int32_t *cmap, ManyDev many, T *factor, T *upd, PivotCtl pv, cudaStream_t st);
+// Extend-add of the large fronts of ManyDev, after launch_assemble_large without children.
+template <typename T>
+void launch_assemble_many(const ManyTask *tasks, int ntasks, SnDev sd, ManyDev many, const AsmChild *children, T *factor,
+                          T *upd, cudaStream_t st);
 template <typename T>
 void launch_assemble_large(const AssembleTile *tiles, int ntiles, int tile_rows, const AssembleTask *tasks, SnDev sd,
                            const AsmChild *children, const int32_t *cmap, T *factor, T *upd, cudaStream_t st);
@@ -289,8 +320,9 @@ void launch_str(bool forward, const StrTask *tasks, int ntasks, const StrReduce 
 // above the cut, 4 x its superblock's first count + its parts - 1.
 template <typename T>
 cudaError_t launch_sb_solve(bool forward, const SbTask *tasks, int ntasks, SnDev sd, const void *maps,
-                            const SbChild *children, const int32_t *cmap, const int32_t *rowcnt, double *X, int64_t ldx,
-                            int nrhs, double *sol, double *scratch, int *flags, int *err, cudaStream_t st);
+                            const SbChild *children, const int32_t *cmap, ManyDev many, const int32_t *rowcnt,
+                            double *X, int64_t ldx, int nrhs, double *sol, double *scratch, int *flags, int *err,
+                            cudaStream_t st);
 // Per child c of the assembly forest, the map from its parent's front (block rows) to its
 // own structure (block index, -1: not in it), at map + off[c].
 void launch_child_maps(const int32_t *parent, const int64_t *off, int nsn, SnDev sd, int32_t *map, cudaStream_t st);
@@ -306,9 +338,9 @@ void launch_sb_inverse(const SbTask *tasks, int ntasks, int max_rows, int ndiag,
 constexpr int kSbDiagMany = 148;
 int solve_rows_per_task();
 int diag_blocks_per_task();             // 64-row blocks per diagonal-chain task (one flag each)
-// Forward / backward solve of whole subtrees of fronts without stored inverses (subs[k] =
-// postorder range [x, y], largest front fmax rows), then of the fronts above them up to the
-// cut (subtree k: tops[top_ptr[k]..top_ptr[k + 1]) in postorder); backward in the other order.
+// Forward / backward solve of whole subtrees of fronts without stored inverses or many
+// children (subs[k] = postorder range [x, y], largest front fmax rows), then of the fronts
+// above them up to the cut (subtree k: tops[top_ptr[k]..top_ptr[k + 1]) in postorder); backward in the other order.
 // fronts per supernode, kids and cmap as for launch_sb_solve.
 template <typename T>
 void launch_subtree_small(bool forward, const int2 *subs, int nsub, int fmax, SnDev sd, const SubFront *fronts,
@@ -316,8 +348,8 @@ void launch_subtree_small(bool forward, const int2 *subs, int nsub, int fmax, Sn
                           double *sol, cudaStream_t st);
 template <typename T>
 void launch_subtree_solve(bool forward, const int32_t *top_ptr, const int32_t *tops, int nsub, int fmax, SnDev sd,
-                          const SubFront *fronts, const SbChild *kids, const int32_t *cmap, const T *factor, double *X,
-                          int64_t ldx, int nrhs, double *sol, cudaStream_t st);
+                          const SubFront *fronts, const SbChild *kids, const int32_t *cmap, ManyDev many,
+                          const T *factor, double *X, int64_t ldx, int nrhs, double *sol, cudaStream_t st);
 
 // Symmetric block SpMV over permuted reduced rows: Y = A X (both ld = n); dotp: partial sums of
 // X . Y per column (reduce_partials_count each); stop: nothing is done once it is set.

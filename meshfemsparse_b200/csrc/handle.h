@@ -75,6 +75,7 @@ struct LevelPlan {
     int all_off = 0, all_count = 0, all_max_front = 0;
     int large_count = 0;
     int asm_off = 0, asm_tiles = 0, asm_rows = 0;   // extend-add: the level's tiles, rows of a tile
+    int many_off = 0, many_n = 0;                    // ... and the column blocks of its fronts with many children
     struct Step {
         int left_off, left_n, left_tiles;   // the block's columns updated by the earlier blocks of its group
         int potrf_off, potrf_n, potrf_maxnb;
@@ -111,6 +112,10 @@ struct DevSym {
     DBuf<AssembleTask> asm_tasks;
     DBuf<AssembleTile> asm_tiles;
     DBuf<AsmChild> asm_children;         // the children of every front, front by front
+    DBuf<ManyTask> many_tasks;           // large fronts with many children: their column blocks
+    DBuf<ManyFront> many_fronts;         // the lists of ManyDev
+    DBuf<int64_t> many_ptr;
+    DBuf<int2> many_ent;
     DBuf<PanelTask> potrf_tasks;
     DBuf<GemmTask> gemm_tasks;
     DBuf<SolveAsmTask> sasm_tasks;
@@ -137,6 +142,7 @@ struct DevSym {
     DBuf<int64_t> prrfr, sperm;
     std::vector<LevelPlan> levels;
     SnDev sd{};
+    ManyDev many{};
     int64_t ax_len = 0;
     std::vector<int64_t> Ap_full, Ai_full;   // caller's pattern (for the element slot map)
     DBuf<int64_t> Ap_full_dev, Ai_full_dev;  // the same on the device
@@ -151,11 +157,14 @@ struct DevSym {
     std::vector<int32_t> large_fronts;       // fronts factored by the tiled (GEMM) path
     DBuf<int32_t> large_dev;                 // the same list on the device
     size_t bytes() const {
-        return w.bytes() * 5 + col0.bytes() + child_ptr.bytes() + child_list.bytes() + struct_rows.bytes() +
-               rel.bytes() + all_list.bytes() + pan_off.bytes() + upd_off.bytes() +
-               sol_off.bytes() + struct_ptr.bytes() + diag_off.bytes() + inv_off.bytes() + plan.bytes() + asm_tasks.bytes() +
-               potrf_tasks.bytes() + gemm_tasks.bytes() + spmv_ptr.bytes() +
-               spmv_src.bytes() + spmv_col.bytes() + spmv_flag.bytes() + prrfr.bytes() + sperm.bytes();
+        auto sum = [](const auto &...b) { return (b.bytes() + ...); };
+        return sum(w, d, f, ld, col0, child_ptr, child_list, struct_rows, rel, all_list, pan_off, upd_off, sol_off,
+                   struct_ptr, diag_off, inv_off, plan, plan_cat, plan_ptr_dev) +
+               sum(small_tasks, asm_tasks, asm_tiles, asm_children, many_tasks, many_fronts, many_ptr, many_ent,
+                   potrf_tasks, gemm_tasks) +
+               sum(sasm_tasks, ftri_tasks, btri_tasks, fstr_tasks, bstr_tasks, fred, bred, fsb_tasks, bsb_tasks,
+                   isb_tasks, sb_children, parent, cmap, cmap_off, rowcnt, subs, sub_fronts, top_ptr, tops, flags) +
+               sum(spmv_ptr, spmv_src, spmv_col, spmv_flag, prrfr, sperm, Ap_full_dev, Ai_full_dev, large_dev);
     }
 };
 

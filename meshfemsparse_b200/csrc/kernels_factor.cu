@@ -102,10 +102,73 @@ __global__ void extract_diag_kernel(const int64_t *__restrict__ diag_off, int64_
 // barriers a column over the whole square the 20-sided cube took 587 us in FP64 (5
 // launches), 150 us now; the batch of 48 cubes in FP32 4,550 us (9 launches), 1,070 us now.
 constexpr int kSmallCols = 4;
+
+// Column c of block row b of a front of ManyDev (its list: entries e0 to e1 - 1): a warp calls
+// add(front row, value) over each child's rows from the column's own on, in child order. 32
+// list entries and their children are loaded at a time, a lane each, then the values of four
+// children before the first is added: what is left between two adds is the add.
+template <typename T, typename Add>
+__device__ __forceinline__ void many_column(const ManyDev &many, const AsmChild *__restrict__ children, const T *upd,
+                                            int64_t e0, int64_t e1, int c, int vb, int lane, Add add) {
+    for (int64_t e = e0; e < e1; e += 32) {
+        const int n = int(min(int64_t(32), e1 - e));
+        int2 en = make_int2(0, 0);
+        AsmChild ch{0, 0, 0, 0};
+        if (lane < n) {
+            en = many.ent[e + lane];
+            ch = children[en.x];
+        }
+#pragma unroll 1
+        for (int k0 = 0; k0 < n; k0 += 4) {
+            T v[4];
+            int ri[4], d[4], jc[4];
+            int64_t map[4], up[4];
+            auto value = [&](int u, int ic) {            // row ic of the child's column
+                const int b = ic / vb;
+                ri[u] = many.rel[map[u] + b] + ic - b * vb;
+                v[u] = upd[up[u] + int64_t(jc[u]) * d[u] + ic];
+            };
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int k = min(k0 + u, n - 1);
+                d[u] = k0 + u < n ? __shfl_sync(0xffffffffu, ch.d, k) : 0;
+                jc[u] = __shfl_sync(0xffffffffu, en.y, k) * vb + c;
+                map[u] = __shfl_sync(0xffffffffu, ch.map, k);
+                up[u] = __shfl_sync(0xffffffffu, ch.upd, k);
+                if (jc[u] + lane < d[u]) value(u, jc[u] + lane);
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                if (jc[u] + lane < d[u]) add(ri[u], v[u]);
+#pragma unroll 4
+                for (int ic = jc[u] + lane + 32; ic < d[u]; ic += 32) {
+                    value(u, ic);
+                    add(ri[u], v[u]);
+                }
+                __syncwarp();                            // (the next child may meet the same rows)
+            }
+        }
+    }
+}
+
+// The children of a small front of ManyDev, added to its triangle F by the CTA. (A call: rare,
+// and inlined it costs the kernel registers.)
+template <typename T>
+__device__ __noinline__ void small_many(const SmallTask *tk, int vb, const ManyDev &many, const AsmChild *children,
+                                        const T *upd, T *F) {
+    const int f = tk->f;
+    const int64_t *ptr = many.ptr + many.fronts[tk->many].rows;
+    for (int j = threadIdx.x >> 5; j < f; j += 8) {
+        T *Fj = F + j * f - ((j * (j + 1)) >> 1);
+        many_column(many, children, upd, ptr[j / vb], ptr[j / vb + 1], j % vb, vb, threadIdx.x & 31,
+                    [&](int i, T x) { Fj[i] += x; });
+    }
+}
+
 template <typename T, int VB, int NSEG, int MINB>
 __global__ void __launch_bounds__(256, MINB)
     small_factor_kernel(const SmallTask *__restrict__ tasks, int vb_, int lp, const AsmChild *__restrict__ children,
-                        const int32_t *__restrict__ cmap, T *__restrict__ factor, T *upd, PivotCtl pv) {
+                        const int32_t *__restrict__ cmap, ManyDev many, T *__restrict__ factor, T *upd, PivotCtl pv) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T *Lp = reinterpret_cast<T *>(smem_raw);             // [4][lp]: the four columns under way
     T *F = Lp + kSmallCols * lp;
@@ -187,6 +250,10 @@ __global__ void __launch_bounds__(256, MINB)
                     if (j < f && i >= j && i < f) F[col(j) + i] = v[u][g];
                 }
         }
+    }
+    if (tk.many >= 0) {
+        __syncthreads();
+        small_many(tasks + blockIdx.x, vb, many, children, upd, F);
     }
     __syncthreads();
     for (int k = 0; k < w; k += kSmallCols) {
@@ -382,6 +449,25 @@ __global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 1024 : 512) / NT)
     }
 }
 
+// The children of a large front of ManyDev, whose panel and (zeroed) U_s are in place: a warp
+// per block column, added to in global memory.
+template <typename T>
+__global__ void __launch_bounds__(256) assemble_many_kernel(const ManyTask *__restrict__ tasks, SnDev sd, ManyDev many,
+                                                            const AsmChild *__restrict__ children,
+                                                            T *factor, T *upd) {
+    const ManyTask tk = tasks[blockIdx.x];
+    const int s = tk.sn, lane = threadIdx.x & 31, b = tk.b + (threadIdx.x >> 5);
+    const int w = sd.w[s], d = sd.d[s], vb = sd.vb;
+    if (b * vb >= w + d) return;
+    const int64_t *ptr = many.ptr + many.fronts[tk.many].rows + b;
+    T *pan = factor + sd.pan_off[s], *Us = upd + sd.upd_off[s];
+    for (int c = 0; c < vb; ++c) {
+        const int j = b * vb + c;
+        T *dst = j < w ? pan + int64_t(j) * sd.ld[s] : Us + int64_t(j - w) * d - w;
+        many_column(many, children, upd, ptr[0], ptr[1], c, vb, lane, [&](int i, T x) { dst[i] += x; });
+    }
+}
+
 inline int grid_for(int64_t n, int threads) {
     int64_t g = (n + threads - 1) / threads;
     if (g > 148 * 32) g = 148 * 32;
@@ -416,13 +502,13 @@ void launch_diag_shift(const int64_t *diag_off, int64_t n, double sigma, T *fact
 
 template <typename T>
 void launch_small_factor(const SmallTask *tasks, int count, int max_front, int vb, const AsmChild *children,
-                         const int32_t *cmap, T *factor, T *upd, PivotCtl pv, cudaStream_t st) {
+                         const int32_t *cmap, ManyDev many, T *factor, T *upd, PivotCtl pv, cudaStream_t st) {
     if (count <= 0) return;
     const int lp = (max_front + 3) & ~3;
     const size_t smem = (size_t(kSmallCols) * lp + size_t(max_front) * (max_front + 1) / 2) * sizeof(T);
     auto go = [&](auto kern, PerDeviceOnce &once) {
         once([kern] { cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmemOptin); });
-        kern<<<count, 256, smem, st>>>(tasks, vb, lp, children, cmap, factor, upd, pv);
+        kern<<<count, 256, smem, st>>>(tasks, vb, lp, children, cmap, many, factor, upd, pv);
     };
     // rows per lane from the level's largest front
     auto by_front = [&](auto k2, auto k3, auto k5, auto k8, PerDeviceOnce(&once)[4]) {
@@ -443,6 +529,14 @@ void launch_small_factor(const SmallTask *tasks, int count, int max_front, int v
     else
         by_front(small_factor_kernel<T, 0, 2, B2>, small_factor_kernel<T, 0, 3, B2>, small_factor_kernel<T, 0, 5, B5>,
                  small_factor_kernel<T, 0, 8, 1>, once0);
+}
+
+template <typename T>
+void launch_assemble_many(const ManyTask *tasks, int ntasks, SnDev sd, ManyDev many, const AsmChild *children, T *factor,
+                          T *upd, cudaStream_t st) {
+    if (ntasks <= 0) return;
+    ++g_kernel_launches;
+    assemble_many_kernel<T><<<ntasks, 256, 0, st>>>(tasks, sd, many, children, factor, upd);
 }
 
 template <typename T>
@@ -472,8 +566,10 @@ void launch_extract_diag(const int64_t *diag_off, int64_t n, const T *factor, do
     template void launch_inject<T>(const PlanEntryDev *, int64_t, int, int, const double *, const double *, double, \
                                    T *, cudaStream_t);                                                            \
     template void launch_diag_shift<T>(const int64_t *, int64_t, double, T *, cudaStream_t);                       \
-    template void launch_small_factor<T>(const SmallTask *, int, int, int, const AsmChild *, const int32_t *, T *, \
-                                         T *, PivotCtl, cudaStream_t);                                            \
+    template void launch_small_factor<T>(const SmallTask *, int, int, int, const AsmChild *, const int32_t *,      \
+                                         ManyDev, T *, T *, PivotCtl, cudaStream_t);                               \
+    template void launch_assemble_many<T>(const ManyTask *, int, SnDev, ManyDev, const AsmChild *, T *, T *,       \
+                                          cudaStream_t);                                                           \
     template void launch_assemble_large<T>(const AssembleTile *, int, int, const AssembleTask *, SnDev,            \
                                            const AsmChild *, const int32_t *, T *, T *, cudaStream_t);                                               \
     template void launch_extract_diag<T>(const int64_t *, int64_t, const T *, double *, cudaStream_t);

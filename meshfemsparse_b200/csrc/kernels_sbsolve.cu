@@ -628,13 +628,49 @@ __device__ __forceinline__ void bwd_vectors(const SbTask *tasks, int ntasks, con
     }
 }
 
+// The own rows of a forward task of a front of ManyDev: its children are waited for, a lane
+// each, then every row adds up its own list. (A call: rare, and inlined it costs the kernel
+// registers.)
+template <int NR>
+__device__ __noinline__ void gather_many(const SbTask *task, int vb, const SbChild *children, const ManyDev &many,
+                                         const double *X, int64_t ldx, int nrhs, const double *sol, const int *flags,
+                                         int *err, double *o) {
+    const int lane = threadIdx.x & 31, w = task->w, f = task->f, K = task->K;
+    const ManyFront mf = many.fronts[task->many];
+    for (int k = lane; k < mf.nwait; k += 32) {
+        const SbChild &c = children[mf.child0 + k];
+        if (c.flag >= 0) spin_count(flags + c.flag, c.need, err);
+    }
+    __syncwarp();
+#pragma unroll 1
+    for (int e = 0; e < 2; ++e) {
+        const int row = (K < 0 ? (w & ~3) : K * SB) + task->pad * 64 + lane + 32 * e, brow = row / vb;
+        const bool live = K < 0 ? (row >= w && row < f) : row < w;
+        double v[NR];
+#pragma unroll
+        for (int r = 0; r < NR; ++r) v[r] = live && K >= 0 && r < nrhs ? X[task->c0 + row + r * ldx] : 0.0;
+        const int64_t q1 = live ? many.ptr[mf.rows + brow + 1] : 0;
+#pragma unroll 2
+        for (int64_t q = live ? many.ptr[mf.rows + brow] : 0; q < q1; ++q) {
+            const int2 en = many.ent[q];
+            const SbChild &c = children[en.x];
+            const double *uc = sol + c.sol * nrhs + en.y * vb + row - brow * vb;
+            const int d = c.d;
+#pragma unroll
+            for (int r = 0; r < NR; ++r) v[r] += r < nrhs ? __ldcg(uc + int64_t(r) * d) : 0.0;
+        }
+#pragma unroll
+        for (int r = 0; r < NR; ++r) o[r * 64 + lane + 32 * e] = v[r];
+    }
+}
+
 // Gather warp `me`: every kGatherWarps-th task with its own rows, [r][64]. Forward: the
 // right-hand side of a diagonal task's rows plus the children's update vectors, in child
 // order; backward: y. What does not depend on a count (the task, its children, their row
 // maps) is loaded a task ahead.
 template <int NR, bool FWD>
 __device__ __forceinline__ void gather_own(const SbTask *tasks, int ntasks, int vb, const SbChild *children,
-                                           const int32_t *cmap, const double *X, int64_t ldx, int nrhs,
+                                           const int32_t *cmap, const ManyDev &many, const double *X, int64_t ldx, int nrhs,
                                            const double *sol, double *own, const SpRing &rg,
                                            const int *flags, int *err, int me) {
     constexpr int OS = own_slots(NR);
@@ -686,6 +722,12 @@ __device__ __forceinline__ void gather_own(const SbTask *tasks, int ntasks, int 
             SbChild ch[2] = {nx.ch[0], nx.ch[1]};
             int m[2][2] = {{nx.m[0][0], nx.m[0][1]}, {nx.m[1][0], nx.m[1][1]}};
             ahead(t + stride);
+            if (tk.many >= 0) {
+                if (it >= OS && !mbar_wait(rg.oempty + 8 * slot, uint32_t(it / OS - 1) & 1u, err)) return;
+                gather_many<NR>(tasks + t, vb, children, many, X, ldx, nrhs, sol, flags, err, own + slot * (NR * 64));
+                mbar_arrive(rg.ofull + 8 * slot);
+                continue;
+            }
             for (int ci = 0; ci < tk.nchild; ci += 2) {
                 if (ci) maps(tk, ci, ch, m);
 #pragma unroll
@@ -725,8 +767,8 @@ __device__ __forceinline__ void gather_own(const SbTask *tasks, int ntasks, int 
 template <typename T, int NST, int NR, int VS>
 __global__ void __launch_bounds__(kSbThreads, 1)
     sp_fwd_kernel(const SbTask *__restrict__ tasks, int ntasks, SnDev sd, const char *__restrict__ maps,
-                  const SbChild *__restrict__ children, const int32_t *__restrict__ cmap, double *X, int64_t ldx,
-                  int nrhs, double *sol, double *scratch, int *flags, int *err) {
+                  const SbChild *__restrict__ children, ManyDev many, const int32_t *__restrict__ cmap, double *X,
+                  int64_t ldx, int nrhs, double *sol, double *scratch, int *flags, int *err) {
     using Lay = SpLayout<T, NST, NR, VS>;
     using P = PT<T>;
     constexpr int FC = SpChunk<T>::FC, CE = SpChunk<T>::ELEMS, per = SB / FC;
@@ -760,7 +802,7 @@ __global__ void __launch_bounds__(kSbThreads, 1)
         return;
     }
     if (wp > 8) {
-        gather_own<NR, true>(tasks, ntasks, sd.vb, children, cmap, X, ldx, nrhs, sol, owns, rg, flags, err,
+        gather_own<NR, true>(tasks, ntasks, sd.vb, children, cmap, many, X, ldx, nrhs, sol, owns, rg, flags, err,
                               wp - 9 - kVecWarps);
         return;
     }
@@ -891,8 +933,8 @@ __global__ void __launch_bounds__(kSbThreads, 1)
 template <typename T, int NST, int NR, int VS>
 __global__ void __launch_bounds__(kSbThreads, 1)
     sp_bwd_kernel(const SbTask *__restrict__ tasks, int ntasks, SnDev sd, const char *__restrict__ maps,
-                  const SbChild *__restrict__ children, const int32_t *__restrict__ rowcnt, double *X, int64_t ldx,
-                  int nrhs, double *sol, double *scratch, int *flags, int *err) {
+                  const SbChild *__restrict__ children, ManyDev many, const int32_t *__restrict__ rowcnt, double *X,
+                  int64_t ldx, int nrhs, double *sol, double *scratch, int *flags, int *err) {
     using Lay = SpLayout<T, NST, NR, VS>;
     using P = PT<T>;
     using B = BwdLanes<T, NR>;
@@ -923,7 +965,7 @@ __global__ void __launch_bounds__(kSbThreads, 1)
     }
     if (wp == 9 + kVecWarps + kGatherWarps) return;      // (forward only)
     if (wp > 8) {
-        gather_own<NR, false>(tasks, ntasks, sd.vb, children, nullptr, X, ldx, nrhs, sol, owns, rg, flags, err,
+        gather_own<NR, false>(tasks, ntasks, sd.vb, children, nullptr, many, X, ldx, nrhs, sol, owns, rg, flags, err,
                                wp - 9 - kVecWarps);
         return;
     }
@@ -1215,8 +1257,8 @@ __global__ void __launch_bounds__(256) sb_diagonal_kernel(const SbTask *__restri
 // NR: the right-hand sides the vectors hold (nrhs <= NR)
 template <typename T, int NST, int NR, int VS>
 cudaError_t launch_sp_impl(bool forward, const SbTask *tasks, int ntasks, SnDev sd, const char *maps,
-                           const SbChild *children, const int32_t *rowmap, double *X, int64_t ldx, int nrhs, double *sol, double *scratch, int *flags, int *err,
-                           cudaStream_t st) {
+                           const SbChild *children, ManyDev many, const int32_t *cmap, const int32_t *rowcnt, double *X,
+                           int64_t ldx, int nrhs, double *sol, double *scratch, int *flags, int *err, cudaStream_t st) {
     using L = SpLayout<T, NST, NR, VS>;
     constexpr size_t smem = L::bytes + 128;
     static_assert(smem + 1024 <= size_t(kMaxSmemOptin), "superblock solve shared memory");
@@ -1229,9 +1271,11 @@ cudaError_t launch_sp_impl(bool forward, const SbTask *tasks, int ntasks, SnDev 
     // one CTA per SM (its shared memory); the parts of a superblock (at most four) must be
     // on different CTAs, which a grid of min(SMs, tasks) gives
     const int grid = std::min(device_sm_count(), ntasks);
-    void *args[] = {(void *)&tasks, (void *)&ntasks, (void *)&sd,   (void *)&maps, (void *)&children,
-                    (void *)&rowmap, (void *)&X,     (void *)&ldx,  (void *)&nrhs, (void *)&sol,
-                    (void *)&scratch, (void *)&flags, (void *)&err};
+    // (the kernels differ in this one argument)
+    const int32_t **rows = forward ? &cmap : &rowcnt;
+    void *args[] = {(void *)&tasks, (void *)&ntasks, (void *)&sd,  (void *)&maps, (void *)&children,
+                    (void *)&many,  (void *)rows,    (void *)&X,   (void *)&ldx,  (void *)&nrhs,
+                    (void *)&sol,   (void *)&scratch, (void *)&flags, (void *)&err};
     ++g_kernel_launches;
     return cudaLaunchCooperativeKernel(kern, dim3(grid), dim3(kSbThreads), args, smem, st);
 }
@@ -1259,13 +1303,15 @@ void launch_child_maps(const int32_t *parent, const int64_t *off, int nsn, SnDev
 
 template <typename T>
 cudaError_t launch_sb_solve(bool forward, const SbTask *tasks, int ntasks, SnDev sd, const void *maps,
-                            const SbChild *children, const int32_t *cmap, const int32_t *rowcnt, double *X, int64_t ldx,
-                            int nrhs, double *sol, double *scratch, int *flags, int *err, cudaStream_t st) {
+                            const SbChild *children, const int32_t *cmap, ManyDev many, const int32_t *rowcnt,
+                            double *X, int64_t ldx, int nrhs, double *sol, double *scratch, int *flags, int *err,
+                            cudaStream_t st) {
     const char *mp = static_cast<const char *>(maps);
     if (ntasks <= 0) return cudaSuccess;
     if (nrhs > kSbMaxRhs) return cudaErrorInvalidValue;
     auto go = [&](auto impl) {
-        return impl(forward, tasks, ntasks, sd, mp, children, forward ? cmap : rowcnt, X, ldx, nrhs, sol, scratch, flags, err, st);
+        return impl(forward, tasks, ntasks, sd, mp, children, many, cmap, rowcnt, X, ldx, nrhs, sol, scratch, flags, err,
+                    st);
     };
     // ring depth and vector buffers: the most that fit beside the sums of nrhs right-hand sides
     if (nrhs == 1) return go(launch_sp_impl<T, 6, 1, 4>);
@@ -1298,8 +1344,8 @@ void launch_sb_inverse(const SbTask *tasks, int ntasks, int max_rows, int ndiag,
 
 #define MFS_SB_INSTANTIATE(T)                                                                                      \
     template cudaError_t launch_sb_solve<T>(bool, const SbTask *, int, SnDev, const void *, const SbChild *,       \
-                                            const int32_t *, const int32_t *, double *, int64_t, int, double *,    \
-                                            double *, int *, int *, cudaStream_t);
+                                            const int32_t *, ManyDev, const int32_t *, double *, int64_t, int,     \
+                                            double *, double *, int *, int *, cudaStream_t);
 MFS_SB_INSTANTIATE(float)
 MFS_SB_INSTANTIATE(double)
 template void launch_sb_inverse<float>(const SbTask *, int, int, int, int, SnDev, float *, cudaStream_t);

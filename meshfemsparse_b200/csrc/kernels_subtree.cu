@@ -253,10 +253,10 @@ __device__ __forceinline__ void bwd_front(int s, const SnDev &sd, BlockDiv div, 
 // one entry from one such block of columns to the next, so that the loop over the blocks
 // is rolled: unrolled, with the block sizes 1 and 3 as template parameters, this file took
 // 674 s to compile and half of the object code was never run.
-template <typename T, int NSEG, int RB>
+template <typename T, int NSEG, int RB, bool MANY>
 __device__ __forceinline__ void fwd_small(const SubFront &sf, const T *__restrict__ factor,
                                           const SbChild *__restrict__ kids, const int32_t *__restrict__ cmap,
-                                          BlockDiv div, double *X, int64_t ldx, int nrhs, int r0, int nr, double *sol) {
+                                          const ManyDev &many, BlockDiv div, double *X, int64_t ldx, int nrhs, int r0, int nr, double *sol) {
     const int lane = threadIdx.x & 31;
     const int w = sf.w, f = sf.f;
     const T *pan = factor + sf.pan;
@@ -294,6 +294,23 @@ __device__ __forceinline__ void fwd_small(const SubFront &sf, const T *__restric
 #pragma unroll
             for (int g = 0; g < NSEG; ++g) v[r][g] += a[r][g];
     }
+    if constexpr (MANY)
+        if (sf.many >= 0) {                              // each row's own list, in child order
+            const int64_t *ptr = many.ptr + many.fronts[sf.many].rows;
+#pragma unroll
+            for (int g = 0; g < NSEG; ++g) {
+                const int i = lane + 32 * g, b = div(i);
+                if (i >= f) continue;
+#pragma unroll 1
+                for (int64_t q = ptr[b]; q < ptr[b + 1]; ++q) {
+                    const int2 en = many.ent[q];
+                    const SbChild ch = kids[en.x];
+                    const double *u = sol + ch.sol * nrhs + int64_t(r0) * ch.d + en.y * div.vb + i - b * div.vb;
+#pragma unroll
+                    for (int r = 0; r < RB; ++r) v[r][g] += r < nr ? u[r * ch.d] : 0.0;
+                }
+            }
+        }
     int jb = 0;
 #pragma unroll 1
     for (;; jb += 32) {
@@ -458,9 +475,9 @@ __device__ __forceinline__ void bwd_small(const SubFront &sf, const T *__restric
 // The same, for a small front in a CTA's walk: a call, so that the walk keeps its registers.
 template <typename T>
 __device__ __noinline__ void fwd_small_call(const SubFront *sf, const T *factor, const SbChild *kids,
-                                            const int32_t *cmap, BlockDiv div, double *X, int64_t ldx, int nrhs,
-                                            int r, double *sol) {
-    fwd_small<T, 8, 1>(*sf, factor, kids, cmap, div, X, ldx, nrhs, r, 1, sol);
+                                            const int32_t *cmap, const ManyDev &many, BlockDiv div, double *X,
+                                            int64_t ldx, int nrhs, int r, double *sol) {
+    fwd_small<T, 8, 1, true>(*sf, factor, kids, cmap, many, div, X, ldx, nrhs, r, 1, sol);
 }
 
 template <typename T>
@@ -495,8 +512,8 @@ __global__ void __launch_bounds__(kSubThreads) subtree_small_fwd_kernel(
                 next = fronts[s + 1];
                 prefetch_panel(next, factor);
             }
-            if (sf.f <= 64) fwd_small<T, 2, RB>(sf, factor, kids, cmap, div, X, ldx, nrhs, r0, nr, sol);
-            else fwd_small<T, NSEG, RB>(sf, factor, kids, cmap, div, X, ldx, nrhs, r0, nr, sol);
+            if (sf.f <= 64) fwd_small<T, 2, RB, false>(sf, factor, kids, cmap, ManyDev{}, div, X, ldx, nrhs, r0, nr, sol);
+            else fwd_small<T, NSEG, RB, false>(sf, factor, kids, cmap, ManyDev{}, div, X, ldx, nrhs, r0, nr, sol);
         }
     }
 }
@@ -507,7 +524,7 @@ template <typename T>
 __global__ void __launch_bounds__(kSubThreads, 3) subtree_fwd_kernel(
     const int32_t *__restrict__ top_ptr, const int32_t *__restrict__ tops, int nsub, SnDev sd, BlockDiv div,
     const SubFront *__restrict__ fronts, const SbChild *__restrict__ kids, const int32_t *__restrict__ cmap,
-    const T *__restrict__ factor, double *X, int64_t ldx, int nrhs, double *sol) {
+    ManyDev many, const T *__restrict__ factor, double *X, int64_t ldx, int nrhs, double *sol) {
     extern __shared__ __align__(16) double sub_smem[];
     double *red = sub_smem, *v = red + kSubRed;
     const int warp = threadIdx.x >> 5;
@@ -518,7 +535,7 @@ __global__ void __launch_bounds__(kSubThreads, 3) subtree_fwd_kernel(
             __syncthreads();                             // the children's u are there
             if (fronts[s].inv < 0) {
                 for (int r = warp; r < nrhs; r += kSubThreads / 32)
-                    fwd_small_call<T>(fronts + s, factor, kids, cmap, div, X, ldx, nrhs, r, sol);
+                    fwd_small_call<T>(fronts + s, factor, kids, cmap, many, div, X, ldx, nrhs, r, sol);
                 continue;
             }
             for (int rg = 0; rg < nrhs; rg += kSubRhs)
@@ -606,8 +623,8 @@ void launch_subtree_small(bool forward, const int2 *subs, int nsub, int fmax, Sn
 
 template <typename T>
 void launch_subtree_solve(bool forward, const int32_t *top_ptr, const int32_t *tops, int nsub, int fmax, SnDev sd,
-                          const SubFront *fronts, const SbChild *kids, const int32_t *cmap, const T *factor, double *X,
-                          int64_t ldx, int nrhs, double *sol, cudaStream_t st) {
+                          const SubFront *fronts, const SbChild *kids, const int32_t *cmap, ManyDev many,
+                          const T *factor, double *X, int64_t ldx, int nrhs, double *sol, cudaStream_t st) {
     if (nsub <= 0) return;
     const size_t smem = (size_t(kSubRed) + size_t(kSubRhs) * fmax) * sizeof(double);
     const int grid = std::min(nsub, 8 * device_sm_count());
@@ -619,8 +636,8 @@ void launch_subtree_solve(bool forward, const int32_t *top_ptr, const int32_t *t
     });
     ++g_kernel_launches;
     if (forward)
-        subtree_fwd_kernel<T><<<grid, kSubThreads, smem, st>>>(top_ptr, tops, nsub, sd, div, fronts, kids, cmap, factor,
-                                                               X, ldx, nrhs, sol);
+        subtree_fwd_kernel<T><<<grid, kSubThreads, smem, st>>>(top_ptr, tops, nsub, sd, div, fronts, kids, cmap, many,
+                                                               factor, X, ldx, nrhs, sol);
     else
         subtree_bwd_kernel<T><<<grid, kSubThreads, smem, st>>>(top_ptr, tops, nsub, sd, div, fronts, factor, X, ldx,
                                                                nrhs);
@@ -631,8 +648,8 @@ void launch_subtree_solve(bool forward, const int32_t *top_ptr, const int32_t *t
                                           const int32_t *, const T *, double *, int64_t, int, double *,              \
                                           cudaStream_t);                                                             \
     template void launch_subtree_solve<T>(bool, const int32_t *, const int32_t *, int, int, SnDev, const SubFront *, \
-                                          const SbChild *, const int32_t *, const T *, double *, int64_t, int,       \
-                                          double *, cudaStream_t);
+                                          const SbChild *, const int32_t *, ManyDev, const T *, double *, int64_t,   \
+                                          int, double *, cudaStream_t);
 MFS_SUBTREE(float)
 MFS_SUBTREE(double)
 #undef MFS_SUBTREE
