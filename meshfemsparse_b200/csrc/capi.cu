@@ -671,7 +671,7 @@ std::shared_ptr<DevSym> upload_symbolic(mfs_handle *h, std::shared_ptr<Symbolic>
     sd.struct_rows = ds->struct_rows.p;
     sd.rel = ds->rel.p;
     sd.vb = S.vb;
-    ds->many = {ds->many_fronts.p, ds->many_ptr.p, ds->many_ent.p, ds->rel.p};
+    ds->many = {many_fronts.empty() ? nullptr : ds->many_fronts.p, ds->many_ptr.p, ds->many_ent.p, ds->rel.p};
     {
         ds->parent.upload(par, st);
         ds->cmap_off.upload(cmap_off, st);

@@ -216,7 +216,7 @@ struct ManyFront {
     int32_t child0, nwait;               // its children; how many of them to look at for a count to wait for
 };
 struct ManyDev {
-    const ManyFront *fronts;
+    const ManyFront *fronts;             // null: there are none
     const int64_t *ptr;
     const int2 *ent;
     const int32_t *rel;                  // the structure rows' places in the parent's front (scalars)

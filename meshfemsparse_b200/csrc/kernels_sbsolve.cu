@@ -668,7 +668,7 @@ __device__ __noinline__ void gather_many(const SbTask *task, int vb, const SbChi
 // right-hand side of a diagonal task's rows plus the children's update vectors, in child
 // order; backward: y. What does not depend on a count (the task, its children, their row
 // maps) is loaded a task ahead.
-template <int NR, bool FWD>
+template <int NR, bool FWD, bool MANY>
 __device__ __forceinline__ void gather_own(const SbTask *tasks, int ntasks, int vb, const SbChild *children,
                                            const int32_t *cmap, const ManyDev &many, const double *X, int64_t ldx, int nrhs,
                                            const double *sol, double *own, const SpRing &rg,
@@ -722,12 +722,14 @@ __device__ __forceinline__ void gather_own(const SbTask *tasks, int ntasks, int 
             SbChild ch[2] = {nx.ch[0], nx.ch[1]};
             int m[2][2] = {{nx.m[0][0], nx.m[0][1]}, {nx.m[1][0], nx.m[1][1]}};
             ahead(t + stride);
-            if (tk.many >= 0) {
-                if (it >= OS && !mbar_wait(rg.oempty + 8 * slot, uint32_t(it / OS - 1) & 1u, err)) return;
-                gather_many<NR>(tasks + t, vb, children, many, X, ldx, nrhs, sol, flags, err, own + slot * (NR * 64));
-                mbar_arrive(rg.ofull + 8 * slot);
-                continue;
-            }
+            if constexpr (MANY)
+                if (tk.many >= 0) {
+                    if (it >= OS && !mbar_wait(rg.oempty + 8 * slot, uint32_t(it / OS - 1) & 1u, err)) return;
+                    gather_many<NR>(tasks + t, vb, children, many, X, ldx, nrhs, sol, flags, err,
+                                    own + slot * (NR * 64));
+                    mbar_arrive(rg.ofull + 8 * slot);
+                    continue;
+                }
             for (int ci = 0; ci < tk.nchild; ci += 2) {
                 if (ci) maps(tk, ci, ch, m);
 #pragma unroll
@@ -764,7 +766,9 @@ __device__ __forceinline__ void gather_own(const SbTask *tasks, int ntasks, int 
     }
 }
 
-template <typename T, int NST, int NR, int VS>
+// MANY: some front has more than kManyChildren children (the branch alone costs the eight-wide
+// form registers: 32 right-hand sides at k = 48 62.3 ms with it, 61.4 ms without).
+template <typename T, int NST, int NR, int VS, bool MANY>
 __global__ void __launch_bounds__(kSbThreads, 1)
     sp_fwd_kernel(const SbTask *__restrict__ tasks, int ntasks, SnDev sd, const char *__restrict__ maps,
                   const SbChild *__restrict__ children, ManyDev many, const int32_t *__restrict__ cmap, double *X,
@@ -802,7 +806,7 @@ __global__ void __launch_bounds__(kSbThreads, 1)
         return;
     }
     if (wp > 8) {
-        gather_own<NR, true>(tasks, ntasks, sd.vb, children, cmap, many, X, ldx, nrhs, sol, owns, rg, flags, err,
+        gather_own<NR, true, MANY>(tasks, ntasks, sd.vb, children, cmap, many, X, ldx, nrhs, sol, owns, rg, flags, err,
                               wp - 9 - kVecWarps);
         return;
     }
@@ -965,7 +969,7 @@ __global__ void __launch_bounds__(kSbThreads, 1)
     }
     if (wp == 9 + kVecWarps + kGatherWarps) return;      // (forward only)
     if (wp > 8) {
-        gather_own<NR, false>(tasks, ntasks, sd.vb, children, nullptr, many, X, ldx, nrhs, sol, owns, rg, flags, err,
+        gather_own<NR, false, false>(tasks, ntasks, sd.vb, children, nullptr, many, X, ldx, nrhs, sol, owns, rg, flags, err,
                                wp - 9 - kVecWarps);
         return;
     }
@@ -1262,10 +1266,13 @@ cudaError_t launch_sp_impl(bool forward, const SbTask *tasks, int ntasks, SnDev 
     using L = SpLayout<T, NST, NR, VS>;
     constexpr size_t smem = L::bytes + 128;
     static_assert(smem + 1024 <= size_t(kMaxSmemOptin), "superblock solve shared memory");
-    void *kern = forward ? (void *)sp_fwd_kernel<T, NST, NR, VS> : (void *)sp_bwd_kernel<T, NST, NR, VS>;
+    void *kern = !forward      ? (void *)sp_bwd_kernel<T, NST, NR, VS>
+                 : many.fronts ? (void *)sp_fwd_kernel<T, NST, NR, VS, true>
+                               : (void *)sp_fwd_kernel<T, NST, NR, VS, false>;
     static PerDeviceOnce once;
     once([] {
-        cudaFuncSetAttribute(sp_fwd_kernel<T, NST, NR, VS>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+        cudaFuncSetAttribute(sp_fwd_kernel<T, NST, NR, VS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+        cudaFuncSetAttribute(sp_fwd_kernel<T, NST, NR, VS, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
         cudaFuncSetAttribute(sp_bwd_kernel<T, NST, NR, VS>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     });
     // one CTA per SM (its shared memory); the parts of a superblock (at most four) must be
