@@ -60,6 +60,14 @@ int small_front_limit(const mfs_handle *h) {
     return h->opt.precision == MFS_PREC_FP32 ? 160 : 128;
 }
 
+// (the copy reads vec until the stream has passed it)
+template <typename B, typename V>
+void upload_array(B &buf, const V &vec, cudaStream_t st) {
+    buf.ensure(vec.size());
+    if (!vec.empty())
+        MFS_CUDA(cudaMemcpyAsync(buf.p, vec.data(), vec.size() * sizeof(vec[0]), cudaMemcpyHostToDevice, st));
+}
+
 std::shared_ptr<DevSym> upload_symbolic(mfs_handle *h, std::shared_ptr<Symbolic> Sp) {
     const Symbolic &S = *Sp;
     cudaStream_t st = h->stream;
@@ -357,15 +365,6 @@ std::shared_ptr<DevSym> upload_symbolic(mfs_handle *h, std::shared_ptr<Symbolic>
         L.syrk_n = int(gemm_tasks.size()) - L.syrk_off;
         L.syrk_tiles = sb;
     }
-    // ---- solve tasks (all supernodes, level by level)
-    const int RB = solve_rows_per_task();
-    const int DG = diag_blocks_per_task();
-    std::vector<int32_t> flag_base(nsn);
-    int nflags = 0;
-    for (idx s = 0; s < nsn; ++s) {
-        flag_base[s] = nflags;
-        nflags += int((S.w[s] + RB - 1) / RB);
-    }
     // Superblock diagonal solves of the levels above the solve cut: one flag and one
     // stored inverse (nrp x nrp, after the 64 x 64 diagonal inverses) per superblock.
     std::vector<SbTask> fsb, bsb, isb;
@@ -440,73 +439,6 @@ std::shared_ptr<DevSym> upload_symbolic(mfs_handle *h, std::shared_ptr<Symbolic>
                       many[s],
                       S.sol_off[s]};
     };
-    std::vector<SolveAsmTask> sasm;
-    std::vector<SolveTask> ftri, btri;
-    std::vector<StrTask> fstr, bstr;
-    std::vector<StrReduce> fred, bred;
-    int64_t max_str = 0;                          // partial-sum entries of one level and one right-hand side
-    for (idx l = 0; l < S.nlevels; ++l) {
-        LevelPlan &L = ds->levels[l];
-        L.sasm_off = int(sasm.size());
-        L.ftri_off = int(ftri.size());
-        L.btri_off = int(btri.size());
-        int base = 0, maxblk = 0, maxnbw = 0;
-        for (idx k = S.level_ptr[l]; k < S.level_ptr[l + 1]; ++k) {
-            const idx s = S.level_list[k];
-            if (S.child_ptr[s + 1] > S.child_ptr[s] || S.d[s] > 0) {
-                sasm.push_back({int32_t(s), base});
-                base += int((S.f[s] + kSolveAsmRows - 1) / kSolveAsmRows);
-            }
-            const int nbw = int((S.w[s] + RB - 1) / RB), nbd = int((S.d[s] + RB - 1) / RB);
-            maxblk = std::max(maxblk, nbw + nbd);
-            maxnbw = std::max(maxnbw, (nbw + DG - 1) / DG);
-        }
-        L.sasm_n = int(sasm.size()) - L.sasm_off;
-        L.sasm_tiles = base;
-        // ascending task (block pair) index across the level's fronts: every dependency
-        // precedes its task
-        for (int b = 0; b < maxnbw; ++b)
-            for (idx k = S.level_ptr[l]; k < S.level_ptr[l + 1]; ++k) {
-                const idx s = S.level_list[k];
-                const int nlk = int((S.w[s] + RB * DG - 1) / (RB * DG));
-                if (b < nlk) ftri.push_back({int32_t(s), b, flag_base[s], 0});
-            }
-        // structure slabs (rows from w rounded down to a multiple of 4): forward kStrRows-row
-        // slabs x kStrCols-column chunks, backward kStrBCols-column slabs x row chunks
-        L.fstr_off = int(fstr.size());
-        L.fred_off = int(fred.size());
-        L.bstr_off = int(bstr.size());
-        L.bred_off = int(bred.size());
-        const idx brows = str_bwd_rows(h->opt.precision != MFS_PREC_FP32);
-        for (idx k = S.level_ptr[l]; k < S.level_ptr[l + 1]; ++k) {
-            const idx s = S.level_list[k];
-            if (S.d[s] == 0) continue;
-            const idx span = S.f[s] - (S.w[s] & ~idx(3));
-            const int nrs = int((span + kStrRows - 1) / kStrRows), ncs = int((S.w[s] + kStrCols - 1) / kStrCols);
-            for (int a = 0; a < nrs; ++a) {
-                fred.push_back({int32_t(s), a, int32_t(fstr.size()) - L.fstr_off, ncs});
-                for (int c = 0; c < ncs; ++c) fstr.push_back({int32_t(s), a, c, 0});
-            }
-            const int nws = int((S.w[s] + kStrBCols - 1) / kStrBCols), nds = int((span + brows - 1) / brows);
-            for (int a = 0; a < nws; ++a) {
-                bred.push_back({int32_t(s), a, int32_t(bstr.size()) - L.bstr_off, nds});
-                for (int c = 0; c < nds; ++c) bstr.push_back({int32_t(s), a, c, 0});
-            }
-        }
-        L.fstr_n = int(fstr.size()) - L.fstr_off;
-        L.fred_n = int(fred.size()) - L.fred_off;
-        L.bstr_n = int(bstr.size()) - L.bstr_off;
-        L.bred_n = int(bred.size()) - L.bred_off;
-        max_str = std::max<int64_t>(max_str, std::max(int64_t(L.fstr_n) * kStrRows, int64_t(L.bstr_n) * kStrBCols));
-        for (int p = 0; p < maxnbw; ++p)
-            for (idx k = S.level_ptr[l]; k < S.level_ptr[l + 1]; ++k) {
-                const idx s = S.level_list[k];
-                const int nlk = int((S.w[s] + RB * DG - 1) / (RB * DG));
-                if (p < nlk) btri.push_back({int32_t(s), nlk - 1 - p, flag_base[s], 0});
-            }
-        L.ftri_n = int(ftri.size()) - L.ftri_off;
-        L.btri_n = int(btri.size()) - L.btri_off;
-    }
     // Tasks of the solves above the cut, in an order in which every dependency precedes
     // its task and the parts of a superblock are adjacent. Forward: levels ascending;
     // inside a level the superblocks in ascending order across the fronts, each front's
@@ -550,11 +482,7 @@ std::shared_ptr<DevSym> upload_symbolic(mfs_handle *h, std::shared_ptr<Symbolic>
     ds->inv_off.upload(inv_off, st);
     // (+64: the solves' 16-byte loads of a panel column may reach 3 elements past its end)
     ds->factor_alloc = inv_end + 64;
-    auto up = [&](auto &buf, const auto &vec) {
-        buf.ensure(vec.size());
-        if (!vec.empty())
-            MFS_CUDA(cudaMemcpyAsync(buf.p, vec.data(), vec.size() * sizeof(vec[0]), cudaMemcpyHostToDevice, st));
-    };
+    auto up = [&](auto &buf, const auto &vec) { upload_array(buf, vec, st); };
     up(ds->small_tasks, small_tasks);
     up(ds->asm_tasks, asm_tasks);
     up(ds->asm_children, asm_children);
@@ -575,13 +503,6 @@ std::shared_ptr<DevSym> upload_symbolic(mfs_handle *h, std::shared_ptr<Symbolic>
         if (g.lower && g.mode == 0) fl = 2.0 * k * (m * n - std::min(m, n) * (std::min(m, n) - 1.0) / 2.0);
         ds->gemm_flops_prefix[t + 1] = ds->gemm_flops_prefix[t] + fl;
     }
-    up(ds->sasm_tasks, sasm);
-    up(ds->ftri_tasks, ftri);
-    up(ds->btri_tasks, btri);
-    up(ds->fstr_tasks, fstr);
-    up(ds->bstr_tasks, bstr);
-    up(ds->fred, fred);
-    up(ds->bred, bred);
     up(ds->fsb_tasks, fsb);
     up(ds->bsb_tasks, bsb);
     ds->isb_host = isb;
@@ -607,7 +528,6 @@ std::shared_ptr<DevSym> upload_symbolic(mfs_handle *h, std::shared_ptr<Symbolic>
         isb.insert(isb.end(), diag.begin(), diag.end());
         up(ds->isb_tasks, isb);
     }
-    ds->max_str_entries = max_str;
     {
         // below the cut: the largest subtrees without stored inverses or many children, and
         // per subtree of the cut the fronts above those
@@ -651,7 +571,7 @@ std::shared_ptr<DevSym> upload_symbolic(mfs_handle *h, std::shared_ptr<Symbolic>
         up(ds->sub_fronts, sf);
         ds->solve_cut = int(S.solve_cut);
     }
-    ds->flags.ensure(size_t(std::max(std::max(nflags, nsbflags), 1)));
+    ds->flags.ensure(size_t(std::max(nsbflags, 1)));
     MFS_CUDA(cudaMemsetAsync(ds->flags.p, 0, ds->flags.bytes(), st));
     MFS_CUDA(cudaStreamSynchronize(st));
 
@@ -995,6 +915,101 @@ void factor_sequence(mfs_handle *h, DevSym &ds, T *factor, T *upd, T *dscr, cons
     MFS_CUDA(cudaGraphLaunch(exec, st));
 }
 
+// Task lists of the level-scheduled solves above the cut (solve_chain = 1), built when a
+// handle first solves that way.
+void ensure_chain_tasks(mfs_handle *h, DevSym &ds) {
+    if (ds.chain_built) return;
+    const Symbolic &S = *ds.S;
+    cudaStream_t st = h->stream;
+    const idx nsn = S.nsn;
+    const int RB = solve_rows_per_task();
+    const int DG = diag_blocks_per_task();
+    std::vector<int32_t> flag_base(nsn);
+    int nflags = 0;
+    for (idx s = 0; s < nsn; ++s) {
+        flag_base[s] = nflags;
+        nflags += int((S.w[s] + RB - 1) / RB);
+    }
+    std::vector<SolveAsmTask> sasm;
+    std::vector<SolveTask> ftri, btri;
+    std::vector<StrTask> fstr, bstr;
+    std::vector<StrReduce> fred, bred;
+    int64_t max_str = 0;                          // partial-sum entries of one level and one right-hand side
+    for (idx l = 0; l < S.nlevels; ++l) {
+        LevelPlan &L = ds.levels[l];
+        L.sasm_off = int(sasm.size());
+        L.ftri_off = int(ftri.size());
+        L.btri_off = int(btri.size());
+        int base = 0, maxblk = 0, maxnbw = 0;
+        for (idx k = S.level_ptr[l]; k < S.level_ptr[l + 1]; ++k) {
+            const idx s = S.level_list[k];
+            if (S.child_ptr[s + 1] > S.child_ptr[s] || S.d[s] > 0) {
+                sasm.push_back({int32_t(s), base});
+                base += int((S.f[s] + kSolveAsmRows - 1) / kSolveAsmRows);
+            }
+            const int nbw = int((S.w[s] + RB - 1) / RB), nbd = int((S.d[s] + RB - 1) / RB);
+            maxblk = std::max(maxblk, nbw + nbd);
+            maxnbw = std::max(maxnbw, (nbw + DG - 1) / DG);
+        }
+        L.sasm_n = int(sasm.size()) - L.sasm_off;
+        L.sasm_tiles = base;
+        // ascending task (block pair) index across the level's fronts: every dependency
+        // precedes its task
+        for (int b = 0; b < maxnbw; ++b)
+            for (idx k = S.level_ptr[l]; k < S.level_ptr[l + 1]; ++k) {
+                const idx s = S.level_list[k];
+                const int nlk = int((S.w[s] + RB * DG - 1) / (RB * DG));
+                if (b < nlk) ftri.push_back({int32_t(s), b, flag_base[s], 0});
+            }
+        // structure slabs (rows from w rounded down to a multiple of 4): forward kStrRows-row
+        // slabs x kStrCols-column chunks, backward kStrBCols-column slabs x row chunks
+        L.fstr_off = int(fstr.size());
+        L.fred_off = int(fred.size());
+        L.bstr_off = int(bstr.size());
+        L.bred_off = int(bred.size());
+        const idx brows = str_bwd_rows(h->opt.precision != MFS_PREC_FP32);
+        for (idx k = S.level_ptr[l]; k < S.level_ptr[l + 1]; ++k) {
+            const idx s = S.level_list[k];
+            if (S.d[s] == 0) continue;
+            const idx span = S.f[s] - (S.w[s] & ~idx(3));
+            const int nrs = int((span + kStrRows - 1) / kStrRows), ncs = int((S.w[s] + kStrCols - 1) / kStrCols);
+            for (int a = 0; a < nrs; ++a) {
+                fred.push_back({int32_t(s), a, int32_t(fstr.size()) - L.fstr_off, ncs});
+                for (int c = 0; c < ncs; ++c) fstr.push_back({int32_t(s), a, c, 0});
+            }
+            const int nws = int((S.w[s] + kStrBCols - 1) / kStrBCols), nds = int((span + brows - 1) / brows);
+            for (int a = 0; a < nws; ++a) {
+                bred.push_back({int32_t(s), a, int32_t(bstr.size()) - L.bstr_off, nds});
+                for (int c = 0; c < nds; ++c) bstr.push_back({int32_t(s), a, c, 0});
+            }
+        }
+        L.fstr_n = int(fstr.size()) - L.fstr_off;
+        L.fred_n = int(fred.size()) - L.fred_off;
+        L.bstr_n = int(bstr.size()) - L.bstr_off;
+        L.bred_n = int(bred.size()) - L.bred_off;
+        max_str = std::max<int64_t>(max_str, std::max(int64_t(L.fstr_n) * kStrRows, int64_t(L.bstr_n) * kStrBCols));
+        for (int p = 0; p < maxnbw; ++p)
+            for (idx k = S.level_ptr[l]; k < S.level_ptr[l + 1]; ++k) {
+                const idx s = S.level_list[k];
+                const int nlk = int((S.w[s] + RB * DG - 1) / (RB * DG));
+                if (p < nlk) btri.push_back({int32_t(s), nlk - 1 - p, flag_base[s], 0});
+            }
+        L.ftri_n = int(ftri.size()) - L.ftri_off;
+        L.btri_n = int(btri.size()) - L.btri_off;
+    }
+    ds.max_str_entries = max_str;
+    upload_array(ds.sasm_tasks, sasm, st);
+    upload_array(ds.ftri_tasks, ftri, st);
+    upload_array(ds.btri_tasks, btri, st);
+    upload_array(ds.fstr_tasks, fstr, st);
+    upload_array(ds.bstr_tasks, bstr, st);
+    upload_array(ds.fred, fred, st);
+    upload_array(ds.bred, bred, st);
+    ds.flags.ensure(size_t(std::max(nflags, 1)));
+    MFS_CUDA(cudaStreamSynchronize(st));
+    ds.chain_built = true;
+}
+
 template <typename T>
 void run_solve(mfs_handle *h, DevSym &ds, const T *factor, double *X, int nrhs) {
     const Symbolic &S = *ds.S;
@@ -1007,6 +1022,7 @@ void run_solve(mfs_handle *h, DevSym &ds, const T *factor, double *X, int nrhs) 
         h->sb_scratch.ensure(size_t(std::max<idx>(S.n, 1)) * chunk);
         ensure_solve_maps(h, ds, factor, int(sizeof(T)));
     } else {
+        ensure_chain_tasks(h, ds);
         h->str_partials.ensure(size_t(std::max<int64_t>(ds.max_str_entries, 1)) * chunk);
     }
     for (int r0 = 0; r0 < nrhs; r0 += pass) {

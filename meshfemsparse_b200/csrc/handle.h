@@ -85,7 +85,7 @@ struct LevelPlan {
     };
     std::vector<Step> steps;
     int syrk_off = 0, syrk_n = 0, syrk_tiles = 0;
-    // solve task lists of this level
+    // task lists of this level in the solves by levels (solve_chain = 1)
     int sasm_off = 0, sasm_n = 0, sasm_tiles = 0;
     int ftri_off = 0, ftri_n = 0;
     int btri_off = 0, btri_n = 0;
@@ -118,6 +118,7 @@ struct DevSym {
     DBuf<int2> many_ent;
     DBuf<PanelTask> potrf_tasks;
     DBuf<GemmTask> gemm_tasks;
+    bool chain_built = false;            // the task lists of solve_chain = 1, down to bred (built on first use)
     DBuf<SolveAsmTask> sasm_tasks;
     DBuf<SolveTask> ftri_tasks, btri_tasks;
     DBuf<StrTask> fstr_tasks, bstr_tasks;
