@@ -75,68 +75,66 @@ __device__ __forceinline__ void fwd_front(int s, const SnDev &sd, BlockDiv div, 
         __syncthreads();
     }
     const int64_t inv = sd.inv_off[s];
-    if (inv >= 0) {
-        const int nbw = (w + 63) / 64;
-        const int i = tid & 63, g = tid >> 6;             // row of the block, k-split group (4)
-        for (int rb = 0; rb < nbw; ++rb) {
-            const int r0 = rb * 64, nrr = min(64, w - r0);
-            if (rb > 0) {
-                // v[r0 + i] -= sum_{j < r0} L(r0 + i, j) y_j, j split over the 4 groups
-                double acc[kSubRhs] = {0.0, 0.0, 0.0, 0.0};
-                if (i < nrr)
-                    for (int j = g; j < r0; j += 4) {
-                        const double l = double(pan[int64_t(j) * ld + r0 + i]);
-#pragma unroll
-                        for (int r = 0; r < kSubRhs; ++r)
-                            if (r < nr) acc[r] += l * v[r * f + j];
-                    }
-#pragma unroll
-                for (int r = 0; r < kSubRhs; ++r) red[(g * kSubRhs + r) * 64 + i] = acc[r];
-                __syncthreads();
-                if (g == 0 && i < nrr)
-#pragma unroll
-                    for (int r = 0; r < kSubRhs; ++r)
-                        if (r < nr)
-                            v[r * f + r0 + i] -= red[r * 64 + i] + red[(kSubRhs + r) * 64 + i] +
-                                                 red[(2 * kSubRhs + r) * 64 + i] + red[(3 * kSubRhs + r) * 64 + i];
-                __syncthreads();
-            }
-            // y = inv(L(rb, rb)) v_block, j split over the 4 groups
-            {
-                const T *ib = factor + inv + int64_t(rb) * 4096;   // column-major 64 x 64
-                double acc[kSubRhs] = {0.0, 0.0, 0.0, 0.0};
-                if (i < nrr)
-                    for (int j = g; j <= i; j += 4) {
-                        const double l = double(ib[j * 64 + i]);
-#pragma unroll
-                        for (int r = 0; r < kSubRhs; ++r)
-                            if (r < nr) acc[r] += l * v[r * f + r0 + j];
-                    }
-#pragma unroll
-                for (int r = 0; r < kSubRhs; ++r) red[(g * kSubRhs + r) * 64 + i] = acc[r];
-                __syncthreads();
-                if (g == 0 && i < nrr)
-#pragma unroll
-                    for (int r = 0; r < kSubRhs; ++r)
-                        if (r < nr)
-                            v[r * f + r0 + i] = red[r * 64 + i] + red[(kSubRhs + r) * 64 + i] +
-                                                red[(2 * kSubRhs + r) * 64 + i] + red[(3 * kSubRhs + r) * 64 + i];
-                __syncthreads();
-            }
-        }
-        // u = v[w:f] - L21 y
-        for (int k = tid; k < d; k += nt) {
+    const int nbw = (w + 63) / 64;
+    const int i = tid & 63, g = tid >> 6;             // row of the block, k-split group (4)
+    for (int rb = 0; rb < nbw; ++rb) {
+        const int r0 = rb * 64, nrr = min(64, w - r0);
+        if (rb > 0) {
+            // v[r0 + i] -= sum_{j < r0} L(r0 + i, j) y_j, j split over the 4 groups
             double acc[kSubRhs] = {0.0, 0.0, 0.0, 0.0};
-            for (int j = 0; j < w; ++j) {
-                const double l = double(pan[int64_t(j) * ld + w + k]);
+            if (i < nrr)
+                for (int j = g; j < r0; j += 4) {
+                    const double l = double(pan[int64_t(j) * ld + r0 + i]);
+#pragma unroll
+                    for (int r = 0; r < kSubRhs; ++r)
+                        if (r < nr) acc[r] += l * v[r * f + j];
+                }
+#pragma unroll
+            for (int r = 0; r < kSubRhs; ++r) red[(g * kSubRhs + r) * 64 + i] = acc[r];
+            __syncthreads();
+            if (g == 0 && i < nrr)
 #pragma unroll
                 for (int r = 0; r < kSubRhs; ++r)
-                    if (r < nr) acc[r] += l * v[r * f + j];
-            }
+                    if (r < nr)
+                        v[r * f + r0 + i] -= red[r * 64 + i] + red[(kSubRhs + r) * 64 + i] +
+                                             red[(2 * kSubRhs + r) * 64 + i] + red[(3 * kSubRhs + r) * 64 + i];
+            __syncthreads();
+        }
+        // y = inv(L(rb, rb)) v_block, j split over the 4 groups
+        {
+            const T *ib = factor + inv + int64_t(rb) * 4096;   // column-major 64 x 64
+            double acc[kSubRhs] = {0.0, 0.0, 0.0, 0.0};
+            if (i < nrr)
+                for (int j = g; j <= i; j += 4) {
+                    const double l = double(ib[j * 64 + i]);
+#pragma unroll
+                    for (int r = 0; r < kSubRhs; ++r)
+                        if (r < nr) acc[r] += l * v[r * f + r0 + j];
+                }
+#pragma unroll
+            for (int r = 0; r < kSubRhs; ++r) red[(g * kSubRhs + r) * 64 + i] = acc[r];
+            __syncthreads();
+            if (g == 0 && i < nrr)
+#pragma unroll
+                for (int r = 0; r < kSubRhs; ++r)
+                    if (r < nr)
+                        v[r * f + r0 + i] = red[r * 64 + i] + red[(kSubRhs + r) * 64 + i] +
+                                            red[(2 * kSubRhs + r) * 64 + i] + red[(3 * kSubRhs + r) * 64 + i];
+            __syncthreads();
+        }
+    }
+    // u = v[w:f] - L21 y
+    for (int k = tid; k < d; k += nt) {
+        double acc[kSubRhs] = {0.0, 0.0, 0.0, 0.0};
+        for (int j = 0; j < w; ++j) {
+            const double l = double(pan[int64_t(j) * ld + w + k]);
 #pragma unroll
             for (int r = 0; r < kSubRhs; ++r)
-                if (r < nr) v[r * f + w + k] -= acc[r];
+                if (r < nr) acc[r] += l * v[r * f + j];
         }
+#pragma unroll
+        for (int r = 0; r < kSubRhs; ++r)
+            if (r < nr) v[r * f + w + k] -= acc[r];
     }
     __syncthreads();
     const bool has_u = d > 0 && sd.sol_off[s] >= 0;
@@ -169,7 +167,7 @@ __device__ __forceinline__ void bwd_front(int s, const SnDev &sd, BlockDiv div, 
     __syncthreads();
     const int64_t inv = sd.inv_off[s];
     // v[0:w] -= L21^T x_struct: one warp per column, lanes over rows
-    if (d > 0 && inv >= 0) {
+    if (d > 0) {
         for (int j = warp; j < w; j += nw) {
             double acc[kSubRhs] = {0.0, 0.0, 0.0, 0.0};
             for (int k = lane; k < d; k += 32) {
@@ -186,57 +184,55 @@ __device__ __forceinline__ void bwd_front(int s, const SnDev &sd, BlockDiv div, 
         }
         __syncthreads();
     }
-    if (inv >= 0) {
-        const int nbw = (w + 63) / 64;
-        for (int rb = nbw - 1; rb >= 0; --rb) {
-            const int r0 = rb * 64, nrr = min(64, w - r0);
-            if (r0 + 64 < w) {
-                // v[r0 + j] -= sum_{i >= r0 + 64} L(i, r0 + j) x_i
-                for (int j = warp; j < nrr; j += nw) {
-                    double acc[kSubRhs] = {0.0, 0.0, 0.0, 0.0};
-                    for (int i = r0 + 64 + lane; i < w; i += 32) {
-                        const double l = double(pan[int64_t(r0 + j) * ld + i]);
+    const int nbw = (w + 63) / 64;
+    for (int rb = nbw - 1; rb >= 0; --rb) {
+        const int r0 = rb * 64, nrr = min(64, w - r0);
+        if (r0 + 64 < w) {
+            // v[r0 + j] -= sum_{i >= r0 + 64} L(i, r0 + j) x_i
+            for (int j = warp; j < nrr; j += nw) {
+                double acc[kSubRhs] = {0.0, 0.0, 0.0, 0.0};
+                for (int i = r0 + 64 + lane; i < w; i += 32) {
+                    const double l = double(pan[int64_t(r0 + j) * ld + i]);
+#pragma unroll
+                    for (int r = 0; r < kSubRhs; ++r)
+                        if (r < nr) acc[r] += l * v[r * f + i];
+                }
+#pragma unroll
+                for (int r = 0; r < kSubRhs; ++r) {
+                    const double sum = warp_sum(acc[r]);
+                    if (lane == 0 && r < nr) v[r * f + r0 + j] -= sum;
+                }
+            }
+            __syncthreads();
+        }
+        // x_block = inv(L(rb, rb))^T v_block, one warp per column of the inverse
+        const T *ib = factor + inv + int64_t(rb) * 4096;
+        for (int j0 = 0; j0 < nrr; j0 += 2 * nw) {          // 2 columns per warp and round
+            double out[2][kSubRhs];
+#pragma unroll
+            for (int t = 0; t < 2; ++t) {
+                const int j = j0 + warp + t * nw;
+                double acc[kSubRhs] = {0.0, 0.0, 0.0, 0.0};
+                if (j < nrr)
+                    for (int i = j + lane; i < nrr; i += 32) {
+                        const double l = double(ib[j * 64 + i]);
 #pragma unroll
                         for (int r = 0; r < kSubRhs; ++r)
-                            if (r < nr) acc[r] += l * v[r * f + i];
+                            if (r < nr) acc[r] += l * v[r * f + r0 + i];
                     }
 #pragma unroll
-                    for (int r = 0; r < kSubRhs; ++r) {
-                        const double sum = warp_sum(acc[r]);
-                        if (lane == 0 && r < nr) v[r * f + r0 + j] -= sum;
-                    }
-                }
-                __syncthreads();
+                for (int r = 0; r < kSubRhs; ++r) out[t][r] = warp_sum(acc[r]);
             }
-            // x_block = inv(L(rb, rb))^T v_block, one warp per column of the inverse
-            const T *ib = factor + inv + int64_t(rb) * 4096;
-            for (int j0 = 0; j0 < nrr; j0 += 2 * nw) {          // 2 columns per warp and round
-                double out[2][kSubRhs];
+            __syncthreads();                              // all reads of this round done
 #pragma unroll
-                for (int t = 0; t < 2; ++t) {
-                    const int j = j0 + warp + t * nw;
-                    double acc[kSubRhs] = {0.0, 0.0, 0.0, 0.0};
-                    if (j < nrr)
-                        for (int i = j + lane; i < nrr; i += 32) {
-                            const double l = double(ib[j * 64 + i]);
+            for (int t = 0; t < 2; ++t) {
+                const int j = j0 + warp + t * nw;
+                if (lane == 0 && j < nrr)
 #pragma unroll
-                            for (int r = 0; r < kSubRhs; ++r)
-                                if (r < nr) acc[r] += l * v[r * f + r0 + i];
-                        }
-#pragma unroll
-                    for (int r = 0; r < kSubRhs; ++r) out[t][r] = warp_sum(acc[r]);
-                }
-                __syncthreads();                              // all reads of this round done
-#pragma unroll
-                for (int t = 0; t < 2; ++t) {
-                    const int j = j0 + warp + t * nw;
-                    if (lane == 0 && j < nrr)
-#pragma unroll
-                        for (int r = 0; r < kSubRhs; ++r)
-                            if (r < nr) v[r * f + r0 + j] = out[t][r];
-                }
-                __syncthreads();
+                    for (int r = 0; r < kSubRhs; ++r)
+                        if (r < nr) v[r * f + r0 + j] = out[t][r];
             }
+            __syncthreads();
         }
     }
     __syncthreads();
