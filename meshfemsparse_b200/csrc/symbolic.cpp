@@ -578,8 +578,21 @@ std::string analyze(idx nblocks, const idx *Ap, const idx *Ai, int bs, const idx
         for (idx s = 0; s < nsn; ++s)
             for (idx l = S.level[s]; l < (S.sn_parent[s] < 0 ? S.nlevels : S.level[S.sn_parent[s]]); ++l)
                 ++roots_at[l];
+        // A subtree is walked as a range of supernodes: [s - size(s) + 1, s] for root s where
+        // the numbering is a postorder there, which natural and user orders need not be. The
+        // cut stays below the lowest subtree that is no range.
+        std::vector<idx> size(nsn, 1), first(nsn);
+        idx whole = S.nlevels;
+        std::iota(first.begin(), first.end(), idx(0));
+        for (idx s = 0; s < nsn; ++s) {
+            if (s - first[s] + 1 != size[s]) whole = std::min(whole, idx(S.level[s]));
+            const idx p = S.sn_parent[s];
+            if (p < 0) continue;
+            size[p] += size[s];
+            first[p] = std::min(first[p], first[s]);
+        }
         for (idx want : {kManySubtrees, kFewSubtrees, kMinSubtrees}) {
-            for (idx l = S.nlevels - 2; l >= 0; --l) {
+            for (idx l = std::min(S.nlevels - 1, whole) - 1; l >= 0; --l) {
                 if (fmax_le[l] > kSubFmax || roots_at[l] < want) continue;
                 S.solve_cut = l;
                 S.sub_fmax = fmax_le[l];
@@ -588,10 +601,6 @@ std::string analyze(idx nblocks, const idx *Ap, const idx *Ai, int bs, const idx
             if (S.solve_cut >= 0) break;
         }
         if (S.solve_cut >= 0) {
-            // subtree of root s = [s - size(s) + 1, s] in postorder
-            std::vector<idx> size(nsn, 1);
-            for (idx s = 0; s < nsn; ++s)
-                if (S.sn_parent[s] >= 0) size[S.sn_parent[s]] += size[s];
             std::vector<std::pair<double, idx>> work;
             for (idx s = 0; s < nsn; ++s) {
                 if (S.level[s] > S.solve_cut) continue;
