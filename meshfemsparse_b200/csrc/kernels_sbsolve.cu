@@ -1090,21 +1090,27 @@ __global__ void __launch_bounds__(kSbThreads, 1)
 }
 
 // inv(L_KK) of superblock K of front s (nr rows), nrp x nrp column-major at
-// factor + tk.inv, one CTA per 16 columns of it (blockIdx.y; columns of 64-column block b):
+// factor + tk.inv, one CTA per NC columns of it (blockIdx.y; columns of 64-column block b):
 //   X_bb = D_b, X_ab = -D_a sum_{c=b}^{a-1} L_ac X_cb for a > b, X_ab = 0 for a < b,
 // with D_a = inv(L_aa) the 64 x 64 diagonal inverses: the panel kernel's stored ones when
 // the front has them, else (given) what sb_diagonal_kernel left in place, else by
 // substitution on L_aa (all threads, a barrier a row). The
 // columns' blocks X_cb stay in shared memory; each L_ac and D_a is loaded into registers
-// while the product before runs and staged there for its own 64 x 64 x 16 one (thread = row
-// i, 4 columns). Bound by the chain of up to nine products of a superblock where there are
-// few of them: with 64 columns a CTA, no loads ahead and one thread per column in the
-// substitution, 90 us for the 7-sided cube and 120 us for the 20-sided one in FP64, 34
-// and 87 us this way.
-template <typename T>
+// while the product before runs and staged there for its own 64 x 64 x NC one (thread = row
+// i, NC / 4 columns).
+// NC: few superblocks are bound by the chain of up to nine products, which 16 columns make the
+// shortest (with 64 columns, no loads ahead and one thread per column in the substitution
+// 90 us for the 7-sided cube and 120 us for the 20-sided one in FP64, 34 and 74 us this
+// way). More than kSbInverseMany of them fill the SMs and are bound by the blocks' loads and
+// staging, which 32 columns halve: FP32, 16 and 32 columns, 166 superblocks 29 and 36 us,
+// 276 41 and 49, 453 54 and 54, 872 99 and 68, 936 127 and 87 us, a batch of 48 cubes 854 and
+// 553 us, the 64-sided cube 1,572 and 1,046 us. 64 columns are one CTA an SM (615 us for the
+// batch). In FP64 32 columns are one CTA an SM, too: the 48-sided cube 996 and 1,052 us.
+constexpr int kSbInverseMany = 512;
+template <typename T, int NC>
 __global__ void __launch_bounds__(256) sb_inverse_kernel(const SbTask *__restrict__ tasks, SnDev sd, bool given,
                                                          T *factor) {
-    constexpr int LD = 65, NC = 16;
+    constexpr int LD = 65, U = NC / 4;                    // columns a thread
     extern __shared__ __align__(16) double inv_smem[];
     T *Xc = reinterpret_cast<T *>(inv_smem);              // [4][NC][LD]: X_cb, c = b .. nbk - 1
     T *Tt = Xc + 4 * NC * LD;                             // [NC][LD]: sum L_ac X_cb
@@ -1173,46 +1179,48 @@ __global__ void __launch_bounds__(256) sb_inverse_kernel(const SbTask *__restric
     {
         const T *D = diagonal(b);
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int j = jg * 4 + u;
+        for (int u = 0; u < U; ++u) {
+            const int j = jg * U + u;
             const T x = D[(j0 + j) * LD + i];
             Xc[j * LD + i] = x;
             if (dinv >= 0 || !given) out[int64_t(b * 64 + j0 + j) * nrp + b * 64 + i] = x;
         }
     }
     for (int a = b + 1; a < nbk; ++a) {
-        T acc[4] = {T(0), T(0), T(0), T(0)};
+        T acc[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) acc[u] = T(0);
         for (int c = b; c < a; ++c) {
             __syncthreads();                               // Ls is free
             stage(Ls);
             fetch(a, c + 1);
             __syncthreads();
-            const T *X = Xc + ((c - b) * NC + jg * 4) * LD;
+            const T *X = Xc + ((c - b) * NC + jg * U) * LD;
 #pragma unroll 8
             for (int m = 0; m < 64; ++m) {
                 const T l = Ls[m * LD + i];
 #pragma unroll
-                for (int u = 0; u < 4; ++u) acc[u] += l * X[u * LD + m];
+                for (int u = 0; u < U; ++u) acc[u] += l * X[u * LD + m];
             }
         }
         __syncthreads();                                   // Ls, Ds and Tt are free
 #pragma unroll
-        for (int u = 0; u < 4; ++u) Tt[(jg * 4 + u) * LD + i] = acc[u];
+        for (int u = 0; u < U; ++u) Tt[(jg * U + u) * LD + i] = acc[u];
         stage(Ds);
         fetch(a + 1, b);
         const T *D = diagonal(a);
-        const T *Tj = Tt + jg * 4 * LD;
+        const T *Tj = Tt + jg * U * LD;
 #pragma unroll
-        for (int u = 0; u < 4; ++u) acc[u] = T(0);
+        for (int u = 0; u < U; ++u) acc[u] = T(0);
 #pragma unroll 8
         for (int m = 0; m < 64; ++m) {
             const T dv = D[m * LD + i];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) acc[u] -= dv * Tj[u * LD + m];
+            for (int u = 0; u < U; ++u) acc[u] -= dv * Tj[u * LD + m];
         }
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int j = jg * 4 + u;
+        for (int u = 0; u < U; ++u) {
+            const int j = jg * U + u;
             Xc[((a - b) * NC + j) * LD + i] = acc[u];
             out[int64_t(b * 64 + j0 + j) * nrp + a * 64 + i] = acc[u];
         }
@@ -1342,11 +1350,20 @@ void launch_sb_inverse(const SbTask *tasks, int ntasks, int max_rows, int ndiag,
         sb_diagonal_kernel<T><<<ndiag, 256, smem, st>>>(tasks + ntasks, sd, ld, factor);
     }
     if (ntasks <= 0) return;
-    const size_t smem = size_t(5 * 16 + 2 * 64) * 65 * sizeof(T);
-    static PerDeviceOnce once;
-    once([smem] { cudaFuncSetAttribute(sb_inverse_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)); });
-    ++g_kernel_launches;
-    sb_inverse_kernel<T><<<dim3(ntasks, 4 * ((max_rows + 63) / 64)), 256, smem, st>>>(tasks, sd, ndiag > 0, factor);
+    auto go = [&](auto cols, PerDeviceOnce &once) {
+        constexpr int NC = decltype(cols)::value;
+        constexpr size_t smem = size_t(5 * NC + 2 * 64) * 65 * sizeof(T);
+        once([] {
+            cudaFuncSetAttribute(sb_inverse_kernel<T, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+        });
+        ++g_kernel_launches;
+        sb_inverse_kernel<T, NC><<<dim3(ntasks, 64 / NC * ((max_rows + 63) / 64)), 256, smem, st>>>(tasks, sd, ndiag > 0,
+                                                                                                   factor);
+    };
+    static PerDeviceOnce once16, once32;
+    if constexpr (sizeof(T) == 4)
+        if (ntasks > kSbInverseMany) return go(std::integral_constant<int, 32>{}, once32);
+    go(std::integral_constant<int, 16>{}, once16);
 }
 
 #define MFS_SB_INSTANTIATE(T)                                                                                      \
