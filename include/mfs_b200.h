@@ -89,16 +89,17 @@ typedef struct {
                                    reuses the previous separator tree, re-dissecting only the subtrees that a
                                    new edge violates (PARTH-style temporal reuse, ParallelNestedDissection/
                                    README.md:86-127); a full dissection every nd_reuse_period analyses */
-    int32_t solve_chain;        /* diagonal-block solves of the fronts above the subtree cut: 0 through the
-                                   inverses of 256-row superblocks of L11 (one CTA per superblock),
-                                   1 through chains of 64-row blocks (one CTA per pair of blocks) */
+    int32_t solve_chain;        /* solves of the fronts above the subtree cut: 0 one launch per direction, through
+                                   the inverses of 256-row superblocks of L11 (a CTA per 64 rows), 1 level by
+                                   level, through chains of 64-row blocks (one CTA per pair of blocks) */
     int32_t factor_group;       /* large fronts: column blocks per group of the blocked factorization (inside a
                                    group left-looking, after it one update of the rest of the front);
                                    0: default (4); read at the symbolic analysis */
     int32_t solve_subtrees;     /* solves: the levels below the highest level with at least this many subtrees
-                                   (fronts of at most 2048 rows) are solved one subtree per CTA, the levels above
-                                   by level kernels; 0: default (the larger of 2368 and 48 per tree of the
-                                   assembly forest); read at the symbolic analysis */
+                                   (fronts of at most 2048 rows, subtrees that are ranges of supernodes) are
+                                   solved subtree by subtree, the levels above as solve_chain says; 0: default (the
+                                   larger of 2368 and 48 per tree of the assembly forest, else 592, else 148);
+                                   read at the symbolic analysis */
     int32_t reserved[2];
 } mfs_options;
 

@@ -74,8 +74,8 @@ __device__ __forceinline__ double partial_sum(const double *__restrict__ partial
 // by one lane, the row's indices coalesced), NR right-hand sides a pass over the matrix.
 // HBM- or L2-bound: every stored block is read for its row and for its column. One thread
 // per scalar row took three passes over the indices, one pass over the matrix per
-// right-hand side and one load at a time: k = 64, four right-hand sides 380 us, one of them
-// about 200 us before, 89 us now.
+// right-hand side and one load at a time: k = 64, four right-hand sides 383 us before, 205 us
+// now; one of them about 200 us before, 89 us now.
 // dotp: kReduceBlocks partial sums of X . Y per column.
 template <int NR>
 __global__ void __launch_bounds__(256) spmv3_kernel(const int64_t *__restrict__ ptr, const int64_t *__restrict__ src,

@@ -18,9 +18,11 @@
 // at a barrier. The fronts above them are a CTA's per subtree of the cut, four right-hand
 // sides at a time, through the stored 64 x 64 inverses, v in shared memory. In one CTA walk for
 // all, with barriers, a division a column and the children one after the other, a pass over
-// the batch of 48 cubes (FP32, 8 right-hand sides) took 1,140 us forward and 1,160 us backward,
-// @@BF@@ and @@BB@@ us this way; k = 64 with 4: 690 us each way, @@KF@@ and @@KB@@ us. Subtrees are
-// assigned round-robin in order of decreasing work.
+// the batch of 48 cubes (FP32, 8 right-hand sides) took 1,160 us forward and 1,170 us backward;
+// now 209 us (small fronts) and 377 us (above them) forward, 406 and 498 us backward. The
+// 64-sided cube with 4: 687 us forward and 694 us backward before, 140 + 366 and 271 + 464 us
+// now (the fronts with stored inverses read L straight from global memory, which is what
+// bounds the larger half). Subtrees are assigned round-robin in order of decreasing work.
 #include "device.h"
 
 #include <algorithm>

@@ -560,11 +560,12 @@ std::string analyze(idx nblocks, const idx *Ap, const idx *Ai, int bs, const idx
     // ---- subtree solve cut: the highest level whose subtrees are many and small
     // (fronts <= kSubFmax rows). One CTA walks a subtree sequentially, so the
     // largest subtree bounds the phase: aim for kManySubtrees (16 per SM of a
-    // 148-SM B200, the measured optimum on the 811k-DOF cube; for a forest of many
-    // independent meshes 48 per tree, measured on a batch of 256: the solve 103.5 ->
-    // 87.9 ms against 2368), else settle for kFewSubtrees (four per SM: a solve of the
-    // 20-sided cube 0.38 ms instead of 0.73 ms with the 148 largest), else for kMinSubtrees
-    // (one per SM).
+    // 148-SM B200, the optimum on the 811k-DOF cube; for a forest of many
+    // independent meshes 48 per tree, on a batch of 256: the solve 103.5 ->
+    // 87.9 ms against 2368; both swept when a CTA walked every subtree whole and the
+    // levels above the cut were launches of their own), else settle for kFewSubtrees (four
+    // per SM: a solve of the 20-sided cube 0.38 ms instead of 0.73 ms with the 148 largest),
+    // else for kMinSubtrees (one per SM).
     {
         idx nroots = 0;
         for (idx s = 0; s < nsn; ++s) nroots += S.sn_parent[s] < 0 ? 1 : 0;
