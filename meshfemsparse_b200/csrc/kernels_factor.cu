@@ -100,7 +100,7 @@ __global__ void extract_diag_kernel(const int64_t *__restrict__ diag_off, int64_
 // roots in a row) for narrow fronts and by the triangle's read and write in shared memory
 // for wide ones, hence rank 4 and not 1. With rank-1 steps, a division per element and three
 // barriers a column over the whole square the 20-sided cube took 587 us in FP64 (5
-// launches), 150 us now; the batch of 48 cubes in FP32 4,550 us (9 launches), 1,070 us now.
+// launches), 150 us now; the batch of 48 cubes in FP32 4,550 us (9 launches), 1,255 us now.
 constexpr int kSmallCols = 4;
 
 // Column c of block row b of a front of ManyDev (its list: entries e0 to e1 - 1): a warp calls

@@ -31,8 +31,8 @@
 // soon as their own children are done, the structure products stream L21 while the
 // chain runs, and no partial sums go through memory. One pass over the factor in FP64
 // with one right-hand side (k = 40, 201,720 variables, 19 levels above the cut):
-// 5.56 ms before (133 launches), 1.56 ms now; FP32 with 32 of them, refined in 4 iterations
-// (k = 48, 345,744 variables): 146 ms before, 71 ms now.
+// 5.56 ms before (133 launches), 1.53 ms now; FP32 with 32 of them, refined in 4 iterations
+// (k = 48, 345,744 variables): 146 ms before, 61 ms now.
 //
 // A CTA is 8 product warps and 8 warps that run ahead of them through the CTA's tasks, so
 // that a small task costs its products and not its chain of dependent loads (a structure
